@@ -10,7 +10,6 @@ int em_plain_estep(fem_em *h);
 int em_plain_mstep(fem_em *h);
 int em_factor(fem_em *h, bool regularize);
 int64_t em_plain_logl_blocks(int64_t n, int d);
-void cov_geometry(int d, int *TB, int *nb, int *nblk);
 int em_post_rows(fem_em *h, int64_t r0, int64_t rows, double *dout);
 int em_classes(fem_em *h, int32_t *dcls);
 
@@ -22,6 +21,9 @@ int em_tc_upload(fem_em *h);    // X -> bf16 hi/lo split
 int em_tc_prepare(fem_em *h);   // factors -> permuted bf16 hi/lo operands + offsets
 int em_tc_estep(fem_em *h);
 int em_tc_mstep(fem_em *h);
+// em_cov.cu: CUDA-core covariance sums and their finalisation
+CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo);
+int em_cov_plain(fem_em *h);
 // the mixed path's covariance on CUDA cores in FP32 (for small components):
 // posteriors as FP16 hi + lo, means as float with row stride mu_ld
 int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld);

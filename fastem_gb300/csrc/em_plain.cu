@@ -405,146 +405,6 @@ __global__ void k_final_means(const double *__restrict__ part, int G, int K, int
   }
 }
 
-// ================================================== M-step: covariances
-// MatrixEMBase::ComputeWeightedTempDataset + BlockCovariances
-// (EM2/MatrixEM.cpp:53-67,90-99): z = sqrt(r_ij) (x_i - mu_j), CovSum_j +=
-// z z^T over the upper block triangle.  Each thread owns one TB x TB block
-// of one component; a CTA owns 256 consecutive (component, block) units.
-constexpr int kCovTP = 32;
-constexpr int kCovFlushTiles = 64;   // FP32 sums span at most 64 tiles (2048 rows)
-
-// posterior (component j, point i): typed component-major array, or the
-// mixed path's FP16 hi + lo pair
-template <typename T>
-struct PostTyped {
-  const T *R;
-  int64_t pitch;
-  __device__ T operator()(int j, int64_t i) const { return R[(size_t)j * pitch + i]; }
-};
-struct PostHiLo {
-  const __half *Rh, *Rl;
-  int64_t pitch;
-  __device__ float operator()(int j, int64_t i) const {
-    const size_t o = (size_t)j * pitch + i;
-    return __half2float(Rh[o]) + __half2float(Rl[o]);
-  }
-};
-
-template <typename T, int TB, class Src>
-__global__ void __launch_bounds__(256)
-k_cov_plain(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T *__restrict__ mu, int mu_ld,
-            double *__restrict__ part, int nb, int nblk, int64_t rows_per_chunk, int upc) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sZ = (T *)smem_raw;  // CJ x TP x d
-  const int tid = threadIdx.x;
-  // this CTA's upc (<= 256, a multiple of 32) units; the components they
-  // span are staged, so small d with many components takes fewer units
-  const int u0 = blockIdx.x * upc;
-  const int j_lo = u0 / nblk;
-  const int j_hi = min(K - 1, (u0 + upc - 1) / nblk);
-  const int CJ = j_hi - j_lo + 1;
-  T *sSr = sZ + (size_t)CJ * kCovTP * d;  // CJ x TP: sqrt(r), once per point and component
-  const int unit = u0 + tid;
-  const bool valid = tid < upc && unit < K * nblk;
-  int j = 0, bi = 0, bj = 0;
-  if (valid) {
-    j = unit / nblk;
-    int b = unit - j * nblk;
-    // upper-triangular enumeration of nb x nb blocks: row bi has nb - bi blocks
-    while (b >= nb - bi) {
-      b -= nb - bi;
-      bi++;
-    }
-    bj = bi + b;
-  }
-  const int64_t c0 = (int64_t)blockIdx.y * rows_per_chunk;
-  const int64_t c1 = min(n, c0 + rows_per_chunk);
-  T acc[TB][TB];
-#pragma unroll
-  for (int a = 0; a < TB; a++)
-#pragma unroll
-    for (int b = 0; b < TB; b++) acc[a][b] = T(0);
-  const int cj = j - j_lo;
-  // this thread's FP64 partial block (owned by it alone): the FP32 sums are
-  // added into it every kCovFlushTiles tiles, so FP32 never sums more than
-  // 2048 rows (ill-conditioned covariances stay positive definite)
-  double *o = valid ? part + (((size_t)blockIdx.y * K + j) * nblk + (unit - j * nblk)) * (TB * TB) : nullptr;
-  if (valid)
-#pragma unroll
-    for (int e = 0; e < TB * TB; e++) o[e] = 0.0;
-  int tiles = 0;
-  for (int64_t t0 = c0; t0 < c1; t0 += kCovTP) {
-    const int tp = (int)min((int64_t)kCovTP, c1 - t0);
-    __syncthreads();
-    for (int e = tid; e < CJ * kCovTP; e += 256) {
-      const int jj = e / kCovTP, p = e - jj * kCovTP;
-      sSr[e] = p < tp ? sqrt((T)R(j_lo + jj, t0 + p)) : T(0);
-    }
-    __syncthreads();
-    const int tot = CJ * kCovTP * d;
-    for (int e = tid; e < tot; e += 256) {
-      const int jj = e / (kCovTP * d);
-      const int rem = e - jj * kCovTP * d;
-      const int p = rem / d, a = rem - p * d;
-      T z = T(0);
-      if (p < tp) {
-        const int64_t row = t0 + p;
-        z = sSr[jj * kCovTP + p] * ((T)X[row * d + a] - mu[(size_t)(j_lo + jj) * mu_ld + a]);
-      }
-      sZ[e] = z;
-    }
-    __syncthreads();
-    if (valid) {
-      const T *zb = sZ + (size_t)cj * kCovTP * d;
-      for (int p = 0; p < kCovTP; p++) {
-        const T *zr = zb + p * d;
-        T va[TB], vb[TB];
-#pragma unroll
-        for (int a = 0; a < TB; a++) va[a] = zr[bi * TB + a];
-#pragma unroll
-        for (int b = 0; b < TB; b++) vb[b] = zr[bj * TB + b];
-#pragma unroll
-        for (int a = 0; a < TB; a++)
-#pragma unroll
-          for (int b = 0; b < TB; b++) acc[a][b] = fma(va[a], vb[b], acc[a][b]);
-      }
-      if (++tiles == kCovFlushTiles || t0 + kCovTP >= c1) {
-        tiles = 0;
-#pragma unroll
-        for (int a = 0; a < TB; a++)
-#pragma unroll
-          for (int b = 0; b < TB; b++) o[a * TB + b] += (double)acc[a][b], acc[a][b] = T(0);
-      }
-    }
-  }
-}
-
-// Covs_j = CovSum_j / PosteriorSum_j, upper mirrored to lower (EM2/MatrixEM.cpp:370-373)
-__global__ void k_final_cov(const double *__restrict__ part, int chunks, int K, int d, int nb,
-                            int nblk, int TB, const double *__restrict__ psum,
-                            double *__restrict__ sigma) {
-  const int j = blockIdx.x;
-  const double inv = 1.0 / psum[j];
-  double *S = sigma + (size_t)j * d * d;
-  const int per = TB * TB;
-  for (int e = threadIdx.x; e < nblk * per; e += blockDim.x) {
-    int b = e / per, w = e - b * per;
-    int bi = 0, bb = b;
-    while (bb >= nb - bi) {
-      bb -= nb - bi;
-      bi++;
-    }
-    const int bj = bi + bb;
-    const int a = bi * TB + w / TB, c = bj * TB + (w % TB);
-    if (a > c) continue;  // lower half of a diagonal block
-    double s = 0.0;
-    for (int ch = 0; ch < chunks; ch++) s += part[(((size_t)ch * K + j) * nblk + b) * per + w];
-    s *= inv;
-    S[(size_t)a * d + c] = s;
-    S[(size_t)c * d + a] = s;
-  }
-}
-
 // ======================================================= factorisation
 // EMAlgorithm::RegularizeCovariances + NormalDensity::Init + CalcLogCoeffs
 // (EM2/EMAlgorithm.cpp:237-244, EM2/NormalDensity.cpp:43-65,
@@ -648,14 +508,6 @@ int64_t em_plain_logl_blocks(int64_t n, int d) {
   }
 }
 
-// tiles of TB x TB covariance entries; TB divides d, so no tile reaches past
-// the last dimension
-void cov_geometry(int d, int *TB, int *nb, int *nblk) {
-  *TB = d % 8 == 0 ? 8 : (d % 4 == 0 ? 4 : (d % 2 == 0 ? 2 : 1));
-  *nb = d / *TB;
-  *nblk = (*nb) * (*nb + 1) / 2;
-}
-
 template <typename T, int C>
 static int launch_means(fem_em *h, int upt, int64_t rpb, size_t sm) {
   const T *R = (const T *)h->R;
@@ -672,56 +524,6 @@ static int launch_means(fem_em *h, int upt, int64_t rpb, size_t sm) {
 #undef FEM_ML
   set_error("means kernel: %d units per thread unsupported", upt);
   return FEM_ERR_UNSUPPORTED;
-}
-
-template <typename T, int TB, class Src>
-static int launch_cov(fem_em *h, int nb, int nblk, int64_t rpc, Src src, const T *mu, int mu_ld) {
-  const int units = h->k * nblk;
-  // z tiles + sqrt(r) of the components that upc consecutive units span
-  auto smem = [&](int upc) {
-    return (size_t)min((upc - 1) / nblk + 2, h->k) * kCovTP * (h->d + 1) * sizeof(T);
-  };
-  int upc = 256;
-  while (upc > 32 && smem(upc) > kMaxDynSmem) upc -= 32;
-  if (smem(upc) > kMaxDynSmem) {
-    set_error("covariance tiles of d = %d need %zu bytes of shared memory", h->d, smem(upc));
-    return FEM_ERR_UNSUPPORTED;
-  }
-  const size_t sm = smem(upc);
-  const int gx = (units + upc - 1) / upc;
-  FEM_CUDA(allow_dyn_smem(k_cov_plain<T, TB, Src>, sm));
-  dim3 grid(gx, h->cchunks);
-  k_cov_plain<T, TB, Src><<<grid, 256, sm, h->stream>>>(h->X, h->n, h->d, h->k, src, mu, mu_ld, h->cpart, nb,
-                                                        nblk, rpc, upc);
-  return FEM_OK;
-}
-
-// the covariance pass for any posterior source: partials + FP64 finalisation
-template <typename T, class Src>
-static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld) {
-  const int d = h->d, K = h->k;
-  int TB, nb, nblk, st;
-  cov_geometry(d, &TB, &nb, &nblk);
-  const int64_t rpc = (h->n + h->cchunks - 1) / h->cchunks;
-  if (TB == 8)
-    st = launch_cov<T, 8>(h, nb, nblk, rpc, src, mu, mu_ld);
-  else if (TB == 4)
-    st = launch_cov<T, 4>(h, nb, nblk, rpc, src, mu, mu_ld);
-  else if (TB == 2)
-    st = launch_cov<T, 2>(h, nb, nblk, rpc, src, mu, mu_ld);
-  else
-    st = launch_cov<T, 1>(h, nb, nblk, rpc, src, mu, mu_ld);
-  FEM_TRY(st);
-  FEM_CUDA(cudaGetLastError());
-  k_final_cov<<<K, 256, 0, h->stream>>>(h->cpart, h->cchunks, K, d, nb, nblk, TB, h->psum, h->sigma);
-  FEM_CUDA(cudaGetLastError());
-  return FEM_OK;
-}
-
-int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld) {
-  FEM_TRY((cov_pass<float, PostHiLo>(h, PostHiLo{Rh, Rl, pitch}, muf, mu_ld)));
-  h->launches += 2;
-  return FEM_OK;
 }
 
 template <typename T>
@@ -751,7 +553,7 @@ static int mstep_plain_t(fem_em *h) {
   k_final_means<T><<<K, 128, 0, h->stream>>>(h->mpart, h->mgrid, K, d, n, h->mu, h->pi, h->psum,
                                              (T *)h->muT);
   FEM_CUDA(cudaGetLastError());
-  FEM_TRY((cov_pass<T, PostTyped<T>>(h, PostTyped<T>{(const T *)h->R, n}, (const T *)h->muT, d)));
+  FEM_TRY(em_cov_plain(h));
   h->launches += 4;
   return FEM_OK;
 }

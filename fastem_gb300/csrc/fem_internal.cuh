@@ -88,9 +88,16 @@ struct DevStatus {
 };
 
 // ------------------------------------------------------------------ EM handle
-enum { EM_PAR_CHUNKS = 0 };
+// schedule of the CUDA-core covariance sums (em_cov.cu)
+struct CovPlan {
+  int TB = 0, tri = 0, nb = 0, nblk = 0;   // block size, one triangular block, blocks per dimension / per component
+  int gx = 0, upc = 0, G = 0, cj = 0;      // CTAs over the units, units per CTA, point groups, components per CTA
+  int TP = 0, xpitch = 0, rpitch = 0;      // points per tile, shared-memory pitches
+  int chunks = 0;                          // row chunks (grid.y)
+  int64_t rows = 0;                        // rows per chunk
+  size_t smem = 0, part = 0;               // shared memory of a CTA, doubles of the partials
+};
 
-struct EmHandle;
 struct TcEmPlan;    // mixed-precision launch plan, d <= 64 (em_tc.cu)
 struct WideEmPlan;  // mixed-precision launch plan, 64 < d <= 256 (em_wide.cu)
 
@@ -126,8 +133,8 @@ struct fem_em {
   // M-step partials (FP64)
   double *mpart = nullptr;      // means: grid x k x (d+1)
   int mgrid = 0;
-  double *cpart = nullptr;      // covariances: chunks x k x nblk x 64
-  int cchunks = 0, cunits_blocks = 0;
+  double *cpart = nullptr;      // CUDA-core covariances: cov.part
+  fem::CovPlan cov;
   double *psum = nullptr;       // k   PosteriorSum
 
   // mixed-precision state (em_tc.cu)

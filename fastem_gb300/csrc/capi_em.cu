@@ -234,8 +234,8 @@ int fem_em_create(int d, int64_t n, int k, const fem_em_config *cfg, fem_em **ou
   } else {
     h->n_logl_part = em_plain_logl_blocks(n, d);
     if ((st = dalloc(&h->logl_part, h->n_logl_part))) return fail(st);
-    h->mgrid = (int)std::min<int64_t>((int64_t)4 * sm_count(), (n + 31) / 32);
-    if ((st = dalloc(&h->mpart, (size_t)h->mgrid * k * (d + 1)))) return fail(st);
+    h->means = means_plan(d, n, k, c.precision == FEM_PREC_FP64);
+    if ((st = dalloc(&h->mpart, h->means.part))) return fail(st);
     h->cov = cov_plan(d, n, k, c.precision == FEM_PREC_FP64, false);
     if ((st = dalloc(&h->cpart, h->cov.part))) return fail(st);
   }

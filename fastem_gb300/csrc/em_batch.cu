@@ -770,8 +770,11 @@ k_b_cov_own(const BFit *__restrict__ fits, const BState *__restrict__ state, con
 __global__ void __launch_bounds__(kBFThreads)
 k_b_factor(const BFit *__restrict__ fits, BState *__restrict__ state, const int2 *__restrict__ comps,
            const double *__restrict__ cpart, double reg, int reduce, int svd) {
-  __shared__ double sA[kBMaxD * kBMaxD];
-  __shared__ double sWi[kBMaxD * kBMaxD];
+  // factor and inverse (row stride factor_ld(d)); the d x d copy of the
+  // condition check reuses the first
+  __shared__ double sA[kBMaxD * (kBMaxD + 1)];
+  __shared__ double sWi[kBMaxD * (kBMaxD + 1)];
+  __shared__ double piv[kBMaxD], rd[kBMaxD], mult[2 * kBMaxD], red[kBFThreads / 32];
   const int2 fc = comps[blockIdx.x];
   const int f = fc.x, j = fc.y, tid = threadIdx.x;
   if (!state[f].active) return;
@@ -834,14 +837,20 @@ k_b_factor(const BFit *__restrict__ fits, BState *__restrict__ state, const int2
     __syncthreads();
   }
   if (reg != 0.0) block_regularize(S, d, reg);
-  if (!block_cholesky(S, d, sA)) {
+  const int ld = factor_ld(d);
+  for (int e = tid; e < d * d; e += kBFThreads) {
+    const int r = e / d, c = e - r * d;
+    if (c <= r) sA[r * ld + c] = S[e];
+  }
+  __syncthreads();
+  if (!block_factor_smem<1>(sA, sWi, piv, rd, mult, d, ld)) {
     if (tid == 0) atomicMin(&state[f].chol_failed, j);
     return;
   }
-  block_lower_inverse(sA, d, sWi);
-  const double ld = block_chol_logdet(sA, d);
+  double ldet[1] = {tid < d ? log(piv[tid]) : 0.0};
+  block_sums(ldet, red);
   if (tid == 0) {
-    const double lc = log(F.pi[j]) - 0.5 * (double)d * log(2.0 * M_PI) - 0.5 * ld;
+    const double lc = log(F.pi[j]) - 0.5 * (double)d * log(2.0 * M_PI) - 0.5 * ldet[0];
     F.logc[j] = lc;
     F.logcT[j] = (float)lc;
   }
@@ -851,7 +860,7 @@ k_b_factor(const BFit *__restrict__ fits, BState *__restrict__ state, const int2
     int kk = 0, off = 0;
     while (off + tri_row(kk) <= e) off += tri_row(kk++);
     const int m = e - off;
-    Wt[e] = (kk < d && m <= kk) ? (float)sWi[kk * d + m] : 0.f;
+    Wt[e] = (kk < d && m <= kk) ? (float)(m < kk ? sWi[kk * ld + m] * rd[kk] : rd[kk]) : 0.f;
   }
   if (svd) {
     __syncthreads();

@@ -1,5 +1,6 @@
-// em_cov.cu -- the CUDA-core covariance sums of the EM sweep (FP32, FP64, and
-// FP32 from the mixed path's FP16 hi/lo posteriors).
+// em_cov.cu -- the CUDA-core M-step sums of the EM sweep: covariances (FP32,
+// FP64, and FP32 from the mixed path's FP16 hi/lo posteriors) and means (FP32,
+// FP64).
 //
 // MatrixEMBase::ComputeWeightedTempDataset + BlockCovariances
 // (EM2/MatrixEM.cpp:53-67,90-99): CovSum_j += r_ij (x_i - mu_j)(x_i - mu_j)^T
@@ -345,17 +346,182 @@ k_final_cov(const double *__restrict__ part, int chunks, int K, int d, int nb, i
   S[(size_t)c * d + a] = v;
 }
 
+// ============================================================== means
+// SimpleMatrixEM::doMStep means part (EM2/MatrixEM.cpp:319-343):
+// PosteriorSum_j = sum_i r_ij and MeanSums_j = sum_i r_ij x_i as the product
+// R^T [X | 1] (column d of a staged row is 1).  A thread owns 4 components x 4
+// columns for every G-th group of 4 points; units, point groups and chunks as
+// in k_cov_units.  FP32 sums span at most kMnRows rows, then go into the
+// thread's FP64 sums; the point groups are combined in FP64, in order.
+// part[chunk][component][0: sum r, 1 + q: sum r x_q].  Per 4 points 8 128-bit
+// shared-memory loads feed 64 products, which is what bounds the FP32 form.
+// Against one component x 8 or 16 columns per thread (GB300): N = 250007,
+// d = 16, K = 200, FP32 239 -> 138 us; N = 100000, d = 8, K = 10, FP64 128 -> 54 us.
+constexpr int kMnRows = 512;
+
+template <typename T>
+__device__ __forceinline__ void mn_load(const T *p, T (&v)[4]);
+template <>
+__device__ __forceinline__ void mn_load(const float *p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4 *>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+template <>
+__device__ __forceinline__ void mn_load(const double *p, double (&v)[4]) {
+  const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCvThreads, 2)
+k_means_units(const float *__restrict__ X, int64_t n, int d, int K, PostTyped<T> R, double *__restrict__ part, int nc,
+              int64_t rows_per_chunk, int upc, int G, int TP, int xpitch, int rpitch, int cjmax) {
+  extern __shared__ __align__(16) unsigned char cv_smem[];
+  const int tid = threadIdx.x;
+  const int units = (K + 3) / 4 * nc, u0 = blockIdx.x * upc;
+  const int b_lo = u0 / nc, b_hi = min(units - 1, u0 + upc - 1) / nc;
+  const int j_lo = 4 * b_lo, cj = min(K, 4 * b_hi + 4) - j_lo;
+  const int g = tid / upc, ul = tid - g * upc, unit = u0 + ul;
+  const bool act = g < G && unit < units;
+  const int jb = act ? unit / nc : b_lo, cb = act ? unit - jb * nc : 0;
+  const size_t xbytes = (size_t)TP * xpitch * sizeof(float);
+  const size_t buf_bytes = xbytes + (size_t)cjmax * rpitch * sizeof(T);
+  const int64_t c0 = (int64_t)blockIdx.y * rows_per_chunk, c1 = min(n, c0 + rows_per_chunk);
+  // what the copies leave alone: columns d (ones) .. 4 nc - 1 (zero) of the
+  // rows, and posteriors of components past K
+  for (int e = tid; e < 2 * TP * (4 * nc - d); e += kCvThreads) {
+    const int row = e / (4 * nc - d), q = d + e - row * (4 * nc - d);
+    float *sx = reinterpret_cast<float *>(cv_smem + (row >= TP ? buf_bytes : 0));
+    sx[(row >= TP ? row - TP : row) * xpitch + q] = q == d ? 1.f : 0.f;
+  }
+  for (int e = tid; e < 2 * (cjmax - cj) * rpitch; e += kCvThreads) {
+    const int b = e / ((cjmax - cj) * rpitch), o = e - b * (cjmax - cj) * rpitch;
+    reinterpret_cast<T *>(cv_smem + b * buf_bytes + xbytes)[cj * rpitch + o] = T(0);
+  }
+  auto stage = [&](int buf, int64_t t0) {
+    float *sx = reinterpret_cast<float *>(cv_smem + buf * buf_bytes);
+    if ((d & 3) == 0) {
+      const int d4 = d >> 2;
+      for (int e = tid; e < TP * d4; e += kCvThreads) {
+        const int p = e / d4, q = 4 * (e - p * d4);
+        const bool v = t0 + p < c1;
+        cv_copy16(sx + p * xpitch + q, X + (v ? (t0 + p) * d + q : 0), v);
+      }
+    } else {
+      for (int e = tid; e < TP * d; e += kCvThreads) {
+        const int p = e / d, q = e - p * d;
+        const bool v = t0 + p < c1;
+        cv_copy4(sx + p * xpitch + q, X + (v ? (t0 + p) * d + q : 0), v);
+      }
+    }
+    R.stage(cv_smem + buf * buf_bytes + xbytes, rpitch, j_lo, cj, t0, TP, c1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  T acc[4][4];
+  double dacc[4][4];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[q][c] = T(0), dacc[q][c] = 0.0;
+  auto fold = [&]() {
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) dacc[q][c] += (double)acc[q][c], acc[q][c] = T(0);
+  };
+  stage(0, c0);
+  int buf = 0, rows = 0;
+  const int tile_rows = TP / G;
+  for (int64_t t0 = c0; t0 < c1; t0 += TP, buf ^= 1) {
+    if (t0 + TP < c1)
+      stage(buf ^ 1, t0 + TP);
+    else
+      asm volatile("cp.async.commit_group;\n" ::: "memory");   // keeps the wait count uniform
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    if (act) {
+      const float *sx = reinterpret_cast<const float *>(cv_smem + buf * buf_bytes) + 4 * cb;
+      const T *sr = reinterpret_cast<const T *>(cv_smem + buf * buf_bytes + xbytes) + 4 * (jb - b_lo) * rpitch;
+      for (int p = 4 * g; p < TP; p += 4 * G) {
+        T r[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) mn_load(sr + q * rpitch + p, r[q]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          float x[4];
+          mn_load(sx + (p + i) * xpitch, x);
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            const T xc = (T)x[c];
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc[q][c] = fma(r[q][i], xc, acc[q][c]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    rows += tile_rows;
+    if (sizeof(T) == 4 && rows + tile_rows > kMnRows) fold(), rows = 0;
+  }
+  fold();
+  double *o = part + (size_t)blockIdx.y * K * (d + 1);
+  auto put = [&](int u, int e, double v) {     // element e of unit u
+    const int b = u / nc, c = 4 * (u - b * nc) + (e & 3), j = 4 * b + (e >> 2);
+    if (j < K && c <= d) o[(size_t)j * (d + 1) + (c == d ? 0 : 1 + c)] = v;
+  };
+  if (G == 1) {
+    if (act)
+#pragma unroll
+      for (int e = 0; e < 16; e++) put(unit, e, dacc[e >> 2][e & 3]);
+    return;
+  }
+  double *red = reinterpret_cast<double *>(cv_smem);   // 16 x 256, over the tiles
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 16; e++) red[e * kCvThreads + tid] = dacc[e >> 2][e & 3];
+  __syncthreads();
+  const int live = min(upc, units - u0);
+  for (int i = tid; i < live * 16; i += kCvThreads) {
+    const int e = i / live, u = i - e * live;
+    double v = red[e * kCvThreads + u];
+    for (int q = 1; q < G; q++) v += red[e * kCvThreads + q * upc + u];
+    put(u0 + u, e, v);
+  }
+}
+
+// gx CTAs of upc units with G point groups each: the split of at most 8 more
+// CTAs than needed that leaves the fewest of the threads without a unit (600
+// units on 3 x 200 threads would idle 22 %; 5 x 120 with two groups idle 6 %)
+void split_units(int units, int *gx, int *upc, int *G) {
+  const int g0 = (units + kCvThreads - 1) / kCvThreads;
+  double best = -1.0;
+  for (int c = g0; c <= std::min(units, g0 + 8); c++) {
+    const int u = (units + c - 1) / c, ctas = (units + u - 1) / u;
+    const int g = std::min(kCvMaxGroups, kCvThreads / u);
+    const double eff = (double)units * g / ((double)ctas * kCvThreads) * (1.0 - 0.01 * (c - g0));
+    if (eff > best) best = eff, *gx = ctas, *upc = u, *G = g;
+  }
+}
+
+// row chunks: the count whose waves over `slots` resident CTAs finish first,
+// counting two tiles' time for a CTA's start and end
+void split_rows(int64_t n, int TP, int gx, int slots, int *chunks, int64_t *rows) {
+  const int64_t tiles = (n + TP - 1) / TP;
+  double bt = 1e300;
+  for (int64_t c = 1; c <= std::min<int64_t>(tiles, (int64_t)3 * slots / gx + 1); c++) {
+    const int64_t tpc = (tiles + c - 1) / c, ch = (tiles + tpc - 1) / tpc;
+    const double t = std::ceil((double)gx * ch / slots) * (tpc + 2.0);
+    if (t < bt) bt = t, *chunks = (int)ch, *rows = tpc * TP;
+  }
+}
+
 }  // namespace
 
 // Schedule of the covariance sums for one handle (fixed by its shape).
 //
 //  TB, tri   8 x 8 blocks; one triangular block when d <= 8 (4 x 4 when d <= 4)
-//  gx, upc   CTAs the units are spread over and units per CTA: the split of
-//            at most 8 more CTAs than needed that leaves the fewest of the
-//            256 threads without a unit (600 units on 3 x 200 threads would
-//            idle 22 %; 5 x 120 with two point groups idle 6 %)
-//  chunks    row chunks: the count whose waves over the SMs finish first,
-//            counting two tiles' time for a CTA's start and flush
+//  units     split as split_units says, rows as split_rows says
 CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
   CovPlan p{};
   p.TB = d <= 4 ? 4 : 8;
@@ -363,14 +529,8 @@ CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
   p.tri = p.nb == 1;
   p.nblk = p.nb * (p.nb + 1) / 2;
   const int ne = p.tri ? p.TB * (p.TB + 1) / 2 : p.TB * p.TB;
-  const int units = k * p.nblk, g0 = (units + kCvThreads - 1) / kCvThreads;
-  double best = -1.0;
-  for (int gx = g0; gx <= std::min(units, g0 + 8); gx++) {
-    const int upc = (units + gx - 1) / gx, ctas = (units + upc - 1) / upc;
-    const int G = std::min(kCvMaxGroups, kCvThreads / upc);
-    const double eff = (double)units * G / ((double)ctas * kCvThreads) * (1.0 - 0.01 * (gx - g0));
-    if (eff > best) best = eff, p.gx = ctas, p.upc = upc, p.G = G;
-  }
+  const int units = k * p.nblk;
+  split_units(units, &p.gx, &p.upc, &p.G);
   const int m = std::max(8, (32 / p.G + 7) / 8 * 8);   // points per thread and tile
   p.TP = p.G * m;
   p.xpitch = p.TB == 4 ? 4 : 8 * p.nb + 4;             // odd multiple of 16 bytes: point groups in different banks
@@ -379,16 +539,47 @@ CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
   const size_t rb = ((size_t)p.cj * p.rpitch * (fp64 ? 8 : 4) + 15) & ~(size_t)15;
   p.smem = 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + rb);
   if (p.G > 1) p.smem = std::max(p.smem, (size_t)ne * kCvThreads * (fp64 ? 8 : 4));
-  const int slots = (fp64 ? 1 : 2) * sm_count();
-  const int64_t tiles = (n + p.TP - 1) / p.TP;
-  double bt = 1e300;
-  for (int64_t c = 1; c <= std::min<int64_t>(tiles, (int64_t)3 * slots / p.gx + 1); c++) {
-    const int64_t tpc = (tiles + c - 1) / c, ch = (tiles + tpc - 1) / tpc;
-    const double waves = std::ceil((double)p.gx * ch / slots), t = waves * (tpc + 2.0);
-    if (t < bt) bt = t, p.chunks = (int)ch, p.rows = tpc * p.TP;
-  }
+  split_rows(n, p.TP, p.gx, (fp64 ? 1 : 2) * sm_count(), &p.chunks, &p.rows);
   p.part = (size_t)p.chunks * units * ne;
   return p;
+}
+
+// Schedule of the means sums (TB = 4: 4 components x 4 columns per unit; nb =
+// column groups of a row and its 1)
+CovPlan means_plan(int d, int64_t n, int k, bool fp64) {
+  CovPlan p{};
+  p.TB = 4;
+  p.nb = (d + 4) / 4;
+  const int units = (k + 3) / 4 * p.nb;
+  split_units(units, &p.gx, &p.upc, &p.G);
+  p.xpitch = 4 * p.nb;
+  p.cj = 4 * std::min((k + 3) / 4, (p.upc + p.nb - 2) / p.nb + 1);
+  const size_t ts = fp64 ? 8 : 4;
+  for (int m = std::max(2, 8 / p.G); m >= 1; m /= 2) {   // groups of 4 points per thread and tile
+    p.TP = 4 * p.G * m;
+    p.rpitch = p.TP + 16 / (int)ts;
+    p.smem = 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + (size_t)p.cj * p.rpitch * ts);
+    if (p.smem <= kCvMaxSmem / 2) break;
+  }
+  if (p.G > 1) p.smem = std::max(p.smem, (size_t)16 * kCvThreads * sizeof(double));
+  split_rows(n, p.TP, p.gx, 2 * sm_count(), &p.chunks, &p.rows);
+  p.part = (size_t)p.chunks * k * (d + 1);
+  return p;
+}
+
+template <typename T>
+static int means_pass(fem_em *h) {
+  const CovPlan &p = h->means;
+  FEM_CUDA(allow_dyn_smem(k_means_units<T>, p.smem));
+  k_means_units<T><<<dim3(p.gx, p.chunks), kCvThreads, p.smem, h->stream>>>(
+      h->X, h->n, h->d, h->k, PostTyped<T>{(const T *)h->R, h->n}, h->mpart, p.nb, p.rows, p.upc, p.G, p.TP, p.xpitch,
+      p.rpitch, p.cj);
+  FEM_CUDA(cudaGetLastError());
+  return FEM_OK;
+}
+
+int em_means_plain(fem_em *h) {
+  return h->cfg.precision == FEM_PREC_FP64 ? means_pass<double>(h) : means_pass<float>(h);
 }
 
 // partials + FP64 finalisation for one posterior source

@@ -26,96 +26,163 @@ __device__ inline void block_regularize(double *S, int d, double reg) {
   __syncthreads();
 }
 
-// NormalDensity::Init (EM2/NormalDensity.cpp:43-65): A <- sym(lower(S)),
-// then right-looking Cholesky in place (L in the lower triangle).  A pivot
-// <= 0 fails, as Eigen's LLT reports.  Returns true on success, the same in
-// every thread.
-__device__ inline bool block_cholesky(const double *S, int d, double *A) {
-  __shared__ double s_piv;
-  __shared__ int s_fail;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < d * d; e += nt) {
-    const int r = e / d, c = e - r * d;
-    A[e] = (c <= r) ? S[e] : S[(size_t)c * d + r];
-  }
-  if (tid == 0) s_fail = 0;
+constexpr int kFactorMaxD = 256;   // largest d of the block factorisation helpers
+constexpr int kFactorThreads = 256;
+
+// N sums over the block in a fixed order; the values in every thread.  red:
+// N doubles per warp
+template <int N>
+__device__ inline void block_sums(double (&v)[N], double *red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
   __syncthreads();
-  for (int k = 0; k < d; k++) {
-    if (tid == 0) {
-      const double x = A[(size_t)k * d + k];
-      if (!(x > 0.0)) {
-        s_fail = 1;
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < N; q++) red[(threadIdx.x >> 5) * N + q] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    v[q] = red[q];
+    for (int w = 1; w < (int)blockDim.x / 32; w++) v[q] += red[w * N + q];
+  }
+}
+
+// u / p for N values of u: the hardware's approximate reciprocal y (relative
+// error below 2^-20) and a third-order correction, u y (1 + e + e^2) with
+// e = 1 - p y (Schulz / Householder iteration): three dependent FP64
+// operations to within 2^-60 before rounding
+template <int N>
+__device__ __forceinline__ void factor_divide(double (&u)[N], double p) {
+  const int ex = (__double2hiint(p) >> 20) & 0x7ff;
+  if (ex < 64 || ex > 1983) {                    // the approximation flushes subnormal results
+#pragma unroll
+    for (int s = 0; s < N; s++) u[s] = u[s] / p;
+    return;
+  }
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+  const double e = fma(-p, y, 1.0), e2 = fma(e, e, e);
+#pragma unroll
+  for (int s = 0; s < N; s++) {
+    const double t = u[s] * y;
+    u[s] = fma(t, e2, t);
+  }
+}
+
+// NormalDensity::Init (EM2/NormalDensity.cpp:43-65) with both matrices in
+// shared memory, as L D L^T: A (row stride ld, lower triangle = the
+// covariance) ends as L sqrt(D) columns before their scaling, W as the rows of
+// the unit inverse, piv[k] = D_k and rd[k] = 1 / sqrt(D_k), so that
+//   L_rc = A[r][c] rd[c] (r > c), L_rr = sqrt(piv[r]),
+//   (L^-1)_rc = W[r][c] rd[r] (r > c), (L^-1)_rr = rd[r]
+// (the upper triangles and the diagonal of W are not written).  A pivot <= 0
+// fails, as Eigen's LLT reports (the pivots are the same); the answer is the
+// same in every thread.  m: 2 d doubles of scratch.  d <= 32 NS.
+//
+// FP64 runs at 2 lanes per clock and SM with a long latency, so the form is
+// chosen for its chain: per column one barrier, and between two barriers warp
+// 0 (lane = row) forms column k + 1, the reciprocal of its pivot and its
+// multipliers, 6 dependent operations where a Cholesky column's square root
+// and divisions are ~25; the square roots wait for the end.  Meanwhile the
+// other warps (warp = row, lane = column) apply column k: row i takes the
+// inverse's columns 0..k and the factor's k + 2..i in one pass.
+// Against one thread per column over matrices in L2 (GB300, the whole kernel):
+// d = 24, K = 21 73 -> 21 us; d = 64, K = 128 263 -> 95 us; d = 99, K = 23
+// 593 -> 284 us.  From d = 48 on the updates' shared-memory round trips and the
+// FP64 pipe set the time; batching 2 or 4 rows per warp to overlap them was
+// slower (d = 99: 335, 369 us: warp 0's chain waits behind the bursts).
+template <int NS>
+__device__ inline bool block_factor_smem(double *A, double *W, double *piv, double *rd, double *m, int d, int ld) {
+  __shared__ int s_fail;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nu = (blockDim.x >> 5) - 1;
+  if (threadIdx.x == 0) s_fail = 0;
+  __syncthreads();
+  for (int k = -1; k < d - 1; k++) {
+    const double *mk = m + (k & 1) * d;
+    if (warp == 0) {
+      const int c = k + 1;
+      double u[NS];
+      const double uc = k >= 0 ? -A[c * ld + k] : 0.0;
+#pragma unroll
+      for (int s = 0; s < NS; s++) {
+        const int r = c + lane + 32 * s;
+        u[s] = 0.0;
+        if (r < d) u[s] = k >= 0 ? fma(mk[r], uc, A[r * ld + c]) : A[r * ld + c];
+      }
+      const double p = __shfl_sync(0xffffffffu, u[0], 0);
+      const long long pb = __double_as_longlong(p);
+      if (pb <= 0 || pb > 0x7ff0000000000000LL) {    // !(p > 0), without waiting for the FP64 pipe
+        if (lane == 0) s_fail = 1;
       } else {
-        const double l = sqrt(x);
-        A[(size_t)k * d + k] = l;
-        s_piv = l;
+        double *mc = m + (c & 1) * d;
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          const int r = c + lane + 32 * s;
+          if (r < d) A[r * ld + c] = u[s];
+        }
+        factor_divide(u, p);
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          const int r = c + lane + 32 * s;
+          if (r < d) mc[r] = u[s];
+        }
+        if (lane == 0) piv[c] = p;
+      }
+    } else if (k >= 0) {
+      double v[NS];
+      double *col[NS];                    // column c of the inverse's or the factor's rows
+#pragma unroll
+      for (int s = 0; s < NS; s++) {
+        const int c = lane + 32 * s;
+        v[s] = c < k ? W[k * ld + c] : (c > k + 1 && c < d ? A[c * ld + k] : 0.0);
+        col[s] = (c <= k ? W : A) + c;
+      }
+      for (int i = k + warp; i < d; i += nu) {
+        const double mi = -mk[i];
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+          const int c = lane + 32 * s;
+          if (c > i || c == k + 1) continue;
+          double *t = col[s] + i * ld;
+          *t = c == k ? mi : fma(mi, v[s], *t);
+        }
       }
     }
     __syncthreads();
     if (s_fail) break;
-    const double lkk = s_piv;
-    for (int i = k + 1 + tid; i < d; i += nt) A[(size_t)i * d + k] /= lkk;
-    __syncthreads();
-    // trailing update of the lower triangle: A[i][c] -= L[i][k] L[c][k], k < c <= i
-    const int m = d - k - 1;
-    for (int e = tid; e < m * m; e += nt) {
-      const int i = e / m, c = e - i * m;
-      if (c > i) continue;
-      const int gi = k + 1 + i, gc = k + 1 + c;
-      A[(size_t)gi * d + gc] -= A[(size_t)gi * d + k] * A[(size_t)gc * d + k];
-    }
-    __syncthreads();
   }
   const bool ok = !s_fail;
+  if (ok)
+    for (int q = threadIdx.x; q < d; q += blockDim.x) rd[q] = 1.0 / sqrt(piv[q]);
   __syncthreads();
   return ok;
 }
 
-constexpr int kFactorMaxD = 256;   // largest d of the block factorisation helpers
-
-// W = L^-1 (lower, row-major) by forward substitution, threads owning columns;
-// L is the lower triangle of A.  The diagonal's reciprocals are formed once,
-// in parallel, so a column's substitution multiplies instead of dividing.
-// d <= kFactorMaxD.
-__device__ inline void block_lower_inverse(const double *A, int d, double *Wi) {
-  __shared__ double s_rd[kFactorMaxD];
-  for (int r = threadIdx.x; r < d; r += blockDim.x) s_rd[r] = 1.0 / A[(size_t)r * d + r];
-  __syncthreads();
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    for (int r = 0; r < c; r++) Wi[(size_t)r * d + c] = 0.0;
-    for (int r = c; r < d; r++) {
-      double s = (r == c) ? 1.0 : 0.0;
-      for (int m2 = c; m2 < r; m2++) s -= A[(size_t)r * d + m2] * Wi[(size_t)m2 * d + c];
-      Wi[(size_t)r * d + c] = s * s_rd[r];
-    }
-  }
-  __syncthreads();
-}
-
 // ------------------------------------------------------------------------
-// Blocked forms of block_cholesky and block_lower_inverse for one CTA of
-// kFactorThreads threads (d <= kFactorMaxD).  Each matrix element goes through
-// the same FP64 operations in the same order as in the unblocked functions (a
-// running a - x y per update, k ascending), so the factors are bit-identical;
-// the blocking only changes where the operands live.  With one CTA per
-// component the unblocked loops wait on L2 for every element update; here the
-// panel being factored and the row block being inverted sit in shared memory,
-// the trailing updates are 4 x 4 register tiles, and the FP64 pipe is the
-// limit (d^3 / 6 fused multiply-adds each for the factor and the inverse).
-constexpr int kFactorThreads = 256;
+// Blocked Cholesky and triangular inverse for one CTA of kFactorThreads
+// threads (kFactorSmemD < d <= kFactorMaxD).  The matrices stay in global
+// memory (L2); the panel being factored and the row block being inverted sit
+// in shared memory, the trailing updates are 4 x 4 register tiles, and the
+// FP64 pipe is the limit (d^3 / 6 fused multiply-adds each for the factor and
+// the inverse).
 constexpr int kPanel = 32;                // columns per Cholesky panel, rows per inverse block
 constexpr int kPanelLd = kPanel + 1;      // panel row stride (doubles)
-constexpr int kFactorBlockedD = 128;      // smallest d that the blocked forms are used for
+// block_factor_smem holds both matrices in shared memory up to this d
+constexpr int kFactorSmemD = 118;
+__host__ __device__ constexpr int factor_ld(int d) { return d | 1; }
 
-// dynamic shared memory of the two functions (the panel, then the row block)
+// dynamic shared memory: both matrices and block_factor_smem's vectors up to
+// kFactorSmemD, else the panel, then the row block
 __host__ __device__ constexpr size_t factor_smem_bytes(int d) {
-  return (size_t)d * kPanelLd * sizeof(double);
+  return (d <= kFactorSmemD ? (size_t)2 * d * factor_ld(d) + 4 * d : (size_t)d * kPanelLd) * sizeof(double);
 }
 
-// block_cholesky with panels of kPanel columns: the panel (rows k0 .. d-1)
+// Right-looking Cholesky of sym(lower(S)) by panels of kPanel columns: the panel (rows k0 .. d-1)
 // is factored in shared memory (thread i owns row k0 + i), written back, and
 // its update of the trailing lower triangle applied as 4 x 4 tiles.  The
-// upper triangle of A keeps the symmetric copy of S, as in block_cholesky.
+// upper triangle of A keeps the symmetric copy of S.
 // P: factor_smem_bytes(d) of shared memory.  Returns true on success, the
 // same in every thread.
 __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, double *P) {
@@ -205,8 +272,8 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
   return ok;
 }
 
-// block_lower_inverse by blocks of kPanel rows, thread c owning column c of
-// W = L^-1 (d <= blockDim.x): the block's rows of L are staged in shared
+// W = L^-1 (lower, row-major) by blocks of kPanel rows, thread c owning column c
+// (d <= blockDim.x): the block's rows of L are staged in shared
 // memory (Lb); the terms of the rows above the block (m < r0) run as a
 // register-blocked product over the thread's own column of W, then the
 // block's triangle is solved row by row with that column's new entries in

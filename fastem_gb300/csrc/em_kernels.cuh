@@ -21,7 +21,9 @@ int em_tc_upload(fem_em *h);    // X -> bf16 hi/lo split
 int em_tc_prepare(fem_em *h);   // factors -> permuted bf16 hi/lo operands + offsets
 int em_tc_estep(fem_em *h);
 int em_tc_mstep(fem_em *h);
-// em_cov.cu: CUDA-core covariance sums and their finalisation
+// em_cov.cu: CUDA-core means sums (partials only), covariance sums and their finalisation
+CovPlan means_plan(int d, int64_t n, int k, bool fp64);
+int em_means_plain(fem_em *h);
 CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo);
 int em_cov_plain(fem_em *h);
 // the mixed path's covariance on CUDA cores in FP32 (for small components):

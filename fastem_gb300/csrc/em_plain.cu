@@ -294,114 +294,41 @@ __global__ void __launch_bounds__(1024) k_reduce_logl(const double *part, int64_
   if (threadIdx.x == 0) st->logl = s;
 }
 
-// ======================================================= M-step: means
-// SimpleMatrixEM::doMStep means part (EM2/MatrixEM.cpp:319-343):
-// PosteriorSum_j = sum_i r_ij and MeanSums_j = sum_i r_ij x_i per block of
-// rows; each thread owns (component, C-column chunk) units.  The last chunk
-// of a row may be partial (C does not divide d): its lanes past column d
-// read staged values of the next row (or the padding after the last one)
-// and are never written out.
-constexpr int kMeanTP = 32;
-
-template <typename T, int C, int UPT>
-__global__ void __launch_bounds__(256)
-k_means_plain(const float *__restrict__ X, int64_t n, int d, int K, const T *__restrict__ R,
-              double *__restrict__ part, int64_t rows_per_block) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float *sX = (float *)smem_raw;                       // TP x d, then C floats of padding
-  T *sR = (T *)(sX + kMeanTP * d + C);                 // K x (TP+1)
-  const int tid = threadIdx.x;
-  const int nch = (d + C - 1) / C, units = K * nch;
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
-  const int64_t r1 = min(n, r0 + rows_per_block);
-  T acc[UPT][C], acc1[UPT];
-  double dacc[UPT][C], dacc1[UPT];
-#pragma unroll
-  for (int u = 0; u < UPT; u++) {
-    acc1[u] = T(0);
-    dacc1[u] = 0.0;
-#pragma unroll
-    for (int a = 0; a < C; a++) acc[u][a] = T(0), dacc[u][a] = 0.0;
-  }
-  int tiles = 0;
-  for (int64_t t0 = r0; t0 < r1; t0 += kMeanTP) {
-    const int tp = (int)min((int64_t)kMeanTP, r1 - t0);
-    __syncthreads();
-    for (int e = tid; e < kMeanTP * d; e += 256) {
-      int p = e / d;
-      sX[e] = (p < tp) ? X[(t0 + p) * d + (e - p * d)] : 0.f;
-    }
-    for (int e = tid; e < K * kMeanTP; e += 256) {
-      int j = e / kMeanTP, p = e - j * kMeanTP;
-      sR[j * (kMeanTP + 1) + p] = (p < tp) ? R[(size_t)j * n + t0 + p] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < UPT; u++) {
-      const int unit = tid + u * 256;
-      if (unit < units) {
-        const int j = unit / nch, c = unit - j * nch;
-        const T *rr = sR + j * (kMeanTP + 1);
-        const float *xx = sX + c * C;
-        for (int p = 0; p < kMeanTP; p++) {
-          const T r = rr[p];
-          acc1[u] += r;
-#pragma unroll
-          for (int a = 0; a < C; a++) acc[u][a] = fma(r, (T)xx[p * d + a], acc[u][a]);
-        }
-      }
-    }
-    // flush the short-range accumulators into FP64 every 16 tiles
-    if (++tiles == 16 || t0 + kMeanTP >= r1) {
-      tiles = 0;
-#pragma unroll
-      for (int u = 0; u < UPT; u++) {
-        dacc1[u] += (double)acc1[u];
-        acc1[u] = T(0);
-#pragma unroll
-        for (int a = 0; a < C; a++) {
-          dacc[u][a] += (double)acc[u][a];
-          acc[u][a] = T(0);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < UPT; u++) {
-    const int unit = tid + u * 256;
-    if (unit < units) {
-      const int j = unit / nch, c = unit - j * nch;
-      double *o = part + ((size_t)blockIdx.x * K + j) * (d + 1);
-      if (c == 0) o[0] = dacc1[u];
-#pragma unroll
-      for (int a = 0; a < C; a++)
-        if (c * C + a < d) o[1 + c * C + a] = dacc[u][a];
-    }
-  }
-}
-
 // PosteriorSum, Means = MeanSums / PosteriorSum, Probs = PosteriorSum / N
 // (EM2/MatrixEM.cpp:341-343,375); one block per component, blocks summed in order
+// and split over the 8 warps of its CTA (lane = column 0, the posterior sum,
+// or 1 + dimension), combined in warp order
 template <typename T>
-__global__ void k_final_means(const double *__restrict__ part, int G, int K, int d, int64_t n,
-                              double *__restrict__ mu, double *__restrict__ pi,
-                              double *__restrict__ psum, T *__restrict__ muT) {
-  const int j = blockIdx.x;
-  __shared__ double s1;
-  if (threadIdx.x == 0) {
+__global__ void __launch_bounds__(256)
+k_final_means(const double *__restrict__ part, int G, int K, int d, int64_t n, double *__restrict__ mu,
+              double *__restrict__ pi, double *__restrict__ psum, T *__restrict__ muT) {
+  const int j = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ double red[8][32], s1;
+  for (int c0 = 0; c0 <= d; c0 += 32) {
+    const int c = c0 + lane;
     double s = 0.0;
-    for (int g = 0; g < G; g++) s += part[((size_t)g * K + j) * (d + 1)];
-    s1 = s;
-    psum[j] = s;
-    pi[j] = s / (double)n;
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < d; q += blockDim.x) {
-    double s = 0.0;
-    for (int g = 0; g < G; g++) s += part[((size_t)g * K + j) * (d + 1) + 1 + q];
-    const double m = s / s1;
-    mu[(size_t)j * d + q] = m;
-    muT[(size_t)j * d + q] = (T)m;
+    if (c <= d) {
+#pragma unroll 8
+      for (int g = w; g < G; g += 8) s += part[((size_t)g * K + j) * (d + 1) + c];
+    }
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && c <= d) {
+#pragma unroll
+      for (int q = 1; q < 8; q++) s += red[q][lane];
+      red[0][lane] = s;
+      if (c == 0) {
+        s1 = s;
+        psum[j] = s;
+        pi[j] = s / (double)n;
+      }
+    }
+    __syncthreads();
+    if (w == 0 && c >= 1 && c <= d) {
+      const double m = red[0][lane] / s1;
+      mu[(size_t)j * d + c - 1] = m;
+      muT[(size_t)j * d + c - 1] = (T)m;
+    }
   }
 }
 
@@ -413,11 +340,74 @@ __global__ void k_final_means(const double *__restrict__ part, int G, int K, int
 // Eigen's LLT), log det = 2 sum log L_ii, W = L^-1 by column substitution,
 // log coefficient log pi_j - d/2 log 2pi - 1/2 log det, and an upper bound
 // of the condition number (block_cond_bound) folded into st->cond_bound.
-// From d = kFactorBlockedD on, the Cholesky and L^-1 run blocked through
-// factor_smem_bytes(d) of dynamic shared memory (block_cholesky_panels,
-// block_lower_inverse_rows: the same bits, 7.8 -> 3.3 ms for 64 components at
-// d = 256); below it the unblocked forms are faster (0.24 against 0.26 ms at
-// d = 64).
+constexpr double kLog2Pi = 1.8378770664093454835606594728112;   // log(2 pi)
+
+// Up to d = kFactorSmemD both matrices live in shared memory (k_factor_smem);
+// above it the Cholesky and L^-1 run blocked over matrices in L2
+// (block_cholesky_panels, block_lower_inverse_rows).
+template <typename T, int NS>
+__global__ void __launch_bounds__(kFactorThreads)
+k_factor_smem(int K, int d, double reg, int regularize, double *__restrict__ sigma, const double *__restrict__ pi,
+              const double *__restrict__ mu, double *__restrict__ work, double *__restrict__ linv,
+              double *__restrict__ logdet, double *__restrict__ logc, T *__restrict__ muT, T *__restrict__ linvT,
+              T *__restrict__ logcT, DevStatus *st) {
+  const int j = blockIdx.x, tid = threadIdx.x, ld = factor_ld(d);
+  extern __shared__ double fsm[];
+  __shared__ double red[3 * kFactorThreads / 32];
+  __shared__ double s_logpi;
+  double *A = fsm, *W = A + d * ld, *piv = W + d * ld, *rd = piv + d, *m = rd + d;
+  double *S = sigma + (size_t)j * d * d;
+  double add = 0.0;
+  const bool rg = regularize && reg != 0.0;
+  if (rg) {
+    // (1 - reg) S + (reg tr(S) / d) I
+    double t[1] = {tid < d ? S[(size_t)tid * d + tid] : 0.0};
+    block_sums(t, red);
+    add = reg * t[0] / (double)d;
+  }
+  double sums[3] = {0.0, 0.0, 0.0};      // ||Sigma||_F^2, ||L^-1||_F^2, log det
+  for (int e = tid; e < d * d; e += kFactorThreads) {
+    const int r = e / d, c = e - r * d;
+    double v = S[e];
+    if (rg) {
+      v = v * (1.0 - reg) + (r == c ? add : 0.0);
+      S[e] = v;
+    }
+    if (c <= r) {
+      A[r * ld + c] = v;
+      sums[0] = fma(c == r ? v : 2.0 * v, v, sums[0]);
+    }
+  }
+  for (int q = tid; q < d; q += kFactorThreads) muT[(size_t)j * d + q] = (T)mu[(size_t)j * d + q];
+  __syncthreads();
+  if (!block_factor_smem<NS>(A, W, piv, rd, m, d, ld)) {
+    if (tid == 0) atomicMin(&st->chol_failed, j);
+    return;
+  }
+  if (tid < d) sums[2] = log(piv[tid]);
+  if (tid == kFactorThreads - 1) s_logpi = log(pi[j]);
+  for (int e = tid; e < d * d; e += kFactorThreads) {
+    const int r = e / d, c = e - r * d;
+    const double w = c > r ? 0.0 : (c == r ? rd[r] : W[r * ld + c] * rd[r]);
+    sums[1] = fma(w, w, sums[1]);
+    linv[(size_t)j * d * d + e] = w;
+    linvT[(size_t)j * d * d + e] = (T)w;
+    // the wide E-step keeps L
+    if (d > 64) work[(size_t)j * d * d + e] = c > r ? 0.0 : (c == r ? sqrt(piv[r]) : A[r * ld + c] * rd[c]);
+  }
+  block_sums(sums, red);
+  if (tid == 0) {
+    // ||Sigma||_F ||L^-1||_F^2 >= cond (see block_cond_bound); non-negative
+    // doubles order like their bit patterns
+    atomicMax(reinterpret_cast<unsigned long long *>(&st->cond_bound),
+              (unsigned long long)__double_as_longlong(sqrt(sums[0]) * sums[1]));
+    logdet[j] = sums[2];
+    const double lc = s_logpi - 0.5 * (double)d * kLog2Pi - 0.5 * sums[2];
+    logc[j] = lc;
+    logcT[j] = (T)lc;
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kFactorThreads)
 k_factor(int K, int d, double reg, int regularize, double *__restrict__ sigma,
@@ -430,15 +420,11 @@ k_factor(int K, int d, double reg, int regularize, double *__restrict__ sigma,
   double *Wi = linv + (size_t)j * d * d;
   extern __shared__ double fsm[];
   if (regularize && reg != 0.0) block_regularize(S, d, reg);
-  const bool blocked = d >= kFactorBlockedD;
-  if (!(blocked ? block_cholesky_panels(S, d, A, fsm) : block_cholesky(S, d, A))) {
+  if (!block_cholesky_panels(S, d, A, fsm)) {
     if (tid == 0) atomicMin(&st->chol_failed, j);
     return;
   }
-  if (blocked)
-    block_lower_inverse_rows(A, d, Wi, fsm);
-  else
-    block_lower_inverse(A, d, Wi);
+  block_lower_inverse_rows(A, d, Wi, fsm);
   const double ld = block_chol_logdet(A, d);
   const double cb = block_cond_bound(S, Wi, d);
   if (tid == 0) {
@@ -508,49 +494,18 @@ int64_t em_plain_logl_blocks(int64_t n, int d) {
   }
 }
 
-template <typename T, int C>
-static int launch_means(fem_em *h, int upt, int64_t rpb, size_t sm) {
-  const T *R = (const T *)h->R;
-#define FEM_ML(U)                                                                          \
-  if (upt == U) {                                                                          \
-    FEM_CUDA(allow_dyn_smem(k_means_plain<T, C, U>, sm));                                  \
-    k_means_plain<T, C, U><<<h->mgrid, 256, sm, h->stream>>>(h->X, h->n, h->d, h->k, R,     \
-                                                             h->mpart, rpb);               \
-    return FEM_OK;                                                                         \
-  }
-  FEM_ML(1)
-  FEM_ML(2)
-  FEM_ML(4)
-#undef FEM_ML
-  set_error("means kernel: %d units per thread unsupported", upt);
-  return FEM_ERR_UNSUPPORTED;
-}
-
 template <typename T>
 static int mstep_plain_t(fem_em *h) {
   const int d = h->d, K = h->k;
   const int64_t n = h->n;
-  // column chunk: the smallest of 4, 8, 16 covering d, else 32 (any d)
+  // the form's limit: components times 4-, 8-, 16- or 32-column chunks
   const int C = d <= 4 ? 4 : (d <= 8 ? 8 : (d <= 16 ? 16 : 32));
-  const int units = K * ((d + C - 1) / C);
-  const int upt = units <= 256 ? 1 : (units <= 512 ? 2 : (units <= 1024 ? 4 : 0));
-  if (upt == 0) {
+  if (K * ((d + C - 1) / C) > 1024) {
     set_error("plain M-step: k*d too large (k=%d d=%d)", K, d);
     return FEM_ERR_UNSUPPORTED;
   }
-  const int64_t rpb = (n + h->mgrid - 1) / h->mgrid;
-  size_t sm = ((size_t)kMeanTP * d + C) * sizeof(float) + (size_t)K * (kMeanTP + 1) * sizeof(T);
-  int st;
-  switch (C) {
-    case 4: st = launch_means<T, 4>(h, upt, rpb, sm); break;
-    case 8: st = launch_means<T, 8>(h, upt, rpb, sm); break;
-    case 16: st = launch_means<T, 16>(h, upt, rpb, sm); break;
-    case 32: st = launch_means<T, 32>(h, upt, rpb, sm); break;
-    default: set_error("unsupported d=%d", d); return FEM_ERR_UNSUPPORTED;
-  }
-  FEM_TRY(st);
-  FEM_CUDA(cudaGetLastError());
-  k_final_means<T><<<K, 128, 0, h->stream>>>(h->mpart, h->mgrid, K, d, n, h->mu, h->pi, h->psum,
+  FEM_TRY(em_means_plain(h));
+  k_final_means<T><<<K, 256, 0, h->stream>>>(h->mpart, h->means.chunks, K, d, n, h->mu, h->pi, h->psum,
                                              (T *)h->muT);
   FEM_CUDA(cudaGetLastError());
   FEM_TRY(em_cov_plain(h));
@@ -608,25 +563,33 @@ int em_max_cond(fem_em *h, double *cond) {
   return FEM_OK;
 }
 
-int em_factor(fem_em *h, bool regularize) {
+template <typename T>
+static int factor_t(fem_em *h, bool regularize) {
   const int K = h->k, d = h->d;
-  const size_t sm = d >= kFactorBlockedD ? factor_smem_bytes(d) : 0;
-  if (h->cfg.precision == FEM_PREC_FP64) {
-    FEM_CUDA(allow_dyn_smem(k_factor<double>, sm));
-    k_factor<double><<<K, kFactorThreads, sm, h->stream>>>(K, d, h->cfg.reg_coef, regularize, h->sigma, h->pi,
-                                               h->mu, h->work, h->linv, h->logdet, h->logc,
-                                               (double *)h->muT, (double *)h->linvT,
-                                               (double *)h->logcT, h->dstat);
-  } else {
-    FEM_CUDA(allow_dyn_smem(k_factor<float>, sm));
-    k_factor<float><<<K, kFactorThreads, sm, h->stream>>>(K, d, h->cfg.reg_coef, regularize, h->sigma, h->pi,
-                                              h->mu, h->work, h->linv, h->logdet, h->logc,
-                                              (float *)h->muT, (float *)h->linvT,
-                                              (float *)h->logcT, h->dstat);
-  }
+  const size_t sm = factor_smem_bytes(d);
+#define FEM_FK(KERNEL)                                                                                                \
+  do {                                                                                                                \
+    FEM_CUDA(allow_dyn_smem(KERNEL, sm));                                                                             \
+    KERNEL<<<K, kFactorThreads, sm, h->stream>>>(K, d, h->cfg.reg_coef, regularize, h->sigma, h->pi, h->mu, h->work,  \
+                                                 h->linv, h->logdet, h->logc, (T *)h->muT, (T *)h->linvT,             \
+                                                 (T *)h->logcT, h->dstat);                                            \
+  } while (0)
+  if (d <= 32)
+    FEM_FK((k_factor_smem<T, 1>));
+  else if (d <= 64)
+    FEM_FK((k_factor_smem<T, 2>));
+  else if (d <= kFactorSmemD)
+    FEM_FK((k_factor_smem<T, 4>));
+  else
+    FEM_FK(k_factor<T>);
+#undef FEM_FK
   FEM_CUDA(cudaGetLastError());
   h->launches += 1;
   return FEM_OK;
+}
+
+int em_factor(fem_em *h, bool regularize) {
+  return h->cfg.precision == FEM_PREC_FP64 ? factor_t<double>(h, regularize) : factor_t<float>(h, regularize);
 }
 
 // ------------------------------------------------ posteriors read-back

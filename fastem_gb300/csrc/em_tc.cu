@@ -545,27 +545,34 @@ k_means_tc(const __grid_constant__ CUtensorMap tm_rh, const __grid_constant__ CU
   if (warp == 1) tmem_dealloc(tbase, 256);
 }
 
-// S1 = sum r, mu = S2 / S1, pi = S1 / N (FP64, blocks summed in order)
-__global__ void k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n,
-                                 double *__restrict__ mu, double *__restrict__ pi,
-                                 double *__restrict__ psum, float *__restrict__ muf) {
-  const int j = blockIdx.x;
-  __shared__ double s1;
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int g = 0; g < G; g++) s += part[((size_t)g * kMeanN + kD) * kMaxK + j];
-    s1 = s;
-    psum[j] = s;
-    pi[j] = s / (double)n;
-  }
+// S1 = sum r, mu = S2 / S1, pi = S1 / N (FP64).  One CTA per component; the
+// CTAs' partials are split over its 4 thread sets (65 threads each: column 64
+// holds S1) and combined in order
+constexpr int kFMSplit = 4, kFMCols = kD + 1;
+__global__ void __launch_bounds__(kFMSplit * kFMCols)
+k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n, double *__restrict__ mu,
+                 double *__restrict__ pi, double *__restrict__ psum, float *__restrict__ muf) {
+  const int j = blockIdx.x, q = threadIdx.x % kFMCols, w = threadIdx.x / kFMCols;
+  __shared__ double red[kFMSplit][kFMCols];
+  double s = 0.0;
+#pragma unroll 8
+  for (int g = w; g < G; g += kFMSplit) s += part[((size_t)g * kMeanN + q) * kMaxK + j];
+  red[w][q] = s;
   __syncthreads();
-  for (int q = threadIdx.x; q < kD; q += blockDim.x) {
-    double s = 0.0;
-    for (int g = 0; g < G; g++) s += part[((size_t)g * kMeanN + q) * kMaxK + j];
-    const double m = s / s1;
-    if (q < d) mu[(size_t)j * d + q] = m;
-    muf[(size_t)j * kD + q] = q < d ? (float)m : 0.f;
+  if (w) return;
+  double s1 = 0.0;
+#pragma unroll
+  for (int u = 0; u < kFMSplit; u++) s1 += red[u][kD];
+  if (q == kD) {
+    psum[j] = s1;
+    pi[j] = s1 / (double)n;
+    return;
   }
+#pragma unroll
+  for (int u = 1; u < kFMSplit; u++) s += red[u][q];
+  const double m = s / s1;
+  if (q < d) mu[(size_t)j * d + q] = m;
+  muf[(size_t)j * kD + q] = q < d ? (float)m : 0.f;
 }
 
 // ========================================================= covariances
@@ -1037,34 +1044,46 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
 // Sigma_j = sym(sum z x^T - (sum z) muf^T) / N_j - (mu - muf)(mu - muf)^T:
 // the scatter around the FP32 means the producers used, moved to the FP64
 // means; chunks summed in order (FP64)
-__global__ void k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d,
-                               const double *__restrict__ psum, const double *__restrict__ mu,
-                               const float *__restrict__ muf, double *__restrict__ sigma) {
+// (a CTA owns rows 16 blockIdx.y .. + 15 of component blockIdx.x)
+constexpr int kFCRows = 16;
+__global__ void __launch_bounds__(512)
+k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const double *__restrict__ psum,
+               const double *__restrict__ mu, const float *__restrict__ muf, double *__restrict__ sigma) {
   const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
+  const int a0 = blockIdx.y * kFCRows;
+  // S[a][b] = sum z_a x_b for the block's 16 rows a, and S[b][a] for its 16 columns
+  __shared__ double sr[kFCRows][kD + 1], sc[kD][kFCRows + 1];
   __shared__ double sz[kD];                    // sum z of component j, per dimension
-  __shared__ double dm[kD];                    // mu - muf
-  for (int a = threadIdx.x; a < kD; a += blockDim.x) {
+  const double *P0 = cpart + ((size_t)grp * 2 + pr) * (kZCols * 128) + slot * 64;
+  const size_t step = (size_t)gx * 2 * (kZCols * 128);
+  for (int e = threadIdx.x; e < 2 * kFCRows * kD + kD; e += blockDim.x) {
+    // rows: (b, a0 + i) at P[b * 128 + a0 + i]; columns: (a0 + i, b) at P[(a0 + i) * 128 + b]; sum z: P[64 * 128 + a]
+    size_t o;
+    double *dst;
+    if (e < kFCRows * kD) {
+      const int i = e % kFCRows, b = e / kFCRows;
+      o = (size_t)b * 128 + a0 + i, dst = &sr[i][b];
+    } else if (e < 2 * kFCRows * kD) {
+      const int r = e - kFCRows * kD, b = r % kD, i = r / kD;
+      o = (size_t)(a0 + i) * 128 + b, dst = &sc[b][i];
+    } else {
+      const int a = e - 2 * kFCRows * kD;
+      o = (size_t)kD * 128 + a, dst = &sz[a];
+    }
     double v = 0.0;
-    for (int ch = 0; ch < gy; ch++)
-      v += cpart[(((size_t)ch * gx + grp) * 2 + pr) * (kZCols * 128) + (size_t)kD * 128 + slot * 64 + a];
-    sz[a] = v;
-    dm[a] = a < d ? mu[(size_t)j * d + a] - (double)muf[(size_t)j * kD + a] : 0.0;
+#pragma unroll 8
+    for (int ch = 0; ch < gy; ch++) v += P0[ch * step + o];
+    *dst = v;
   }
   __syncthreads();
   const double inv = 1.0 / psum[j];
   double *Sg = sigma + (size_t)j * d * d;
-  for (int e = threadIdx.x; e < d * d; e += blockDim.x) {
-    const int a = e / d, b = e - a * d;
-    if (b < a) continue;
-    double sab = 0.0, sba = 0.0;
-    for (int ch = 0; ch < gy; ch++) {
-      const double *P = cpart + (((size_t)ch * gx + grp) * 2 + pr) * (kZCols * 128) + slot * 64;
-      sab += P[(size_t)b * 128 + a];
-      sba += P[(size_t)a * 128 + b];
-    }
-    const double ca = sab - sz[a] * (double)muf[(size_t)j * kD + b];
-    const double cb = sba - sz[b] * (double)muf[(size_t)j * kD + a];
-    const double v = 0.5 * (ca + cb) * inv - dm[a] * dm[b];
+  for (int e = threadIdx.x; e < kFCRows * kD; e += blockDim.x) {
+    const int i = e / kD, a = a0 + i, b = e - i * kD;
+    if (a >= d || b >= d || b < a) continue;
+    const double ma = muf[(size_t)j * kD + a], mb = muf[(size_t)j * kD + b];
+    const double ca = sr[i][b] - sz[a] * mb, cb = sc[b][i] - sz[b] * ma;
+    const double v = 0.5 * (ca + cb) * inv - (mu[(size_t)j * d + a] - ma) * (mu[(size_t)j * d + b] - mb);
     Sg[a * d + b] = v;
     Sg[b * d + a] = v;
   }
@@ -1188,11 +1207,15 @@ __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half 
   if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
 }
 
+// one warp, a lane's terms first, then a fixed tree
 __global__ void k_reduce_parts(const double *__restrict__ part, int np, DevStatus *st,
                                const int *__restrict__ err) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < np; b++) s += part[b];
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = threadIdx.x; b < np; b += 32) s += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) {
     st->logl = s;
     if (*err) st->timeout = 1;
   }
@@ -1409,7 +1432,7 @@ int em_tc_mstep(fem_em *h) {
   k_means_tc<<<p->mgrid, 192, msmem_bytes(), h->stream>>>(p->tm_rh, p->tm_rl, p->tm_xht, p->tm_xlt, h->n,
                                                            p->mpart, p->err);
   FEM_CUDA(cudaGetLastError());
-  k_final_means_tc<<<K, 64, 0, h->stream>>>(p->mpart, p->mgrid, K, h->d, h->n, h->mu, h->pi, h->psum, p->muf);
+  k_final_means_tc<<<K, kFMSplit * kFMCols, 0, h->stream>>>(p->mpart, p->mgrid, K, h->d, h->n, h->mu, h->pi, h->psum, p->muf);
   FEM_CUDA(cudaGetLastError());
   if (em_tc_small_components(h->n, h->k, h->d)) {
     timing_begin(h, 8);
@@ -1427,7 +1450,7 @@ int em_tc_mstep(fem_em *h) {
                                                                            h->n, bpc, p->cpart, p->err);
     FEM_CUDA(cudaGetLastError());
     timing_begin(h, 9);
-    k_final_cov_zx<<<K, 256, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, h->sigma);
+    k_final_cov_zx<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, h->sigma);
   } else {
     k_cov_tc<<<dim3(p->cgx, p->cgy), kCThreads, csmem_bytes(), h->stream>>>(p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf,
                                                                            h->n, bpc, p->cpart, p->dpart, p->err);

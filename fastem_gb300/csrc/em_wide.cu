@@ -918,10 +918,14 @@ __global__ void k_wide_amax(const float *__restrict__ X, int64_t m, float *__res
   if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(v));
 }
 
+// one warp, a lane's terms first, then a fixed tree
 __global__ void k_wide_reduce(const double *__restrict__ part, int np, DevStatus *st, const int *__restrict__ err) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < np; b++) s += part[b];
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = threadIdx.x; b < np; b += 32) s += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) {
     st->logl = s;
     if (*err) st->timeout = 1;
   }

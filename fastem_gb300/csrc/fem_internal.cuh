@@ -88,7 +88,7 @@ struct DevStatus {
 };
 
 // ------------------------------------------------------------------ EM handle
-// schedule of the CUDA-core covariance sums (em_cov.cu)
+// schedule of the CUDA-core means or covariance sums (em_cov.cu)
 struct CovPlan {
   int TB = 0, tri = 0, nb = 0, nblk = 0;   // block size, one triangular block, blocks per dimension / per component
   int gx = 0, upc = 0, G = 0, cj = 0;      // CTAs over the units, units per CTA, point groups, components per CTA
@@ -131,8 +131,8 @@ struct fem_em {
   double *logl_part = nullptr;
   int64_t n_logl_part = 0;
   // M-step partials (FP64)
-  double *mpart = nullptr;      // means: grid x k x (d+1)
-  int mgrid = 0;
+  double *mpart = nullptr;      // CUDA-core means: means.part
+  fem::CovPlan means;
   double *cpart = nullptr;      // CUDA-core covariances: cov.part
   fem::CovPlan cov;
   double *psum = nullptr;       // k   PosteriorSum

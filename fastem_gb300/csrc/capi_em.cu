@@ -226,7 +226,7 @@ int fem_em_create(int d, int64_t n, int k, const fem_em_config *cfg, fem_em **ou
   if (c.precision == FEM_PREC_MIXED) {
     st = em_tc_create(h);
     if (st) return fail(st);
-    if (em_tc_small_components(n, k, d)) {
+    if (em_tc_cuda_core_cov(h)) {
       // partials of the FP32 CUDA-core covariance used for small components
       h->cov = cov_plan(d, n, k, false, true);
       if ((st = dalloc(&h->cpart, h->cov.part))) return fail(st);

@@ -504,19 +504,19 @@ void split_units(int units, int *gx, int *upc, int *G) {
   }
 }
 
+}  // namespace
+
 // row chunks: the count whose waves over `slots` resident CTAs finish first,
-// counting two tiles' time for a CTA's start and end
-void split_rows(int64_t n, int TP, int gx, int slots, int *chunks, int64_t *rows) {
+// counting `extra` tiles' time for a CTA's start and end
+void split_rows(int64_t n, int TP, int gx, int slots, double extra, int *chunks, int64_t *rows) {
   const int64_t tiles = (n + TP - 1) / TP;
   double bt = 1e300;
   for (int64_t c = 1; c <= std::min<int64_t>(tiles, (int64_t)3 * slots / gx + 1); c++) {
     const int64_t tpc = (tiles + c - 1) / c, ch = (tiles + tpc - 1) / tpc;
-    const double t = std::ceil((double)gx * ch / slots) * (tpc + 2.0);
+    const double t = std::ceil((double)gx * ch / slots) * (tpc + extra);
     if (t < bt) bt = t, *chunks = (int)ch, *rows = tpc * TP;
   }
 }
-
-}  // namespace
 
 // Schedule of the covariance sums for one handle (fixed by its shape).
 //
@@ -539,7 +539,7 @@ CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
   const size_t rb = ((size_t)p.cj * p.rpitch * (fp64 ? 8 : 4) + 15) & ~(size_t)15;
   p.smem = 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + rb);
   if (p.G > 1) p.smem = std::max(p.smem, (size_t)ne * kCvThreads * (fp64 ? 8 : 4));
-  split_rows(n, p.TP, p.gx, (fp64 ? 1 : 2) * sm_count(), &p.chunks, &p.rows);
+  split_rows(n, p.TP, p.gx, (fp64 ? 1 : 2) * sm_count(), 2.0, &p.chunks, &p.rows);
   p.part = (size_t)p.chunks * units * ne;
   return p;
 }
@@ -562,7 +562,7 @@ CovPlan means_plan(int d, int64_t n, int k, bool fp64) {
     if (p.smem <= kCvMaxSmem / 2) break;
   }
   if (p.G > 1) p.smem = std::max(p.smem, (size_t)16 * kCvThreads * sizeof(double));
-  split_rows(n, p.TP, p.gx, 2 * sm_count(), &p.chunks, &p.rows);
+  split_rows(n, p.TP, p.gx, 2 * sm_count(), 2.0, &p.chunks, &p.rows);
   p.part = (size_t)p.chunks * k * (d + 1);
   return p;
 }

@@ -143,15 +143,49 @@ static_assert(sizeof(ZSmem) + 1024 <= 232448, "covariance kernel shared memory")
 static_assert(kZSets % kZSplit == 0 && (kBlk / 16) % kZSplit == 0, "covariance producer split");
 static_assert(kZACol + kZA * kZAStage <= 512 && 3 * kZDCol + kZN <= kZACol, "covariance kernel TMEM columns");
 
+// covariance kernel, split z x^T form: 4 components per CTA (2 pairs), 64-point blocks of four 16-point steps
+constexpr int kSIn = 4;                  // input ring (blocks)
+constexpr int kSSteps = kBlk / 16;
+constexpr int kSA = 6;                   // TMEM A ring (steps)
+constexpr int kSAcc = 16;                // blocks a zh xh^T accumulator spans
+constexpr int kSWin = 64;                // blocks an FP32 register sum spans (4096 rows)
+constexpr int kSRows = 2048;             // rows an FP32 diagonal sum spans
+// TMEM columns: [pair] zh [xh; 1]^T, [pair] the small products, A ring (per pair 8 hi + 8 lo a step)
+constexpr int kSN = kD + 16;             // accumulator columns per pair: 64 sums, sum z, 15 unused
+constexpr uint32_t kSCross = 2 * kSN, kSACol = 4 * kSN, kSAStage = 32;
+// warps 0 TMA, 1 MMA, 2 posteriors, 3 none; 4..19 producers (4 groups); 20..27 flush (a group of 4 per pair)
+constexpr int kSThreads = 28 * 32;
+constexpr int kSProd0 = 4, kSFlush0 = 20;
+// registers per thread after the split: 128 threads x 24 + 512 x 72 + 256 x
+// 96 = 64512 = the launch's 896 x 72
+constexpr int kSRegLaunch = 72, kSRegCtl = 24, kSRegProd = 72, kSRegFlush = 96;
+static_assert(128 * kSRegCtl + 512 * kSRegProd + 256 * kSRegFlush <= kSThreads * kSRegLaunch, "register split");
+static_assert(kSACol + kSA * kSAStage <= 512, "split covariance TMEM columns");
+struct __align__(1024) SSmem {
+  __half bh[kSIn][kSN * kBlk];                       // rows 0..63 xh^T (TMA, SW128), row 64 ones, 65..79 zero
+  __half bl[kSIn][kD * kBlk], bm[kSIn][kD * kBlk];   // xl^T, xm^T
+  float x[kSIn][kBlk * kD];                          // FP32 rows (TMA)
+  __half rh[kSIn][4 * kBlk], rl[kSIn][4 * kBlk];     // posteriors of the CTA's 4 components
+  float rf[kSIn][4 * kBlk];                          // hi + lo
+  float mu[4][kD];                                   // means of the CTA's components in column units
+  float zs[4][kD], zm[4][kD];                        // 1 / zunit, -mu / zunit
+  uint64_t in_full[kSIn], rf_full[kSIn], in_empty[kSIn], a_full[kSA], a_empty[kSA], acc_full, acc_empty, cross_full,
+      mma_done;
+  uint32_t tmem_base;
+};
+static_assert(sizeof(SSmem) + 1024 <= 232448, "split covariance shared memory");
+
 struct TcEmPlan {
   CUtensorMap tm_xh, tm_xl, tm_wh, tm_wl;      // E-step
   CUtensorMap tm_rh, tm_rl, tm_xht, tm_xlt;    // means
+  CUtensorMap tm_xmt;                          // split covariance
   CUtensorMap tm_x32, tm_rh4, tm_rl4;          // covariances
   __half *Wh = nullptr, *Wl = nullptr;  // (K*d) x d, permuted rows
   float *bias = nullptr;                // K*d, permuted
   float *clo = nullptr;                 // log coefficient - float(log coefficient)
   __half *Rh = nullptr, *Rl = nullptr;  // K x np posteriors hi / lo
-  __half *XhT = nullptr, *XlT = nullptr;  // d x np
+  __half *XhT = nullptr, *XlT = nullptr;  // d x np, in units of each dimension (x_unit)
+  __half *XmT = nullptr;                // their remainder (split covariance only)
   int64_t np = 0;                       // padded row pitch (multiple of 64)
   float *lsc = nullptr;                 // E-step scratch: egrid x 2 x K x 256
   double *epart = nullptr;              // per-CTA log-likelihood
@@ -162,9 +196,11 @@ struct TcEmPlan {
   float *chi = nullptr;                 // float(log coefficient); -inf for padding components
   float *X64 = nullptr;                 // n x 64 zero-padded FP32 rows when d < 64
   int *err = nullptr;                   // device status of the bounded waits
-  float *amax = nullptr;                // upload: largest |x| (FP16 range check)
+  float *amax = nullptr;                // upload: largest |x| of every dimension, then of all (FP16 range check)
+  float *zunit = nullptr;               // split covariance: unit of z per component and dimension
   int *roles = nullptr;                 // bounded-wait expiry self-test: which waits gave up
   int egrid = 0, mgrid = 0, cgx = 0, cgy = 0;
+  int64_t srows = 0;                    // split form: rows per chunk (0: not used)
   int kp = 0, d = 0;                    // components padded to a multiple of 4; true dimension
 };
 
@@ -176,6 +212,28 @@ __device__ __forceinline__ void store_post(__half *Rh, __half *Rl, size_t o, flo
   const __half h = __float2half_rn(r);
   Rh[o] = h;
   Rl[o] = __float2half_rn(r - __half2float(h));
+}
+
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+
+// Columns of X^T are held in units of a power of two, h = 2^(E - 10) with 2^E
+// <= max |x| < 2^(E + 1) over the column: x = h (xh + xl), xh an integer of at
+// most 2^11 (exact in FP16), |xl| <= 1/2 in FP16 (2^-24 of the column's
+// maximum); the split covariance adds what is left, xm.  Products of xh with a weight on a grid add up exactly in FP32
+// while they stay below 2^24 units, where the tensor core's truncation of a
+// floating split would cut every addition.
+__device__ __forceinline__ int x_unit_exp(float cmax) { return cmax > 0.f ? max(ilogbf(cmax), -110) - 10 : 0; }
+__device__ __forceinline__ float x_unit(float cmax) { return ldexpf(1.f, x_unit_exp(cmax)); }
+
+// unit of z = r (x - mu) in the split covariance: 2^-9 of the standard
+// deviation that the E-step used (sigma: its covariance's diagonal entry), so
+// most rows are integers below 2^11, but no less than keeps |z| <= 2 max|x|
+// below 2^15 units whatever sigma says
+__device__ __forceinline__ float z_unit(double var, float cmax) {
+  const int lo = x_unit_exp(cmax) - 3;
+  int e = lo;
+  if (var > 1e-60 && var < 1e60) e = max(lo, ilogb(sqrt(var)) - 9);
+  return ldexpf(1.f, min(e, 100));
 }
 
 // ============================================================== E-step
@@ -545,13 +603,15 @@ k_means_tc(const __grid_constant__ CUtensorMap tm_rh, const __grid_constant__ CU
   if (warp == 1) tmem_dealloc(tbase, 256);
 }
 
-// S1 = sum r, mu = S2 / S1, pi = S1 / N (FP64).  One CTA per component; the
+// S1 = sum r, mu = S2 / S1, pi = S1 / N (FP64), and the units of the split
+// covariance from the E-step's covariances.  One CTA per component; the
 // CTAs' partials are split over its 4 thread sets (65 threads each: column 64
 // holds S1) and combined in order
 constexpr int kFMSplit = 4, kFMCols = kD + 1;
 __global__ void __launch_bounds__(kFMSplit * kFMCols)
 k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n, double *__restrict__ mu,
-                 double *__restrict__ pi, double *__restrict__ psum, float *__restrict__ muf) {
+                 double *__restrict__ pi, double *__restrict__ psum, float *__restrict__ muf,
+                 const float *__restrict__ cmax, const double *__restrict__ sigma, float *__restrict__ zunit) {
   const int j = blockIdx.x, q = threadIdx.x % kFMCols, w = threadIdx.x / kFMCols;
   __shared__ double red[kFMSplit][kFMCols];
   double s = 0.0;
@@ -570,9 +630,10 @@ k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n
   }
 #pragma unroll
   for (int u = 1; u < kFMSplit; u++) s += red[u][q];
-  const double m = s / s1;
+  const double m = s * (double)x_unit(cmax[q]) / s1;
   if (q < d) mu[(size_t)j * d + q] = m;
   muf[(size_t)j * kD + q] = q < d ? (float)m : 0.f;
+  zunit[(size_t)j * kD + q] = q < d ? z_unit(sigma[((size_t)j * d + q) * d + q], cmax[q]) : 1.f;
 }
 
 // ========================================================= covariances
@@ -848,7 +909,8 @@ __global__ void k_final_cov_tc(const double *__restrict__ cpart, const double *_
 // kFlushBlocks blocks (double buffered in TMEM).
 __global__ void __launch_bounds__(kZThreads, 1)
 k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUtensorMap tm_xlt,
-         const __grid_constant__ CUtensorMap tm_rh4, const float *__restrict__ muf, int64_t n,
+         const __grid_constant__ CUtensorMap tm_rh4, const float *__restrict__ muf, const float *__restrict__ cmax,
+         int64_t n,
          int64_t blocks_per_chunk, double *__restrict__ cpart, int *err) {
   extern __shared__ uint8_t smem_raw[];
   ZSmem &S = smem_aligned<ZSmem>(smem_raw);
@@ -946,6 +1008,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
     const int a = 32 * (quad & 1) + lane;        // dimension = TMEM lane within the slot
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     float mu[2];
+    const float2 hx = f2(x_unit(cmax[a]));       // x = hx (xh + xl)
 #pragma unroll
     for (int pr = 0; pr < 2; pr++) mu[pr] = muf[(size_t)(cg * 4 + 2 * pr + slot) * kD + a];
     bool ok = true;
@@ -958,7 +1021,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
       const uint8_t *rowl = reinterpret_cast<const uint8_t *>(S.bl[st]) + a * 128;
 #pragma unroll 1
       for (int kb = part * kSteps; kb < (part + 1) * kSteps; kb++) {
-        // x = xh + xl (exact in FP32) of the 16 points of this K step, dimension a
+        // x / hx = xh + xl (exact in FP32) of the 16 points of this K step, dimension a
         float2 x[8];
 #pragma unroll
         for (int hc = 0; hc < 2; hc++) {
@@ -982,7 +1045,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
           uint32_t packed[8];
 #pragma unroll
           for (int q = 0; q < 8; q++) {
-            const float2 dz = __fadd2_rn(x[q], nm);
+            const float2 dz = __ffma2_rn(x[q], hx, nm);
             const __half2 z = __hmul2(__floats2half2_rn(dz.x, dz.y), *reinterpret_cast<const __half2 *>(&rw[q]));
             packed[q] = *reinterpret_cast<const uint32_t *>(&z);
           }
@@ -1048,7 +1111,8 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
 constexpr int kFCRows = 16;
 __global__ void __launch_bounds__(512)
 k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const double *__restrict__ psum,
-               const double *__restrict__ mu, const float *__restrict__ muf, double *__restrict__ sigma) {
+               const double *__restrict__ mu, const float *__restrict__ muf, const float *__restrict__ cmax,
+               double *__restrict__ sigma) {
   const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
   const int a0 = blockIdx.y * kFCRows;
   // S[a][b] = sum z_a x_b for the block's 16 rows a, and S[b][a] for its 16 columns
@@ -1082,8 +1146,362 @@ k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const do
     const int i = e / kD, a = a0 + i, b = e - i * kD;
     if (a >= d || b >= d || b < a) continue;
     const double ma = muf[(size_t)j * kD + a], mb = muf[(size_t)j * kD + b];
-    const double ca = sr[i][b] - sz[a] * mb, cb = sc[b][i] - sz[b] * ma;
+    // the sums' columns are in units of the x column
+    const double ca = sr[i][b] * x_unit(cmax[b]) - sz[a] * mb, cb = sc[b][i] * x_unit(cmax[a]) - sz[b] * ma;
     const double v = 0.5 * (ca + cb) * inv - (mu[(size_t)j * d + a] - ma) * (mu[(size_t)j * d + b] - mb);
+    Sg[a * d + b] = v;
+    Sg[b * d + a] = v;
+  }
+}
+
+// ================================================ covariances (split z x^T)
+// The z x^T form above with z = r (x - mu) split into FP16 hi + lo as well,
+// for fits whose components hold too few points for z's single rounding to
+// average out:  sum z x^T = sum zh xh^T + (sum zh (xl + xm)^T + sum zl (xh + xl)^T).
+// To reach the accuracy of FP32 sums on CUDA cores:
+//  * the tensor core truncates its FP32 accumulator, so z is put on a grid as x
+//    is (z_unit: zh an integer, |zl| <= 1/2): zh xh^T then adds up exactly below
+//    2^24 units, which kSAcc blocks of a component rarely reach (beyond it,
+//    truncation is as for any FP32 sum).  With a floating split every addition
+//    truncates: 4e-8 to 7e-8 off where FP32 sums on CUDA cores are at 1e-8;
+//  * the small products have an accumulator of their own over the chunk; z
+//    comes from the FP32 rows, and x on the B side has a third part xm;
+//  * x on the B side is shared by all components and so not centred: a sum
+//    holds (sum z) mu^T, random and |mu| / sigma times larger than what is
+//    wanted.  A row of ones in B gives sum zh (exact) and sum zl beside the
+//    sums, and flush warps take the product off before they add to FP32
+//    registers (round to nearest); those go to FP64 every kSWin blocks;
+//  * the diagonal is summed by the producers from the unrounded z (FP32 over
+//    at most kSRows rows, then FP64).
+// Sums are in units of z (rows) and x (columns), whatever the data's scale.
+// Warp roles: 0 TMA, 1 MMA, 2 turns the posteriors into FP32 once per block;
+// four producer groups of 4 warps, group g forming step g of every block (a
+// warp's lanes and dimensions as in k_cov_zx); a flush group of 4 warps per pair, 64 sums per thread (which is why the
+// registers are split unevenly).
+// What bounds it: shared memory, read by producers (x, posteriors) and by the
+// 40 MMAs of a block (B), written by TMA, ~1800 of the ~3000 cycles a block
+// takes; without 24 of the MMAs it is 13 % faster, with waits that sleep
+// instead of polling no different.  GB300, with its finalisation, against the
+// FP32 CUDA-core form: N = 2^20, d = 64, K = 128 20.7 -> 5.4 ms, N = 200000,
+// d = 64, K = 32 1.19 -> 0.32 ms; error of Sigma (Frobenius) against 64-bit
+// sums over the same posteriors 8e-9 and 9e-9 (CUDA cores 8e-9 and 1.6e-8).
+__global__ void __launch_bounds__(kSThreads, 1)
+k_cov_split(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUtensorMap tm_xlt,
+            const __grid_constant__ CUtensorMap tm_xmt, const __grid_constant__ CUtensorMap tm_x32,
+            const __grid_constant__ CUtensorMap tm_rh4, const __grid_constant__ CUtensorMap tm_rl4,
+            const float *__restrict__ muf, const float *__restrict__ cmax, const float *__restrict__ zunit, int64_t n,
+            int64_t rows_per_chunk, double *__restrict__ cpart, double *__restrict__ dpart, int *err) {
+  extern __shared__ uint8_t smem_raw[];
+  SSmem &S = smem_aligned<SSmem>(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cg = blockIdx.x;
+  const int64_t r0 = (int64_t)blockIdx.y * rows_per_chunk, r1 = std::min<int64_t>(n, r0 + rows_per_chunk);
+  const int mine = (int)((r1 - r0 + kBlk - 1) / kBlk);     // blocks of this chunk
+  const size_t cta = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+
+  if (threadIdx.x == 0) {
+    // a block is read by the MMA and by the 16 producer warps
+    for (int st = 0; st < kSIn; st++)
+      mbar_init(&S.in_full[st], 1), mbar_init(&S.rf_full[st], 1), mbar_init(&S.in_empty[st], 17);
+    for (int sl = 0; sl < kSA; sl++) mbar_init(&S.a_full[sl], 4), mbar_init(&S.a_empty[sl], 1);
+    mbar_init(&S.acc_full, 1);
+    mbar_init(&S.acc_empty, 8);
+    mbar_init(&S.cross_full, 1);
+    mbar_init(&S.mma_done, 1);
+    fence_mbar_init();
+  }
+  // 16-byte chunk c of row r stored at c ^ (r & 7)
+  for (int e = threadIdx.x; e < kSIn * 16 * kBlk; e += blockDim.x) {
+    const int st = e / (16 * kBlk), rem = e - st * 16 * kBlk;
+    const int r = kD + rem / kBlk, col = rem % kBlk;
+    S.bh[st][r * kBlk + (((col >> 3) ^ (r & 7)) << 3) + (col & 7)] = __float2half(r == kD ? 1.f : 0.f);
+  }
+  fence_proxy_async_smem();
+  for (int e = threadIdx.x; e < 4 * kD; e += blockDim.x) {
+    const float m = muf[(size_t)cg * 4 * kD + e];
+    const int ez = ilogbf(zunit[(size_t)cg * 4 * kD + e]);
+    S.mu[e / kD][e % kD] = ldexpf(m, -x_unit_exp(cmax[e % kD]));
+    S.zs[e / kD][e % kD] = ldexpf(1.f, -ez);
+    S.zm[e / kD][e % kD] = ldexpf(-m, -ez);
+  }
+  if (warp == 1) tmem_alloc(&S.tmem_base, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = S.tmem_base;
+  constexpr uint32_t kInBytes = 3 * kD * kBlk * 2 + kBlk * kD * 4 + 2 * 4 * kBlk * 2;
+
+  // no function calls behind this point: a call may use registers that the
+  // split has taken away
+  if (warp < kSProd0) {
+    reg_dec<kSRegCtl>();
+    if (warp == 0) {
+      // ---------------------------------------------- TMA
+      if (elect_one()) {
+        bool ok = true;
+        for (int t = 0; t < mine && ok; t++) {
+          const int st = t % kSIn;
+          if (!(ok = mbar_wait_lazy(&S.in_empty[st], ((t / kSIn) & 1) ^ 1, err, 128))) break;
+          const int p0 = (int)(r0 + (int64_t)t * kBlk);
+          mbar_expect_tx(&S.in_full[st], kInBytes);
+          tma_load_2d(S.bh[st], &tm_xht, &S.in_full[st], p0, 0);
+          tma_load_2d(S.bl[st], &tm_xlt, &S.in_full[st], p0, 0);
+          tma_load_2d(S.bm[st], &tm_xmt, &S.in_full[st], p0, 0);
+          tma_load_2d(S.x[st], &tm_x32, &S.in_full[st], 0, p0);
+          tma_load_2d(S.rh[st], &tm_rh4, &S.in_full[st], p0, cg * 4);
+          tma_load_2d(S.rl[st], &tm_rl4, &S.in_full[st], p0, cg * 4);
+        }
+        for (int u = mine - 1; u >= 0 && u >= mine - kSIn; u--)
+          mbar_wait_drain(&S.in_full[u % kSIn], (u / kSIn) & 1);
+      }
+    } else if (warp == 1) {
+      // ---------------------------------------------- MMA
+      if (elect_one()) {
+        bool ok = true;
+        constexpr uint32_t id = idesc_f16(128, kD), idn = idesc_f16(128, kSN);
+        uint32_t sl = 0, sp = 0;                   // operand slot and its phase
+        for (int t = 0; t < mine && ok; t++) {
+          const int st = t % kSIn;
+          if (!(ok = mbar_wait(&S.in_full[st], (t / kSIn) & 1, err))) break;
+          const uint64_t dbh = sdesc_sw128(smem_u32(S.bh[st])), dbl = sdesc_sw128(smem_u32(S.bl[st]));
+          const uint64_t dbm = sdesc_sw128(smem_u32(S.bm[st]));
+#pragma unroll 1
+          for (int kb = 0; kb < kSSteps; kb++) {
+            if (!(ok = mbar_wait(&S.a_full[sl], sp, err))) break;
+            tc_fence_after();
+            const uint32_t at = tbase + kSACol + sl * kSAStage;
+#pragma unroll
+            for (int pr = 0; pr < 2; pr++) {
+              // +32 bytes per 16-point step inside the 128-byte swizzle row
+              const uint32_t dc = tbase + kSCross + pr * kSN, ah = at + 16 * pr, al = ah + 8;
+              mma_f16_ta(dc, al, dbh + 2 * kb, idn, (t | kb) != 0);
+              mma_f16_ta(dc, al, dbl + 2 * kb, id, 1);
+              mma_f16_ta(dc, ah, dbl + 2 * kb, id, 1);
+              mma_f16_ta(dc, ah, dbm + 2 * kb, id, 1);
+            }
+            if (t % kSAcc == 0 && kb == 0) {
+              if (!(ok = mbar_wait(&S.acc_empty, ((t / kSAcc) & 1) ^ 1, err))) break;
+              tc_fence_after();
+            }
+#pragma unroll
+            for (int pr = 0; pr < 2; pr++)
+              mma_f16_ta(tbase + pr * kSN, at + 16 * pr, dbh + 2 * kb, idn, (t % kSAcc != 0) || kb);
+            mma_commit(&S.a_empty[sl]);
+            if (++sl == kSA) sl = 0, sp ^= 1;
+          }
+          if (!ok) break;
+          mma_commit(&S.in_empty[st]);
+          if (t % kSAcc == kSAcc - 1 || t + 1 == mine) mma_commit(&S.acc_full);
+        }
+        if (ok) mma_commit(&S.cross_full);
+        mma_commit(&S.mma_done);
+        mbar_wait_drain(&S.mma_done, 0);
+      }
+    } else if (warp == 2) {
+      // ---------------------------------------------- posteriors: lane = 8 points of component lane / 8
+      bool ok = true;
+      for (int t = 0; t < mine && ok; t++) {
+        const int st = t % kSIn;
+        if (!(ok = mbar_wait_lazy_warp(&S.in_full[st], (t / kSIn) & 1, err, 64))) break;
+        const uint4 vh = reinterpret_cast<const uint4 *>(S.rh[st])[lane];
+        const uint4 vl = reinterpret_cast<const uint4 *>(S.rl[st])[lane];
+        const uint32_t wh[4] = {vh.x, vh.y, vh.z, vh.w}, wl[4] = {vl.x, vl.y, vl.z, vl.w};
+        float2 r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          r[q] = __fadd2_rn(__half22float2(*reinterpret_cast<const __half2 *>(&wh[q])),
+                            __half22float2(*reinterpret_cast<const __half2 *>(&wl[q])));
+        float4 *o = reinterpret_cast<float4 *>(S.rf[st]) + 2 * lane;
+        o[0] = make_float4(r[0].x, r[0].y, r[1].x, r[1].y);
+        o[1] = make_float4(r[2].x, r[2].y, r[3].x, r[3].y);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.rf_full[st]);
+      }
+    }
+  } else if (warp < kSFlush0) {
+    reg_dec<kSRegProd>();
+    // ------------------------------------------------ producers
+    const int grp = (warp - kSProd0) >> 2, quad = warp & 3;   // group = the step it forms of every block
+    const int slot = quad >> 1;                  // component slot within each pair
+    const int a = 32 * (quad & 1) + lane;        // dimension = TMEM lane within the slot
+    const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
+    // (x - mu) / zunit = x xs + nm, one rounding: the unit is a power of two
+    float2 xs[2], nm[2], dg[2];
+    double ddg[2] = {0.0, 0.0};
+#pragma unroll
+    for (int pr = 0; pr < 2; pr++) {
+      xs[pr] = f2(S.zs[2 * pr + slot][a]);
+      nm[pr] = f2(S.zm[2 * pr + slot][a]);
+      dg[pr] = make_float2(0.f, 0.f);
+    }
+    // w + c0 - c0 is w rounded to an integer (c0 = 1.5 2^23)
+    const float2 c0 = f2(12582912.f), n0 = f2(-12582912.f);
+    bool ok = true;
+    int rows = 0;
+    int sl = grp, sp = 0;                          // operand slot of step 4 t + grp (mod kSA) and its phase
+    for (int t = 0; t < mine && ok; t++) {
+      const int st = t % kSIn;
+      if (!(ok = mbar_wait_warp(&S.in_full[st], (t / kSIn) & 1, err))) break;
+      float2 x[8];                                 // the step's 16 points, dimension a
+      const float *xr = S.x[st] + 16 * grp * kD + a;
+#pragma unroll
+      for (int q = 0; q < 8; q++) x[q] = make_float2(xr[2 * q * kD], xr[(2 * q + 1) * kD]);
+      if (!(ok = mbar_wait_warp(&S.rf_full[st], (t / kSIn) & 1, err))) break;
+      if (!(ok = mbar_wait_warp(&S.a_empty[sl], sp ^ 1, err))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int pr = 0; pr < 2; pr++) {
+        const float4 *r4 = reinterpret_cast<const float4 *>(S.rf[st] + (2 * pr + slot) * kBlk + 16 * grp);
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const float4 r = r4[q];
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const float2 dz = __ffma2_rn(x[2 * q + u], xs[pr], nm[pr]);
+            const float2 rr = u ? make_float2(r.z, r.w) : make_float2(r.x, r.y);
+            const float2 w = __fmul2_rn(dz, rr);
+            dg[pr] = __ffma2_rn(w, dz, dg[pr]);
+            const float2 wi = __fadd2_rn(__ffma2_rn(dz, rr, c0), n0);
+            const __half2 h = __floats2half2_rn(wi.x, wi.y);
+            const float2 hf = __half22float2(h);
+            const float2 wl = __fadd2_rn(w, make_float2(-hf.x, -hf.y));
+            const __half2 l = __floats2half2_rn(wl.x, wl.y);
+            hi[2 * q + u] = *reinterpret_cast<const uint32_t *>(&h);
+            lo[2 * q + u] = *reinterpret_cast<const uint32_t *>(&l);
+          }
+        }
+        const uint32_t at = tbase + lane_addr + kSACol + sl * kSAStage + 16 * pr;
+        tmem_st8(at, hi);
+        tmem_st8(at + 8, lo);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&S.a_full[sl]);
+        mbar_arrive(&S.in_empty[st]);
+      }
+      sl += kSSteps;
+      if (sl >= kSA) sl -= kSA, sp ^= 1;
+      rows += 16;
+      if (rows == kSRows) {
+        rows = 0;
+#pragma unroll
+        for (int pr = 0; pr < 2; pr++) {
+          ddg[pr] += (double)(dg[pr].x + dg[pr].y);
+          dg[pr] = make_float2(0.f, 0.f);
+        }
+      }
+    }
+#pragma unroll
+    for (int pr = 0; pr < 2; pr++)   // [cta][producer group][component][dimension]
+      dpart[((cta * 4 + grp) * 4 + 2 * pr + slot) * kD + a] = ddg[pr] + (double)(dg[pr].x + dg[pr].y);
+  } else {
+    reg_inc<kSRegFlush>();
+    // ------------------------------------------------ flush warps: TMEM lane = row of the pair tile
+    const int pr = (warp - kSFlush0) >> 2, quad = warp & 3, lrow = quad * 32 + lane;
+    // this CTA's FP64 partials, column-major per pair: column c of pair pr at
+    // cpart[..][(pr * 64 + c) * 128], so a warp's 32 rows are 256 contiguous bytes
+    double *o = cpart + cta * (size_t)(2 * kD * 128) + (size_t)pr * (kD * 128) + lrow;
+    const float *mu = S.mu[2 * pr + (quad >> 1)];
+    float acc[kD];
+#pragma unroll
+    for (int c = 0; c < kD; c++) acc[c] = 0.f;
+    const uint32_t ta = tbase + ((uint32_t)(quad * 32) << 16) + pr * kSN;
+    auto take = [&](uint32_t from) {
+      uint32_t v[16];
+      tmem_ld16(from + kD, v);
+      tmem_wait_ld();
+      const float sz = __uint_as_float(v[0]);
+#pragma unroll
+      for (int c0 = 0; c0 < kD; c0 += 16) {
+        tmem_ld16(from + c0, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          const float4 m = *reinterpret_cast<const float4 *>(mu + c0 + c);
+          acc[c0 + c] += fmaf(-sz, m.x, __uint_as_float(v[c]));
+          acc[c0 + c + 1] += fmaf(-sz, m.y, __uint_as_float(v[c + 1]));
+          acc[c0 + c + 2] += fmaf(-sz, m.z, __uint_as_float(v[c + 2]));
+          acc[c0 + c + 3] += fmaf(-sz, m.w, __uint_as_float(v[c + 3]));
+        }
+      }
+    };
+    bool ok = true, first = true;
+    for (int t0 = 0; t0 < mine && ok; t0 += kSAcc) {
+      const int t1 = std::min(mine, t0 + kSAcc);
+      if (!(ok = mbar_wait_lazy_warp(&S.acc_full, (t0 / kSAcc) & 1, err, 500))) break;
+      tc_fence_after();
+      take(ta);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.acc_empty);
+      if (t1 == mine) {
+        if (!(ok = mbar_wait_warp(&S.cross_full, 0, err))) break;
+        tc_fence_after();
+        take(ta + kSCross);
+      }
+      if (t1 == mine || t1 % kSWin == 0) {
+#pragma unroll
+        for (int c = 0; c < kD; c++) {
+          double *q = o + (size_t)c * 128;
+          *q = first ? (double)acc[c] : *q + (double)acc[c];
+          acc[c] = 0.f;
+        }
+        first = false;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tbase, 512);
+}
+
+// Sigma_j = sym(sum z (x - muf)^T) / N_j - (mu - muf)(mu - muf)^T, the
+// producers' sums on the diagonal; chunks summed in order (FP64).
+// A CTA owns rows 16 blockIdx.y .. + 15 of component blockIdx.x.
+__global__ void __launch_bounds__(512)
+k_final_cov_split(const double *__restrict__ cpart, const double *__restrict__ dpart, int gx, int gy, int d,
+                  const double *__restrict__ psum, const double *__restrict__ mu, const float *__restrict__ muf,
+                  const float *__restrict__ cmax, const float *__restrict__ zunit, double *__restrict__ sigma) {
+  const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
+  const int a0 = blockIdx.y * kFCRows;
+  __shared__ double sr[kFCRows][kD + 1], sc[kD][kFCRows + 1], sd[kFCRows];
+  const double *P0 = cpart + ((size_t)grp * 2 + pr) * (kD * 128) + slot * 64;
+  const size_t step = (size_t)gx * 2 * (kD * 128);
+  for (int e = threadIdx.x; e < 2 * kFCRows * kD + kFCRows; e += blockDim.x) {
+    double v = 0.0;
+    if (e < 2 * kFCRows * kD) {
+      // rows: (b, a0 + i) at P[b * 128 + a0 + i]; columns: (a0 + i, b) at P[(a0 + i) * 128 + b]
+      const int r = e % (kFCRows * kD);
+      const bool rowpart = e < kFCRows * kD;
+      const int i = rowpart ? r % kFCRows : r / kD, b = rowpart ? r / kFCRows : r % kD;
+      const size_t o = rowpart ? (size_t)b * 128 + a0 + i : (size_t)(a0 + i) * 128 + b;
+#pragma unroll 8
+      for (int ch = 0; ch < gy; ch++) v += P0[ch * step + o];
+      (rowpart ? sr[i][b] : sc[b][i]) = v;
+    } else {
+      const int i = e - 2 * kFCRows * kD;
+      for (int ch = 0; ch < gy; ch++)
+#pragma unroll
+        for (int g = 0; g < 4; g++) v += dpart[((((size_t)ch * gx + grp) * 4 + g) * 4 + c) * kD + a0 + i];
+      sd[i] = v;
+    }
+  }
+  __syncthreads();
+  const double inv = 1.0 / psum[j];
+  double *Sg = sigma + (size_t)j * d * d;
+  for (int e = threadIdx.x; e < kFCRows * kD; e += blockDim.x) {
+    const int i = e / kD, a = a0 + i, b = e - i * kD;
+    if (a >= d || b >= d || b < a) continue;
+    const double da = mu[(size_t)j * d + a] - (double)muf[(size_t)j * kD + a];
+    const double db = mu[(size_t)j * d + b] - (double)muf[(size_t)j * kD + b];
+    const double ga = zunit[(size_t)j * kD + a], gb = zunit[(size_t)j * kD + b];
+    const double t = a == b ? sd[i] * ga * ga
+                            : 0.5 * (sr[i][b] * (ga * x_unit(cmax[b])) + sc[b][i] * (gb * x_unit(cmax[a])));
+    const double v = t * inv - da * db;
     Sg[a * d + b] = v;
     Sg[b * d + a] = v;
   }
@@ -1167,14 +1585,39 @@ __global__ void k_prep_w(const double *__restrict__ linv, const double *__restri
   }
 }
 
-// x -> xh = fp16(x), xl = fp16(x - xh), row-major and transposed (d x np)
-// (rows of d < 64 values are zero-padded to 64; X64 receives the padded FP32
-// rows when it is not null)
+// largest |x| of every dimension (cmax[0..63], zero for dimensions >= d) and
+// of all (cmax[64]); cmax starts at zero
+__global__ void __launch_bounds__(256)
+k_col_max(const float *__restrict__ X, int64_t n, int d, float *__restrict__ cmax) {
+  __shared__ int sm[kD];
+  if (threadIdx.x < kD) sm[threadIdx.x] = 0;
+  __syncthreads();
+  // a thread stays in one column: blocks and strides are whole rows
+  const int rows = 256 / d, c = threadIdx.x % d, r = threadIdx.x / d;
+  float m = 0.f;
+  if (r < rows) {
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * rows + r; i < n; i += (int64_t)gridDim.x * rows)
+      m = fmaxf(m, fabsf(X[i * d + c]));
+    atomicMax(&sm[c], __float_as_int(m));
+  }
+  __syncthreads();
+  if (threadIdx.x < d) {
+    // non-negative floats order like their bits
+    atomicMax(reinterpret_cast<int *>(cmax) + threadIdx.x, sm[threadIdx.x]);
+    atomicMax(reinterpret_cast<int *>(cmax) + kD, sm[threadIdx.x]);
+  }
+}
+
+// row-major: x -> xh = fp16(x), xl = fp16(x - xh); transposed (d x np): x /
+// x_unit -> its nearest integer xh, the rest xl, and with XmT what FP16 leaves of it
 __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half *__restrict__ Xh,
                           __half *__restrict__ Xl, __half *__restrict__ XhT, __half *__restrict__ XlT,
-                          int64_t np, float *__restrict__ X64, float *__restrict__ amax) {
-  __shared__ __half th[kD][65], tl[kD][65];
-  float m = 0.f;
+                          __half *__restrict__ XmT, int64_t np, float *__restrict__ X64, const float *__restrict__ cmax) {
+  __shared__ __half th[kD][65], tl[kD][65], tm[kD][65];
+  __shared__ float sinv[kD];
+  if (threadIdx.x < kD) sinv[threadIdx.x] = ldexpf(1.f, -x_unit_exp(cmax[threadIdx.x]));
+  __syncthreads();
   const int64_t nt = (n + 63) / 64;
   for (int64_t tile = blockIdx.x; tile < nt; tile += gridDim.x) {
     const int64_t r0 = tile * 64;
@@ -1187,9 +1630,11 @@ __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half 
         const __half l = __float2half_rn(x - __half2float(h));
         Xh[(r0 + r) * kD + c] = h;
         Xl[(r0 + r) * kD + c] = l;
-        th[c][r] = h;
-        tl[c][r] = l;
-        m = fmaxf(m, fabsf(x));
+        const float u = x * sinv[c], ui = rintf(u);
+        th[c][r] = __float2half_rn(ui);
+        const __half ul = __float2half_rn(u - ui);
+        tl[c][r] = ul;
+        if (XmT) tm[c][r] = __float2half_rn((u - ui) - __half2float(ul));
       }
     }
     __syncthreads();
@@ -1198,13 +1643,11 @@ __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half 
       if (r0 + r < n) {
         XhT[(size_t)c * np + r0 + r] = th[c][r];
         XlT[(size_t)c * np + r0 + r] = tl[c][r];
+        if (XmT) XmT[(size_t)c * np + r0 + r] = tm[c][r];
       }
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
 }
 
 // one warp, a lane's terms first, then a fixed tree
@@ -1257,6 +1700,7 @@ static size_t esmem_bytes() { return sizeof(ESmem) + 1024; }
 static size_t msmem_bytes() { return sizeof(MSmem) + 1024; }
 static size_t csmem_bytes() { return sizeof(CSmem) + 1024; }
 static size_t zsmem_bytes() { return sizeof(ZSmem) + 1024; }
+static size_t ssmem_bytes() { return sizeof(SSmem) + 1024; }
 
 static int fp16_map(CUtensorMap *m, const void *base, uint64_t cols, uint64_t rows, uint64_t pitch_elems,
                     uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swz) {
@@ -1274,7 +1718,7 @@ bool em_tc_supported(int d, int k) {
 // over the points of a component (relative ~2^-12 / sqrt(N_j)).  With fewer
 // than 16384 points per component on average it would not, so such fits take
 // the FP32 CUDA-core covariance (its cost is small at that size).
-bool em_tc_small_components(int64_t n, int k, int d) { return d <= kD && n < (int64_t)16384 * k; }
+static bool em_tc_small_components(int64_t n, int k, int d) { return d <= kD && n < (int64_t)16384 * k; }
 
 // covariance kernel selection while both forms are compared (FEM_COV_KERNEL=zz
 // selects the z z^T form)
@@ -1284,6 +1728,22 @@ static bool cov_zx_enabled() {
     return !(v && v[0] == 'z' && v[1] == 'z');
   }();
   return zx;
+}
+
+// Small components: the split tensor-core form or the CUDA-core one.  The
+// split form pads to 64 dimensions and 4 components, the CUDA-core form costs
+// 8 x 8 blocks of the triangle, so it is ahead up to d = 32 (N = 10^5, K = 12,
+// d = 32: 86 against 130 us; N = 200003, K = 21, d = 24: 147 against 240) and
+// the split form above (N = 500000, K = 64, d = 48: 1.3 against 3.5 ms; N =
+// 2^20, K = 128, d = 64: 5.4 against 20.7 ms), once every SM has 16 or more of
+// its (64-point block, 4-component group) units to pay for a CTA's start and
+// end (K = 8, d = 64: N = 20000, 4 a SM, 57 against 102 us; N = 100000, 20 a
+// SM, 227 against 143 us).
+static bool cov_split_wins(int64_t n, int d, int kp) {
+  cudaFuncAttributes a;
+  // its register split presumes the launch's share
+  if (cudaFuncGetAttributes(&a, k_cov_split) != cudaSuccess || a.numRegs < kSRegLaunch) return false;
+  return d > 32 && (n + kBlk - 1) / kBlk * (kp / 4) >= (int64_t)16 * sm_count();
 }
 
 int em_tc_create(fem_em *h) {
@@ -1312,7 +1772,9 @@ int em_tc_create(fem_em *h) {
   if (h->d < kD) FEM_TRY(dalloc(&p->X64, (size_t)n * kD));
   FEM_TRY(dalloc(&p->err, 1));
   FEM_CUDA(cudaMemset(p->err, 0, sizeof(int)));
-  FEM_TRY(dalloc(&p->amax, 1));
+  FEM_TRY(dalloc(&p->amax, kD + 1));
+  FEM_CUDA(cudaMemset(p->amax, 0, (kD + 1) * sizeof(float)));
+  FEM_TRY(dalloc(&p->zunit, (size_t)K * kD));
   FEM_TRY(dalloc(&p->roles, 4));
   const int64_t npairs = ((n + kTileM - 1) / kTileM + 1) / 2;
   p->egrid = (int)std::min<int64_t>(sms, npairs);
@@ -1322,9 +1784,21 @@ int em_tc_create(fem_em *h) {
   p->mgrid = (int)std::min<int64_t>(sms, nblocks);
   FEM_TRY(dalloc(&p->mpart, (size_t)p->mgrid * kMaxK * kMeanN));
   p->cgx = K / 4;
-  p->cgy = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks, (4 * sms + p->cgx - 1) / p->cgx));
-  FEM_TRY(dalloc(&p->cpart, (size_t)p->cgx * p->cgy * std::max(4 * kD * kD, 2 * kZCols * 128)));
-  FEM_TRY(dalloc(&p->dpart, (size_t)p->cgx * p->cgy * 4 * kD));
+  if (em_tc_small_components(n, h->k, h->d)) {
+    if (cov_split_wins(n, h->d, K)) {
+      // a CTA's start and end (TMEM, pipeline fill, FP64 stores) cost about 12 blocks
+      split_rows(n, kBlk, p->cgx, sms, 12.0, &p->cgy, &p->srows);
+      FEM_TRY(dalloc(&p->cpart, (size_t)p->cgx * p->cgy * 2 * kD * 128));
+      FEM_TRY(dalloc(&p->dpart, (size_t)p->cgx * p->cgy * 4 * 4 * kD));
+      FEM_TRY(dalloc(&p->XmT, (size_t)kD * p->np));
+      FEM_TRY(encode_tmap_2d(&p->tm_xmt, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p->XmT, (uint64_t)n, kD, kBlk, kD,
+                             CU_TENSOR_MAP_SWIZZLE_128B, (uint64_t)p->np * 2));
+    }
+  } else {
+    p->cgy = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks, (4 * sms + p->cgx - 1) / p->cgx));
+    FEM_TRY(dalloc(&p->cpart, (size_t)p->cgx * p->cgy * std::max(4 * kD * kD, 2 * kZCols * 128)));
+    FEM_TRY(dalloc(&p->dpart, (size_t)p->cgx * p->cgy * 4 * kD));
+  }
   // E-step operands
   FEM_TRY(fp16_map(&p->tm_xh, h->Xhi, kD, n, kD, kD, kTileM, CU_TENSOR_MAP_SWIZZLE_128B));
   FEM_TRY(fp16_map(&p->tm_xl, h->Xlo, kD, n, kD, kD, kTileM, CU_TENSOR_MAP_SWIZZLE_128B));
@@ -1351,7 +1825,12 @@ int em_tc_create(fem_em *h) {
   FEM_CUDA(cudaFuncSetAttribute(k_means_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem_bytes()));
   FEM_CUDA(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem_bytes()));
   FEM_CUDA(cudaFuncSetAttribute(k_cov_zx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem_bytes()));
+  FEM_CUDA(cudaFuncSetAttribute(k_cov_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem_bytes()));
   return FEM_OK;
+}
+
+bool em_tc_cuda_core_cov(const fem_em *h) {
+  return h->tc && em_tc_small_components(h->n, h->k, h->d) && !h->tc->srows;
 }
 
 void em_tc_destroy(fem_em *h) {
@@ -1366,6 +1845,7 @@ void em_tc_destroy(fem_em *h) {
   dfree(p->Rl);
   dfree(p->XhT);
   dfree(p->XlT);
+  dfree(p->XmT);
   dfree(p->lsc);
   dfree(p->epart);
   dfree(p->mpart);
@@ -1376,6 +1856,7 @@ void em_tc_destroy(fem_em *h) {
   dfree(p->X64);
   dfree(p->err);
   dfree(p->amax);
+  dfree(p->zunit);
   dfree(p->roles);
   delete p;
   h->tc = nullptr;
@@ -1385,11 +1866,13 @@ int em_tc_upload(fem_em *h) {
   if (h->wide) return em_wide_upload(h);
   TcEmPlan *p = h->tc;
   float *amax = p->amax;
-  FEM_CUDA(cudaMemsetAsync(amax, 0, sizeof(float), h->stream));
+  FEM_CUDA(cudaMemsetAsync(amax, 0, (kD + 1) * sizeof(float), h->stream));
   const int blocks = (int)std::min<int64_t>(4 * sm_count(), (h->n + 63) / 64);
-  k_split_x<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, h->Xhi, h->Xlo, p->XhT, p->XlT, p->np, p->X64, amax);
+  k_col_max<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, amax);
+  k_split_x<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, h->Xhi, h->Xlo, p->XhT, p->XlT, p->XmT, p->np,
+                                            p->X64, amax);
   float m = 0.f;
-  cudaMemcpyAsync(&m, amax, sizeof(float), cudaMemcpyDeviceToHost, h->stream);
+  cudaMemcpyAsync(&m, amax + kD, sizeof(float), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
     set_error("dataset split failed: %s", cudaGetErrorString(e));
@@ -1432,12 +1915,25 @@ int em_tc_mstep(fem_em *h) {
   k_means_tc<<<p->mgrid, 192, msmem_bytes(), h->stream>>>(p->tm_rh, p->tm_rl, p->tm_xht, p->tm_xlt, h->n,
                                                            p->mpart, p->err);
   FEM_CUDA(cudaGetLastError());
-  k_final_means_tc<<<K, kFMSplit * kFMCols, 0, h->stream>>>(p->mpart, p->mgrid, K, h->d, h->n, h->mu, h->pi, h->psum, p->muf);
+  k_final_means_tc<<<K, kFMSplit * kFMCols, 0, h->stream>>>(p->mpart, p->mgrid, K, h->d, h->n, h->mu, h->pi, h->psum,
+                                                               p->muf, p->amax, h->sigma, p->zunit);
   FEM_CUDA(cudaGetLastError());
   if (em_tc_small_components(h->n, h->k, h->d)) {
     timing_begin(h, 8);
-    FEM_TRY(em_cov_hilo(h, p->Rh, p->Rl, p->np, p->muf, kD));
-    timing_begin(h, 9);
+    if (p->srows) {
+      k_cov_split<<<dim3(p->cgx, p->cgy), kSThreads, ssmem_bytes(), h->stream>>>(
+          p->tm_xht, p->tm_xlt, p->tm_xmt, p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf, p->amax, p->zunit, h->n, p->srows, p->cpart, p->dpart,
+          p->err);
+      FEM_CUDA(cudaGetLastError());
+      timing_begin(h, 9);
+      k_final_cov_split<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(
+          p->cpart, p->dpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, p->amax, p->zunit, h->sigma);
+      FEM_CUDA(cudaGetLastError());
+      h->launches += 2;
+    } else {
+      FEM_TRY(em_cov_hilo(h, p->Rh, p->Rl, p->np, p->muf, kD));
+      timing_begin(h, 9);
+    }
     k_flag_timeout<<<1, 32, 0, h->stream>>>(h->dstat, p->err);
     h->launches += 3;
     return FEM_OK;
@@ -1446,11 +1942,12 @@ int em_tc_mstep(fem_em *h) {
   const int64_t bpc = (nblocks + p->cgy - 1) / p->cgy;
   timing_begin(h, 8);
   if (cov_zx_enabled()) {
-    k_cov_zx<<<dim3(p->cgx, p->cgy), kZThreads, zsmem_bytes(), h->stream>>>(p->tm_xht, p->tm_xlt, p->tm_rh4, p->muf,
-                                                                           h->n, bpc, p->cpart, p->err);
+    k_cov_zx<<<dim3(p->cgx, p->cgy), kZThreads, zsmem_bytes(), h->stream>>>(
+        p->tm_xht, p->tm_xlt, p->tm_rh4, p->muf, p->amax, h->n, bpc, p->cpart, p->err);
     FEM_CUDA(cudaGetLastError());
     timing_begin(h, 9);
-    k_final_cov_zx<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, h->sigma);
+    k_final_cov_zx<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, p->amax,
+                                                                          h->sigma);
   } else {
     k_cov_tc<<<dim3(p->cgx, p->cgy), kCThreads, csmem_bytes(), h->stream>>>(p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf,
                                                                            h->n, bpc, p->cpart, p->dpart, p->err);

@@ -163,13 +163,12 @@ struct fem_km {
   int64_t next_repair = 0;         // next row of FEM_KM_REPAIR_NEXT
 
   float *X = nullptr;              // n x d
-  __nv_bfloat16 *Xb = nullptr;     // n x d (mixed)
-  float *xnorm = nullptr;          // n   ||x_i|| (mixed bound)
   int32_t *labels = nullptr;       // n
   double *cent = nullptr;          // k x d (FP64 centroids, device)
   float *centf = nullptr;          // k x d float copy
-  __nv_bfloat16 *centb = nullptr;  // k x d bf16 copy (mixed)
-  float *cnorm = nullptr;          // k   ||c_j|| and ||c_j||^2
+  float *cnorm = nullptr;          // k   ||c_j||
+  float *centg = nullptr;          // k x d c_j - g (FP32 path)
+  float *hnorm = nullptr;          // k   ||c_j - g||^2 / 2 (FP32 path)
   long long *acc = nullptr;        // grid x k x d  fixed-point partial sums
   int *cnt = nullptr;              // grid x k
   int grid = 0;

@@ -86,19 +86,31 @@ k_km_stats(const float *__restrict__ X, int64_t n, int d, int64_t rows_per_block
   }
 }
 
-// centroids -> float copy and norms
-__global__ void k_km_prep(const double *__restrict__ cent, int K, int d, float *__restrict__ centf,
-                          float *__restrict__ cnorm, __nv_bfloat16 *__restrict__ centb) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// centroids -> float copy and norm, and for the FP32 path the copy around the
+// data mean (as float) and half its squared norm; one warp per centroid
+__global__ void __launch_bounds__(128)
+k_km_prep(const double *__restrict__ cent, const double *__restrict__ g, int K, int d, float *__restrict__ centf,
+          float *__restrict__ cnorm, float *__restrict__ centg, float *__restrict__ hnorm) {
+  const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= K) return;
-  double s = 0.0;
-  for (int q = 0; q < d; q++) {
+  double s = 0.0, h = 0.0;
+  for (int q = lane; q < d; q += 32) {
     const double c = cent[(size_t)j * d + q];
     centf[(size_t)j * d + q] = (float)c;
-    if (centb) centb[(size_t)j * d + q] = __float2bfloat16_rn((float)c);
-    s += c * c;
+    s = fma(c, c, s);
+    if (centg) {
+      const double cg = c - (double)(float)g[q];
+      centg[(size_t)j * d + q] = (float)cg;
+      h = fma(cg, cg, h);
+    }
   }
-  cnorm[j] = (float)sqrt(s);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, o), h += __shfl_xor_sync(0xffffffffu, h, o);
+  if (lane == 0) {
+    cnorm[j] = (float)sqrt(s);
+    if (centg) hnorm[j] = (float)(0.5 * h);
+  }
 }
 
 // FP64 difference form in column order, no contraction: bit-identical to
@@ -120,158 +132,302 @@ __device__ __forceinline__ float bound_f32(float s, float cn, int d) {
 }
 
 // =================================================== FP32 assignment
-// One CTA per SM streams 256-row tiles; per row: FP32 difference-form
-// distances to all centroids, candidate test, FP64 recheck if needed;
-// then exact fixed-point accumulation of the rows into per-CTA sums.
+// Every warp takes its own share of the rows, 32 R at a time (R rows per
+// lane, in registers), and screens all centroids by
+//   w_j = ||c'_j||^2 / 2 - x'.c'_j     (x' = x - g, c' = c - g; ||x - c||^2 =
+//                                       ||x'||^2 + 2 w_j),
+// D products per (row, centroid) where the difference form takes 2 D
+// operations, keeping the two smallest.  With u = 2^-24 the computed w_j is within
+//   B = 1.05 (D + 6) u (||x'|| ||c'||max + ||c'||max^2 / 2)
+// of the exact one (rounding of x', c', ||c'||^2 and the D-term sum), so a row
+// whose two smallest differ by more than 2 B is decided.  The others, few, go
+// through the difference form by the whole warp (lane = centroid): FP32 with
+// the bound of bound_f32, then the reference's FP64 sums among the centroids
+// that remain, lowest index on ties.  Rows are added to exact fixed-point sums
+// in shared memory (a float times 2^shift is exact), so the order is free.
+// Bound by the FP32 pipe, and by the broadcast loads of the centroids where R <
+// 4 (R = 4 loads 16 bytes per 16 products).  N = 1000003, D = 16, K = 100 on
+// the GB300: 442 -> 128 us an iteration (difference form, one row per thread).
 template <int D>
-__global__ void __launch_bounds__(256)
-k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const float *__restrict__ centf,
-                const float *__restrict__ cnorm, const double *__restrict__ cent,
-                int32_t *__restrict__ labels, long long *__restrict__ accg, int *__restrict__ cntg,
-                double scale, DevStatus *st) {
+struct KmShape {
+  static constexpr int R = D <= 32 ? 4 : 2;               // rows per lane
+  static constexpr int kThreads = D <= 16 ? 512 : 256;
+};
+
+__device__ __forceinline__ float2 km_ffma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// two smallest w and the first's index for NR rows per lane
+template <int D, int NR>
+__device__ __forceinline__ void km_screen(const float2 (*x)[D / 2], const float *sC, const float *sH, int K, float *m1,
+                                          float *m2, int *j1) {
+#pragma unroll
+  for (int r = 0; r < NR; r++) m1[r] = INFINITY, m2[r] = INFINITY, j1[r] = -1;
+#pragma unroll 1
+  for (int j = 0; j < K; j++) {
+    const float *c = sC + j * D;
+    float2 w[NR];
+    const float h = sH[j];
+#pragma unroll
+    for (int r = 0; r < NR; r++) w[r] = make_float2(h, 0.f);
+    if constexpr (D >= 4) {
+#pragma unroll
+      for (int q = 0; q < D / 4; q++) {
+        const float4 c4 = reinterpret_cast<const float4 *>(c)[q];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+          w[r] = km_ffma2(x[r][2 * q], make_float2(c4.x, c4.y), w[r]);
+          w[r] = km_ffma2(x[r][2 * q + 1], make_float2(c4.z, c4.w), w[r]);
+        }
+      }
+    } else {
+      const float2 c2 = *reinterpret_cast<const float2 *>(c);
+#pragma unroll
+      for (int r = 0; r < NR; r++) w[r] = km_ffma2(x[r][0], c2, w[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      const float v = w[r].x + w[r].y;
+      m2[r] = fminf(m2[r], fmaxf(m1[r], v));
+      if (v < m1[r]) j1[r] = j;
+      m1[r] = fminf(m1[r], v);
+    }
+  }
+}
+
+// the reference's choice for one row, by the whole warp: -1 when no centroid
+// compares (a row with NaN); *fp64 when FP64 had to decide
+template <int D>
+__device__ int km_decide(const float *__restrict__ x, const float *__restrict__ centf, const float *__restrict__ cnorm,
+                         const double *__restrict__ cent, int K, bool *fp64) {
+  const int lane = threadIdx.x & 31;
+  float xr[D];
+#pragma unroll
+  for (int q = 0; q < D; q++) xr[q] = x[q];
+  float U = INFINITY;
+  for (int j = lane; j < K; j += 32) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < D; q++) {
+      const float t = xr[q] - centf[(size_t)j * D + q];
+      s = fmaf(t, t, s);
+    }
+    U = fminf(U, s + bound_f32(s, cnorm[j], D));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) U = fminf(U, __shfl_xor_sync(0xffffffffu, U, o));
+  double best = DBL_MAX;
+  int lab = INT_MAX, cand = 0, only = INT_MAX;
+  for (int j = lane; j < K; j += 32) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < D; q++) {
+      const float t = xr[q] - centf[(size_t)j * D + q];
+      s = fmaf(t, t, s);
+    }
+    if (s - bound_f32(s, cnorm[j], D) <= U) cand++, only = min(only, j);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    cand += __shfl_xor_sync(0xffffffffu, cand, o);
+    only = min(only, __shfl_xor_sync(0xffffffffu, only, o));
+  }
+  *fp64 = cand > 1;
+  if (cand <= 1) return cand == 1 ? only : -1;
+  for (int j = lane; j < K; j += 32) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < D; q++) {
+      const float t = xr[q] - centf[(size_t)j * D + q];
+      s = fmaf(t, t, s);
+    }
+    if (s - bound_f32(s, cnorm[j], D) <= U) {
+      const double s64 = dist64(cent + (size_t)j * D, xr, D);
+      if (s64 < best) best = s64, lab = j;       // a lane's centroids come in index order
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int ol = __shfl_xor_sync(0xffffffffu, lab, o);
+    if (ob < best || (ob == best && ol < lab)) best = ob, lab = ol;
+  }
+  return lab == INT_MAX ? -1 : lab;
+}
+
+template <int D>
+__global__ void __launch_bounds__(KmShape<D>::kThreads)
+k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const double *__restrict__ gmean,
+                const float *__restrict__ centg, const float *__restrict__ hnorm, const float *__restrict__ centf,
+                const float *__restrict__ cnorm, const double *__restrict__ cent, int32_t *__restrict__ labels,
+                long long *__restrict__ accg, int *__restrict__ cntg, float scale, DevStatus *st) {
+  constexpr int R = KmShape<D>::R, T = KmShape<D>::kThreads;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   long long *sAcc = (long long *)smem_raw;              // K x D
-  float *sC = (float *)(sAcc + (size_t)K * D);          // K x D
-  float *sCn = sC + (size_t)K * D;                      // K
-  int *sCnt = (int *)(sCn + K);                         // K
-  int *sLab = sCnt + K;                                 // 256
-  float *sX = (float *)(sLab + 256);                    // 256 x (D+1)
-  const int tid = threadIdx.x;
-  for (int e = tid; e < K * D; e += 256) {
+  float *sC = (float *)(sAcc + (size_t)K * D);          // K x D, around g
+  float *sH = sC + (size_t)K * D;                       // K
+  int *sCnt = (int *)(sH + K);                          // K
+  __shared__ __align__(16) float sG[D < 4 ? 4 : D];
+  __shared__ float sMax[T / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float hmax = 0.f;
+  for (int e = tid; e < K * D; e += T) {
     sAcc[e] = 0;
-    sC[e] = centf[e];
+    sC[e] = -centg[e];                                  // w = h + x'.(-c')
   }
-  for (int j = tid; j < K; j += 256) {
+  for (int j = tid; j < K; j += T) {
+    const float h = hnorm[j];
     sCnt[j] = 0;
-    sCn[j] = cnorm[j];
+    sH[j] = h;
+    hmax = fmaxf(hmax, h);
   }
-  int64_t rechecks = 0;
-  const int64_t ntiles = (n + 255) / 256;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t base = tile * 256;
-    const int rows = (int)min((int64_t)256, n - base);
-    __syncthreads();
-    for (int e = tid; e < 256 * D; e += 256) {
-      const int p = e / D, q = e - p * D;
-      sX[p * (D + 1) + q] = (p < rows) ? X[base * D + e] : 0.f;
-    }
-    __syncthreads();
-    int lab = -1;
-    if (tid < rows) {
-      float x[D];
+  if (tid < D) sG[tid] = (float)gmean[tid];
 #pragma unroll
-      for (int q = 0; q < D; q++) x[q] = sX[tid * (D + 1) + q];
-      float U = INFINITY, lb1 = INFINITY, lb2 = INFINITY;
-      int j1 = -1;
-      for (int j = 0; j < K; j++) {
-        const float *c = sC + j * D;
-        float s = 0.f;
-#pragma unroll
-        for (int q = 0; q < D; q++) {
-          const float t = x[q] - c[q];
-          s = fmaf(t, t, s);
-        }
-        const float b = bound_f32(s, sCn[j], D);
-        const float lb = s - b, ub = s + b;
-        U = fminf(U, ub);
-        if (lb < lb1) {
-          lb2 = lb1;
-          lb1 = lb;
-          j1 = j;
-        } else if (lb < lb2) {
-          lb2 = lb;
-        }
-      }
-      if (lb2 > U) {
-        lab = j1;
-      } else {
-        // candidates within the bounds: decide in FP64, index order, strict <
-        rechecks++;
-        double best = DBL_MAX;
-        for (int j = 0; j < K; j++) {
-          const float *c = sC + j * D;
-          float s = 0.f;
-#pragma unroll
-          for (int q = 0; q < D; q++) {
-            const float t = x[q] - c[q];
-            s = fmaf(t, t, s);
-          }
-          if (s - bound_f32(s, sCn[j], D) <= U) {
-            const double s64 = dist64(cent + (size_t)j * D, x, D);
-            if (s64 < best) {
-              best = s64;
-              lab = j;
-            }
-          }
-        }
-      }
-      if (st->track_changes && labels[base + tid] != lab) st->changed = 1;
-      labels[base + tid] = lab;
-      atomicAdd(&sCnt[lab], 1);
-    }
-    sLab[tid] = lab;
-    __syncthreads();
-    // exact accumulation: warp w folds rows 32w..32w+31 into sAcc
-    const int w = tid >> 5, l = tid & 31;
-    for (int idx = l; idx < 32 * D; idx += 32) {
-      const int p = 32 * w + idx / D, q = idx % D;
-      const int lb = sLab[p];
-      if (lb >= 0) {
-        const long long v = __double2ll_rn((double)sX[p * (D + 1) + q] * scale);
-        atomicAdd((unsigned long long *)&sAcc[lb * D + q], (unsigned long long)v);
-      }
-    }
-  }
+  for (int o = 16; o > 0; o >>= 1) hmax = fmaxf(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
+  if (lane == 0) sMax[warp] = hmax;
   __syncthreads();
-  for (int e = tid; e < K * D; e += 256) accg[(size_t)blockIdx.x * K * D + e] = sAcc[e];
-  for (int j = tid; j < K; j += 256) cntg[(size_t)blockIdx.x * K + j] = sCnt[j];
+#pragma unroll
+  for (int w = 0; w < T / 32; w++) hmax = fmaxf(hmax, sMax[w]);
+  const float cmax = sqrtf(2.f * hmax) * 1.00001f;
+  const bool track = st->track_changes;
+  constexpr float kU = 5.9604645e-8f * 1.05f * (D + 6);
+  int64_t rechecks = 0;
+  bool changed = false;
+  // this warp's rows: an even share, in whole groups of 32
+  const int64_t nw = (int64_t)gridDim.x * (T / 32), gw = (int64_t)blockIdx.x * (T / 32) + warp;
+  const int64_t groups = (n + 31) / 32;
+  const int64_t r0 = gw * groups / nw * 32, r1 = min(n, (gw + 1) * groups / nw * 32);
+  for (int64_t base = r0; base < r1; base += 32 * R) {
+    float2 x[R][D / 2];
+    float xn[R], m1[R], m2[R];
+    int j1[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int64_t row = base + 32 * r + lane;
+      const float *xr = X + (row < r1 ? row : r0) * D;
+      float ss = 0.f;
+      if constexpr (D >= 4) {
+#pragma unroll
+        for (int q = 0; q < D / 4; q++) {
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(xr) + q);
+          const float4 g4 = reinterpret_cast<const float4 *>(sG)[q];
+          x[r][2 * q] = make_float2(v.x - g4.x, v.y - g4.y);
+          x[r][2 * q + 1] = make_float2(v.z - g4.z, v.w - g4.w);
+        }
+      } else {
+        x[r][0] = make_float2(xr[0] - sG[0], xr[1] - sG[1]);
+      }
+#pragma unroll
+      for (int q = 0; q < D / 2; q++) ss = fmaf(x[r][q].x, x[r][q].x, fmaf(x[r][q].y, x[r][q].y, ss));
+      xn[r] = sqrtf(ss) * 1.00001f;
+    }
+    const int live = (int)min((int64_t)R, (r1 - base + 31) / 32);   // row groups of this pass
+    if (live == R)
+      km_screen<D, R>(x, sC, sH, K, m1, m2, j1);
+    else if (R > 2 && live == 3)
+      km_screen<D, R - 1>(x, sC, sH, K, m1, m2, j1);
+    else if (R > 2 && live == 2)
+      km_screen<D, 2>(x, sC, sH, K, m1, m2, j1);
+    else
+      km_screen<D, 1>(x, sC, sH, K, m1, m2, j1);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (r >= live) break;
+      const int64_t row = base + 32 * r + lane;
+      const bool in = row < r1;
+      // the last term covers the reference's own FP64 rounding
+      const float B = fmaf(kU, fmaf(xn[r], cmax, 0.5f * cmax * cmax), 1e-13f * fmaf(xn[r], xn[r], cmax * cmax)) + 1e-30f;
+      int lab = j1[r];
+      unsigned open = __ballot_sync(0xffffffffu, in && !(m2[r] - m1[r] > 2.1f * B));
+      while (open) {
+        const int b = __ffs(open) - 1;
+        open &= open - 1;
+        bool fp64 = false;
+        const int l = km_decide<D>(X + (base + 32 * r + b) * D, centf, cnorm, cent, K, &fp64);
+        if (lane == b) {
+          lab = l;
+          if (fp64) rechecks++;
+        }
+      }
+      if (in) {
+        if (track && labels[row] != lab) changed = true;
+        labels[row] = lab;
+        if (lab >= 0) atomicAdd(&sCnt[lab], 1);
+      } else {
+        lab = -1;
+      }
+      // exact sums: the 32 rows again, lanes along the dimensions
+#pragma unroll 4
+      for (int i = lane; i < 32 * D; i += 32) {
+        const int p = i / D, l = __shfl_sync(0xffffffffu, lab, p);
+        if (l >= 0) {
+          const float xv = __ldg(X + (base + 32 * r) * D + i);
+          atomicAdd((unsigned long long *)&sAcc[l * D + i % D], (unsigned long long)__float2ll_rn(xv * scale));
+        }
+      }
+    }
+  }
+  if (changed) st->changed = 1;
   if (rechecks) atomicAdd((unsigned long long *)&st->rechecked, (unsigned long long)rechecks);
+  __syncthreads();
+  for (int e = tid; e < K * D; e += T) accg[(size_t)blockIdx.x * K * D + e] = sAcc[e];
+  for (int j = tid; j < K; j += T) cntg[(size_t)blockIdx.x * K + j] = sCnt[j];
 }
 
 // sums the per-CTA partials (exact), forms the new centroids and the fit terms
-__global__ void k_km_final(const long long *__restrict__ accg, const int *__restrict__ cntg, int G,
-                           int K, int d, double inv_scale, const double *__restrict__ cent,
-                           const double *__restrict__ g, double *__restrict__ out) {
-  const int j = blockIdx.x;
-  __shared__ long long s_n;
-  __shared__ double red[32];
-  if (threadIdx.x == 0) {
-    long long c = 0;
-    for (int b = 0; b < G; b++) c += cntg[(size_t)b * K + j];
-    s_n = c;
-  }
+// (one CTA per centroid, the CTAs' partials split over its 8 warps: the sums
+// are integers, so their order is free)
+__global__ void __launch_bounds__(256)
+k_km_final(const long long *__restrict__ accg, const int *__restrict__ cntg, int G, int K, int d, double inv_scale,
+           const double *__restrict__ cent, const double *__restrict__ g, double *__restrict__ out) {
+  const int j = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ long long red[8][32], s_n[8];
+  long long c = 0;
+  for (int b = threadIdx.x; b < G; b += 256) c += cntg[(size_t)b * K + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (lane == 0) s_n[w] = c;
   __syncthreads();
-  const long long nj = s_n;
+  long long nj = 0;
+#pragma unroll
+  for (int q = 0; q < 8; q++) nj += s_n[q];
   double term = 0.0;
-  for (int q = threadIdx.x; q < d; q += blockDim.x) {
+  for (int q0 = 0; q0 < d; q0 += 32) {
+    const int q = q0 + lane;
     long long S = 0;
-    for (int b = 0; b < G; b++) S += accg[((size_t)b * K + j) * d + q];
-    const double sum = (double)S * inv_scale;
-    out[(size_t)j * d + q] = nj > 0 ? sum * (1.0 / (double)nj) : 0.0;
-    const double cg = cent[(size_t)j * d + q] - g[q];
-    term += -2.0 * cg * (sum - (double)nj * g[q]) + (double)nj * cg * cg;
+    if (q < d) {
+#pragma unroll 4
+      for (int b = w; b < G; b += 8) S += accg[((size_t)b * K + j) * d + q];
+    }
+    __syncthreads();
+    red[w][lane] = S;
+    __syncthreads();
+    if (w == 0 && q < d) {
+#pragma unroll
+      for (int u = 1; u < 8; u++) S += red[u][lane];
+      const double sum = (double)S * inv_scale;
+      out[(size_t)j * d + q] = nj > 0 ? sum * (1.0 / (double)nj) : 0.0;
+      const double cg = cent[(size_t)j * d + q] - g[q];
+      term += -2.0 * cg * (sum - (double)nj * g[q]) + (double)nj * cg * cg;
+    }
   }
-  term = warp_sum_d(term);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = term;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < (int)(blockDim.x + 31) / 32; w++) s += red[w];
-    out[(size_t)K * d + j] = (double)nj;
-    out[(size_t)K * d + K + j] = s;
+  if (w == 0) {
+    term = warp_sum_d(term);
+    if (lane == 0) {
+      out[(size_t)K * d + j] = (double)nj;
+      out[(size_t)K * d + K + j] = term;
+    }
   }
 }
 
 int km_launch_assign_f32(fem_km *h) {
   const int D = h->d, K = h->k;
-  const size_t sm = (size_t)K * D * 8 + (size_t)K * D * 4 + (size_t)K * 4 + (size_t)K * 4 + 256 * 4 +
-                    (size_t)256 * (D + 1) * 4;
-#define FEM_KA(DD)                                                                              \
-  case DD:                                                                                      \
-    FEM_CUDA(allow_dyn_smem(k_km_assign_f32<DD>, sm));                                          \
-    k_km_assign_f32<DD><<<h->grid, 256, sm, h->stream>>>(h->X, h->n, K, h->centf, h->cnorm,     \
-                                                         h->cent, h->labels, h->acc, h->cnt,    \
-                                                         ldexp(1.0, h->shift), h->dstat);       \
+  const size_t sm = (size_t)K * D * 12 + (size_t)K * 8;
+#define FEM_KA(DD)                                                                                             \
+  case DD:                                                                                                     \
+    FEM_CUDA(allow_dyn_smem(k_km_assign_f32<DD>, sm));                                                         \
+    k_km_assign_f32<DD><<<h->grid, KmShape<DD>::kThreads, sm, h->stream>>>(                                    \
+        h->X, h->n, K, h->g, h->centg, h->hnorm, h->centf, h->cnorm, h->cent, h->labels, h->acc, h->cnt,       \
+        ldexpf(1.f, h->shift), h->dstat);                                                                      \
     break;
   switch (D) {
     FEM_KA(2)
@@ -308,12 +464,11 @@ int check(fem_km *h) {
 
 void free_km(fem_km *h) {
   dfree(h->X);
-  dfree(h->Xb);
-  dfree(h->xnorm);
   dfree(h->labels);
   dfree(h->cent);
   dfree(h->centf);
-  dfree(h->centb);
+  dfree(h->centg);
+  dfree(h->hnorm);
   dfree(h->cnorm);
   dfree(h->acc);
   dfree(h->cnt);
@@ -465,6 +620,8 @@ int fem_km_create(int d, int64_t n, int k, const fem_km_config *cfg, fem_km **ou
   if (cudaMallocHost(&h->hout, ((size_t)k * d + 2 * k) * 8) != cudaSuccess ||
       cudaMallocHost(&h->hstat, sizeof(DevStatus)) != cudaSuccess)
     return fail(FEM_ERR_CUDA);
+  if (c.precision == FEM_PREC_FP32 && ((st = dalloc(&h->centg, (size_t)k * d)) || (st = dalloc(&h->hnorm, k))))
+    return fail(st);
   if (c.precision == FEM_PREC_MIXED && (st = km_tc_create(h))) return fail(st);
   FEM_CUDA(cudaMemsetAsync(h->labels, 0, n * 4, h->stream));
   *out = h;
@@ -541,7 +698,7 @@ static int km_iterate(fem_km *h, double *centroids, double *fit, int64_t *counts
   *h->hstat = z;
   FEM_CUDA(cudaMemcpyAsync(h->dstat, h->hstat, sizeof(DevStatus), cudaMemcpyHostToDevice, h->stream));
   FEM_CUDA(cudaMemcpyAsync(h->cent, centroids, kd * 8, cudaMemcpyHostToDevice, h->stream));
-  k_km_prep<<<(K + 127) / 128, 128, 0, h->stream>>>(h->cent, K, d, h->centf, h->cnorm, h->centb);
+  k_km_prep<<<(K + 3) / 4, 128, 0, h->stream>>>(h->cent, h->g, K, d, h->centf, h->cnorm, h->centg, h->hnorm);
   FEM_CUDA(cudaGetLastError());
   FEM_CUDA(cudaEventRecord(h->ev[0], h->stream));
   if (h->cfg.precision == FEM_PREC_MIXED)
@@ -549,7 +706,7 @@ static int km_iterate(fem_km *h, double *centroids, double *fit, int64_t *counts
   else
     FEM_TRY(km_launch_assign_f32(h));
   FEM_CUDA(cudaEventRecord(h->ev[1], h->stream));
-  k_km_final<<<K, 64, 0, h->stream>>>(h->acc, h->cnt, h->grid, K, d, ldexp(1.0, -h->shift), h->cent,
+  k_km_final<<<K, 256, 0, h->stream>>>(h->acc, h->cnt, h->grid, K, d, ldexp(1.0, -h->shift), h->cent,
                                       h->g, h->out);
   FEM_CUDA(cudaGetLastError());
   FEM_CUDA(cudaEventRecord(h->ev[2], h->stream));

@@ -173,6 +173,7 @@ struct fem_km {
   int *cnt = nullptr;              // grid x k
   int grid = 0;
   int shift = 0;                   // fixed-point scale 2^shift
+  float xmax = 0.f;                // max |x|
   double xg2 = 0.0;                // sum_i ||x_i - g||^2
   double *g = nullptr;             // data mean (device, d)
   double *hg = nullptr;            // data mean (host)

@@ -539,6 +539,7 @@ int upload_km(fem_km *h, const float *X, int64_t ld, cudaMemcpyKind kind) {
   }
   // |x| * 2^shift * n < 2^62: the per-CTA and the final int64 sums cannot overflow
   const double lg = std::log2((double)std::max(mx, 1e-30f)) + std::log2((double)n);
+  h->xmax = mx;
   h->shift = (int)std::min(40.0, std::floor(61.0 - std::ceil(lg)));
   FEM_CUDA(cudaMemcpyAsync(h->g, h->hg, d * 8, cudaMemcpyHostToDevice, h->stream));
   h->have_data = true;

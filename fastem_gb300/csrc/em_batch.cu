@@ -40,6 +40,7 @@
 #include <cuda_fp16.h>
 
 #include "em_factor.cuh"
+#include "em_tri.cuh"
 #include "fem_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -60,13 +61,6 @@ constexpr int kBatchSyncEvery = 8;
 constexpr int kTimeMarks = 15;   // timing events per sweep (see collect_timing)
 constexpr int kClasses = 4;      // D = 4, 8, 16, 32
 
-// padded lower triangle: row kk holds kk + 1 entries in 4 * ceil((kk + 1) / 4) floats
-__host__ __device__ constexpr int tri_row(int kk) { return 4 * ((kk + 4) / 4); }
-__host__ __device__ constexpr int tri_off(int kk) {
-  int s = 0;
-  for (int r = 0; r < kk; r++) s += tri_row(r);
-  return s;
-}
 __host__ __device__ constexpr int class_tb(int D) { return D >= 16 ? 8 : 4; }
 __host__ __device__ constexpr int class_nblk(int D) { return (D / class_tb(D)) * (D / class_tb(D) + 1) / 2; }
 // covariance sums: D <= 16 by component owners (k_b_cov_own), D = 32 by TB x TB blocks (k_b_cov)
@@ -132,15 +126,6 @@ __device__ double bblock_sum(double v, double *red) {
   return s;
 }
 
-__device__ __forceinline__ void blse_push(float l, float &mx, float &se) {
-  if (l > mx) {
-    se = se * expf(mx - l) + 1.f;
-    mx = l;
-  } else if (l > -INFINITY) {
-    se += expf(l - mx);
-  }
-}
-
 // 4-byte asynchronous global -> shared copy; `valid` false writes zero
 __device__ __forceinline__ void cp_async4(float *dst, const float *src, bool valid) {
   const unsigned da = (unsigned)__cvta_generic_to_shared(dst);
@@ -155,125 +140,88 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// s_p += ||row KK of W . t_p||^2 for rows KK.. D-1 of a padded lower
-// triangle W, P centred points; rows by compile-time recursion so every
-// column bound is a constant, two interleaved accumulators per row for
-// instruction-level parallelism
-template <int D, int P, int KK>
-__device__ __forceinline__ void tri_rows(const float (&t)[P][D], const float *__restrict__ w, float (&s)[P]) {
-  float y0[P], y1[P];
-#pragma unroll
-  for (int p = 0; p < P; p++) y0[p] = 0.f, y1[p] = 0.f;
-  const float *wr = w + tri_off(KK);
-#pragma unroll
-  for (int m4 = 0; m4 <= KK / 4; m4++) {
-    const float4 wv = *reinterpret_cast<const float4 *>(wr + 4 * m4);
-    const float we[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      if (4 * m4 + e <= KK) {
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-          if (m4 & 1) y1[p] = fmaf(t[p][4 * m4 + e], we[e], y1[p]);
-          else y0[p] = fmaf(t[p][4 * m4 + e], we[e], y0[p]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < P; p++) {
-    const float y = y0[p] + y1[p];
-    s[p] = fmaf(y, y, s[p]);
-  }
-  if constexpr (KK + 1 < D) tri_rows<D, P, KK + 1>(t, w, s);
-}
-
-// s_p = ||W t_p||^2
-template <int D, int P>
-__device__ __forceinline__ void tri_norms(const float (&t)[P][D], const float *__restrict__ w, float (&s)[P]) {
-#pragma unroll
-  for (int p = 0; p < P; p++) s[p] = 0.f;
-  tri_rows<D, P, 0>(t, w, s);
-}
-
 // ================================================================ E-step
 // MatrixEMBase::BlockDensities + PostProcessDensityMatrix
 // (EM2/MatrixEM.cpp:39-51,69-81) for one item: 128 P points of one fit.
-// The item's rows are staged once in shared memory, transposed (a column of
-// 128 P values per dimension, stride kBEXs: conflict-free stores and reads).
-// Components are staged kc at a time; per component each thread centres its
-// P points on the mean, forms ||W_j (x - mu_j)||^2, writes l_ij to R and
-// keeps an online log-sum-exp; a second pass turns l_ij into
-// exp(l_ij - LSE_i).
+// The item's rows are staged once in shared memory as columns of pairs
+// (2 q, 2 q + 1) x 128 P points.  Components are staged KC at a time; per
+// component each thread centres its P points on the mean, forms
+// ||W_j (x - mu_j)||^2 (two columns per instruction, em_tri.cuh), writes l_ij to
+// R and keeps an online log-sum-exp; a second pass turns l_ij into
+// exp(l_ij - LSE_i).  Bound by the FMA pipe; KC is what lets three CTAs of D = 32
+// share an SM (KC 4, 2, 1: 973, 1033, 1137 us over a batch of 192 fits of
+// 2000..200000 rows; 880 with the row staging's loads in flight together).  Fits of d <= 24 in the D = 32 class multiply 24 columns of its
+// layout.  With single products, a branching log-sum-exp and KC = 8 that launch
+// took 2160 us.
 constexpr int kBEP = 4;                          // points per thread
 constexpr int kBEPoints = kBEThreads * kBEP;     // points per item
-constexpr int kBEXs = kBEPoints + 1;             // transposed row stride (floats)
+constexpr int kBEXs = kBEPoints + 1;             // column-pair stride (float2)
+
+// components staged at a time
+__host__ __device__ constexpr int estep_kc(int D) { return D >= 24 ? 4 : D >= 16 ? 8 : 16; }
 
 template <int D>
 constexpr size_t estep_smem() {
-  constexpr int KC = D >= 32 ? 8 : 16;
+  constexpr int KC = estep_kc(D);
   return ((size_t)D * kBEXs + 2 * (size_t)((KC * tri_off(D) + KC * D + KC + 3) & ~3)) * sizeof(float);
 }
 
-template <int D, int P>
-__global__ void __launch_bounds__(kBEThreads)
-k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const EItem *__restrict__ items,
-          double *__restrict__ epart) {
-  static_assert(P == kBEP, "points per thread");
-  constexpr int TRI = tri_off(D);
-  constexpr int KC = D >= 32 ? 8 : 16;
+// D: columns computed (d <= D, even); CD: the fit's class, whose layout muT and WT have
+template <int D, int CD>
+__device__ __forceinline__ void b_estep_item(const BFit &F, int p0, float *smem, double *red, double *out) {
+  constexpr int P = kBEP, TRI = tri_off(D), CTRI = tri_off(CD), KC = estep_kc(D);
   constexpr int CB = KC * TRI + KC * D + KC;      // one component buffer: W, means, log coefficients
   constexpr int CBP = (CB + 3) & ~3;
-  extern __shared__ __align__(16) float sXt[];   // D x kBEXs, then two component buffers
-  __shared__ double red[kBEThreads / 32];
-  const EItem item = items[blockIdx.x];
-  if (!state[item.fit].active) return;
-  const BFit &F = fits[item.fit];
+  float2 *sX = reinterpret_cast<float2 *>(smem);  // D / 2 x kBEXs, then two component buffers
   const float *__restrict__ X = F.X;
   float *__restrict__ R = F.R;
   const int64_t n = F.n;
   const int d = F.d, K = F.k, tid = threadIdx.x;
-  float *cbuf = sXt + D * kBEXs;
+  float *cbuf = smem + (((size_t)D * kBEXs + 3) & ~(size_t)3);
   // components [j0, j0 + kc) into buffer b (16-byte copies; W rows and means are 16-byte multiples)
   auto stage = [&](int b, int j0) {
     const int kc = min(KC, K - j0);
     float *w = cbuf + b * CBP, *m = w + KC * TRI, *l = m + KC * D;
-    for (int e = tid; e < kc * TRI / 4; e += kBEThreads) cp_async16(w + 4 * e, F.WT + (size_t)j0 * TRI + 4 * e);
-    for (int e = tid; e < kc * D / 4; e += kBEThreads) cp_async16(m + 4 * e, F.muT + (size_t)j0 * D + 4 * e);
+    for (int e = tid; e < kc * (TRI / 4); e += kBEThreads) {
+      const int jj = e / (TRI / 4), q = e % (TRI / 4);
+      cp_async16(w + 4 * e, F.WT + (size_t)(j0 + jj) * CTRI + 4 * q);
+    }
+    for (int e = tid; e < kc * (D / 4); e += kBEThreads) {
+      const int jj = e / (D / 4), q = e % (D / 4);
+      cp_async16(m + 4 * e, F.muT + (size_t)(j0 + jj) * CD + 4 * q);
+    }
     for (int e = tid; e < kc; e += kBEThreads) cp_async4(l + e, F.logcT + j0 + e, true);
     cp_async_commit();
   };
   stage(0, 0);
-  const int npts = (int)min((int64_t)kBEPoints, n - item.p0);
-  // rows -> transposed columns (zero past the last point and past column d)
+  const int npts = (int)min((int64_t)kBEPoints, n - p0);
+  // rows -> columns of pairs (zero past the last point and past column d)
   if (d == D) {
-    const float4 *src = reinterpret_cast<const float4 *>(X + (size_t)item.p0 * D);
+    const float4 *src = reinterpret_cast<const float4 *>(X + (size_t)p0 * D);
+#pragma unroll 4
     for (int e = tid; e < kBEPoints * D / 4; e += kBEThreads) {
       const int pt = (4 * e) / D, q = (4 * e) % D;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (pt < npts) v = src[e];
-      sXt[(q + 0) * kBEXs + pt] = v.x;
-      sXt[(q + 1) * kBEXs + pt] = v.y;
-      sXt[(q + 2) * kBEXs + pt] = v.z;
-      sXt[(q + 3) * kBEXs + pt] = v.w;
+      if (pt < npts) v = __ldg(src + e);
+      sX[(q / 2 + 0) * kBEXs + pt] = make_float2(v.x, v.y);
+      sX[(q / 2 + 1) * kBEXs + pt] = make_float2(v.z, v.w);
     }
   } else {
-    const float *src = X + (size_t)item.p0 * d;
+    const float *src = X + (size_t)p0 * d;
+    float *sx = smem;
+#pragma unroll 8
     for (int e = tid; e < kBEPoints * D; e += kBEThreads) {
-      const int pt = e / D, q = e - pt * D;
-      sXt[q * kBEXs + pt] = (pt < npts && q < d) ? src[(size_t)pt * d + q] : 0.f;
+      const int pt = e / D, q = e % D;
+      sx[2 * ((q / 2) * kBEXs + pt) + (q & 1)] = (pt < npts && q < d) ? __ldg(src + pt * d + q) : 0.f;
     }
   }
-  int64_t idx[P];
   bool valid[P];
-#pragma unroll
-  for (int p = 0; p < P; p++) {
-    idx[p] = (int64_t)item.p0 + tid + p * kBEThreads;
-    valid[p] = idx[p] < n;
-  }
   float mx[P], se[P];
 #pragma unroll
-  for (int p = 0; p < P; p++) mx[p] = -INFINITY, se[p] = 0.f;
+  for (int p = 0; p < P; p++) {
+    valid[p] = tid + p * kBEThreads < npts;
+    mx[p] = -INFINITY, se[p] = 0.f;
+  }
   int b = 0;
   for (int j0 = 0; j0 < K; j0 += KC, b ^= 1) {
     const int kc = min(KC, K - j0);
@@ -283,23 +231,24 @@ k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const
     __syncthreads();
     const float *sW = cbuf + b * CBP, *smu = sW + KC * TRI, *slc = smu + KC * D;
     for (int jj = 0; jj < kc; jj++) {
-      const float *m = smu + jj * D;
-      float t[P][D];
+      const uint64_t *m = reinterpret_cast<const uint64_t *>(smu + jj * D);
+      uint64_t t[P][D / 2];
 #pragma unroll
-      for (int q = 0; q < D; q++) {
-        const float mq = m[q];
+      for (int q = 0; q < D / 2; q++) {
+        const uint64_t mq = m[q];
 #pragma unroll
-        for (int p = 0; p < P; p++) t[p][q] = sXt[q * kBEXs + tid + p * kBEThreads] - mq;
+        for (int p = 0; p < P; p++)
+          t[p][q] = f2_sub(reinterpret_cast<const uint64_t *>(sX)[q * kBEXs + tid + p * kBEThreads], mq);
       }
       float s[P];
       tri_norms<D, P>(t, sW + jj * TRI, s);
       const float lc = slc[jj];
-      float *Rj = R + (size_t)(j0 + jj) * n;
+      float *Rj = R + (size_t)(j0 + jj) * n + p0 + tid;
 #pragma unroll
       for (int p = 0; p < P; p++) {
         const float l = lc - 0.5f * s[p];
-        if (valid[p]) Rj[idx[p]] = l;
-        blse_push(l, mx[p], se[p]);
+        if (valid[p]) Rj[p * kBEThreads] = l;
+        lse_add(l, mx[p], se[p]);
       }
     }
     __syncthreads();
@@ -314,13 +263,28 @@ k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const
   }
 #pragma unroll 4
   for (int j = 0; j < K; j++) {
-    float *Rj = R + (size_t)j * n;
+    float *Rj = R + (size_t)j * n + p0 + tid;
 #pragma unroll
     for (int p = 0; p < P; p++)
-      if (valid[p]) Rj[idx[p]] = expf(Rj[idx[p]] - lse[p]);
+      if (valid[p]) Rj[p * kBEThreads] = expf(Rj[p * kBEThreads] - lse[p]);
   }
   const double sum = bblock_sum<kBEThreads>(v, red);
-  if (tid == 0) epart[blockIdx.x] = sum;
+  if (tid == 0) *out = sum;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kBEThreads)
+k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const EItem *__restrict__ items,
+          double *__restrict__ epart) {
+  extern __shared__ __align__(16) float esm[];
+  __shared__ double red[kBEThreads / 32];
+  const EItem item = items[blockIdx.x];
+  if (!state[item.fit].active) return;
+  const BFit &F = fits[item.fit];
+  if (D == 32 && F.d <= 24)
+    b_estep_item<D == 32 ? 24 : D, D>(F, item.p0, esm, red, epart + blockIdx.x);
+  else
+    b_estep_item<D, D>(F, item.p0, esm, red, epart + blockIdx.x);
 }
 
 // ======================================================= M-step: means
@@ -1151,7 +1115,7 @@ k_bt_estep(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
             if (j < K) {
               const float l = (chi[(size_t)(F.wg + g) * 4 + q] - 0.5f * (s0 + s1)) + clo[(size_t)(F.wg + g) * 4 + q];
               if (valid) F.R[(size_t)j * n + i] = l;
-              blse_push(l, mx, se);
+              lse_add(l, mx, se);
             }
           }
         }
@@ -1348,10 +1312,10 @@ int launch_sweep(fem_em_batch *b, int it, int svd, int slot) {
       continue;
     }
     switch (c) {
-      case 0: k_b_estep<4, kBEP><<<cnt, kBEThreads, estep_smem<4>(), b->stream>>>(fits, st, it0, ep); break;
-      case 1: k_b_estep<8, kBEP><<<cnt, kBEThreads, estep_smem<8>(), b->stream>>>(fits, st, it0, ep); break;
-      case 2: k_b_estep<16, kBEP><<<cnt, kBEThreads, estep_smem<16>(), b->stream>>>(fits, st, it0, ep); break;
-      default: k_b_estep<32, kBEP><<<cnt, kBEThreads, estep_smem<32>(), b->stream>>>(fits, st, it0, ep); break;
+      case 0: k_b_estep<4><<<cnt, kBEThreads, estep_smem<4>(), b->stream>>>(fits, st, it0, ep); break;
+      case 1: k_b_estep<8><<<cnt, kBEThreads, estep_smem<8>(), b->stream>>>(fits, st, it0, ep); break;
+      case 2: k_b_estep<16><<<cnt, kBEThreads, estep_smem<16>(), b->stream>>>(fits, st, it0, ep); break;
+      default: k_b_estep<32><<<cnt, kBEThreads, estep_smem<32>(), b->stream>>>(fits, st, it0, ep); break;
     }
     FEM_CUDA(cudaGetLastError());
     b->launches++;
@@ -1646,10 +1610,10 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     set_error("event creation failed");
     return fail(FEM_ERR_CUDA);
   }
-  if (allow_dyn_smem(k_b_estep<4, kBEP>, estep_smem<4>()) != cudaSuccess ||
-      allow_dyn_smem(k_b_estep<8, kBEP>, estep_smem<8>()) != cudaSuccess ||
-      allow_dyn_smem(k_b_estep<16, kBEP>, estep_smem<16>()) != cudaSuccess ||
-      allow_dyn_smem(k_b_estep<32, kBEP>, estep_smem<32>()) != cudaSuccess ||
+  if (allow_dyn_smem(k_b_estep<4>, estep_smem<4>()) != cudaSuccess ||
+      allow_dyn_smem(k_b_estep<8>, estep_smem<8>()) != cudaSuccess ||
+      allow_dyn_smem(k_b_estep<16>, estep_smem<16>()) != cudaSuccess ||
+      allow_dyn_smem(k_b_estep<32>, estep_smem<32>()) != cudaSuccess ||
       allow_dyn_smem(k_b_means<4>, b->m_smem[0]) != cudaSuccess ||
       allow_dyn_smem(k_b_means<8>, b->m_smem[1]) != cudaSuccess ||
       allow_dyn_smem(k_b_means<16>, b->m_smem[2]) != cudaSuccess ||

@@ -17,6 +17,7 @@
 #include "fem_internal.cuh"
 #include "em_kernels.cuh"
 #include "em_factor.cuh"
+#include "em_tri.cuh"
 
 namespace fem {
 
@@ -61,15 +62,259 @@ __device__ __forceinline__ void lse_push(T l, T &mx, T &se) {
 
 // ================================================================ E-step
 // MatrixEMBase::BlockDensities + PostProcessDensityMatrix
-// (EM2/MatrixEM.cpp:39-51,69-81): one thread per point, components staged
-// through shared memory; l_ij is written to R, then overwritten by
-// exp(l_ij - LSE_i).  D > 0: compile-time dimension with the centred point
-// in registers.
-template <typename T, int D>
+// (EM2/MatrixEM.cpp:39-51,69-81) for d <= D (columns d..D-1 are zero in the
+// rows and the factors).  A CTA takes 128 P points, P per thread; the factors'
+// lower triangles, means and log coefficients of KC components are copied
+// asynchronously one group ahead.  Per component a thread centres its points,
+// forms ||W_j (x - mu_j)||^2 and writes l_ij to R.
+// FP32 is bound by the FMA pipe and the 16-byte broadcast loads of the factor,
+// which serve P points; columns are multiplied in pairs (em_tri.cuh) and the
+// log-sum-exp takes one exponential and no branch.  Against one point per
+// thread, one component at a time and a branch (GB300): 250007 x 16 x 200
+// 893 -> 548 us, 400000 x 32 x 40 808 -> 501, 300000 x 4 x 200 276 -> 228; where
+// the dimension had no kernel of its own, 250007 x 13 x 135 1590 -> 445,
+// 200000 x 40 x 60 5264 -> 726.
+// FP64: 100000 x 8 x 10 231 -> 167 us, 100000 x 13 x 10 375 -> 332,
+// 20000 x 4 x 5 29 -> 19.
+constexpr int kEPThreads = 128;
+
+template <typename T, int D, int KC>
+struct EstepBuf {
+  static constexpr int TRI = tri_off(D);
+  static constexpr int CB = KC * (TRI + D + 4);     // elements (log coefficients at the end)
+};
+
+template <typename T, int BYTES>
+__device__ __forceinline__ void ep_copy(T *dst, const T *src, bool valid) {
+  const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(da), "l"(src), "n"(BYTES), "r"(valid ? BYTES : 0)
+               : "memory");
+}
+
+// components [j0, j0 + kc) into buf; rows of the triangle from d on and columns
+// from d on become zero.  16-byte copies when a row of the factors is a
+// multiple of 16 bytes.
+template <typename T, int D, int KC>
+__device__ __forceinline__ void ep_stage(T *buf, const T *__restrict__ mu, const T *__restrict__ W,
+                                         const T *__restrict__ logc, int d, int j0, int kc) {
+  constexpr int TRI = tri_off(D), V = 16 / sizeof(T);
+  T *m = buf + KC * TRI, *l = m + KC * D;
+  const int tid = threadIdx.x;
+  const T *Wj = W + (size_t)j0 * d * d, *mj = mu + (size_t)j0 * d;
+  auto copy = [&](auto vec) {
+    constexpr int E = decltype(vec)::value, Q = D / E;
+    for (int e = tid; e < kc * D * Q; e += kEPThreads) {
+      const int jj = e / (D * Q), r = (e / Q) % D, c = E * (e % Q);
+      if (c >= tri_row(r)) continue;
+      const bool v = r < d && c < d;
+      ep_copy<T, E * (int)sizeof(T)>(buf + jj * TRI + tri_off(r) + c, Wj + (v ? (jj * d + r) * d + c : 0), v);
+    }
+    for (int e = tid; e < kc * Q; e += kEPThreads) {
+      const int jj = e / Q, q = E * (e % Q);
+      ep_copy<T, E * (int)sizeof(T)>(m + jj * D + q, mj + (q < d ? jj * d + q : 0), q < d);
+    }
+  };
+  if (d % V == 0)
+    copy(std::integral_constant<int, V>());
+  else
+    copy(std::integral_constant<int, 1>());
+  for (int e = tid; e < kc; e += kEPThreads) ep_copy<T, (int)sizeof(T)>(l + e, logc + j0 + e, true);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// FP32, with an online log-sum-exp; a second pass turns R into exp(l - LSE).
+// Rows in registers, or (XS) as columns of pairs in shared memory.
+template <int D, int P, bool XS, int KC>
+__global__ void __launch_bounds__(kEPThreads)
+k_estep_f32(const float *__restrict__ X, int64_t n, int d, int K, const float *__restrict__ mu,
+            const float *__restrict__ W, const float *__restrict__ logc, float *__restrict__ R,
+            double *__restrict__ part) {
+  using S = EstepBuf<float, D, KC>;
+  constexpr int TRI = S::TRI, PS = kEPThreads * P + 1;
+  extern __shared__ __align__(16) float esm[];
+  __shared__ double red[kEPThreads / 32];
+  float *cbuf = esm;
+  uint64_t *sx = reinterpret_cast<uint64_t *>(esm + 2 * S::CB) + threadIdx.x;
+  const int tid = threadIdx.x;
+  const int64_t p0 = (int64_t)blockIdx.x * kEPThreads * P;
+  ep_stage<float, D, KC>(cbuf, mu, W, logc, d, 0, min(KC, K));
+  uint64_t x[P][XS ? 1 : D / 2];
+  bool live[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) live[p] = p0 + tid + p * kEPThreads < n;
+  if constexpr (XS) {
+    float *sf = esm + 2 * S::CB;
+    const int np = (int)min((int64_t)kEPThreads * P, n - p0);
+    const float *src = X + (size_t)p0 * d;
+#pragma unroll 8
+    for (int e = tid; e < kEPThreads * P * D; e += kEPThreads) {
+      const int pt = e / D, q = e % D;
+      sf[2 * ((q / 2) * PS + pt) + (q & 1)] = (pt < np && q < d) ? __ldg(src + pt * d + q) : 0.f;
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+      const float *xr = X + (live[p] ? p0 + tid + p * kEPThreads : 0) * d;
+      if (d == D) {
+#pragma unroll
+        for (int q = 0; q < D / 4; q++) {
+          const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(xr) + q);
+          x[p][2 * q] = v.x, x[p][2 * q + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < D / 2; q++)
+          x[p][q] = f2_pack(2 * q < d ? __ldg(xr + 2 * q) : 0.f, 2 * q + 1 < d ? __ldg(xr + 2 * q + 1) : 0.f);
+      }
+    }
+  }
+  float mx[P], se[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) mx[p] = -INFINITY, se[p] = 0.f;
+  int b = 0;
+  for (int j0 = 0; j0 < K; j0 += KC, b ^= 1) {
+    const int kc = min(KC, K - j0);
+    if (j0 + KC < K)
+      ep_stage<float, D, KC>(cbuf + (b ^ 1) * S::CB, mu, W, logc, d, j0 + KC, min(KC, K - j0 - KC));
+    else
+      asm volatile("cp.async.commit_group;\n" ::: "memory");   // keeps the wait count uniform
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    const float *sW = cbuf + b * S::CB, *sm = sW + KC * TRI, *sl = sm + KC * D;
+    float *Rj = R + (size_t)j0 * n + p0 + tid;
+#pragma unroll 1
+    for (int jj = 0; jj < kc; jj++, Rj += n) {
+      const uint64_t *m = reinterpret_cast<const uint64_t *>(sm + jj * D);
+      uint64_t t[P][D / 2];
+#pragma unroll
+      for (int q = 0; q < D / 2; q++) {
+        const uint64_t mq = m[q];
+#pragma unroll
+        for (int p = 0; p < P; p++) t[p][q] = f2_sub(XS ? sx[q * PS + p * kEPThreads] : x[p][XS ? 0 : q], mq);
+      }
+      float s[P];
+      tri_norms<D, P>(t, sW + jj * TRI, s);
+      const float lc = sl[jj];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+        const float l = lc - 0.5f * s[p];
+        if (live[p]) Rj[p * kEPThreads] = l;
+        lse_add(l, mx[p], se[p]);
+      }
+    }
+    __syncthreads();
+  }
+  double v = 0.0;
+  float lse[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) {
+    lse[p] = mx[p] + logf(se[p]);
+    if (live[p]) v += (double)lse[p];
+  }
+  float *Rt = R + p0 + tid;
+#pragma unroll 4
+  for (int j = 0; j < K; j++)
+#pragma unroll
+    for (int p = 0; p < P; p++)
+      if (live[p]) {
+        float *q = Rt + (size_t)j * n + p * kEPThreads;
+        *q = expf(*q - lse[p]);
+      }
+  const double s = block_sum<kEPThreads>(v, red);
+  if (tid == 0) part[blockIdx.x] = s;
+}
+
+// FP64 is bound by its pipe, of which an exponential takes half a d = 8
+// component's share: the maximum only is kept and each exponential is taken
+// once.  R holds l, then exp(l - max), then that over its sum.
+template <int D, int P, int KC>
+__global__ void __launch_bounds__(kEPThreads)
+k_estep_f64(const float *__restrict__ X, int64_t n, int d, int K, const double *__restrict__ mu,
+            const double *__restrict__ W, const double *__restrict__ logc, double *__restrict__ R,
+            double *__restrict__ part) {
+  using S = EstepBuf<double, D, KC>;
+  constexpr int TRI = S::TRI;
+  extern __shared__ __align__(16) double dsm[];
+  __shared__ double red[kEPThreads / 32];
+  const int tid = threadIdx.x;
+  const int64_t p0 = (int64_t)blockIdx.x * kEPThreads * P;
+  ep_stage<double, D, KC>(dsm, mu, W, logc, d, 0, min(KC, K));
+  float x[P][D];
+  bool live[P];
+  double mx[P], se[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) {
+    live[p] = p0 + tid + p * kEPThreads < n;
+    mx[p] = -INFINITY, se[p] = 0.0;
+    const float *xr = X + (live[p] ? p0 + tid + p * kEPThreads : 0) * d;
+#pragma unroll
+    for (int q = 0; q < D; q++) x[p][q] = q < d ? __ldg(xr + q) : 0.f;
+  }
+  double *Rt = R + p0 + tid;
+  int b = 0;
+  for (int j0 = 0; j0 < K; j0 += KC, b ^= 1) {
+    const int kc = min(KC, K - j0);
+    if (j0 + KC < K)
+      ep_stage<double, D, KC>(dsm + (b ^ 1) * S::CB, mu, W, logc, d, j0 + KC, min(KC, K - j0 - KC));
+    else
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    const double *sW = dsm + b * S::CB, *sm = sW + KC * TRI, *sl = sm + KC * D;
+    for (int jj = 0; jj < kc; jj++) {
+      double t[P][D], s[P];
+#pragma unroll
+      for (int q = 0; q < D; q++) {
+        const double mq = sm[jj * D + q];
+#pragma unroll
+        for (int p = 0; p < P; p++) t[p][q] = (double)x[p][q] - mq;
+      }
+      tri_norms<D, P>(t, sW + jj * TRI, s);
+      const double lc = sl[jj];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+        const double l = lc - 0.5 * s[p];
+        if (live[p]) Rt[(size_t)(j0 + jj) * n + p * kEPThreads] = l;
+        mx[p] = l > mx[p] ? l : mx[p];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll 4
+  for (int j = 0; j < K; j++)
+#pragma unroll
+    for (int p = 0; p < P; p++)
+      if (live[p]) {
+        double *q = Rt + (size_t)j * n + p * kEPThreads;
+        const double l = *q, e = exp(l - mx[p]);
+        if (l > -INFINITY) se[p] += e;
+        *q = e;
+      }
+  double v = 0.0, c[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) {
+    c[p] = 1.0 / se[p];
+    if (live[p]) v += mx[p] + log(se[p]);
+  }
+#pragma unroll 4
+  for (int j = 0; j < K; j++)
+#pragma unroll
+    for (int p = 0; p < P; p++)
+      if (live[p]) Rt[(size_t)j * n + p * kEPThreads] *= c[p];
+  const double s = block_sum<kEPThreads>(v, red);
+  if (tid == 0) part[blockIdx.x] = s;
+}
+
+// d = 64: one point per thread, components one at a time.  The unrolled triangle
+// of the kernels above no longer fits the instruction cache (FP32, 20000 rows,
+// 10 components: 108 us against 75 here) or, in FP64, the registers (30000 rows,
+// 10 components: 3446 us against 1458; k_estep_plain_generic takes 1776).
+template <typename T>
 __global__ void __launch_bounds__(128)
-k_estep_plain(const float *__restrict__ X, int64_t n, int K, const T *__restrict__ mu,
+k_estep_64(const float *__restrict__ X, int64_t n, int K, const T *__restrict__ mu,
               const T *__restrict__ W, const T *__restrict__ logc, T *__restrict__ R,
               double *__restrict__ part) {
+  constexpr int D = 64;
   __shared__ __align__(16) T sW[D * D];
   __shared__ __align__(16) T smu[D];
   __shared__ double red[4];
@@ -440,44 +685,121 @@ k_factor(int K, int d, double reg, int regularize, double *__restrict__ sigma,
 }
 
 // =========================================================== launchers
+// P points per thread once there are two CTAs of that many per SM; below that
+// one, which spreads the rows over more SMs.  With one point the rows are in
+// registers up to D = 32 (20000 x 24 x 20: 37 us, in shared memory 39).
+template <int D, int P, bool XS, int KC>
+static int estep_f32(fem_em *h, int64_t *nb) {
+  constexpr bool XS1 = XS && D > 32;
+  const bool wide = P > 1 && h->n >= (int64_t)2 * sm_count() * kEPThreads * P;
+  const int pw = wide ? P : 1, pts = kEPThreads * pw;
+  const size_t sm = (2 * (size_t)EstepBuf<float, D, KC>::CB + ((wide ? XS : XS1) ? (size_t)D * (kEPThreads * pw + 1) : 0)) * sizeof(float);
+  *nb = (h->n + pts - 1) / pts;
+  auto launch = [&](auto kern) -> int {
+    FEM_CUDA(allow_dyn_smem(kern, sm));
+    kern<<<(unsigned)*nb, kEPThreads, sm, h->stream>>>(h->X, h->n, h->d, h->k, (const float *)h->muT, (const float *)h->linvT,
+                                                       (const float *)h->logcT, (float *)h->R, h->logl_part);
+    return FEM_OK;
+  };
+  return wide ? launch(k_estep_f32<D, P, XS, KC>) : launch(k_estep_f32<D, 1, XS1, KC>);
+}
+
+template <int D, int P, int KC>
+static int estep_f64(fem_em *h, int64_t *nb) {
+  const bool wide = P > 1 && h->n >= (int64_t)2 * sm_count() * kEPThreads * P;
+  const int pts = kEPThreads * (wide ? P : 1);
+  const size_t sm = 2 * (size_t)EstepBuf<double, D, KC>::CB * sizeof(double);
+  *nb = (h->n + pts - 1) / pts;
+  auto launch = [&](auto kern) -> int {
+    FEM_CUDA(allow_dyn_smem(kern, sm));
+    kern<<<(unsigned)*nb, kEPThreads, sm, h->stream>>>(h->X, h->n, h->d, h->k, (const double *)h->muT, (const double *)h->linvT,
+                                                       (const double *)h->logcT, (double *)h->R, h->logl_part);
+    return FEM_OK;
+  };
+  return wide ? launch(k_estep_f64<D, P, KC>) : launch(k_estep_f64<D, 1, KC>);
+}
+
 template <typename T>
 static int estep_plain_t(fem_em *h) {
   const int64_t n = h->n;
   const int d = h->d, K = h->k;
   const T *mu = (const T *)h->muT, *W = (const T *)h->linvT, *lc = (const T *)h->logcT;
   T *R = (T *)h->R;
-  cudaStream_t s = h->stream;
-  int64_t nb;
-#define FEM_EPL(DD)                                                                        \
-  case DD:                                                                                 \
-    nb = (n + 127) / 128;                                                                  \
-    k_estep_plain<T, DD><<<(unsigned)nb, 128, 0, s>>>(h->X, n, K, mu, W, lc, R, h->logl_part); \
-    break;
-  switch (d) {
-    FEM_EPL(4)
-    FEM_EPL(8)
-    FEM_EPL(16)
-    FEM_EPL(32)
-    FEM_EPL(64)
-    default: {
-      constexpr int PT = sizeof(T) == 4 ? 4 : 2;   // 128 FP32 or 64 FP64 points per CTA
-      const size_t smt = estep_tiled_smem<T, PT>(d);
-      if (d > 64 && smt <= kMaxDynSmem) {
-        nb = (n + 32 * PT - 1) / (32 * PT);
-        FEM_CUDA(allow_dyn_smem(k_estep_plain_tiled<T, PT>, smt));
-        k_estep_plain_tiled<T, PT><<<(unsigned)nb, 256, smt, s>>>(h->X, n, d, K, mu, W, lc, R, h->logl_part);
-      } else {
-        nb = (n + 63) / 64;
-        size_t sm = (size_t)64 * (d + 1) * sizeof(T);
-        FEM_CUDA(allow_dyn_smem(k_estep_plain_generic<T>, sm));
-        k_estep_plain_generic<T><<<(unsigned)nb, 64, sm, s>>>(h->X, n, d, K, mu, W, lc, R,
-                                                              h->logl_part);
-      }
+  int64_t nb = 0;
+  int st = FEM_OK;
+  bool done = true;
+  // FP32 below 64 columns: the next D.  P, rows in registers or shared memory and
+  // KC by measurement: D = 16 in registers P = 2, 3, 4: 609, 548, 619 us
+  // (250007 x 16 x 200), in shared memory P = 4: 636; D = 32 in shared memory
+  // P = 2, 3, 4: 554, 517, 633 (400000 x 32 x 40), one point in registers 808.
+  // FP64 up to 16 and at 32 (60000 x 32 x 10: 833 us, generic form 873): from 17
+  // on the generic form, which has no padding, is the faster one (60000 x 20 x 10:
+  // 394 against 495 us padded to 24).
+  if constexpr (sizeof(T) == 4) {
+    if (d <= 4)
+      st = estep_f32<4, 4, false, 16>(h, &nb);
+    else if (d <= 8)
+      st = estep_f32<8, 4, false, 8>(h, &nb);
+    else if (d <= 12)
+      st = estep_f32<12, 3, false, 4>(h, &nb);
+    else if (d <= 16)
+      st = estep_f32<16, 3, false, 4>(h, &nb);
+    else if (d <= 20)
+      st = estep_f32<20, 2, true, 2>(h, &nb);
+    else if (d <= 24)
+      st = estep_f32<24, 2, true, 2>(h, &nb);
+    else if (d <= 28)
+      st = estep_f32<28, 3, true, 2>(h, &nb);
+    else if (d <= 32)
+      st = estep_f32<32, 3, true, 2>(h, &nb);
+    else if (d <= 40)
+      st = estep_f32<40, 2, true, 2>(h, &nb);
+    else if (d <= 48)
+      st = estep_f32<48, 2, true, 2>(h, &nb);
+    else if (d < 64)
+      st = estep_f32<64, 2, true, 1>(h, &nb);
+    else
+      done = false;
+  } else {
+    if (d <= 4)
+      st = estep_f64<4, 2, 8>(h, &nb);
+    else if (d <= 6)
+      st = estep_f64<6, 2, 8>(h, &nb);
+    else if (d <= 8)
+      st = estep_f64<8, 2, 8>(h, &nb);
+    else if (d <= 10)
+      st = estep_f64<10, 1, 8>(h, &nb);
+    else if (d <= 12)
+      st = estep_f64<12, 1, 8>(h, &nb);
+    else if (d <= 14)
+      st = estep_f64<14, 1, 8>(h, &nb);
+    else if (d <= 16)
+      st = estep_f64<16, 1, 8>(h, &nb);
+    else if (d == 32)
+      st = estep_f64<32, 1, 2>(h, &nb);
+    else
+      done = false;
+  }
+  FEM_TRY(st);
+  if (!done) {
+    constexpr int PT = sizeof(T) == 4 ? 4 : 2;   // 128 FP32 or 64 FP64 points per CTA
+    const size_t smt = estep_tiled_smem<T, PT>(d);
+    if (d > 64 && smt <= kMaxDynSmem) {
+      nb = (n + 32 * PT - 1) / (32 * PT);
+      FEM_CUDA(allow_dyn_smem(k_estep_plain_tiled<T, PT>, smt));
+      k_estep_plain_tiled<T, PT><<<(unsigned)nb, 256, smt, h->stream>>>(h->X, n, d, K, mu, W, lc, R, h->logl_part);
+    } else if (d == 64) {
+      nb = (n + 127) / 128;
+      k_estep_64<T><<<(unsigned)nb, 128, 0, h->stream>>>(h->X, n, K, mu, W, lc, R, h->logl_part);
+    } else {
+      nb = (n + 63) / 64;
+      const size_t sm = (size_t)64 * (d + 1) * sizeof(T);
+      FEM_CUDA(allow_dyn_smem(k_estep_plain_generic<T>, sm));
+      k_estep_plain_generic<T><<<(unsigned)nb, 64, sm, h->stream>>>(h->X, n, d, K, mu, W, lc, R, h->logl_part);
     }
   }
-#undef FEM_EPL
   FEM_CUDA(cudaGetLastError());
-  k_reduce_logl<<<1, 1024, 0, s>>>(h->logl_part, nb, h->dstat);
+  k_reduce_logl<<<1, 1024, 0, h->stream>>>(h->logl_part, nb, h->dstat);
   FEM_CUDA(cudaGetLastError());
   h->launches += 2;
   return FEM_OK;
@@ -487,12 +809,7 @@ int em_plain_estep(fem_em *h) {
   return h->cfg.precision == FEM_PREC_FP64 ? estep_plain_t<double>(h) : estep_plain_t<float>(h);
 }
 
-int64_t em_plain_logl_blocks(int64_t n, int d) {
-  switch (d) {
-    case 4: case 8: case 16: case 32: case 64: return (n + 127) / 128;
-    default: return (n + 63) / 64;
-  }
-}
+int64_t em_plain_logl_blocks(int64_t n, int d) { (void)d; return (n + 63) / 64; }
 
 template <typename T>
 static int mstep_plain_t(fem_em *h) {

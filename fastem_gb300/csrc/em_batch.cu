@@ -19,14 +19,14 @@
 //
 // Layout in HBM: the fits' rows are packed one fit after another (each fit
 // starting on a 16-byte boundary); posteriors are component-major per fit
-// (k x n); W_j = L_j^-1 is stored as a lower triangle whose rows are padded
+// (k x n, rows of a component on 16-byte boundaries); W_j = L_j^-1 is stored as a lower triangle whose rows are padded
 // to multiples of 4 floats so the E-step reads it with 16-byte loads.
 //
 // Work items are built on the host when the batch is created (the shapes
 // are fixed): E-step items of 128 P points, means items and covariance items
 // of a per-class number of points (fem_em_batch_tuning; defaults kBMChunk,
-// kBCChunk) x one range of <= 256 (component,
-// TB x TB block) units.  Item lists are grouped by dimension class; each
+// kBCChunk) x one range of <= 256 (component, 8 x 8
+// block) units.  Item lists are grouped by dimension class; each
 // class is one launch per phase.
 #include <algorithm>
 #include <cfloat>
@@ -40,6 +40,7 @@
 #include <cuda_fp16.h>
 
 #include "em_factor.cuh"
+#include "em_kernels.cuh"
 #include "em_tri.cuh"
 #include "fem_internal.cuh"
 #include "tc_ptx.cuh"
@@ -50,35 +51,30 @@ namespace {
 constexpr int kBMaxD = 32;
 constexpr int kBMaxK = 64;
 constexpr int kBEThreads = 128;
-constexpr int kBMThreads = 128;
+constexpr int kBMThreads = 256;
 constexpr int kBCThreads = 256;
 constexpr int kBFThreads = 256;
 constexpr int kBMChunk = 2048;   // points per means item
 constexpr int kBCChunk = 4096;   // points per covariance item
 constexpr int kBMTile = 128;     // points staged per means tile
-constexpr int kBCTile = 16;      // points staged per covariance tile
+constexpr int kBCTile = 128;     // points staged per covariance tile
 constexpr int kBatchSyncEvery = 8;
 constexpr int kTimeMarks = 15;   // timing events per sweep (see collect_timing)
 constexpr int kClasses = 4;      // D = 4, 8, 16, 32
 
-__host__ __device__ constexpr int class_tb(int D) { return D >= 16 ? 8 : 4; }
-__host__ __device__ constexpr int class_nblk(int D) { return (D / class_tb(D)) * (D / class_tb(D) + 1) / 2; }
-// covariance sums: D <= 16 by component owners (k_b_cov_own), D = 32 by TB x TB blocks (k_b_cov)
-__host__ __device__ constexpr bool class_owner(int D) { return D <= 16; }
-__host__ __device__ constexpr int own_S(int D) { return D >= 16 ? 2 : 1; }          // threads per component
-__host__ __device__ constexpr int own_pairs(int D) { return D / 2 / own_S(D); }     // row pairs per thread
-__host__ __device__ constexpr int own_NE(int D) { return own_pairs(D) * (D + 1); }  // sums per thread
-__host__ __device__ constexpr int own_TP(int D) { return D >= 16 ? 32 : 128; }      // points per tile
+// covariance sums: D = 4 by component owners (k_b_cov_own), above by 8 x 8 blocks (k_b_cov)
+__host__ __device__ constexpr bool class_owner(int D) { return D <= 4; }
+constexpr int kOwnD = 4, kOwnNE = 10, kOwnTP = 128;   // owner form: dimensions, sums per component, points per tile
 int class_of(int d) { return d <= 4 ? 0 : d <= 8 ? 1 : d <= 16 ? 2 : 3; }
 int class_dim(int c) { return 4 << c; }
 
 // device descriptor of one fit
 struct BFit {
   const float *X;        // n x d rows
-  float *R;              // k x n, component-major
-  int64_t n;
+  float *R;              // k x ld, component-major
+  int64_t n, ld;         // rows; n rounded up to 4
   int d, k, D;
-  int nug;               // covariance unit ranges: ceil(k nblk / 256)
+  int nug;               // covariance unit ranges
   int e_first, e_count;  // E-step items (global indices)
   int m_first, m_count;  // means items
   int64_t m_part;        // first means partial (doubles): m_count blocks of k (D + 4)
@@ -112,6 +108,20 @@ __device__ __forceinline__ double bwarp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
+// sum of n FP32 values `stride` apart, in order, to FP64: the rounding errors of
+// the FP32 additions are carried along exactly (two-sum), so three FP64
+// operations suffice instead of 2 n, which the FP64 pipe's rate would make a
+// tenth of a covariance item's time
+__device__ __forceinline__ double group_sum(const float *v, int n, int stride) {
+  float hi = v[0], lo = 0.f;
+  for (int g = 1; g < n; g++) {
+    const float x = v[g * stride], t = __fadd_rn(hi, x), b = __fsub_rn(t, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(x, b)));
+    hi = t;
+  }
+  return n > 1 ? (double)hi + (double)lo : (double)hi;
+}
+
 // deterministic block sum, result in thread 0
 template <int NT>
 __device__ double bblock_sum(double v, double *red) {
@@ -135,6 +145,11 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src, bool val
 __device__ __forceinline__ void cp_async16(float *dst, const float *src) {
   const unsigned da = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(da), "l"(src) : "memory");
+}
+// the same for the first `bytes` of the 16, zeros behind them
+__device__ __forceinline__ void cp_async16z(float *dst, const float *src, int bytes) {
+  const unsigned da = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(da), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
@@ -175,7 +190,7 @@ __device__ __forceinline__ void b_estep_item(const BFit &F, int p0, float *smem,
   float2 *sX = reinterpret_cast<float2 *>(smem);  // D / 2 x kBEXs, then two component buffers
   const float *__restrict__ X = F.X;
   float *__restrict__ R = F.R;
-  const int64_t n = F.n;
+  const int64_t n = F.n, ld = F.ld;
   const int d = F.d, K = F.k, tid = threadIdx.x;
   float *cbuf = smem + (((size_t)D * kBEXs + 3) & ~(size_t)3);
   // components [j0, j0 + kc) into buffer b (16-byte copies; W rows and means are 16-byte multiples)
@@ -243,7 +258,7 @@ __device__ __forceinline__ void b_estep_item(const BFit &F, int p0, float *smem,
       float s[P];
       tri_norms<D, P>(t, sW + jj * TRI, s);
       const float lc = slc[jj];
-      float *Rj = R + (size_t)(j0 + jj) * n + p0 + tid;
+      float *Rj = R + (size_t)(j0 + jj) * ld + p0 + tid;
 #pragma unroll
       for (int p = 0; p < P; p++) {
         const float l = lc - 0.5f * s[p];
@@ -263,7 +278,7 @@ __device__ __forceinline__ void b_estep_item(const BFit &F, int p0, float *smem,
   }
 #pragma unroll 4
   for (int j = 0; j < K; j++) {
-    float *Rj = R + (size_t)j * n + p0 + tid;
+    float *Rj = R + (size_t)j * ld + p0 + tid;
 #pragma unroll
     for (int p = 0; p < P; p++)
       if (valid[p]) Rj[p * kBEThreads] = expf(Rj[p * kBEThreads] - lse[p]);
@@ -287,68 +302,84 @@ k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const
     b_estep_item<D, D>(F, item.p0, esm, red, epart + blockIdx.x);
 }
 
+// Posteriors of components j0 .. j0 + cj - 1 and points t0 .. t0 + tp - 1 into
+// shared memory, component-major with `pitch` floats between components, zeros
+// from tp to TP.  t0 is a multiple of 4 (items start on multiples of 128, tiles
+// of 4)
+template <int NT, int TP>
+__device__ __forceinline__ void stage_posteriors(float *sr, int pitch, const float *__restrict__ R, int64_t ld, int j0,
+                                                 int cj, int t0, int tp) {
+  for (int e = threadIdx.x; e < cj * (TP / 4); e += NT) {
+    const int jj = e / (TP / 4), p = 4 * (e % (TP / 4)), m = max(0, min(4, tp - p));
+    cp_async16z(sr + jj * pitch + p, R + (size_t)(j0 + jj) * ld + (m ? t0 + p : 0), 4 * m);
+  }
+}
+
 // ======================================================= M-step: means
 // SimpleMatrixEM::doMStep means part (EM2/MatrixEM.cpp:319-343) for one item:
 // sums_j[c] = sum_i r_ij [x_i | 1][c] over the item's points, as a K x (D+4)
-// block of FP64 partials (column D holds PosteriorSum_j).  Threads own 4 x 4
-// micro-tiles of (component, column); when there are fewer micro-tiles than
-// threads, point groups split each tile's points and are summed at the end.
-// Tiles of kBMTile points are copied with cp.async one tile ahead into two
-// shared buffers (rows x (D + 4) with the ones column, posteriors point-major
-// with an odd stride).  FP32 sums over the item.
+// block of FP64 partials (column D holds PosteriorSum_j).  A unit is 4
+// components x 4 columns of [x | 1]; thread t owns unit t % units for every
+// 4 G-th group of four points (G = 256 / units), so four 16-byte loads of
+// posteriors and four of rows feed 64 products.  Tiles of kBMTile points are
+// copied with cp.async one tile ahead into two shared buffers.  FP32 sums over
+// the item, the groups' sums by group_sum.  Bound by shared-memory loads and,
+// for short tiles, the copies' instructions.  Against point-major posteriors,
+// 4-byte copies and units rounded up to warps (192 fits of 2000..200000 rows, a
+// sweep): D = 32 359 -> 172 us, 16 84 -> 50, 8 151 -> 98, 4 117 -> 75.
 template <int D>
 __host__ __device__ constexpr size_t means_buf_floats(int kmax) {
-  return (((size_t)kBMTile * (D + 4) + (size_t)kBMTile * (((kmax + 3) & ~3) + 1)) + 3) & ~(size_t)3;
+  return (size_t)kBMTile * (D + 4) + (size_t)((kmax + 3) & ~3) * (kBMTile + 4);
 }
 
 template <int D>
 __global__ void __launch_bounds__(kBMThreads)
 k_b_means(const BFit *__restrict__ fits, const BState *__restrict__ state, const MItem *__restrict__ items,
           double *__restrict__ mpart, int kmax) {
-  constexpr int XC = D + 4, NQB = XC / 4, TP = kBMTile;
-  constexpr int UPT = (kBMaxK / 4 * NQB + kBMThreads - 1) / kBMThreads;
+  constexpr int XC = D + 4, TP = kBMTile, RP = TP + 4;
+  static_assert(kBMaxK / 4 * (XC / 4) <= kBMThreads, "a thread per unit");
   extern __shared__ __align__(16) float msm[];
   const MItem item = items[blockIdx.x];
   if (!state[item.fit].active) return;
   const BFit &F = fits[item.fit];
   const float *__restrict__ X = F.X;
-  const float *__restrict__ R = F.R;
-  const int64_t n = F.n;
   const int d = F.d, K = F.k, tid = threadIdx.x;
-  const int K4 = (K + 3) & ~3, SR = ((kmax + 3) & ~3) + 1, nmt = (K4 / 4) * NQB;
+  const int nc = d / 4 + 1, K4 = (K + 3) & ~3, units = (K4 / 4) * nc, G = kBMThreads / units;
+  const int g = tid / units, unit = tid - g * units, jb = unit / nc, qb = unit - jb * nc;
+  const bool act = g < G;
   const size_t bufsz = means_buf_floats<D>(kmax);
-  const bool grouped = nmt <= kBMThreads;
-  const int UG = grouped ? (nmt + 31) & ~31 : kBMThreads;
-  const int MG = grouped ? kBMThreads / UG : 1;
-  const int g = grouped ? tid / UG : 0;
-  const bool gok = g < MG;
-  int mt[UPT];
-#pragma unroll
-  for (int u = 0; u < UPT; u++) mt[u] = grouped ? (u == 0 ? tid % UG : nmt) : tid + u * kBMThreads;
-  // columns d..D-1 and D+1..D+3 stay zero; posterior columns K..K4-1 too
-  for (size_t e = tid; e < 2 * bufsz; e += kBMThreads) msm[e] = 0.f;
-  __syncthreads();
+  // what the copies leave alone: the ones column d, columns d + 1 .. and the components past K
+  for (int e = tid; e < 2 * TP * (XC - d); e += kBMThreads) {
+    const int row = e / (XC - d), q = d + e - row * (XC - d);
+    msm[(row >= TP ? bufsz : 0) + (row % TP) * XC + q] = q == d ? 1.f : 0.f;
+  }
+  for (int e = tid; e < 2 * (K4 - K) * RP; e += kBMThreads) {
+    const int b = e / ((K4 - K) * RP);
+    msm[b * bufsz + TP * XC + K * RP + (e - b * (K4 - K) * RP)] = 0.f;
+  }
   auto stage = [&](int buf, int t0) {
-    float *sx = msm + buf * bufsz, *sr = sx + TP * XC;
+    float *sx = msm + buf * bufsz;
     const int tp = min(TP, item.p1 - t0);
-    for (int e = tid; e < TP * d; e += kBMThreads) {
-      const int p = e / d, c = e - p * d;
-      cp_async4(sx + p * XC + c, X + (p < tp ? (size_t)(t0 + p) * d + c : 0), p < tp);
+    if ((d & 3) == 0) {
+      const int d4 = d >> 2;
+      for (int e = tid; e < TP * d4; e += kBMThreads) {
+        const int p = e / d4, q = 4 * (e - p * d4);
+        cp_async16z(sx + p * XC + q, X + (p < tp ? (size_t)(t0 + p) * d + q : 0), p < tp ? 16 : 0);
+      }
+    } else {
+      for (int e = tid; e < TP * d; e += kBMThreads) {
+        const int p = e / d, c = e - p * d;
+        cp_async4(sx + p * XC + c, X + (p < tp ? (size_t)(t0 + p) * d + c : 0), p < tp);
+      }
     }
-    for (int e = tid; e < K * TP; e += kBMThreads) {
-      const int j = e / TP, p = e - j * TP;
-      cp_async4(sr + p * SR + j, R + (size_t)j * n + (p < tp ? t0 + p : 0), p < tp);
-    }
-    for (int p = tid; p < TP; p += kBMThreads) sx[p * XC + D] = p < tp ? 1.f : 0.f;
+    stage_posteriors<kBMThreads, TP>(sx + TP * XC, RP, F.R, F.ld, 0, K, t0, tp);
     cp_async_commit();
   };
-  float acc[UPT][4][4];
+  float acc[4][4];
 #pragma unroll
-  for (int u = 0; u < UPT; u++)
+  for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) acc[u][a][b] = 0.f;
+    for (int b = 0; b < 4; b++) acc[a][b] = 0.f;
   stage(0, item.p0);
   int buf = 0;
   for (int t0 = item.p0; t0 < item.p1; t0 += TP, buf ^= 1) {
@@ -356,334 +387,304 @@ k_b_means(const BFit *__restrict__ fits, const BState *__restrict__ state, const
     else cp_async_commit();
     cp_async_wait_prev();
     __syncthreads();
-    const float *sx = msm + buf * bufsz, *sr = sx + TP * XC;
-    if (gok) {
+    if (act) {
+      const float *sx = msm + buf * bufsz + 4 * qb, *sr = msm + buf * bufsz + TP * XC + 4 * jb * RP;
+#pragma unroll 1
+      for (int p = 4 * g; p < TP; p += 4 * G) {
+        float4 r[4];
 #pragma unroll
-      for (int u = 0; u < UPT; u++) {
-        if (mt[u] < nmt) {
-          const int jb = mt[u] / NQB, qb = mt[u] - jb * NQB;
-          for (int p = g; p < TP; p += MG) {
-            const float *rp = sr + p * SR + 4 * jb;
-            const float4 xv = *reinterpret_cast<const float4 *>(sx + p * XC + 4 * qb);
-            const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
+        for (int a = 0; a < 4; a++) r[a] = *reinterpret_cast<const float4 *>(sr + a * RP + p);
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
-              const float r = rp[a];
+        for (int i = 0; i < 4; i++) {
+          const float4 x = *reinterpret_cast<const float4 *>(sx + (p + i) * XC);
 #pragma unroll
-              for (int b = 0; b < 4; b++) acc[u][a][b] = fmaf(r, xs[b], acc[u][a][b]);
-            }
+          for (int a = 0; a < 4; a++) {
+            const float w = i == 0 ? r[a].x : i == 1 ? r[a].y : i == 2 ? r[a].z : r[a].w;
+            acc[a][0] = fmaf(w, x.x, acc[a][0]);
+            acc[a][1] = fmaf(w, x.y, acc[a][1]);
+            acc[a][2] = fmaf(w, x.z, acc[a][2]);
+            acc[a][3] = fmaf(w, x.w, acc[a][3]);
           }
         }
       }
     }
     __syncthreads();
   }
-  if (MG > 1) {
-    // point groups 1.. hand their sums to group 0 (in group order)
-    float *red = msm;
-    if (gok && g > 0 && mt[0] < nmt)
+  cp_async_wait_all();
+  float *red = msm;                                 // 16 x 256, over the tiles
 #pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) red[((g - 1) * UG + mt[0]) * 16 + a * 4 + b] = acc[0][a][b];
-    __syncthreads();
-    if (g == 0 && mt[0] < nmt)
-      for (int gg = 1; gg < MG; gg++)
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++) acc[0][a][b] += red[((gg - 1) * UG + mt[0]) * 16 + a * 4 + b];
-  }
-  if (g != 0) return;
+  for (int e = 0; e < 16; e++) red[e * kBMThreads + tid] = acc[e >> 2][e & 3];
+  __syncthreads();
   double *o = mpart + item.part;
-#pragma unroll
-  for (int u = 0; u < UPT; u++) {
-    if (mt[u] < nmt) {
-      const int jb = mt[u] / NQB, qb = mt[u] - jb * NQB;
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        const int j = 4 * jb + a;
-        if (j < K)
-#pragma unroll
-          for (int b = 0; b < 4; b++) o[(size_t)j * XC + 4 * qb + b] = (double)acc[u][a][b];
-      }
-    }
+  for (int i = tid; i < units * 16; i += kBMThreads) {
+    const int e = i / units, u = i - e * units;
+    const double v = group_sum(red + e * kBMThreads + u, G, units);
+    const int j = 4 * (u / nc) + (e >> 2), q = 4 * (u % nc) + (e & 3);
+    if (j < K && q <= d) o[(size_t)j * XC + (q == d ? D : q)] = v;
   }
 }
 
 // PosteriorSum, Means = MeanSums / PosteriorSum, Probs = PosteriorSum / N
-// (EM2/MatrixEM.cpp:341-343,375) and LogL = sum_i LSE_i, one CTA per fit;
-// partials summed in item order.
-template <int NT>
-__global__ void __launch_bounds__(NT)
-k_b_final_means(const BFit *__restrict__ fits, BState *__restrict__ state, const double *__restrict__ epart,
-                const double *__restrict__ mpart) {
-  __shared__ double red[NT / 32];
-  const int f = blockIdx.x, tid = threadIdx.x;
+// (EM2/MatrixEM.cpp:341-343,375), one CTA per (fit, component), and LogL =
+// sum_i LSE_i in the CTA of component 0.  Lane q holds column q; the warps
+// take every 8th item's partials, combined in a fixed order.  (A CTA per fit
+// with a thread per column walked the items one dependent load after another:
+// 190 us a sweep over 192 fits, here 39.)
+__global__ void __launch_bounds__(256)
+k_b_final_means(const BFit *__restrict__ fits, BState *__restrict__ state, const int2 *__restrict__ comps,
+                const double *__restrict__ epart, const double *__restrict__ mpart) {
+  __shared__ double red[8], sm[8][33];
+  const int f = comps[blockIdx.x].x, j = comps[blockIdx.x].y, tid = threadIdx.x;
   if (!state[f].active) return;
   const BFit &F = fits[f];
-  const int K = F.k, d = F.d, D = F.D, XC = D + 4;
-  double v = 0.0;
-  for (int e = tid; e < F.e_count; e += NT) v += epart[F.e_first + e];
-  const double ll = bblock_sum<NT>(v, red);
-  if (tid == 0) state[f].logl = ll;
-  const double *mp = mpart + F.m_part;
-  const size_t stride = (size_t)K * XC;
-  for (int j = tid; j < K; j += NT) {
-    double s = 0.0;
-    for (int c = 0; c < F.m_count; c++) s += mp[c * stride + (size_t)j * XC + D];
-    F.psum[j] = s;
-    F.pi[j] = s / (double)F.n;
+  const int K = F.k, d = F.d, D = F.D, XC = D + 4, w = tid >> 5, q = tid & 31;
+  if (j == 0) {
+    double v = 0.0;
+    for (int e = tid; e < F.e_count; e += 256) v += epart[F.e_first + e];
+    const double ll = bblock_sum<256>(v, red);
+    if (tid == 0) state[f].logl = ll;
   }
+  const size_t stride = (size_t)K * XC;
+  const double *mp = mpart + F.m_part + (size_t)j * XC;
+  double s = 0.0, ps = 0.0;
+#pragma unroll 4
+  for (int c = w; c < F.m_count; c += 8) {
+    ps += mp[c * stride + D];
+    if (q < d) s += mp[c * stride + q];
+  }
+  sm[w][q] = s;
+  if (q == 0) sm[w][32] = ps;
   __syncthreads();
-  for (int e = tid; e < K * D; e += NT) {
-    const int j = e / D, q = e - j * D;
-    if (q < d) {
-      double s = 0.0;
-      for (int c = 0; c < F.m_count; c++) s += mp[c * stride + (size_t)j * XC + q];
-      const double m = s / F.psum[j];
-      F.mu[(size_t)j * d + q] = m;
-      F.muT[e] = (float)m;
-    } else {
-      F.muT[e] = 0.f;
-    }
+  if (w) return;
+  s = ps = 0.0;
+#pragma unroll
+  for (int c = 0; c < 8; c++) s += sm[c][q], ps += sm[c][32];
+  if (q == 0) {
+    F.psum[j] = ps;
+    F.pi[j] = ps / (double)F.n;
+  }
+  if (q < D) {
+    const double m = s / ps;
+    if (q < d) F.mu[(size_t)j * d + q] = m;
+    F.muT[(size_t)j * D + q] = q < d ? (float)m : 0.f;
   }
 }
 
 // ================================================== M-step: covariances
 // MatrixEMBase::ComputeWeightedTempDataset + BlockCovariances
-// (EM2/MatrixEM.cpp:53-67,90-99) for one item: z = sqrt(r_ij) (x_i - mu_j)
-// around the new means, CovSum_j += z z^T over the upper block triangle.
-// A unit is one TB x TB block of one component; the item's units
-// [u0, u1) take UG = roundup32(u1 - u0) threads and the CTA's 256 / UG
-// point groups split each tile's points.  Per tile of kBCTile points the x
-// rows and sqrt(r) are staged in shared memory (loaded into registers one
-// tile ahead, so the loads overlap the previous tile's work), z is built
-// there for the item's components, then each unit accumulates its block.
-// FP32 sums over the item's points; each (group, unit) writes its TB x TB
-// block as FP64 partials.
-template <int D>
-struct CovGeom {
-  static constexpr int TB = class_tb(D), NB = D / TB, NBLK = class_nblk(D);
-  static constexpr int ZP = D + 4;                                   // z / x row pitch (floats)
-  static constexpr int CJMAX = kBMaxK < 256 / NBLK + 2 ? kBMaxK : 256 / NBLK + 2;
-  static constexpr int ZCS = kBCTile * ZP + 4;                       // z stride per component (bank skew)
-  static constexpr int XT = kBCTile * D;                             // x tile values
-  static constexpr int XPT = (XT + kBCThreads - 1) / kBCThreads;
-  static constexpr int RPT = (CJMAX * kBCTile + kBCThreads - 1) / kBCThreads;
-  // smem floats: mu (CJ x ZP), x tile (TP x ZP), w (CJ x TP), z (CJ x ZCS)
-  static constexpr size_t floats(int cj) {
-    return (size_t)cj * ZP + (size_t)kBCTile * ZP + (((size_t)cj * kBCTile + 3) & ~(size_t)3) + (size_t)cj * ZCS;
-  }
-};
+// (EM2/MatrixEM.cpp:53-67,90-99) for one item of a class above D = 4:
+// CovSum_j += r_ij (x_i - mu_j)(x_i - mu_j)^T over the upper block triangle
+// around the new means.  A unit is one 8 x 8 block of one component; thread t
+// owns unit u0 + t % upc of the item's upc = u1 - u0 units for the points
+// t / upc, t / upc + G, ... of every tile (G = 256 / upc groups), keeps its
+// sums in registers and forms x - mu and r (x - mu) from the staged rows, so a
+// tile costs one barrier and nothing per component passes through shared
+// memory.  Tiles of kBCTile points are copied asynchronously one tile ahead.
+// FP32 sums over the item, the groups' sums added without loss (group_sum); one
+// 8 x 8 FP64 block per unit.  Bound by the FP32 pipe (64 of 88 operations per
+// point and unit are the products; they are issued two columns at a time) with
+// the 16-byte shared-memory loads behind it.  Against a kernel that wrote
+// sqrt(r) (x - mu) of every component to shared memory, took four blocks per
+// dimension for d <= 24 too and left threads idle where the units did not divide
+// by 32 (GB300, a batch of 192 fits of 2000..200000 rows): D = 32 2442 -> 1443 us
+// a sweep; against component owners D = 16 396 -> 226 us, D = 8 282 -> 271.
+constexpr int kBUPitch = kBCThreads + 1;         // element stride of the group reduction
 
-template <int D>
+// position of dimension q in a staged row of nb 8-column blocks: the blocks'
+// first and second 16-byte halves apart, so lanes on neighbouring blocks read
+// neighbouring words
+__device__ __forceinline__ int bu_pos(int q, int nb) { return ((q >> 2) & 1) * (4 * nb) + (q >> 3) * 4 + (q & 3); }
+__host__ __device__ constexpr int bu_xpitch(int nb) { return 8 * nb + 4; }
+
+// floats of shared memory for items of at most cj components
+constexpr size_t bu_floats(int cj) {
+  const size_t tiles = 2 * ((size_t)kBCTile * bu_xpitch(4) + (size_t)cj * (kBCTile + 4)), red = 64 * (size_t)kBUPitch;
+  return tiles > red ? tiles : red;
+}
+
+// a block's columns as four pairs: its 16-byte halves are `half` floats apart
+__device__ __forceinline__ void bu_load(const float *x, int half, uint64_t (&v)[4]) {
+  const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(x);
+  const ulonglong2 hi = *reinterpret_cast<const ulonglong2 *>(x + half);
+  v[0] = lo.x, v[1] = lo.y, v[2] = hi.x, v[3] = hi.y;
+}
+
 __global__ void __launch_bounds__(kBCThreads, 2)
 k_b_cov(const BFit *__restrict__ fits, const BState *__restrict__ state, const CItem *__restrict__ items,
         double *__restrict__ cpart) {
-  using G = CovGeom<D>;
-  constexpr int TB = G::TB, NB = G::NB, NBLK = G::NBLK, ZP = G::ZP, ZCS = G::ZCS, TP = kBCTile;
+  constexpr int TM = kBCTile, RP = TM + 4;
   extern __shared__ __align__(16) float csm[];
   const CItem item = items[blockIdx.x];
   if (!state[item.fit].active) return;
   const BFit &F = fits[item.fit];
   const float *__restrict__ X = F.X;
-  const float *__restrict__ R = F.R;
-  const int64_t n = F.n;
-  const int d = F.d, tid = threadIdx.x;
-  const int nunits = item.u1 - item.u0;
-  const int UG = (nunits + 31) & ~31, NG = kBCThreads / UG;
-  const int ul = tid % UG, g = tid / UG;
-  const bool act = ul < nunits && g < NG;
-  const int j_lo = item.u0 / NBLK, j_hi = (item.u1 - 1) / NBLK, CJ = j_hi - j_lo + 1;
-  float *smu = csm;                                   // CJ x ZP
-  float *sx = smu + (size_t)CJ * ZP;                  // TP x ZP
-  float *sw = sx + (size_t)TP * ZP;                   // CJ x TP
-  float *sZ = sw + (((size_t)CJ * TP + 3) & ~(size_t)3);   // CJ x ZCS
-  int cj = 0, bi = 0, bj = 0;
+  const int d = F.d, D = F.D, tid = threadIdx.x;
+  const int nb = (d + 7) / 8, nblk = nb * (nb + 1) / 2, xp = bu_xpitch(nb);
+  const int upc = item.u1 - item.u0, G = min(TM / 4, kBCThreads / upc);
+  const int TP = TM / (4 * G) * (4 * G);            // points per tile: as many for every group, a multiple of 4
+  const int g = tid / upc, unit = item.u0 + tid - g * upc;
+  const bool act = g < G;
+  const int j_lo = item.u0 / nblk, cj = (item.u1 - 1) / nblk - j_lo + 1;
+  const size_t bufsz = ((size_t)TM * xp + (size_t)cj * RP + 3) & ~(size_t)3;
+  int j = j_lo, bi = 0, bj = 0;
   if (act) {
-    const int unit = item.u0 + ul;
-    const int j = unit / NBLK;
-    int b = unit - j * NBLK;
-    while (b >= NB - bi) {
-      b -= NB - bi;
+    j = unit / nblk;
+    int b = unit - j * nblk;
+    while (b >= nb - bi) {
+      b -= nb - bi;
       bi++;
     }
     bj = bi + b;
-    cj = j - j_lo;
   }
-  for (int e = tid; e < CJ * ZP; e += kBCThreads) {
-    const int jj = e / ZP, q = e - jj * ZP;
-    smu[e] = q < D ? F.muT[(size_t)(j_lo + jj) * D + q] : 0.f;
+  uint64_t ma[4], mb[4];                            // means, zero from column d on
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    ma[a] = reinterpret_cast<const uint64_t *>(F.muT + (size_t)j * D + 8 * bi)[a];
+    mb[a] = reinterpret_cast<const uint64_t *>(F.muT + (size_t)j * D + 8 * bj)[a];
   }
-  // register prefetch of one tile's x values and posteriors
-  float xr[G::XPT], rr[G::RPT];
-  auto fetch = [&](int t0) {
+  uint64_t acc[32];                                 // rows of the block, two columns each
+#pragma unroll
+  for (int e = 0; e < 32; e++) acc[e] = 0;
+  // columns d .. 8 nb - 1 of the staged rows stay zero
+  const int dp = 8 * nb;
+  if (d < dp)
+    for (int e = tid; e < 2 * TM * (dp - d); e += kBCThreads) {
+      const int row = e / (dp - d), q = d + e - row * (dp - d);
+      csm[(row >= TM ? bufsz : 0) + (row % TM) * xp + bu_pos(q, nb)] = 0.f;
+    }
+  auto stage = [&](int buf, int t0) {
+    float *sx = csm + buf * bufsz, *sr = sx + TM * xp;
     const int tp = min(TP, item.p1 - t0);
-#pragma unroll
-    for (int u = 0; u < G::XPT; u++) {
-      const int e = tid + u * kBCThreads, p = e / D, q = e - p * D;
-      xr[u] = (e < G::XT && p < tp && q < d) ? X[(size_t)(t0 + p) * d + q] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < G::RPT; u++) {
-      const int e = tid + u * kBCThreads, jj = e / TP, p = e - jj * TP;
-      rr[u] = (jj < CJ && p < tp) ? R[(size_t)(j_lo + jj) * n + t0 + p] : 0.f;
-    }
-  };
-  fetch(item.p0);
-  float acc[TB][TB];
-#pragma unroll
-  for (int a = 0; a < TB; a++)
-#pragma unroll
-    for (int b = 0; b < TB; b++) acc[a][b] = 0.f;
-  for (int t0 = item.p0; t0 < item.p1; t0 += TP) {
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < G::XPT; u++) {
-      const int e = tid + u * kBCThreads, p = e / D, q = e - p * D;
-      if (e < G::XT) sx[p * ZP + q] = xr[u];
-    }
-#pragma unroll
-    for (int u = 0; u < G::RPT; u++) {
-      const int e = tid + u * kBCThreads;
-      if (e < CJ * TP) sw[e] = sqrtf(rr[u]);
-    }
-    __syncthreads();
-    if (t0 + TP < item.p1) fetch(t0 + TP);
-#pragma unroll 1
-    for (int e = tid; e < CJ * TP * (D / 4); e += kBCThreads) {
-      const int row = e / (D / 4), q4 = e - row * (D / 4);
-      const int jj = row / TP, p = row - jj * TP;
-      const float w = sw[row];
-      const float4 xv = *reinterpret_cast<const float4 *>(sx + p * ZP + 4 * q4);
-      const float4 mv = *reinterpret_cast<const float4 *>(smu + jj * ZP + 4 * q4);
-      float4 z;
-      z.x = w * (xv.x - mv.x);
-      z.y = w * (xv.y - mv.y);
-      z.z = w * (xv.z - mv.z);
-      z.w = w * (xv.w - mv.w);
-      *reinterpret_cast<float4 *>(sZ + (size_t)jj * ZCS + p * ZP + 4 * q4) = z;
-    }
-    __syncthreads();
-    if (act) {
-      const float *zb = sZ + (size_t)cj * ZCS;
-#pragma unroll 1
-      for (int p = g; p < TP; p += NG) {
-        const float *zr = zb + p * ZP;
-        float va[TB], vb[TB];
-#pragma unroll
-        for (int a4 = 0; a4 < TB / 4; a4++) {
-          const float4 u = *reinterpret_cast<const float4 *>(zr + bi * TB + 4 * a4);
-          const float4 v = *reinterpret_cast<const float4 *>(zr + bj * TB + 4 * a4);
-          va[4 * a4 + 0] = u.x, va[4 * a4 + 1] = u.y, va[4 * a4 + 2] = u.z, va[4 * a4 + 3] = u.w;
-          vb[4 * a4 + 0] = v.x, vb[4 * a4 + 1] = v.y, vb[4 * a4 + 2] = v.z, vb[4 * a4 + 3] = v.w;
-        }
-#pragma unroll
-        for (int a = 0; a < TB; a++)
-#pragma unroll
-          for (int b = 0; b < TB; b++) acc[a][b] = fmaf(va[a], vb[b], acc[a][b]);
+    if ((d & 3) == 0) {
+      const int d4 = d >> 2;
+      for (int e = tid; e < tp * d4; e += kBCThreads) {
+        const int p = e / d4, q = 4 * (e - p * d4);
+        cp_async16(sx + p * xp + bu_pos(q, nb), X + (size_t)(t0 + p) * d + q);
+      }
+    } else {
+      for (int e = tid; e < tp * d; e += kBCThreads) {
+        const int p = e / d, q = e - p * d;
+        cp_async4(sx + p * xp + bu_pos(q, nb), X + (size_t)(t0 + p) * d + q, true);
       }
     }
+    stage_posteriors<kBCThreads, TM>(sr, RP, F.R, F.ld, j_lo, cj, t0, tp);
+    cp_async_commit();
+  };
+  stage(0, item.p0);
+  int buf = 0;
+  for (int t0 = item.p0; t0 < item.p1; t0 += TP, buf ^= 1) {
+    if (t0 + TP < item.p1) stage(buf ^ 1, t0 + TP);
+    else cp_async_commit();
+    cp_async_wait_prev();
+    __syncthreads();
+    const float *sx = csm + buf * bufsz, *sr = sx + TM * xp + (j - j_lo) * RP;
+    if (act) {
+      const int live = min(TP, item.p1 - t0);
+      const float *xa = sx + g * xp + 4 * bi, *xb = sx + g * xp + 4 * bj, *pr = sr + g;
+      const int xs = G * xp;
+#pragma unroll 1
+      for (int p = g; p < live; p += G, xa += xs, xb += xs, pr += G) {
+        const float r = *pr;
+        uint64_t ua[4], ub[4];
+        bu_load(xa, 4 * nb, ua);
+        bu_load(xb, 4 * nb, ub);
+#pragma unroll
+        for (int a = 0; a < 4; a++) ua[a] = f2_sub(ua[a], ma[a]), ub[a] = f2_sub(ub[a], mb[a]);
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          float u0, u1;
+          f2_unpack(ua[a], u0, u1);
+          const float w0 = r * u0, w1 = r * u1;
+          const uint64_t ww0 = f2_pack(w0, w0), ww1 = f2_pack(w1, w1);
+#pragma unroll
+          for (int b = 0; b < 4; b++) {
+            acc[8 * a + b] = f2_fma(ww0, ub[b], acc[8 * a + b]);
+            acc[8 * a + 4 + b] = f2_fma(ww1, ub[b], acc[8 * a + 4 + b]);
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
-  if (act) {
-    double *o = cpart + item.part + ((size_t)g * nunits + ul) * (TB * TB);
+  cp_async_wait_all();
 #pragma unroll
-    for (int a = 0; a < TB; a++)
-#pragma unroll
-      for (int b = 0; b < TB; b++) o[a * TB + b] = (double)acc[a][b];
+  for (int e = 0; e < 32; e++) f2_unpack(acc[e], csm[2 * e * kBUPitch + tid], csm[(2 * e + 1) * kBUPitch + tid]);
+  __syncthreads();
+  double *o = cpart + item.part;
+  for (int i = tid; i < upc * 64; i += kBCThreads) {
+    o[i] = group_sum(csm + (i & 63) * kBUPitch + (i >> 6), G, upc);
   }
 }
 
-// Partial geometry of covariance unit range `ug` of a fit with k components
-// in class D: units [u0, u1), ng point groups, per doubles per unit; the
-// range's partials are ng x (u1 - u0) x per doubles.  Block layout (D = 32):
-// a unit is one TB x TB block of one component, ranges of <= 256 units.
-// Owner layout (D <= 16): one range whose units are the k components, each
-// owned by own_S(D) threads of own_NE(D) sums.
-__host__ __device__ inline void unit_range(int k, int D, int ug, int *u0, int *u1, int *ng, int *per) {
+// Partial geometry of covariance unit range `ug` of `nug` of a fit with k
+// components of d columns in class D: units [u0, u1), ng point groups, per
+// doubles per unit; the range's partials are ng x (u1 - u0) x per doubles.
+// Block layout (D > 4): a unit is one 8 x 8 block of one component, nug equal
+// ranges (split_units).  Owner layout (D = 4): one range whose units are the k
+// components.
+__host__ __device__ inline int cov_blocks(int d) {
+  const int nb = (d + 7) / 8;
+  return nb * (nb + 1) / 2;
+}
+__host__ __device__ inline void unit_range(int k, int d, int D, int ug, int nug, int *u0, int *u1, int *ng, int *per) {
+  *ng = 1;
   if (class_owner(D)) {
     *u0 = 0;
     *u1 = k;
-    *ng = 256 / (own_S(D) * ((k + 31) & ~31));
-    *per = own_S(D) * own_NE(D);
+    *per = kOwnNE;
     return;
   }
-  const int total = k * class_nblk(D);
-  *u0 = ug * 256;
-  *u1 = min(total, *u0 + 256);
-  const int UG = (*u1 - *u0 + 31) & ~31;
-  *ng = 256 / UG;
-  *per = class_tb(D) * class_tb(D);
+  const int total = k * cov_blocks(d), each = (total + nug - 1) / nug;
+  *u0 = min(total, ug * each);
+  *u1 = min(total, *u0 + each);
+  *per = 64;
 }
 
-// one point's contribution r u u^T to the sums of row pairs I.. of the
-// thread set SS: pair q covers rows q (columns q..D-1) and D-1-q (columns
-// D-1-q..D-1), D + 1 sums; compile-time recursion keeps every index constant
-template <int D, int SS, int I>
-__device__ __forceinline__ void own_pairs_acc(const float (&u)[D], float r, float (&acc)[own_NE(D)]) {
-  constexpr int S = own_S(D), q = SS + S * I, q2 = D - 1 - q, base = I * (D + 1);
-  const float ra = r * u[q], rb = r * u[q2];
-#pragma unroll
-  for (int c = q; c < D; c++) acc[base + c - q] = fmaf(ra, u[c], acc[base + c - q]);
-#pragma unroll
-  for (int c = q2; c < D; c++) acc[base + (D - q) + c - q2] = fmaf(rb, u[c], acc[base + (D - q) + c - q2]);
-  if constexpr (I + 1 < own_pairs(D)) own_pairs_acc<D, SS, I + 1>(u, r, acc);
-}
-
-// shared memory of k_b_cov_own<D> for classes with at most kmax components:
-// two buffers of (TP x D rows, kmax x (TP + 1) posteriors); the odd row
-// stride keeps the lanes of a warp (consecutive components, one point) in
-// different banks
-__host__ __device__ constexpr size_t own_buf_floats(int D, int kmax) {
-  return ((size_t)own_TP(D) * D + (size_t)kmax * (own_TP(D) + 1) + 3) & ~(size_t)3;
-}
+// shared memory of k_b_cov_own for classes with at most kmax components: two
+// buffers of (TP x 4 rows, kmax x (TP + 4) posteriors), at least the groups' sums
+constexpr size_t own_buf_floats(int kmax) { return (size_t)kOwnTP * kOwnD + (size_t)kmax * (kOwnTP + 4); }
 
 // MatrixEMBase::ComputeWeightedTempDataset + BlockCovariances
-// (EM2/MatrixEM.cpp:53-67,90-99) for D <= 16: CovSum_j += r_ij u u^T with
-// u = x_i - mu_j formed on the fly from a staged tile of rows.  A component
-// is owned by own_S(D) threads (a warp-uniform split of its row pairs), the
-// CTA's 256 / (own_S roundup32(k)) point groups split each tile's points.
-// Tiles are copied asynchronously one tile ahead into two shared buffers.
-// FP32 sums over the item; partials [group][thread set][component][own_NE]
-// in FP64.
-template <int D>
-__global__ void __launch_bounds__(kBCThreads, D >= 16 ? 1 : 2)
+// (EM2/MatrixEM.cpp:53-67,90-99) for d <= 4: CovSum_j += r_ij u u^T with
+// u = x_i - mu_j formed on the fly from a staged tile of rows.  Thread t owns
+// component t % k for every G-th group of four points (G = 256 / k).  Tiles are
+// copied asynchronously one tile ahead into two shared buffers.  FP32 sums over
+// the item, the groups' sums by group_sum.  With 32 lanes for any k <= 32 and
+// 4-byte copies a sweep over 40 fits took 111 us, here 76.
+__global__ void __launch_bounds__(kBCThreads, 2)
 k_b_cov_own(const BFit *__restrict__ fits, const BState *__restrict__ state, const CItem *__restrict__ items,
             double *__restrict__ cpart, int kmax) {
-  constexpr int S = own_S(D), NE = own_NE(D), TP = own_TP(D);
+  constexpr int D = kOwnD, NE = kOwnNE, TP = kOwnTP, RP = TP + 4;
   extern __shared__ __align__(16) float osm[];
   const CItem item = items[blockIdx.x];
   if (!state[item.fit].active) return;
   const BFit &F = fits[item.fit];
   const float *__restrict__ X = F.X;
-  const float *__restrict__ R = F.R;
-  const int64_t n = F.n;
   const int d = F.d, K = F.k, tid = threadIdx.x;
-  const int KG = (K + 31) & ~31, UG = S * KG, NG = kBCThreads / UG;
-  const int ul = tid % UG, g = tid / UG, ts = ul / KG, j = ul - ts * KG;
-  const bool act = j < K && g < NG;
-  const size_t bufsz = own_buf_floats(D, kmax);
+  const int G = kBCThreads / K, g = tid / K, j = tid - g * K;
+  const bool act = g < G;
+  const size_t bufsz = own_buf_floats(kmax);
   float mu[D];
 #pragma unroll
-  for (int q = 0; q < D; q++) mu[q] = act ? F.muT[(size_t)j * D + q] : 0.f;
+  for (int q = 0; q < D; q++) mu[q] = F.muT[(size_t)j * D + q];
   float acc[NE];
 #pragma unroll
   for (int e = 0; e < NE; e++) acc[e] = 0.f;
-  // one tile of rows (TP x D, zero past d and past the item) and posteriors (K x TP)
+  // one tile of rows (TP x 4, zero past d and past the item) and posteriors (K x TP)
   auto stage = [&](int buf, int t0) {
-    float *sx = osm + buf * bufsz, *sr = sx + TP * D;
+    float *sx = osm + buf * bufsz;
     const int tp = min(TP, item.p1 - t0);
-    for (int e = tid; e < TP * D; e += kBCThreads) {
-      const int p = e / D, q = e - p * D;
-      const bool v = p < tp && q < d;
-      cp_async4(sx + e, X + (v ? (size_t)(t0 + p) * d + q : 0), v);
+    if (d == D) {
+      for (int p = tid; p < TP; p += kBCThreads)
+        cp_async16z(sx + 4 * p, X + (p < tp ? (size_t)(t0 + p) * D : 0), p < tp ? 16 : 0);
+    } else {
+      for (int e = tid; e < TP * D; e += kBCThreads) {
+        const int p = e / D, q = e - p * D;
+        const bool v = p < tp && q < d;
+        cp_async4(sx + e, X + (v ? (size_t)(t0 + p) * d + q : 0), v);
+      }
     }
-    for (int e = tid; e < K * TP; e += kBCThreads) {
-      const int jj = e / TP, p = e - jj * TP;
-      const bool v = p < tp;
-      cp_async4(sr + jj * (TP + 1) + p, R + (size_t)jj * n + (v ? t0 + p : 0), v);
-    }
+    stage_posteriors<kBCThreads, TP>(sx + TP * D, RP, F.R, F.ld, 0, K, t0, tp);
     cp_async_commit();
   };
   stage(0, item.p0);
@@ -693,34 +694,36 @@ k_b_cov_own(const BFit *__restrict__ fits, const BState *__restrict__ state, con
     else cp_async_commit();                 // an empty group keeps the wait count uniform
     cp_async_wait_prev();
     __syncthreads();
-    const float *sx = osm + buf * bufsz, *sr = sx + TP * D;
-    const int tp = min(TP, item.p1 - t0);
+    const float *sx = osm + buf * bufsz, *sr = sx + TP * D + j * RP;
     if (act) {
-      for (int p = g; p < tp; p += NG) {
-        const float r = sr[j * (TP + 1) + p];
-        float u[D];
+#pragma unroll 1
+      for (int p = 4 * g; p < TP; p += 4 * G) {
+        const float4 r4 = *reinterpret_cast<const float4 *>(sr + p);
 #pragma unroll
-        for (int q4 = 0; q4 < D / 4; q4++) {
-          const float4 xv = *reinterpret_cast<const float4 *>(sx + p * D + 4 * q4);
-          u[4 * q4 + 0] = xv.x - mu[4 * q4 + 0];
-          u[4 * q4 + 1] = xv.y - mu[4 * q4 + 1];
-          u[4 * q4 + 2] = xv.z - mu[4 * q4 + 2];
-          u[4 * q4 + 3] = xv.w - mu[4 * q4 + 3];
-        }
-        if constexpr (S == 1) {
-          own_pairs_acc<D, 0, 0>(u, r, acc);
-        } else {
-          if (ts == 0) own_pairs_acc<D, 0, 0>(u, r, acc);
-          else own_pairs_acc<D, 1, 0>(u, r, acc);
+        for (int i = 0; i < 4; i++) {
+          const float r = i == 0 ? r4.x : i == 1 ? r4.y : i == 2 ? r4.z : r4.w;
+          const float4 x = *reinterpret_cast<const float4 *>(sx + 4 * (p + i));
+          const float u[D] = {x.x - mu[0], x.y - mu[1], x.z - mu[2], x.w - mu[3]};
+          int e = 0;
+#pragma unroll
+          for (int a = 0; a < D; a++) {
+            const float w = r * u[a];
+#pragma unroll
+            for (int c = a; c < D; c++) acc[e] = fmaf(w, u[c], acc[e]), e++;
+          }
         }
       }
     }
     __syncthreads();
   }
-  if (act) {
-    double *o = cpart + item.part + ((size_t)(g * S + ts) * K + j) * NE;
+  cp_async_wait_all();
 #pragma unroll
-    for (int e = 0; e < NE; e++) o[e] = (double)acc[e];
+  for (int e = 0; e < NE; e++) osm[e * kBUPitch + tid] = acc[e];
+  __syncthreads();
+  double *o = cpart + item.part;
+  for (int i = tid; i < K * NE; i += kBCThreads) {
+    const int jj = i / NE, e = i - jj * NE;
+    o[i] = group_sum(osm + e * kBUPitch + jj, G, K);
   }
 }
 
@@ -743,56 +746,39 @@ k_b_factor(const BFit *__restrict__ fits, BState *__restrict__ state, const int2
   const int f = fc.x, j = fc.y, tid = threadIdx.x;
   if (!state[f].active) return;
   const BFit &F = fits[f];
-  const int d = F.d, D = F.D, K = F.k;
+  const int d = F.d, D = F.D;
   double *S = F.sigma + (size_t)j * d * d;
   if (reduce) {
     const double inv = 1.0 / F.psum[j];
     if (class_owner(D)) {
-      const int Sd = own_S(D), NE = own_NE(D);
-      int u0 = 0, u1 = 0, ng = 0, per = 0;
-      unit_range(K, D, 0, &u0, &u1, &ng, &per);
+      // row a of the upper triangle of 4 x 4: 4 - a sums
+      const double *pj = cpart + F.c_part + (size_t)j * kOwnNE;
       for (int e = tid; e < d * d; e += kBFThreads) {
         const int a = e / d, c = e - a * d;
         if (a > c) continue;
-        const bool first = a < D / 2;
-        const int q = first ? a : D - 1 - a;
-        const int ts = q % Sd, i = q / Sd;
-        const int w = i * (D + 1) + (first ? c - a : (D - q) + (c - a));
+        const int w = a * kOwnD - a * (a - 1) / 2 + c - a;
         double s2 = 0.0;
-        for (int ch = 0; ch < F.c_chunks; ch++) {
-          const double *pp = cpart + F.c_part + ch * F.c_stride + ((size_t)ts * K + j) * NE + w;
-          for (int gg = 0; gg < ng; gg++) s2 += pp[(size_t)gg * Sd * K * NE];
-        }
+#pragma unroll 8
+        for (int ch = 0; ch < F.c_chunks; ch++) s2 += pj[ch * F.c_stride + w];
         s2 *= inv;
         S[(size_t)a * d + c] = s2;
         S[(size_t)c * d + a] = s2;
       }
     } else {
-      const int TB = class_tb(D), NB = D / TB, NBLK = class_nblk(D), per = TB * TB;
-      for (int e = tid; e < NBLK * per; e += kBFThreads) {
-        const int b = e / per, w = e - b * per;
-        int bi = 0, bb = b;
-        while (bb >= NB - bi) {
-          bb -= NB - bi;
+      // the ranges' partials of a chunk follow one another: unit-major over the whole fit
+      const int nb = (d + 7) / 8, nblk = cov_blocks(d);
+      const double *pj = cpart + F.c_part + (size_t)j * nblk * 64;
+      for (int e = tid; e < nblk * 64; e += kBFThreads) {
+        int bi = 0, bb = e >> 6;
+        while (bb >= nb - bi) {
+          bb -= nb - bi;
           bi++;
         }
-        const int bj = bi + bb;
-        const int a = bi * TB + w / TB, c = bj * TB + (w % TB);
+        const int a = bi * 8 + ((e >> 3) & 7), c = (bi + bb) * 8 + (e & 7);
         if (a > c || c >= d) continue;
-        const int unit = j * NBLK + b, ug = unit / 256, ul = unit - ug * 256;
-        int64_t off = 0;
-        int u0 = 0, u1 = 0, ng = 0, pr = 0;
-        for (int q = 0; q < ug; q++) {
-          unit_range(K, D, q, &u0, &u1, &ng, &pr);
-          off += (int64_t)ng * (u1 - u0) * pr;
-        }
-        unit_range(K, D, ug, &u0, &u1, &ng, &pr);
-        const int nu = u1 - u0;
         double s2 = 0.0;
-        for (int ch = 0; ch < F.c_chunks; ch++) {
-          const double *pp = cpart + F.c_part + ch * F.c_stride + off + (size_t)ul * per + w;
-          for (int gg = 0; gg < ng; gg++) s2 += pp[(size_t)gg * nu * per];
-        }
+#pragma unroll 8
+        for (int ch = 0; ch < F.c_chunks; ch++) s2 += pj[ch * F.c_stride + e];
         s2 *= inv;
         S[(size_t)a * d + c] = s2;
         S[(size_t)c * d + a] = s2;
@@ -1114,7 +1100,7 @@ k_bt_estep(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
             }
             if (j < K) {
               const float l = (chi[(size_t)(F.wg + g) * 4 + q] - 0.5f * (s0 + s1)) + clo[(size_t)(F.wg + g) * 4 + q];
-              if (valid) F.R[(size_t)j * n + i] = l;
+              if (valid) F.R[(size_t)j * F.ld + i] = l;
               lse_add(l, mx, se);
             }
           }
@@ -1123,7 +1109,7 @@ k_bt_estep(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
         const float lse = mx + logf(se);
         if (valid) {
           lsum += (double)lse;
-          for (int j = 0; j < K; j++) F.R[(size_t)j * n + i] = expf(F.R[(size_t)j * n + i] - lse);
+          for (int j = 0; j < K; j++) F.R[(size_t)j * F.ld + i] = expf(F.R[(size_t)j * F.ld + i] - lse);
         }
       }
       // the item's LogL partial, summed in a fixed order over the 4 warps
@@ -1338,7 +1324,7 @@ int launch_sweep(fem_em_batch *b, int it, int svd, int slot) {
     b->launches++;
     mark(b, slot, 5 + c);
   }
-  k_b_final_means<128><<<b->nfits, 128, 0, b->stream>>>(fits, st, b->epart, b->mpart);
+  k_b_final_means<<<b->ncomps, 256, 0, b->stream>>>(fits, st, b->comps, b->epart, b->mpart);
   FEM_CUDA(cudaGetLastError());
   b->launches++;
   mark(b, slot, 9);
@@ -1351,10 +1337,8 @@ int launch_sweep(fem_em_batch *b, int it, int svd, int slot) {
     const CItem *it0 = b->citems + b->c_beg[c];
     const size_t sm = b->c_smem[c];
     switch (c) {
-      case 0: k_b_cov_own<4><<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart, b->c_kmax[c]); break;
-      case 1: k_b_cov_own<8><<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart, b->c_kmax[c]); break;
-      case 2: k_b_cov_own<16><<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart, b->c_kmax[c]); break;
-      default: k_b_cov<32><<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart); break;
+      case 0: k_b_cov_own<<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart, b->c_kmax[c]); break;
+      default: k_b_cov<<<cnt, kBCThreads, sm, b->stream>>>(fits, st, it0, b->cpart); break;
     }
     FEM_CUDA(cudaGetLastError());
     b->launches++;
@@ -1456,7 +1440,7 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     const int D = class_dim(class_of(d[f]));
     ox[f] = nx, orr[f] = nr, ok_[f] = nk, okd[f] = nkd, okdd[f] = nkdd, okD[f] = nkD, okT[f] = nkT;
     nx += (n[f] * d[f] + 3) & ~(int64_t)3;
-    nr += n[f] * k[f];
+    nr += ((n[f] + 3) & ~(int64_t)3) * k[f];
     nk += k[f];
     nkd += (int64_t)k[f] * d[f];
     nkdd += (int64_t)k[f] * d[f] * d[f];
@@ -1480,6 +1464,7 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     F.X = b->X + ox[f];
     F.R = b->R + orr[f];
     F.n = n[f];
+    F.ld = (n[f] + 3) & ~(int64_t)3;
     F.d = d[f];
     F.k = k[f];
     F.D = class_dim(class_of(d[f]));
@@ -1524,12 +1509,16 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
         mp += (int64_t)F.k * (F.D + 4);
       }
       F.m_count = (int)mi.size() - F.m_first;
-      F.nug = class_owner(F.D) ? 1 : (F.k * class_nblk(F.D) + 255) / 256;
+      F.nug = 1;
+      if (!class_owner(F.D)) {
+        int upc, G;
+        split_units(F.k * cov_blocks(F.d), &F.nug, &upc, &G);
+      }
       F.c_part = cp;
       F.c_stride = 0;
       for (int ug = 0; ug < F.nug; ug++) {
         int u0, u1, ng, per;
-        unit_range(F.k, F.D, ug, &u0, &u1, &ng, &per);
+        unit_range(F.k, F.d, F.D, ug, F.nug, &u0, &u1, &ng, &per);
         F.c_stride += (int64_t)ng * (u1 - u0) * per;
       }
       F.c_chunks = 0;
@@ -1537,7 +1526,7 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
         int64_t off = cp;
         for (int ug = 0; ug < F.nug; ug++) {
           int u0, u1, ng, per;
-          unit_range(F.k, F.D, ug, &u0, &u1, &ng, &per);
+          unit_range(F.k, F.d, F.D, ug, F.nug, &u0, &u1, &ng, &per);
           ci.push_back(CItem{f, (int)p, (int)std::min<int64_t>(F.n, p + cch), u0, u1, off});
           off += (int64_t)ng * (u1 - u0) * per;
         }
@@ -1545,8 +1534,8 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
         F.c_chunks++;
       }
     }
-    const int D = class_dim(c), nblk = class_nblk(D);
-    const int cj = std::max(1, std::min(kmax, 256 / nblk + 2));
+    const int D = class_dim(c);
+    const int cj = std::max(1, std::min(kmax, 256 / cov_blocks(D / 2 + 1) + 2));   // components an item's units touch
     b->c_kmax[c] = std::max(kmax, 1);
     {
       size_t mf = 0;
@@ -1556,10 +1545,11 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
         case 2: mf = means_buf_floats<16>(b->c_kmax[c]); break;
         default: mf = means_buf_floats<32>(b->c_kmax[c]); break;
       }
-      // two tile buffers; the point-group reduction reuses them (<= 128 x 16 floats)
+      // two tile buffers; the point-group reduction reuses them
       b->m_smem[c] = std::max<size_t>(2 * mf, (size_t)kBMThreads * 16) * sizeof(float);
     }
-    b->c_smem[c] = (class_owner(D) ? 2 * own_buf_floats(D, b->c_kmax[c]) : CovGeom<32>::floats(cj)) * sizeof(float);
+    b->c_smem[c] = (class_owner(D) ? std::max(2 * own_buf_floats(b->c_kmax[c]), (size_t)kOwnNE * kBUPitch) : bu_floats(cj)) *
+                   sizeof(float);
   }
   b->e_beg[kClasses] = (int)ei.size();
   b->m_beg[kClasses] = (int)mi.size();
@@ -1618,10 +1608,8 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
       allow_dyn_smem(k_b_means<8>, b->m_smem[1]) != cudaSuccess ||
       allow_dyn_smem(k_b_means<16>, b->m_smem[2]) != cudaSuccess ||
       allow_dyn_smem(k_b_means<32>, b->m_smem[3]) != cudaSuccess ||
-      allow_dyn_smem(k_b_cov_own<4>, b->c_smem[0]) != cudaSuccess ||
-      allow_dyn_smem(k_b_cov_own<8>, b->c_smem[1]) != cudaSuccess ||
-      allow_dyn_smem(k_b_cov_own<16>, b->c_smem[2]) != cudaSuccess ||
-      allow_dyn_smem(k_b_cov<32>, b->c_smem[3]) != cudaSuccess) {
+      allow_dyn_smem(k_b_cov_own, b->c_smem[0]) != cudaSuccess ||
+      allow_dyn_smem(k_b_cov, std::max({b->c_smem[1], b->c_smem[2], b->c_smem[3]})) != cudaSuccess) {
     set_error("batched kernels' shared-memory limits could not be raised");
     return fail(FEM_ERR_CUDA);
   }

@@ -490,6 +490,8 @@ k_means_units(const float *__restrict__ X, int64_t n, int d, int K, PostTyped<T>
   }
 }
 
+}  // namespace
+
 // gx CTAs of upc units with G point groups each: the split of at most 8 more
 // CTAs than needed that leaves the fewest of the threads without a unit (600
 // units on 3 x 200 threads would idle 22 %; 5 x 120 with two groups idle 6 %)
@@ -503,8 +505,6 @@ void split_units(int units, int *gx, int *upc, int *G) {
     if (eff > best) best = eff, *gx = ctas, *upc = u, *G = g;
   }
 }
-
-}  // namespace
 
 // row chunks: the count whose waves over `slots` resident CTAs finish first,
 // counting `extra` tiles' time for a CTA's start and end

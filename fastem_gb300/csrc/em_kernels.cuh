@@ -21,6 +21,8 @@ int em_tc_upload(fem_em *h);    // X -> bf16 hi/lo split
 int em_tc_prepare(fem_em *h);   // factors -> permuted bf16 hi/lo operands + offsets
 int em_tc_estep(fem_em *h);
 int em_tc_mstep(fem_em *h);
+// gx CTAs of upc <= 256 units with G point groups each (em_cov.cu)
+void split_units(int units, int *gx, int *upc, int *G);
 // row chunks of a grid gx x chunks over n rows in tiles of TP (em_cov.cu)
 void split_rows(int64_t n, int TP, int gx, int slots, double extra, int *chunks, int64_t *rows);
 // em_cov.cu: CUDA-core means sums (partials only), covariance sums and their finalisation

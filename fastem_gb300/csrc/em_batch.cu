@@ -59,6 +59,7 @@ constexpr int kBCChunk = 4096;   // points per covariance item
 constexpr int kBMTile = 128;     // points staged per means tile
 constexpr int kBCTile = 128;     // points staged per covariance tile
 constexpr int kBatchSyncEvery = 8;
+constexpr size_t kStageDoubles = (size_t)1 << 19;   // parameter staging ring (4 MB)
 constexpr int kTimeMarks = 15;   // timing events per sweep (see collect_timing)
 constexpr int kClasses = 4;      // D = 4, 8, 16, 32
 
@@ -81,7 +82,8 @@ struct BFit {
   int c_chunks;          // covariance chunks (items = c_chunks x nug)
   int64_t c_part;        // first covariance partial; chunk stride c_stride
   int64_t c_stride;
-  double *pi, *mu, *sigma, *psum, *logc;   // k, k d, k d d, k, k
+  double *pi, *mu, *sigma;                 // k, k d, k d d: one block in this order
+  double *psum, *logc;                     // k, k
   float *muT, *WT, *logcT;                 // k D, k tri(D), k
   int64_t xrow;          // mixed form, d <= 32 class: first row in the FP16 split copies (-1: none)
   int wg;                // first 4-component W group of the tensor-core E-step
@@ -748,6 +750,9 @@ k_b_factor(const BFit *__restrict__ fits, BState *__restrict__ state, const int2
   const BFit &F = fits[f];
   const int d = F.d, D = F.D;
   double *S = F.sigma + (size_t)j * d * d;
+  if (!reduce)                                      // the start's means, which came from the host in FP64
+    for (int q = tid; q < D; q += kBFThreads)
+      F.muT[(size_t)j * D + q] = q < d ? (float)F.mu[(size_t)j * d + q] : 0.f;
   if (reduce) {
     const double inv = 1.0 / F.psum[j];
     if (class_owner(D)) {
@@ -1143,10 +1148,12 @@ struct fem_em_batch {
   BFit *fits = nullptr;
   BState *state = nullptr;
   float *X = nullptr, *R = nullptr, *muT = nullptr, *WT = nullptr, *logcT = nullptr;
-  double *pi = nullptr, *mu = nullptr, *sigma = nullptr, *psum = nullptr, *logc = nullptr;
+  double *params = nullptr, *psum = nullptr, *logc = nullptr;
   double *epart = nullptr, *mpart = nullptr, *cpart = nullptr;
   double *trace = nullptr, *etrace = nullptr;
   int *nactive = nullptr, *hnactive = nullptr;   // device / pinned host
+  double *stage = nullptr;          // pinned staging ring of the parameters (doubles)
+  size_t stage_n = 0, stage_at = 0;
   EItem *eitems = nullptr;
   MItem *mitems = nullptr;
   CItem *citems = nullptr;
@@ -1204,9 +1211,8 @@ void free_batch(fem_em_batch *b) {
   dfree(b->muT);
   dfree(b->WT);
   dfree(b->logcT);
-  dfree(b->pi);
-  dfree(b->mu);
-  dfree(b->sigma);
+  dfree(b->params);
+  if (b->stage) cudaFreeHost(b->stage);
   dfree(b->psum);
   dfree(b->logc);
   dfree(b->epart);
@@ -1448,9 +1454,8 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     nkT += (int64_t)k[f] * tri_off(D);
   }
   if ((st = dalloc(&b->X, nx)) || (st = dalloc(&b->R, nr)) || (st = dalloc(&b->muT, nkD)) ||
-      (st = dalloc(&b->WT, nkT)) || (st = dalloc(&b->logcT, nk)) || (st = dalloc(&b->pi, nk)) ||
-      (st = dalloc(&b->mu, nkd)) || (st = dalloc(&b->sigma, nkdd)) || (st = dalloc(&b->psum, nk)) ||
-      (st = dalloc(&b->logc, nk)))
+      (st = dalloc(&b->WT, nkT)) || (st = dalloc(&b->logcT, nk)) || (st = dalloc(&b->params, nk + nkd + nkdd)) ||
+      (st = dalloc(&b->psum, nk)) || (st = dalloc(&b->logc, nk)))
     return fail(st);
   // work items, grouped by dimension class
   std::vector<EItem> ei;
@@ -1468,9 +1473,9 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     F.d = d[f];
     F.k = k[f];
     F.D = class_dim(class_of(d[f]));
-    F.pi = b->pi + ok_[f];
-    F.mu = b->mu + okd[f];
-    F.sigma = b->sigma + okdd[f];
+    F.pi = b->params + ok_[f] + okd[f] + okdd[f];
+    F.mu = F.pi + k[f];
+    F.sigma = F.mu + (int64_t)k[f] * d[f];
     F.psum = b->psum + ok_[f];
     F.logc = b->logc + ok_[f];
     F.muT = b->muT + okD[f];
@@ -1586,7 +1591,10 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
       return fail(FEM_ERR_CUDA);
     }
   }
-  if (cudaMallocHost((void **)&b->hnactive, sizeof(int)) != cudaSuccess) {
+  b->stage_n = kStageDoubles;
+  for (int f = 0; f < nfits; f++) b->stage_n = std::max(b->stage_n, (size_t)k[f] * (1 + d[f] + d[f] * d[f]));
+  if (cudaMallocHost((void **)&b->stage, b->stage_n * sizeof(double)) != cudaSuccess ||
+      cudaMallocHost((void **)&b->hnactive, sizeof(int)) != cudaSuccess) {
     set_error("pinned allocation failed");
     return fail(FEM_ERR_CUDA);
   }
@@ -1660,6 +1668,20 @@ extern "C" int fem_em_batch_upload_packed(fem_em_batch *b, const float *X) {
   return FEM_OK;
 }
 
+// n doubles of the pinned staging ring: parameters go in and out in one copy per
+// fit, and a copy in need not have finished when the call returns (192 fits:
+// 27 us a call with three or four waited-for pageable copies).  Wrapping around
+// waits for the copies in flight.
+static int stage_params(fem_em_batch *b, size_t n, double **h) {
+  if (b->stage_at + n > b->stage_n) {
+    FEM_CUDA(cudaStreamSynchronize(b->stream));
+    b->stage_at = 0;
+  }
+  *h = b->stage + b->stage_at;
+  b->stage_at += n;
+  return FEM_OK;
+}
+
 extern "C" int fem_em_batch_set_params(fem_em_batch *b, int fit, const double *pi, const double *mu,
                                        const double *sigma) {
   FEM_TRY(check_fit(b, fit));
@@ -1668,16 +1690,14 @@ extern "C" int fem_em_batch_set_params(fem_em_batch *b, int fit, const double *p
     return FEM_ERR_BAD_ARG;
   }
   const BFit &F = b->hfits[fit];
-  const int k = F.k, d = F.d, D = F.D;
-  std::vector<float> muT((size_t)k * D, 0.f);
-  for (int j = 0; j < k; j++)
-    for (int q = 0; q < d; q++) muT[(size_t)j * D + q] = (float)mu[(size_t)j * d + q];
+  const size_t nk = F.k, nm = nk * F.d, ns = nm * F.d;
   FEM_CUDA(cudaSetDevice(b->cfg.device));
-  FEM_CUDA(cudaMemcpyAsync(F.pi, pi, (size_t)k * sizeof(double), cudaMemcpyHostToDevice, b->stream));
-  FEM_CUDA(cudaMemcpyAsync(F.mu, mu, (size_t)k * d * sizeof(double), cudaMemcpyHostToDevice, b->stream));
-  FEM_CUDA(cudaMemcpyAsync(F.sigma, sigma, (size_t)k * d * d * sizeof(double), cudaMemcpyHostToDevice, b->stream));
-  FEM_CUDA(cudaMemcpyAsync(F.muT, muT.data(), muT.size() * sizeof(float), cudaMemcpyHostToDevice, b->stream));
-  FEM_CUDA(cudaStreamSynchronize(b->stream));
+  double *h = nullptr;
+  FEM_TRY(stage_params(b, nk + nm + ns, &h));
+  memcpy(h, pi, nk * sizeof(double));
+  memcpy(h + nk, mu, nm * sizeof(double));
+  memcpy(h + nk + nm, sigma, ns * sizeof(double));
+  FEM_CUDA(cudaMemcpyAsync(F.pi, h, (nk + nm + ns) * sizeof(double), cudaMemcpyHostToDevice, b->stream));
   b->have_params[fit] = 1;
   return FEM_OK;
 }
@@ -1686,13 +1706,15 @@ extern "C" int fem_em_batch_get_params(fem_em_batch *b, int fit, double *pi, dou
   FEM_TRY(check_fit(b, fit));
   const BFit &F = b->hfits[fit];
   FEM_CUDA(cudaSetDevice(b->cfg.device));
-  if (pi) FEM_CUDA(cudaMemcpyAsync(pi, F.pi, (size_t)F.k * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-  if (mu)
-    FEM_CUDA(cudaMemcpyAsync(mu, F.mu, (size_t)F.k * F.d * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-  if (sigma)
-    FEM_CUDA(cudaMemcpyAsync(sigma, F.sigma, (size_t)F.k * F.d * F.d * sizeof(double), cudaMemcpyDeviceToHost,
-                             b->stream));
+  const size_t nk = F.k, nm = nk * F.d, ns = nm * F.d;
+  double *h = nullptr;
+  FEM_TRY(stage_params(b, nk + nm + ns, &h));
+  const size_t want = sigma ? nk + nm + ns : mu ? nk + nm : pi ? nk : 0;   // up to the last one asked for
+  if (want) FEM_CUDA(cudaMemcpyAsync(h, F.pi, want * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   FEM_CUDA(cudaStreamSynchronize(b->stream));
+  if (pi) memcpy(pi, h, nk * sizeof(double));
+  if (mu) memcpy(mu, h + nk, nm * sizeof(double));
+  if (sigma) memcpy(sigma, h + nk + nm, ns * sizeof(double));
   return FEM_OK;
 }
 

@@ -14,16 +14,19 @@
 // FP32 pipe: 64 of the 88 FP32 operations per point and unit are the products
 // (16 subtractions and 8 multiplications by r beside them) and, at 77 % of its
 // rate, by the 128-bit shared-memory loads; in FP64 by the FP64 pipe (2 per
-// clock and SM).  On the GB300, against a kernel that wrote sqrt(r) (x - mu)
+// clock and SM).  FP32 8 x 8 blocks multiply two columns per instruction
+// (N = 250007, d = 16, K = 200: 0.89 -> 0.68 ms; copies without a division per
+// element 0.65).  On the GB300, against a kernel that wrote sqrt(r) (x - mu)
 // of every component to shared memory and used one thread per block:
 //   N = 2^20, d = 64, K = 128, FP32 from FP16 hi/lo   82.9 -> 20.7 ms
-//   N = 250007, d = 16, K = 200, FP32                  8.20 -> 0.89 ms
-//   N = 200003, d = 24, K = 21, FP32 from FP16 hi/lo   0.75 -> 0.14 ms
+//   N = 250007, d = 16, K = 200, FP32                  8.20 -> 0.61 ms
+//   N = 200003, d = 24, K = 21, FP32 from FP16 hi/lo   0.75 -> 0.115 ms
 //   N = 100000, d = 8, K = 10, FP64                    1.52 -> 0.14 ms
 #include <algorithm>
 #include <cmath>
 
 #include "em_kernels.cuh"
+#include "em_tri.cuh"
 #include "fem_internal.cuh"
 
 namespace fem {
@@ -34,6 +37,7 @@ constexpr int kCvThreads = 256;
 constexpr int kCvRows = 2048;              // rows an FP32 sum may span before it is added into FP64
 constexpr int kCvMaxGroups = 64;
 constexpr size_t kCvMaxSmem = 232448;
+constexpr int kCvTile = 128;               // points per tile
 
 __device__ __forceinline__ void cv_copy4(void *dst, const void *src, bool valid) {
   const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
@@ -53,6 +57,18 @@ __device__ __forceinline__ void cv_copy16(void *dst, const void *src, bool valid
 // (rows past `end` as zero) and reads one of them back.  `pitch` is the
 // number of elements between two components there.
 
+// thread t's elements t, t + 256, ... of a row-major array of `width` columns,
+// without a division per element
+struct CvWalk {
+  int row, col, width, drow, dcol;
+  __device__ __forceinline__ explicit CvWalk(int w)
+      : row(threadIdx.x / w), col(threadIdx.x % w), width(w), drow(kCvThreads / w), dcol(kCvThreads % w) {}
+  __device__ __forceinline__ void next() {
+    row += drow, col += dcol;
+    if (col >= width) col -= width, row++;
+  }
+};
+
 // component-major array of T, rows n apart (any alignment)
 template <typename T>
 struct PostTyped {
@@ -61,8 +77,8 @@ struct PostTyped {
   static constexpr size_t kBytes = sizeof(T);
   __device__ void stage(unsigned char *buf, int pitch, int j0, int cj, int64_t t0, int TP, int64_t end) const {
     T *s = reinterpret_cast<T *>(buf);
-    for (int e = threadIdx.x; e < cj * TP; e += kCvThreads) {
-      const int j = e / TP, p = e - j * TP;
+    for (CvWalk w(TP); w.row < cj; w.next()) {
+      const int j = w.row, p = w.col;
       const bool v = t0 + p < end;
       const T *src = R + (size_t)(j0 + j) * ld + (v ? t0 + p : 0);
       if (sizeof(T) == 4)
@@ -119,6 +135,13 @@ __device__ __forceinline__ void cv_load(const float *row, int b, int nb, float (
   }
 }
 
+// a block's eight columns as pairs, its 16-byte halves `half` floats apart
+__device__ __forceinline__ void cv_load2(const float *x, int half, uint64_t (&v)[4]) {
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(x);
+  const ulonglong2 c = *reinterpret_cast<const ulonglong2 *>(x + half);
+  v[0] = a.x, v[1] = a.y, v[2] = c.x, v[3] = c.y;
+}
+
 constexpr int cv_ne(int TB, bool TRI) { return TRI ? TB * (TB + 1) / 2 : TB * TB; }
 
 // The (component, upper block) units u0 = blockIdx.x upc .. + upc - 1, rows of
@@ -132,6 +155,8 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
             double *__restrict__ part, int nb, int nblk, int64_t rows_per_chunk, int upc, int G, int TP, int xpitch,
             int rpitch, int cjmax) {
   constexpr int NE = cv_ne(TB, TRI);
+  // FP32 blocks of 8 x 8: two columns per instruction
+  constexpr bool PK = sizeof(T) == 4 && TB == 8 && !TRI;
   extern __shared__ __align__(16) unsigned char cv_smem[];
   const int tid = threadIdx.x;
   const int units = K * nblk;
@@ -161,8 +186,16 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
     mb[a] = act && qb < d ? mu[(size_t)j * mu_ld + qb] : T(0);
   }
   T acc[NE];
+  uint64_t ma2[4], mb2[4], acc2[PK ? NE / 2 : 1];
 #pragma unroll
   for (int e = 0; e < NE; e++) acc[e] = T(0);
+#pragma unroll
+  for (int e = 0; e < (PK ? NE / 2 : 1); e++) acc2[e] = 0;
+  if constexpr (PK) {
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+      ma2[a] = f2_pack(ma[2 * a], ma[2 * a + 1]), mb2[a] = f2_pack(mb[2 * a], mb[2 * a + 1]);
+  }
 
   const int64_t c0 = (int64_t)blockIdx.y * rows_per_chunk, c1 = min(n, c0 + rows_per_chunk);
   // dimensions d .. nb TB - 1 of every staged row stay zero
@@ -177,14 +210,14 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
     float *sx = reinterpret_cast<float *>(cv_smem + buf * buf_bytes);
     if ((d & 3) == 0) {
       const int d4 = d >> 2;
-      for (int e = tid; e < TP * d4; e += kCvThreads) {
-        const int p = e / d4, q = 4 * (e - p * d4);
+      for (CvWalk w(d4); w.row < TP; w.next()) {
+        const int p = w.row, q = 4 * w.col;
         const bool v = t0 + p < c1;
         cv_copy16(sx + p * xpitch + cv_pos<TB>(q, nb), X + (v ? (t0 + p) * d + q : 0), v);
       }
     } else {
-      for (int e = tid; e < TP * d; e += kCvThreads) {
-        const int p = e / d, q = e - p * d;
+      for (CvWalk w(d); w.row < TP; w.next()) {
+        const int p = w.row, q = w.col;
         const bool v = t0 + p < c1;
         cv_copy4(sx + p * xpitch + cv_pos<TB>(q, nb), X + (v ? (t0 + p) * d + q : 0), v);
       }
@@ -197,6 +230,10 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
   // adds the FP32 sums into this CTA's FP64 partials (or stores them); the
   // groups' sums of a unit are added in T first, in group order
   auto flush = [&](bool more) {
+    if constexpr (PK) {
+#pragma unroll
+      for (int e = 0; e < NE / 2; e++) f2_unpack(acc2[e], acc[2 * e], acc[2 * e + 1]);
+    }
     double *o = part + (size_t)blockIdx.y * NE * units + u0;
     if (G == 1) {
       if (act) {
@@ -230,6 +267,8 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
     if (more) {
 #pragma unroll
       for (int e = 0; e < NE; e++) acc[e] = T(0);
+#pragma unroll
+      for (int e = 0; e < (PK ? NE / 2 : 1); e++) acc2[e] = 0;
     }
   };
 
@@ -248,33 +287,57 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
     const unsigned char *sr = cv_smem + buf * buf_bytes + xbytes;
     if (act) {
       const int live = (int)min((int64_t)TP, c1 - t0);
-#pragma unroll(TRI ? 2 : 1)
-      for (int p = g; p < live; p += G) {
-        const T r = R.get(sr, roff + p, rlo);
-        float xa[TB];
-        cv_load<TB>(sx + p * xpitch, bi, nb, xa);
-        T ua[TB];
+      if constexpr (PK) {
+        const float *xa = sx + g * xpitch + 4 * bi, *xb = sx + g * xpitch + 4 * bj;
+        const int xs = G * xpitch, half = 4 * nb;
+        int o = roff + g;
+#pragma unroll 1
+        for (int p = g; p < live; p += G, xa += xs, xb += xs, o += G) {
+          const float r = R.get(sr, o, rlo);
+          uint64_t ua[4], ub[4];
+          cv_load2(xa, half, ua);
+          cv_load2(xb, half, ub);
 #pragma unroll
-        for (int a = 0; a < TB; a++) ua[a] = (T)xa[a] - ma[a];
-        if constexpr (TRI) {
-          int e = 0;
+          for (int a = 0; a < 4; a++) ua[a] = f2_sub(ua[a], ma2[a]), ub[a] = f2_sub(ub[a], mb2[a]);
 #pragma unroll
-          for (int a = 0; a < TB; a++) {
-            const T w = r * ua[a];
+          for (int a = 0; a < 8; a++) {
+            float u0, u1;
+            f2_unpack(ua[a / 2], u0, u1);
+            const float w = r * (a & 1 ? u1 : u0);
+            const uint64_t ww = f2_pack(w, w);
 #pragma unroll
-            for (int b = a; b < TB; b++) acc[e] = fma(w, ua[b], acc[e]), e++;
+            for (int b = 0; b < 4; b++) acc2[4 * a + b] = f2_fma(ww, ub[b], acc2[4 * a + b]);
           }
-        } else {
-          float xb[TB];
-          cv_load<TB>(sx + p * xpitch, bj, nb, xb);
-          T ub[TB];
+        }
+      } else {
+#pragma unroll(TRI ? 2 : 1)
+        for (int p = g; p < live; p += G) {
+          const T r = R.get(sr, roff + p, rlo);
+          float xa[TB];
+          cv_load<TB>(sx + p * xpitch, bi, nb, xa);
+          T ua[TB];
 #pragma unroll
-          for (int b = 0; b < TB; b++) ub[b] = (T)xb[b] - mb[b];
+          for (int a = 0; a < TB; a++) ua[a] = (T)xa[a] - ma[a];
+          if constexpr (TRI) {
+            int e = 0;
 #pragma unroll
-          for (int a = 0; a < TB; a++) {
-            const T w = r * ua[a];
+            for (int a = 0; a < TB; a++) {
+              const T w = r * ua[a];
 #pragma unroll
-            for (int b = 0; b < TB; b++) acc[a * TB + b] = fma(w, ub[b], acc[a * TB + b]);
+              for (int b = a; b < TB; b++) acc[e] = fma(w, ua[b], acc[e]), e++;
+            }
+          } else {
+            float xb[TB];
+            cv_load<TB>(sx + p * xpitch, bj, nb, xb);
+            T ub[TB];
+#pragma unroll
+            for (int b = 0; b < TB; b++) ub[b] = (T)xb[b] - mb[b];
+#pragma unroll
+            for (int a = 0; a < TB; a++) {
+              const T w = r * ua[a];
+#pragma unroll
+              for (int b = 0; b < TB; b++) acc[a * TB + b] = fma(w, ub[b], acc[a * TB + b]);
+            }
           }
         }
       }
@@ -402,14 +465,14 @@ k_means_units(const float *__restrict__ X, int64_t n, int d, int K, PostTyped<T>
     float *sx = reinterpret_cast<float *>(cv_smem + buf * buf_bytes);
     if ((d & 3) == 0) {
       const int d4 = d >> 2;
-      for (int e = tid; e < TP * d4; e += kCvThreads) {
-        const int p = e / d4, q = 4 * (e - p * d4);
+      for (CvWalk w(d4); w.row < TP; w.next()) {
+        const int p = w.row, q = 4 * w.col;
         const bool v = t0 + p < c1;
         cv_copy16(sx + p * xpitch + q, X + (v ? (t0 + p) * d + q : 0), v);
       }
     } else {
-      for (int e = tid; e < TP * d; e += kCvThreads) {
-        const int p = e / d, q = e - p * d;
+      for (CvWalk w(d); w.row < TP; w.next()) {
+        const int p = w.row, q = w.col;
         const bool v = t0 + p < c1;
         cv_copy4(sx + p * xpitch + q, X + (v ? (t0 + p) * d + q : 0), v);
       }
@@ -531,13 +594,17 @@ CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
   const int ne = p.tri ? p.TB * (p.TB + 1) / 2 : p.TB * p.TB;
   const int units = k * p.nblk;
   split_units(units, &p.gx, &p.upc, &p.G);
-  const int m = std::max(8, (32 / p.G + 7) / 8 * 8);   // points per thread and tile
-  p.TP = p.G * m;
   p.xpitch = p.TB == 4 ? 4 : 8 * p.nb + 4;             // odd multiple of 16 bytes: point groups in different banks
   p.cj = std::min(k, (p.upc + p.nblk - 2) / p.nblk + 1);
-  p.rpitch = hilo ? p.TP + 8 : p.TP + (fp64 ? 2 : 4);
-  const size_t rb = ((size_t)p.cj * p.rpitch * (fp64 ? 8 : 4) + 15) & ~(size_t)15;
-  p.smem = 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + rb);
+  // kCvTile points a tile (250007 x 16 x 200: 32, 64, 128, 256 points 653, 625,
+  // 605, 605 us), fewer where two CTAs would no longer share an SM
+  for (int tile = kCvTile; tile >= 32; tile /= 2) {
+    p.TP = p.G * std::max(8, (tile / p.G + 7) / 8 * 8);
+    p.rpitch = hilo ? p.TP + 8 : p.TP + (fp64 ? 2 : 4);
+    const size_t rb = ((size_t)p.cj * p.rpitch * (fp64 ? 8 : 4) + 15) & ~(size_t)15;
+    p.smem = 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + rb);
+    if (p.smem <= kCvMaxSmem / 2 - 1024) break;
+  }
   if (p.G > 1) p.smem = std::max(p.smem, (size_t)ne * kCvThreads * (fp64 ? 8 : 4));
   split_rows(n, p.TP, p.gx, (fp64 ? 1 : 2) * sm_count(), 2.0, &p.chunks, &p.rows);
   p.part = (size_t)p.chunks * units * ne;

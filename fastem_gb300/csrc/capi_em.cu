@@ -125,6 +125,7 @@ void free_all(fem_em *h) {
   dfree(h->logdet);
   dfree(h->logc);
   dfree(h->work);
+  dfree(h->fpart);
   if (h->muT) cudaFree(h->muT);
   if (h->linvT) cudaFree(h->linvT);
   if (h->logcT) cudaFree(h->logcT);
@@ -209,7 +210,7 @@ int fem_em_create(int d, int64_t n, int k, const fem_em_config *cfg, fem_em **ou
   if ((st = dalloc(&h->X, (size_t)n * d)) || (st = dalloc(&h->pi, k)) || (st = dalloc(&h->mu, kd)) ||
       (st = dalloc(&h->sigma, kdd)) || (st = dalloc(&h->linv, kdd)) || (st = dalloc(&h->logdet, k)) ||
       (st = dalloc(&h->logc, k)) || (st = dalloc(&h->work, kdd)) || (st = dalloc(&h->psum, k)) ||
-      (st = dalloc(&h->dstat, 1)))
+      (st = dalloc(&h->dstat, 1)) || (st = dalloc(&h->fpart, em_factor_parts(d, k))))
     return fail(st);
   // posteriors: k x n in T for the CUDA-core forms; the mixed form keeps FP16 hi/lo pairs
   const size_t rbytes = (c.precision == FEM_PREC_MIXED) ? 0 : (size_t)k * n * ts;

@@ -161,39 +161,43 @@ __device__ inline bool block_factor_smem(double *A, double *W, double *piv, doub
 }
 
 // ------------------------------------------------------------------------
-// Blocked Cholesky and triangular inverse for one CTA of kFactorThreads
-// threads (kFactorSmemD < d <= kFactorMaxD).  The matrices stay in global
-// memory (L2); the panel being factored and the row block being inverted sit
-// in shared memory, the trailing updates are 4 x 4 register tiles, and the
-// FP64 pipe is the limit (d^3 / 6 fused multiply-adds each for the factor and
-// the inverse).
-constexpr int kPanel = 32;                // columns per Cholesky panel, rows per inverse block
+// Blocked Cholesky for one CTA of kFactorThreads threads (kFactorSmemD < d <=
+// kFactorMaxD).  The matrix stays in global memory (L2); the panel being
+// factored sits in shared memory, the trailing updates are 4 x 4 register
+// tiles, and the FP64 pipe is the limit (d^3 / 6 fused multiply-adds).
+constexpr int kPanel = 32;                // columns per Cholesky panel
 constexpr int kPanelLd = kPanel + 1;      // panel row stride (doubles)
 // block_factor_smem holds both matrices in shared memory up to this d
 constexpr int kFactorSmemD = 118;
 __host__ __device__ constexpr int factor_ld(int d) { return d | 1; }
 
 // dynamic shared memory: both matrices and block_factor_smem's vectors up to
-// kFactorSmemD, else the panel, then the row block
+// kFactorSmemD, else the panel
 __host__ __device__ constexpr size_t factor_smem_bytes(int d) {
   return (d <= kFactorSmemD ? (size_t)2 * d * factor_ld(d) + 4 * d : (size_t)d * kPanelLd) * sizeof(double);
 }
 
-// Right-looking Cholesky of sym(lower(S)) by panels of kPanel columns: the panel (rows k0 .. d-1)
-// is factored in shared memory (thread i owns row k0 + i), written back, and
-// its update of the trailing lower triangle applied as 4 x 4 tiles.  The
-// upper triangle of A keeps the symmetric copy of S.
+// Right-looking Cholesky of sym(lower(S)) by panels of kPanel columns, the
+// trailing lower triangle updated as 4 x 4 tiles.  The upper triangle of A keeps
+// the symmetric copy of S.  In a panel (rows k0 .. d-1) thread i holds row
+// k0 + i in registers, and the panel's own triangle is warp 0, lane = row: per
+// column the warp divides the column by its pivot (L D L^T; the square roots
+// wait for the end of the panel) and one barrier later every row takes the
+// column off.  With the panel in shared memory, a square root and a division per
+// column and two barriers, the kernel took 1391 us at d = 256 and 350 at d = 119,
+// here 1317 and 330; the trailing updates, at the FP64 pipe's rate, are the rest.
 // P: factor_smem_bytes(d) of shared memory.  Returns true on success, the
 // same in every thread.
 __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, double *P) {
-  __shared__ double s_diag[kPanel];
+  __shared__ double s_m[2][kPanel], s_piv[kPanel], s_rd[kPanel];
+  __shared__ int s_bad;
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < d * d; e += nt) {
     const int r = e / d, c = e - r * d;
     A[e] = (c <= r) ? S[e] : S[(size_t)c * d + r];
   }
+  if (tid == 0) s_bad = 0;
   __syncthreads();
-  bool ok = true;
   for (int k0 = 0; k0 < d; k0 += kPanel) {
     const int w = min(kPanel, d - k0), m = d - k0;
     for (int e = tid; e < m * w; e += nt) {
@@ -202,28 +206,41 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
     }
     __syncthreads();
     const int i = tid;                    // panel row owned by this thread
-    for (int q = 0; q < w; q++) {
-      const double x = P[q * kPanelLd + q];   // the same value in every thread
-      if (!(x > 0.0)) {
-        ok = false;
-        break;
+    double x[kPanel];
+#pragma unroll
+    for (int q = 0; q < kPanel; q++) x[q] = i < m && q < w ? P[i * kPanelLd + q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kPanel; q++) {
+      if (q >= w) break;
+      if (tid < 32) {
+        const double p = __shfl_sync(0xffffffffu, x[q], q);
+        if (!(p > 0.0)) {
+          if (tid == 0) s_bad = 1;
+        } else {
+          double u[1] = {x[q]};
+          factor_divide(u, p);
+          s_m[q & 1][tid] = u[0];
+          if (tid == q) s_piv[q] = p;
+        }
       }
-      const double l = sqrt(x);
-      if (i == q) s_diag[q] = l;
-      if (i > q && i < m) P[i * kPanelLd + q] = P[i * kPanelLd + q] / l;
       __syncthreads();
-      if (i > q && i < m) {
-        const double lik = P[i * kPanelLd + q];
-        const int ce = min(i, w - 1);
-        for (int c = q + 1; c <= ce; c++)
-          P[i * kPanelLd + c] = fma(-lik, P[c * kPanelLd + q], P[i * kPanelLd + c]);
-      }
-      __syncthreads();
+      if (s_bad) break;
+      // the entries right of a row's own diagonal are never used
+#pragma unroll
+      for (int c = q + 1; c < kPanel; c++) x[c] = fma(-x[q], s_m[q & 1][c], x[c]);
     }
-    if (!ok) break;
+    if (s_bad) break;
+    if (tid < w) s_rd[tid] = 1.0 / sqrt(s_piv[tid]);
+    __syncthreads();
+    if (i < m) {
+#pragma unroll
+      for (int q = 0; q < kPanel; q++)
+        if (q < w) P[i * kPanelLd + q] = i == q ? sqrt(s_piv[q]) : x[q] * s_rd[q];
+    }
+    __syncthreads();
     for (int e = tid; e < m * w; e += nt) {
       const int r = e / w, q = e - r * w;
-      if (q <= r) A[(size_t)(k0 + r) * d + k0 + q] = (q == r) ? s_diag[q] : P[r * kPanelLd + q];
+      if (q <= r) A[(size_t)(k0 + r) * d + k0 + q] = P[r * kPanelLd + q];
     }
     // trailing update: A[r][c] -= sum_q L[r][q] L[c][q], w <= c <= r < m
     // (panel-relative), over 4 x 4 tiles of the lower triangle
@@ -269,56 +286,7 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
     __syncthreads();
   }
   __syncthreads();
-  return ok;
-}
-
-// W = L^-1 (lower, row-major) by blocks of kPanel rows, thread c owning column c
-// (d <= blockDim.x): the block's rows of L are staged in shared
-// memory (Lb); the terms of the rows above the block (m < r0) run as a
-// register-blocked product over the thread's own column of W, then the
-// block's triangle is solved row by row with that column's new entries in
-// registers.  Terms with m < c multiply an exact zero of W and leave the
-// running sum unchanged, so the loops need no per-column bounds.
-__device__ inline void block_lower_inverse_rows(const double *A, int d, double *Wi, double *Lb) {
-  __shared__ double s_rd[kFactorMaxD];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int r = tid; r < d; r += nt) s_rd[r] = 1.0 / A[(size_t)r * d + r];
-  const int c = tid;
-  for (int r0 = 0; r0 < d; r0 += kPanel) {
-    const int rb = min(kPanel, d - r0), mw = r0 + rb;   // block rows, columns of L used
-    __syncthreads();                                    // Lb free (and s_rd formed)
-    for (int e = tid; e < kPanel * mw; e += nt) {
-      const int rr = e / mw, m = e - rr * mw;
-      Lb[rr * mw + m] = rr < rb ? A[(size_t)(r0 + rr) * d + m] : 0.0;
-    }
-    __syncthreads();
-    if (c >= d) continue;
-    if (c >= mw) {                                      // above the diagonal
-      for (int rr = 0; rr < rb; rr++) Wi[(size_t)(r0 + rr) * d + c] = 0.0;
-      continue;
-    }
-    double acc[kPanel];
-#pragma unroll
-    for (int rr = 0; rr < kPanel; rr++) acc[rr] = 0.0;
-    for (int m = c; m < r0; m++) {                      // rows above the block
-      const double wm = Wi[(size_t)m * d + c];
-#pragma unroll
-      for (int rr = 0; rr < kPanel; rr++) acc[rr] = fma(-Lb[rr * mw + m], wm, acc[rr]);
-    }
-    double wb[kPanel];
-#pragma unroll
-    for (int rr = 0; rr < kPanel; rr++) {               // the block's triangle
-      if (rr < rb) {
-        const int r = r0 + rr;
-        double s = c < r0 ? acc[rr] : (r == c ? 1.0 : 0.0);
-#pragma unroll
-        for (int mm = 0; mm < rr; mm++) s = fma(-Lb[rr * mw + r0 + mm], wb[mm], s);
-        wb[rr] = r < c ? 0.0 : s * s_rd[r];
-        Wi[(size_t)r * d + c] = wb[rr];
-      }
-    }
-  }
-  __syncthreads();
+  return !s_bad;
 }
 
 // log det = 2 sum log L_ii (L in the lower triangle of A): the logarithms in
@@ -340,37 +308,15 @@ __device__ inline double block_chol_logdet(const double *A, int d) {
   return v;
 }
 
-// An upper bound of the condition number lambda_max / lambda_min of the
-// positive definite sym(lower(S)) = L L^T, from norms only:
-//   lambda_max <= ||Sigma||_F and 1 / lambda_min = ||L^-1||_2^2 <= ||L^-1||_F^2.
-// S is row-major (its lower triangle is used), Wi = L^-1 (lower).  At most
-// d^1.5 times the true value; the caller runs the exact eigenvalues
-// (block_jacobi_cond) only when the bound does not settle a test.  Sums in a
-// fixed order; the value in every thread.  blockDim.x <= 256.
-__device__ inline double block_cond_bound(const double *S, const double *Wi, int d) {
-  __shared__ double red_s[256], red_w[256];
-  __shared__ double s_b;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  double fs = 0.0, fw = 0.0;
-  for (int e = tid; e < d * d; e += nt) {
+// ||sym(lower(S))||_F^2, in every thread.  red: a double per warp.
+__device__ inline double block_frob2(const double *S, int d, double *red) {
+  double v[1] = {0.0};
+  for (int e = threadIdx.x; e < d * d; e += blockDim.x) {
     const int r = e / d, c = e - r * d;
-    if (c > r) continue;
-    const double v = S[e], w = Wi[e];
-    fs += (c == r ? 1.0 : 2.0) * v * v;
-    fw += w * w;
+    if (c <= r) v[0] = fma(c == r ? S[e] : 2.0 * S[e], S[e], v[0]);
   }
-  red_s[tid] = fs;
-  red_w[tid] = fw;
-  __syncthreads();
-  if (tid == 0) {
-    double a = 0.0, b = 0.0;
-    for (int t = 0; t < nt; t++) a += red_s[t], b += red_w[t];
-    s_b = sqrt(a) * b;
-  }
-  __syncthreads();
-  const double v = s_b;
-  __syncthreads();
-  return v;
+  block_sums(v, red);
+  return v[0];
 }
 
 // NormalDensity::ComputeConditionNumber (EM2/NormalDensity.cpp:67-71): the

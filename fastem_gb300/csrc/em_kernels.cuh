@@ -9,6 +9,7 @@ namespace fem {
 int em_plain_estep(fem_em *h);
 int em_plain_mstep(fem_em *h);
 int em_factor(fem_em *h, bool regularize);
+size_t em_factor_parts(int d, int k);   // doubles of fem_em::fpart
 int64_t em_plain_logl_blocks(int64_t n, int d);
 int em_post_rows(fem_em *h, int64_t r0, int64_t rows, double *dout);
 int em_classes(fem_em *h, int32_t *dcls);

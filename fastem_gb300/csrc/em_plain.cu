@@ -582,14 +582,17 @@ k_final_means(const double *__restrict__ part, int G, int K, int d, int64_t n, d
 // (EM2/EMAlgorithm.cpp:237-244, EM2/NormalDensity.cpp:43-65,
 // EM2/MatrixEM.cpp:83-87) in FP64, one CTA per component: symmetric copy of
 // the lower triangle, right-looking Cholesky (a pivot <= 0 fails, as in
-// Eigen's LLT), log det = 2 sum log L_ii, W = L^-1 by column substitution,
-// log coefficient log pi_j - d/2 log 2pi - 1/2 log det, and an upper bound
-// of the condition number (block_cond_bound) folded into st->cond_bound.
+// Eigen's LLT), log det = 2 sum log L_ii, W = L^-1, log coefficient
+// log pi_j - d/2 log 2pi - 1/2 log det, and an upper bound of the condition
+// number lambda_max / lambda_min folded into st->cond_bound: lambda_max <=
+// ||Sigma||_F and 1 / lambda_min = ||L^-1||_2^2 <= ||L^-1||_F^2, at most d^1.5
+// times the true value; the caller runs the exact eigenvalues
+// (block_jacobi_cond) only when the bound does not settle a test.
 constexpr double kLog2Pi = 1.8378770664093454835606594728112;   // log(2 pi)
 
 // Up to d = kFactorSmemD both matrices live in shared memory (k_factor_smem);
-// above it the Cholesky and L^-1 run blocked over matrices in L2
-// (block_cholesky_panels, block_lower_inverse_rows).
+// above it the Cholesky runs blocked over matrices in L2 (k_factor) and L^-1 by
+// column blocks on SMs of their own (k_factor_inverse).
 template <typename T, int NS>
 __global__ void __launch_bounds__(kFactorThreads)
 k_factor_smem(int K, int d, double reg, int regularize, double *__restrict__ sigma, const double *__restrict__ pi,
@@ -642,8 +645,7 @@ k_factor_smem(int K, int d, double reg, int regularize, double *__restrict__ sig
   }
   block_sums(sums, red);
   if (tid == 0) {
-    // ||Sigma||_F ||L^-1||_F^2 >= cond (see block_cond_bound); non-negative
-    // doubles order like their bit patterns
+    // non-negative doubles order like their bit patterns
     atomicMax(reinterpret_cast<unsigned long long *>(&st->cond_bound),
               (unsigned long long)__double_as_longlong(sqrt(sums[0]) * sums[1]));
     logdet[j] = sums[2];
@@ -653,35 +655,131 @@ k_factor_smem(int K, int d, double reg, int regularize, double *__restrict__ sig
   }
 }
 
+constexpr int kInvThreads = 128;
+// fpart, doubles per component: ||L^-1||_F^2 of each column block, ||Sigma||_F^2
+// (negative: no factor)
+constexpr int kFactorParts = kFactorMaxD / 32 + 1;
+
 template <typename T>
 __global__ void __launch_bounds__(kFactorThreads)
 k_factor(int K, int d, double reg, int regularize, double *__restrict__ sigma,
          const double *__restrict__ pi, const double *__restrict__ mu, double *__restrict__ work,
-         double *__restrict__ linv, double *__restrict__ logdet, double *__restrict__ logc,
-         T *__restrict__ muT, T *__restrict__ linvT, T *__restrict__ logcT, DevStatus *st) {
+         double *__restrict__ fpart, double *__restrict__ logdet, double *__restrict__ logc,
+         T *__restrict__ muT, T *__restrict__ logcT, DevStatus *st) {
   const int j = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   double *S = sigma + (size_t)j * d * d;
   double *A = work + (size_t)j * d * d;
-  double *Wi = linv + (size_t)j * d * d;
+  double *part = fpart + (size_t)j * kFactorParts;
   extern __shared__ double fsm[];
+  __shared__ double red[kFactorThreads / 32];
   if (regularize && reg != 0.0) block_regularize(S, d, reg);
   if (!block_cholesky_panels(S, d, A, fsm)) {
-    if (tid == 0) atomicMin(&st->chol_failed, j);
+    if (tid == 0) {
+      atomicMin(&st->chol_failed, j);
+      part[kFactorParts - 1] = -1.0;
+    }
     return;
   }
-  block_lower_inverse_rows(A, d, Wi, fsm);
   const double ld = block_chol_logdet(A, d);
-  const double cb = block_cond_bound(S, Wi, d);
+  const double fs = block_frob2(S, d, red);
   if (tid == 0) {
-    // non-negative doubles order like their bit patterns
-    atomicMax(reinterpret_cast<unsigned long long *>(&st->cond_bound), (unsigned long long)__double_as_longlong(cb));
+    part[kFactorParts - 1] = fs;
     logdet[j] = ld;
     const double lc = log(pi[j]) - 0.5 * (double)d * log(2.0 * M_PI) - 0.5 * ld;
     logc[j] = lc;
     logcT[j] = (T)lc;
   }
-  for (int e = tid; e < d * d; e += nt) linvT[(size_t)j * d * d + e] = (T)Wi[e];
   for (int q = tid; q < d; q += nt) muT[(size_t)j * d + q] = (T)mu[(size_t)j * d + q];
+}
+
+// Columns 32 b .. 32 b + 31 of W_j = L_j^-1 (lower, row-major; lane = column),
+// j = blockIdx.x % K and b = blockIdx.x / K, so the blocks with the most rows
+// start first.  The columns of an inverse are independent, and one SM's FP64
+// pipe (2 lanes per clock) is the limit of a whole matrix: spread like this
+// K = 64 components of d = 256 use every SM.  By blocks of 32 rows: the rows of
+// L are staged in shared memory, the terms of the rows above the block are a
+// product over W's own column, 8 rows per warp, and one warp solves the block's
+// triangle, each new entry at once taken off all later rows (32 independent
+// chains; a running sum per row would wait for the FP64 latency at every term).
+// Against one CTA per component for factor and inverse, with running sums (GB300):
+// d = 256, K = 64 3438 -> 1317 + 757 us, d = 128, K = 64 877 -> 367 + 195,
+// d = 119, K = 5 919 -> 328 + 187.
+template <typename T>
+__global__ void __launch_bounds__(kInvThreads)
+k_factor_inverse(int K, int d, const double *__restrict__ work, double *linv, T *__restrict__ linvT,
+                 double *__restrict__ fpart) {
+  extern __shared__ double fsm[];                   // 32 rows of L from column c0 on
+  __shared__ double s_acc[32][33], s_rd[32];
+  const int j = blockIdx.x % K, b = blockIdx.x / K, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int c0 = 32 * b, c = c0 + lane;
+  const double *A = work + (size_t)j * d * d;
+  double *Wi = linv + (size_t)j * d * d, *part = fpart + (size_t)j * kFactorParts;
+  T *Wt = linvT + (size_t)j * d * d;
+  if (part[kFactorParts - 1] < 0.0) return;
+  for (int r = w; r < c0; r += kInvThreads / 32)
+    if (c < d) {
+      Wi[(size_t)r * d + c] = 0.0;
+      Wt[(size_t)r * d + c] = T(0);
+    }
+  double fw = 0.0;
+  for (int r0 = c0; r0 < d; r0 += 32) {
+    const int rb = min(32, d - r0), mp = r0 - c0, mw = mp + rb;
+    __syncthreads();                                // the previous block's rows are used up, its W is written
+#pragma unroll 4
+    for (int rr = w; rr < 32; rr += kInvThreads / 32)
+      for (int m = lane; m < mw; m += 32) fsm[rr * mw + m] = rr < rb ? A[(size_t)(r0 + rr) * d + c0 + m] : 0.0;
+    if (tid < rb) s_rd[tid] = 1.0 / A[(size_t)(r0 + tid) * d + r0 + tid];
+    __syncthreads();
+    double acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[i] = 0.0;
+    if (c < d) {
+      const double *Lw = fsm + 8 * w * mw;
+#pragma unroll 4
+      for (int m = 0; m < mp; m++) {
+        const double wm = Wi[(size_t)(c0 + m) * d + c];   // zero above the diagonal
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = fma(-Lw[i * mw + m], wm, acc[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) s_acc[8 * w + i][lane] = acc[i];
+    __syncthreads();
+    if (w == 0) {
+      double s[32];
+#pragma unroll
+      for (int rr = 0; rr < 32; rr++) s[rr] = r0 + rr == c ? 1.0 : s_acc[rr][lane];
+#pragma unroll
+      for (int rr = 0; rr < 32; rr++) {
+        if (rr >= rb) break;
+        const double v = r0 + rr < c ? 0.0 : s[rr] * s_rd[rr];
+#pragma unroll
+        for (int q = rr + 1; q < 32; q++) s[q] = fma(-fsm[q * mw + mp + rr], v, s[q]);
+        if (c < d) {
+          Wi[(size_t)(r0 + rr) * d + c] = v;
+          Wt[(size_t)(r0 + rr) * d + c] = (T)v;
+          fw = fma(v, v, fw);
+        }
+      }
+    }
+  }
+  if (w == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) fw += __shfl_xor_sync(0xffffffffu, fw, o);
+    if (lane == 0) part[b] = fw;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+k_factor_bound(int K, int nb, const double *__restrict__ fpart, DevStatus *st) {
+  for (int j = threadIdx.x; j < K; j += 256) {
+    const double *part = fpart + (size_t)j * kFactorParts;
+    if (part[kFactorParts - 1] < 0.0) continue;
+    double s = 0.0;
+    for (int b = 0; b < nb; b++) s += part[b];
+    atomicMax(reinterpret_cast<unsigned long long *>(&st->cond_bound),
+              (unsigned long long)__double_as_longlong(sqrt(part[kFactorParts - 1]) * s));
+  }
 }
 
 // =========================================================== launchers
@@ -809,6 +907,8 @@ int em_plain_estep(fem_em *h) {
   return h->cfg.precision == FEM_PREC_FP64 ? estep_plain_t<double>(h) : estep_plain_t<float>(h);
 }
 
+size_t em_factor_parts(int d, int k) { return d > kFactorSmemD ? (size_t)k * kFactorParts : 0; }
+
 int64_t em_plain_logl_blocks(int64_t n, int d) { (void)d; return (n + 63) / 64; }
 
 template <typename T>
@@ -897,8 +997,19 @@ static int factor_t(fem_em *h, bool regularize) {
     FEM_FK((k_factor_smem<T, 2>));
   else if (d <= kFactorSmemD)
     FEM_FK((k_factor_smem<T, 4>));
-  else
-    FEM_FK(k_factor<T>);
+  else {
+    FEM_CUDA(allow_dyn_smem(k_factor<T>, sm));
+    k_factor<T><<<K, kFactorThreads, sm, h->stream>>>(K, d, h->cfg.reg_coef, regularize, h->sigma, h->pi, h->mu, h->work,
+                                                      h->fpart, h->logdet, h->logc, (T *)h->muT, (T *)h->logcT, h->dstat);
+    FEM_CUDA(cudaGetLastError());
+    const int nb = (d + 31) / 32;
+    const size_t si = (size_t)32 * d * sizeof(double);
+    FEM_CUDA(allow_dyn_smem(k_factor_inverse<T>, si));
+    k_factor_inverse<T><<<K * nb, kInvThreads, si, h->stream>>>(K, d, h->work, h->linv, (T *)h->linvT, h->fpart);
+    FEM_CUDA(cudaGetLastError());
+    k_factor_bound<<<1, 256, 0, h->stream>>>(K, nb, h->fpart, h->dstat);
+    h->launches += 2;
+  }
 #undef FEM_FK
   FEM_CUDA(cudaGetLastError());
   h->launches += 1;

@@ -120,6 +120,7 @@ struct fem_em {
   double *linv = nullptr;            // k*d*d  L^-1 (lower), row-major
   double *logdet = nullptr, *logc = nullptr;  // k
   double *work = nullptr;            // k*d*d  factorisation scratch
+  double *fpart = nullptr;           // norms of the blocked factorisation
 
   // kernel-side copies: T = double (FP64) or float (FP32 / mixed)
   void *muT = nullptr, *linvT = nullptr, *logcT = nullptr;

@@ -165,11 +165,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // component each thread centres its P points on the mean, forms
 // ||W_j (x - mu_j)||^2 (two columns per instruction, em_tri.cuh), writes l_ij to
 // R and keeps an online log-sum-exp; a second pass turns l_ij into
-// exp(l_ij - LSE_i).  Bound by the FMA pipe; KC is what lets three CTAs of D = 32
-// share an SM (KC 4, 2, 1: 973, 1033, 1137 us over a batch of 192 fits of
-// 2000..200000 rows; 880 with the row staging's loads in flight together).  Fits of d <= 24 in the D = 32 class multiply 24 columns of its
-// layout.  With single products, a branching log-sum-exp and KC = 8 that launch
-// took 2160 us.
+// exp(l_ij - LSE_i).  Bound by the FMA pipe (58 % busy at D = 32) and the
+// broadcast loads of the factors, which serve P points; more CTAs per SM do not
+// help (KC = 2 and three CTAs of D = 32, four of D = 24: 856 us over a batch of
+// 192 fits of 2000..200000 rows; KC = 4, two and three: 842; KC = 8: 840).
+// Fits of d <= 24 in the D = 32 class multiply 24 columns of its layout, in a
+// launch of their own (in one kernel with both bodies: 903 us).  With single
+// products, a branching log-sum-exp and 32 columns throughout: 2160 us.
 constexpr int kBEP = 4;                          // points per thread
 constexpr int kBEPoints = kBEThreads * kBEP;     // points per item
 constexpr int kBEXs = kBEPoints + 1;             // column-pair stride (float2)
@@ -289,19 +291,15 @@ __device__ __forceinline__ void b_estep_item(const BFit &F, int p0, float *smem,
   if (tid == 0) *out = sum;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kBEThreads)
+template <int D, int CD = D>
+__global__ void __launch_bounds__(kBEThreads, D >= 32 ? 2 : D >= 24 ? 3 : 4)
 k_b_estep(const BFit *__restrict__ fits, const BState *__restrict__ state, const EItem *__restrict__ items,
           double *__restrict__ epart) {
   extern __shared__ __align__(16) float esm[];
   __shared__ double red[kBEThreads / 32];
   const EItem item = items[blockIdx.x];
   if (!state[item.fit].active) return;
-  const BFit &F = fits[item.fit];
-  if (D == 32 && F.d <= 24)
-    b_estep_item<D == 32 ? 24 : D, D>(F, item.p0, esm, red, epart + blockIdx.x);
-  else
-    b_estep_item<D, D>(F, item.p0, esm, red, epart + blockIdx.x);
+  b_estep_item<D, CD>(fits[item.fit], item.p0, esm, red, epart + blockIdx.x);
 }
 
 // Posteriors of components j0 .. j0 + cj - 1 and points t0 .. t0 + tp - 1 into
@@ -1159,6 +1157,7 @@ struct fem_em_batch {
   CItem *citems = nullptr;
   int2 *comps = nullptr;
   int ncomps = 0;
+  int e_mid = 0;                    // first E-step item of the D = 32 class's fits above 24 columns
   int e_beg[kClasses + 1] = {}, m_beg[kClasses + 1] = {}, c_beg[kClasses + 1] = {};
   size_t c_smem[kClasses] = {};
   int c_kmax[kClasses] = {};       // largest k of the class's fits
@@ -1307,7 +1306,14 @@ int launch_sweep(fem_em_batch *b, int it, int svd, int slot) {
       case 0: k_b_estep<4><<<cnt, kBEThreads, estep_smem<4>(), b->stream>>>(fits, st, it0, ep); break;
       case 1: k_b_estep<8><<<cnt, kBEThreads, estep_smem<8>(), b->stream>>>(fits, st, it0, ep); break;
       case 2: k_b_estep<16><<<cnt, kBEThreads, estep_smem<16>(), b->stream>>>(fits, st, it0, ep); break;
-      default: k_b_estep<32><<<cnt, kBEThreads, estep_smem<32>(), b->stream>>>(fits, st, it0, ep); break;
+      default: {
+        // the class's fits of at most 24 columns come first
+        const int c24 = b->e_mid - b->e_beg[c];
+        if (c24) k_b_estep<24, 32><<<c24, kBEThreads, estep_smem<24>(), b->stream>>>(fits, st, it0, ep);
+        if (c24 && c24 < cnt) b->launches++;
+        if (c24 < cnt)
+          k_b_estep<32><<<cnt - c24, kBEThreads, estep_smem<32>(), b->stream>>>(fits, st, it0 + c24, ep + c24);
+      }
     }
     FEM_CUDA(cudaGetLastError());
     b->launches++;
@@ -1498,14 +1504,20 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
     b->m_beg[c] = (int)mi.size();
     b->c_beg[c] = (int)ci.size();
     int kmax = 0;
+    for (int wide = 0; wide < 2; wide++) {           // E-step items: the fits of at most 24 columns first
+      if (wide) b->e_mid = (int)ei.size();
+      for (int f = 0; f < nfits; f++) {
+        BFit &F = b->hfits[f];
+        if (class_of(F.d) != c || (F.d > 24) != (wide != 0)) continue;
+        F.e_first = (int)ei.size();
+        for (int64_t p = 0; p < F.n; p += kBEPoints) ei.push_back(EItem{f, (int)p});
+        F.e_count = (int)ei.size() - F.e_first;
+      }
+    }
     for (int f = 0; f < nfits; f++) {
       BFit &F = b->hfits[f];
       if (class_of(F.d) != c) continue;
       kmax = std::max(kmax, F.k);
-      const int ep = kBEPoints;
-      F.e_first = (int)ei.size();
-      for (int64_t p = 0; p < F.n; p += ep) ei.push_back(EItem{f, (int)p});
-      F.e_count = (int)ei.size() - F.e_first;
       F.m_first = (int)mi.size();
       F.m_part = mp;
       const int mch = tune.means_chunk[c], cch = tune.cov_chunk[c];
@@ -1611,6 +1623,7 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
   if (allow_dyn_smem(k_b_estep<4>, estep_smem<4>()) != cudaSuccess ||
       allow_dyn_smem(k_b_estep<8>, estep_smem<8>()) != cudaSuccess ||
       allow_dyn_smem(k_b_estep<16>, estep_smem<16>()) != cudaSuccess ||
+      allow_dyn_smem(k_b_estep<24, 32>, estep_smem<24>()) != cudaSuccess ||
       allow_dyn_smem(k_b_estep<32>, estep_smem<32>()) != cudaSuccess ||
       allow_dyn_smem(k_b_means<4>, b->m_smem[0]) != cudaSuccess ||
       allow_dyn_smem(k_b_means<8>, b->m_smem[1]) != cudaSuccess ||

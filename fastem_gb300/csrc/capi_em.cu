@@ -213,7 +213,7 @@ int fem_em_create(int d, int64_t n, int k, const fem_em_config *cfg, fem_em **ou
       (st = dalloc(&h->dstat, 1)) || (st = dalloc(&h->fpart, em_factor_parts(d, k))))
     return fail(st);
   // posteriors: k x n in T for the CUDA-core forms; the mixed form keeps FP16 hi/lo pairs
-  const size_t rbytes = (c.precision == FEM_PREC_MIXED) ? 0 : (size_t)k * n * ts;
+  const size_t rbytes = (c.precision == FEM_PREC_MIXED) ? 0 : (size_t)k * post_ld(n) * ts;
   if (cudaMalloc(&h->muT, kd * ts) != cudaSuccess || cudaMalloc(&h->linvT, kdd * ts) != cudaSuccess ||
       cudaMalloc(&h->logcT, k * ts) != cudaSuccess ||
       (rbytes && cudaMalloc(&h->R, rbytes) != cudaSuccess)) {

@@ -145,9 +145,9 @@ extern "C" int fem_em_posterior_correlation(fem_em *h, double *corr) {
     em_tc_posteriors(h, &rh, &rl, &pitch);
     st = launch_corr<float>(h, PostSplit{rh, rl, pitch}, dout);
   } else if (h->cfg.precision == FEM_PREC_FP64) {
-    st = launch_corr<double>(h, PostPlainD{(const double *)h->R, h->n}, dout);
+    st = launch_corr<double>(h, PostPlainD{(const double *)h->R, post_ld(h->n)}, dout);
   } else {
-    st = launch_corr<float>(h, PostPlainF{(const float *)h->R, h->n}, dout);
+    st = launch_corr<float>(h, PostPlainF{(const float *)h->R, post_ld(h->n)}, dout);
   }
   if (st == FEM_OK &&
       cudaMemcpy(corr, dout, (size_t)K * K * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) {

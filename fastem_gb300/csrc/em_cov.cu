@@ -19,7 +19,7 @@
 // element 0.65).  On the GB300, against a kernel that wrote sqrt(r) (x - mu)
 // of every component to shared memory and used one thread per block:
 //   N = 2^20, d = 64, K = 128, FP32 from FP16 hi/lo   82.9 -> 20.7 ms
-//   N = 250007, d = 16, K = 200, FP32                  8.20 -> 0.61 ms
+//   N = 250007, d = 16, K = 200, FP32                  8.20 -> 0.58 ms
 //   N = 200003, d = 24, K = 21, FP32 from FP16 hi/lo   0.75 -> 0.115 ms
 //   N = 100000, d = 8, K = 10, FP64                    1.52 -> 0.14 ms
 #include <algorithm>
@@ -43,9 +43,10 @@ __device__ __forceinline__ void cv_copy4(void *dst, const void *src, bool valid)
   const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(da), "l"(src), "r"(valid ? 4 : 0) : "memory");
 }
-__device__ __forceinline__ void cv_copy8(void *dst, const void *src, bool valid) {
+// the first `bytes` of 16, zeros behind them
+__device__ __forceinline__ void cv_copy16z(void *dst, const void *src, int bytes) {
   const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(da), "l"(src), "r"(valid ? 8 : 0) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(da), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cv_copy16(void *dst, const void *src, bool valid) {
   const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
@@ -69,22 +70,20 @@ struct CvWalk {
   }
 };
 
-// component-major array of T, rows n apart (any alignment)
+// component-major array of T, rows post_ld(n) apart: 16 bytes at a time (TP and
+// t0 are multiples of 4; element by element over unpadded rows 250007 x 16 x 200
+// took 605 us here and 125 in k_means_units, now 578 and 91)
 template <typename T>
 struct PostTyped {
   const T *R;
   int64_t ld;
   static constexpr size_t kBytes = sizeof(T);
   __device__ void stage(unsigned char *buf, int pitch, int j0, int cj, int64_t t0, int TP, int64_t end) const {
+    constexpr int V = 16 / sizeof(T);
     T *s = reinterpret_cast<T *>(buf);
-    for (CvWalk w(TP); w.row < cj; w.next()) {
-      const int j = w.row, p = w.col;
-      const bool v = t0 + p < end;
-      const T *src = R + (size_t)(j0 + j) * ld + (v ? t0 + p : 0);
-      if (sizeof(T) == 4)
-        cv_copy4(s + j * pitch + p, src, v);
-      else
-        cv_copy8(s + j * pitch + p, src, v);
+    for (CvWalk w(TP / V); w.row < cj; w.next()) {
+      const int p = V * w.col, m = (int)max((int64_t)0, min((int64_t)V, end - t0 - p));
+      cv_copy16z(s + w.row * pitch + p, R + (size_t)(j0 + w.row) * ld + (m ? t0 + p : 0), m * (int)sizeof(T));
     }
   }
   __device__ __forceinline__ T get(const unsigned char *buf, int o, int) const {
@@ -639,7 +638,7 @@ static int means_pass(fem_em *h) {
   const CovPlan &p = h->means;
   FEM_CUDA(allow_dyn_smem(k_means_units<T>, p.smem));
   k_means_units<T><<<dim3(p.gx, p.chunks), kCvThreads, p.smem, h->stream>>>(
-      h->X, h->n, h->d, h->k, PostTyped<T>{(const T *)h->R, h->n}, h->mpart, p.nb, p.rows, p.upc, p.G, p.TP, p.xpitch,
+      h->X, h->n, h->d, h->k, PostTyped<T>{(const T *)h->R, post_ld(h->n)}, h->mpart, p.nb, p.rows, p.upc, p.G, p.TP, p.xpitch,
       p.rpitch, p.cj);
   FEM_CUDA(cudaGetLastError());
   return FEM_OK;
@@ -689,9 +688,9 @@ int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, co
 
 int em_cov_plain(fem_em *h) {
   if (h->cfg.precision == FEM_PREC_FP64)
-    return cov_pass<double, PostTyped<double>>(h, PostTyped<double>{(const double *)h->R, h->n},
+    return cov_pass<double, PostTyped<double>>(h, PostTyped<double>{(const double *)h->R, post_ld(h->n)},
                                                (const double *)h->muT, h->d);
-  return cov_pass<float, PostTyped<float>>(h, PostTyped<float>{(const float *)h->R, h->n}, (const float *)h->muT,
+  return cov_pass<float, PostTyped<float>>(h, PostTyped<float>{(const float *)h->R, post_ld(h->n)}, (const float *)h->muT,
                                            h->d);
 }
 

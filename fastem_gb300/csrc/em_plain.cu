@@ -6,7 +6,7 @@
 // (EM2/MatrixEM.cpp:275-378, EM2/EMAlgorithm.cpp:139-191).
 //
 // Layout in HBM: X is n x d float rows; posteriors R are component-major
-// (k x n) so every per-component pass streams contiguous memory; the
+// (k rows, post_ld(n) apart) so every per-component pass streams contiguous memory; the
 // inverse Cholesky factors are stored as W_j = L_j^-1 (lower, row-major), so
 // the Mahalanobis term of point x is ||W_j (x - mu_j)||^2 (the reference
 // multiplies by CholInvC = W_j^T from the right, EM2/MatrixEM.cpp:76).
@@ -181,9 +181,9 @@ k_estep_f32(const float *__restrict__ X, int64_t n, int d, int K, const float *_
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
     const float *sW = cbuf + b * S::CB, *sm = sW + KC * TRI, *sl = sm + KC * D;
-    float *Rj = R + (size_t)j0 * n + p0 + tid;
+    float *Rj = R + (size_t)j0 * post_ld(n) + p0 + tid;
 #pragma unroll 1
-    for (int jj = 0; jj < kc; jj++, Rj += n) {
+    for (int jj = 0; jj < kc; jj++, Rj += post_ld(n)) {
       const uint64_t *m = reinterpret_cast<const uint64_t *>(sm + jj * D);
       uint64_t t[P][D / 2];
 #pragma unroll
@@ -217,7 +217,7 @@ k_estep_f32(const float *__restrict__ X, int64_t n, int d, int K, const float *_
 #pragma unroll
     for (int p = 0; p < P; p++)
       if (live[p]) {
-        float *q = Rt + (size_t)j * n + p * kEPThreads;
+        float *q = Rt + (size_t)j * post_ld(n) + p * kEPThreads;
         *q = expf(*q - lse[p]);
       }
   const double s = block_sum<kEPThreads>(v, red);
@@ -274,7 +274,7 @@ k_estep_f64(const float *__restrict__ X, int64_t n, int d, int K, const double *
 #pragma unroll
       for (int p = 0; p < P; p++) {
         const double l = lc - 0.5 * s[p];
-        if (live[p]) Rt[(size_t)(j0 + jj) * n + p * kEPThreads] = l;
+        if (live[p]) Rt[(size_t)(j0 + jj) * post_ld(n) + p * kEPThreads] = l;
         mx[p] = l > mx[p] ? l : mx[p];
       }
     }
@@ -285,7 +285,7 @@ k_estep_f64(const float *__restrict__ X, int64_t n, int d, int K, const double *
 #pragma unroll
     for (int p = 0; p < P; p++)
       if (live[p]) {
-        double *q = Rt + (size_t)j * n + p * kEPThreads;
+        double *q = Rt + (size_t)j * post_ld(n) + p * kEPThreads;
         const double l = *q, e = exp(l - mx[p]);
         if (l > -INFINITY) se[p] += e;
         *q = e;
@@ -300,7 +300,7 @@ k_estep_f64(const float *__restrict__ X, int64_t n, int d, int K, const double *
   for (int j = 0; j < K; j++)
 #pragma unroll
     for (int p = 0; p < P; p++)
-      if (live[p]) Rt[(size_t)j * n + p * kEPThreads] *= c[p];
+      if (live[p]) Rt[(size_t)j * post_ld(n) + p * kEPThreads] *= c[p];
   const double s = block_sum<kEPThreads>(v, red);
   if (tid == 0) part[blockIdx.x] = s;
 }
@@ -342,13 +342,13 @@ k_estep_64(const float *__restrict__ X, int64_t n, int K, const T *__restrict__ 
       s = fma(y, y, s);
     }
     const T l = logc[j] - T(0.5) * s;
-    if (valid) R[(size_t)j * n + i] = l;
+    if (valid) R[(size_t)j * post_ld(n) + i] = l;
     lse_push(l, mx, se);
   }
   const T lse = mx + t_log(se);
   if (valid)
     for (int j = 0; j < K; j++) {
-      T *p = R + (size_t)j * n + i;
+      T *p = R + (size_t)j * post_ld(n) + i;
       *p = t_exp(*p - lse);
     }
   double s = block_sum<128>(valid ? (double)lse : 0.0, red);
@@ -381,13 +381,13 @@ k_estep_plain_generic(const float *__restrict__ X, int64_t n, int d, int K,
       s = fma(y, y, s);
     }
     const T l = logc[j] - T(0.5) * s;
-    if (valid) R[(size_t)j * n + i] = l;
+    if (valid) R[(size_t)j * post_ld(n) + i] = l;
     lse_push(l, mx, se);
   }
   const T lse = mx + t_log(se);
   if (valid)
     for (int j = 0; j < K; j++) {
-      T *p = R + (size_t)j * n + i;
+      T *p = R + (size_t)j * post_ld(n) + i;
       *p = t_exp(*p - lse);
     }
   double s = block_sum<64>(valid ? (double)lse : 0.0, red);
@@ -505,7 +505,7 @@ k_estep_plain_tiled(const float *__restrict__ X, int64_t n, int d, int K, const 
       for (int i = 0; i < PT; i++) {
         const int64_t pi = i0 + tp + 32 * i;
         const T l = lc - T(0.5) * s[i];
-        if (pi < n) R[(size_t)j * n + pi] = l;
+        if (pi < n) R[(size_t)j * post_ld(n) + pi] = l;
         lse_push(l, mx[i], se[i]);
       }
     }
@@ -522,7 +522,7 @@ k_estep_plain_tiled(const float *__restrict__ X, int64_t n, int d, int K, const 
   for (int e = tid; e < K * P; e += 256) {
     const int j = e / P, p = e - j * P;
     if (i0 + p < n) {
-      T *q = R + (size_t)j * n + i0 + p;
+      T *q = R + (size_t)j * post_ld(n) + i0 + p;
       *q = t_exp(*q - sLse[p]);
     }
   }
@@ -1028,7 +1028,7 @@ __global__ void k_post_rows(const T *__restrict__ R, int64_t n, int K, int64_t r
   if (e >= rows * K) return;
   const int64_t i = e / K;
   const int j = (int)(e - i * K);
-  out[e] = (double)R[(size_t)j * n + r0 + i];
+  out[e] = (double)R[(size_t)j * post_ld(n) + r0 + i];
 }
 
 // EMAlgorithm::RetrieveClasses: first index of the largest posterior
@@ -1039,7 +1039,7 @@ __global__ void k_classes(const T *__restrict__ R, int64_t n, int K, int32_t *__
   double best = -1.0;
   int bj = -1;
   for (int j = 0; j < K; j++) {
-    const double v = (double)R[(size_t)j * n + i];
+    const double v = (double)R[(size_t)j * post_ld(n) + i];
     if (v > best) {
       best = v;
       bj = j;

@@ -859,8 +859,9 @@ k_wide_gather(const double *__restrict__ cpart, const double *__restrict__ spart
 
 // C = A B over 64 x 64 output tiles (FP64): mode 0, C = L M (L lower: inner
 // blocks kk <= I) for the tiles J <= I that mode 1 reads (30 of 40 inner tiles
-// at d = 256, K = 64: both modes together 2452 -> 2010 us); mode 1, C = T L^T for lower tiles I >= J (inner blocks
-// kk <= J), mirrored to the upper triangle.  grid = (tiles, tiles, K).
+// at d = 256; with K = 64 both modes together 2452 -> 2010 us); mode 1, C = T L^T
+// for lower tiles I >= J (inner blocks kk <= J), mirrored to the upper triangle.
+// grid = (tiles, tiles, K).
 __global__ void __launch_bounds__(256)
 k_wide_gemm(const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C, int d, int mode) {
   const int I = blockIdx.y, J = blockIdx.x, j = blockIdx.z;

@@ -87,6 +87,10 @@ struct DevStatus {
   double cond_bound;   // EM: max over components of ||Sigma_j||_F ||L_j^-1||_F^2 (>= cond(Sigma_j))
 };
 
+// elements between two components' rows of the CUDA-core posteriors: every row
+// starts on a 16-byte boundary
+__host__ __device__ constexpr int64_t post_ld(int64_t n) { return (n + 3) & ~(int64_t)3; }
+
 // ------------------------------------------------------------------ EM handle
 // schedule of the CUDA-core means or covariance sums (em_cov.cu)
 struct CovPlan {

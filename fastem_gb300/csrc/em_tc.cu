@@ -237,6 +237,13 @@ __device__ __forceinline__ float z_unit(double var, float cmax) {
 }
 
 // ============================================================== E-step
+// MB = ceil(d / 16): only the 16-wide blocks of dimensions that exist are
+// multiplied and read back. A group's accumulator columns run from the last
+// block of outputs to the first, and the zero blocks of d < 64 would take as
+// much of the tensor core and of the epilogue as real ones (GB300, N = 200003,
+// K = 24 padded: d = 24 76.7 -> 61.0 us; N = 3001,
+// K = 4: d = 5 6.9 -> 5.9 us).
+template <int MB>
 __global__ void __launch_bounds__(kEThreads, 1)
 k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CUtensorMap tm_xl,
            const __grid_constant__ CUtensorMap tm_wh, const __grid_constant__ CUtensorMap tm_wl,
@@ -245,6 +252,7 @@ k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
            __half *__restrict__ Rl, int64_t np, double *__restrict__ part, int64_t n, int K, int *err) {
   extern __shared__ uint8_t smem_raw[];
   ESmem &S = smem_aligned<ESmem>(smem_raw);
+  constexpr int kCol0 = 32 * (kD / 16 - MB);        // first accumulator column and B row in use
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = K / kCompPerGroup;
   const int64_t ntiles = (n + kTileM - 1) / kTileM;
@@ -337,9 +345,10 @@ k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
                 const uint64_t da = (p == 1) ? dxl[t] : dxh[t];
                 const uint64_t db = (p == 0) ? dwl : dwh;
 #pragma unroll
-                for (int kb = 0; kb < kD / 16; kb++) {
+                for (int kb = 0; kb < MB; kb++) {
                   // +32 bytes per 16-element K step inside the 128-byte swizzle row
-                  mma_f16(dt, da + 2 * kb, db + 2 * kb, idesc_f16(kTileM, kGroupN - 32 * kb), (p | kb) != 0);
+                  mma_f16(dt + kCol0, da + 2 * kb, db + kCol0 * 8 + 2 * kb, idesc_f16(kTileM, 32 * (MB - kb)),
+                          (p | kb) != 0);
                 }
               }
             }
@@ -396,17 +405,13 @@ k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
         if (live) {
           const float *bg = S.bias + g * kGroupN;
           // 32-column block bp holds k-block (3 - bp) of both components:
-          // column 32 bp + 16 q + t belongs to component q; two 64-column
-          // loads per group, column pairs in packed FP32 arithmetic
+          // column 32 bp + 16 q + t belongs to component q; 64-column loads
+          // (32 first for an odd MB), column pairs in packed FP32 arithmetic
           float2 s2[kCompPerGroup] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll 1
-          for (int hp = 0; hp < kGroupN / 64; hp++) {
-            uint32_t v[64];
-            tmem_ld64(tbase + lane_addr + (2 * ab + tile) * kGroupN + hp * 64, v);
-            tmem_wait_ld();
-            const float4 *b4 = reinterpret_cast<const float4 *>(bg + hp * 64);
+          auto add = [&](auto &v, int c0) {
+            const float4 *b4 = reinterpret_cast<const float4 *>(bg + c0);
 #pragma unroll
-            for (int u = 0; u < 16; u++) {
+            for (int u = 0; u < (int)(sizeof(v) / 16); u++) {
               const float4 b = b4[u];
               const int q = (u >> 2) & 1;         // columns 4u .. 4u + 3
               const float2 y0 = __fadd2_rn(make_float2(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1])),
@@ -416,6 +421,20 @@ k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
               s2[q] = __ffma2_rn(y0, y0, s2[q]);
               s2[q] = __ffma2_rn(y1, y1, s2[q]);
             }
+          };
+          const uint32_t ta = tbase + lane_addr + (2 * ab + tile) * kGroupN;
+          if constexpr (MB & 1) {
+            uint32_t v[32];
+            tmem_ld32(ta + kCol0, v);
+            tmem_wait_ld();
+            add(v, kCol0);
+          }
+#pragma unroll 1
+          for (int c0 = kCol0 + 32 * (MB & 1); c0 < kGroupN; c0 += 64) {
+            uint32_t v[64];
+            tmem_ld64(ta + c0, v);
+            tmem_wait_ld();
+            add(v, c0);
           }
           s[0] = s2[0].x + s2[0].y;
           s[1] = s2[1].x + s2[1].y;
@@ -1746,6 +1765,10 @@ static bool cov_split_wins(int64_t n, int d, int kp) {
   return d > 32 && (n + kBlk - 1) / kBlk * (kp / 4) >= (int64_t)16 * sm_count();
 }
 
+static decltype(&k_estep_tc<4>) estep_tc_kernel(int d) {
+  return d <= 16 ? k_estep_tc<1> : d <= 32 ? k_estep_tc<2> : d <= 48 ? k_estep_tc<3> : k_estep_tc<4>;
+}
+
 int em_tc_create(fem_em *h) {
   if (h->d > kD) return em_wide_create(h);
   TcEmPlan *p = new TcEmPlan();
@@ -1821,7 +1844,7 @@ int em_tc_create(fem_em *h) {
                          CU_TENSOR_MAP_SWIZZLE_NONE, (uint64_t)p->np * 2));
   FEM_TRY(encode_tmap_2d(&p->tm_rl4, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p->Rl, (uint64_t)n, (uint64_t)K, kBlk, 4,
                          CU_TENSOR_MAP_SWIZZLE_NONE, (uint64_t)p->np * 2));
-  FEM_CUDA(cudaFuncSetAttribute(k_estep_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem_bytes()));
+  FEM_CUDA(cudaFuncSetAttribute(estep_tc_kernel(h->d), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem_bytes()));
   FEM_CUDA(cudaFuncSetAttribute(k_means_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem_bytes()));
   FEM_CUDA(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem_bytes()));
   FEM_CUDA(cudaFuncSetAttribute(k_cov_zx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem_bytes()));
@@ -1898,7 +1921,7 @@ int em_tc_prepare(fem_em *h) {
 int em_tc_estep(fem_em *h) {
   if (h->wide) return em_wide_estep(h);
   TcEmPlan *p = h->tc;
-  k_estep_tc<<<p->egrid, kEThreads, esmem_bytes(), h->stream>>>(
+  estep_tc_kernel(h->d)<<<p->egrid, kEThreads, esmem_bytes(), h->stream>>>(
       p->tm_xh, p->tm_xl, p->tm_wh, p->tm_wl, p->bias, p->chi, p->clo, h->logc, p->lsc, p->Rh, p->Rl, p->np,
       p->epart, h->n, p->kp, p->err);
   FEM_CUDA(cudaGetLastError());

@@ -82,6 +82,32 @@ def test_posteriors_match_numpy(gpu_lib, precision, n, d, k):
     assert abs(logl - lse.sum()) <= bound
 
 
+@pytest.mark.parametrize("d", [1, 15, 16, 17, 32, 33, 48, 49, 64])
+def test_mixed_posteriors_match_numpy(gpu_lib, d):
+    """the tensor-core E-step at the edges of its 16-wide blocks of dimensions"""
+    n, k = 1000, 5
+    X, G = problem(n, d, k, 50 + d)
+    with CudaMatrixEM(d, n, k, precision="mixed") as em:
+        em.CopyDataset(X)
+        em.SetMixture(G)
+        em.InitDensities()
+        em.PrecomputeDensityMatrix()
+        R = em.Posteriors()
+    # x and W carry 22 bits each without the product of their low halves, and an
+    # accumulator is cut to 24 bits up to 12 times: W x to 2^-19 of |W| |x|
+    ref, _, _ = reference(X, G, U32)
+    X64, dl = X.astype(np.float64), np.zeros(n)
+    for j in range(k):
+        W = solve_triangular(cholesky(G.covs[j], lower=True), np.eye(d), lower=True)
+        y = (X64 - G.means[j]) @ W.T
+        dy = 2.0 ** -19 * (np.abs(X64) + np.abs(G.means[j])) @ np.abs(W).T
+        e = np.sum(np.abs(y) * dy + 0.5 * dy * dy, axis=1) + (d + 8) * U32 * (np.sum(y * y, axis=1) + d)
+        dl = np.maximum(dl, e)
+    # FP16 hi + lo posteriors: 22 bits down to FP16's smallest steps
+    tol = ref * (np.expm1(2 * dl) + (k + 16) * 2.0 ** -22)[:, None] + 2.0 ** -24
+    assert np.all(np.abs(R - ref) <= tol), float(np.max(np.abs(R - ref) / tol))
+
+
 def test_batch_weights_match_numpy(gpu_lib):
     shapes = [(1, 17, 1), (511, 20, 5), (513, 24, 4), (1025, 23, 13), (512, 25, 3), (700, 32, 9), (600, 16, 9),
               (600, 9, 8), (600, 8, 17), (600, 5, 16), (600, 3, 33)]

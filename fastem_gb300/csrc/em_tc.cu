@@ -1126,31 +1126,35 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
 // Sigma_j = sym(sum z x^T - (sum z) muf^T) / N_j - (mu - muf)(mu - muf)^T:
 // the scatter around the FP32 means the producers used, moved to the FP64
 // means; chunks summed in order (FP64)
-// (a CTA owns rows 16 blockIdx.y .. + 15 of component blockIdx.x)
-constexpr int kFCRows = 16;
+// (a CTA owns rows 8 blockIdx.y .. + 7 of component blockIdx.x; a thread's sum
+// over the chunks, up to 304 of them, is a chain of L2 loads, so the time is the
+// number of sums per thread: only rows and columns below d, and 8 rows a CTA
+// instead of 16: N = 600000, K = 6, d = 8 251 -> 57 us, K = 10, d = 60 171 -> 78)
+constexpr int kFCRows = 8;
 __global__ void __launch_bounds__(512)
 k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const double *__restrict__ psum,
                const double *__restrict__ mu, const float *__restrict__ muf, const float *__restrict__ cmax,
                double *__restrict__ sigma) {
   const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
   const int a0 = blockIdx.y * kFCRows;
-  // S[a][b] = sum z_a x_b for the block's 16 rows a, and S[b][a] for its 16 columns
+  // S[a][b] = sum z_a x_b for the block's rows a, and S[b][a] for its columns
   __shared__ double sr[kFCRows][kD + 1], sc[kD][kFCRows + 1];
   __shared__ double sz[kD];                    // sum z of component j, per dimension
   const double *P0 = cpart + ((size_t)grp * 2 + pr) * (kZCols * 128) + slot * 64;
   const size_t step = (size_t)gx * 2 * (kZCols * 128);
-  for (int e = threadIdx.x; e < 2 * kFCRows * kD + kD; e += blockDim.x) {
+  const int ri = min(kFCRows, d - a0);         // rows that exist; columns from d on are not summed
+  for (int e = threadIdx.x; e < 2 * ri * d + d; e += blockDim.x) {
     // rows: (b, a0 + i) at P[b * 128 + a0 + i]; columns: (a0 + i, b) at P[(a0 + i) * 128 + b]; sum z: P[64 * 128 + a]
     size_t o;
     double *dst;
-    if (e < kFCRows * kD) {
-      const int i = e % kFCRows, b = e / kFCRows;
+    if (e < ri * d) {
+      const int i = e % ri, b = e / ri;
       o = (size_t)b * 128 + a0 + i, dst = &sr[i][b];
-    } else if (e < 2 * kFCRows * kD) {
-      const int r = e - kFCRows * kD, b = r % kD, i = r / kD;
+    } else if (e < 2 * ri * d) {
+      const int r = e - ri * d, b = r % d, i = r / d;
       o = (size_t)(a0 + i) * 128 + b, dst = &sc[b][i];
     } else {
-      const int a = e - 2 * kFCRows * kD;
+      const int a = e - 2 * ri * d;
       o = (size_t)kD * 128 + a, dst = &sz[a];
     }
     double v = 0.0;

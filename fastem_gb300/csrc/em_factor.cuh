@@ -95,12 +95,11 @@ __device__ __forceinline__ void factor_divide(double (&u)[N], double p) {
 // slower (d = 99: 335, 369 us: warp 0's chain waits behind the bursts).
 template <int NS>
 __device__ inline bool block_factor_smem(double *A, double *W, double *piv, double *rd, double *m, int d, int ld) {
-  __shared__ int s_fail;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nu = (blockDim.x >> 5) - 1;
-  if (threadIdx.x == 0) s_fail = 0;
-  __syncthreads();
+  bool ok = true;
   for (int k = -1; k < d - 1; k++) {
     const double *mk = m + (k & 1) * d;
+    int bad = 0;
     if (warp == 0) {
       const int c = k + 1;
       double u[NS];
@@ -114,7 +113,7 @@ __device__ inline bool block_factor_smem(double *A, double *W, double *piv, doub
       const double p = __shfl_sync(0xffffffffu, u[0], 0);
       const long long pb = __double_as_longlong(p);
       if (pb <= 0 || pb > 0x7ff0000000000000LL) {    // !(p > 0), without waiting for the FP64 pipe
-        if (lane == 0) s_fail = 1;
+        bad = 1;
       } else {
         double *mc = m + (c & 1) * d;
 #pragma unroll
@@ -150,10 +149,13 @@ __device__ inline bool block_factor_smem(double *A, double *W, double *piv, doub
         }
       }
     }
-    __syncthreads();
-    if (s_fail) break;
+    // the barrier carries the verdict: a flag in shared memory could already hold
+    // the next column's when a slow warp reads it, and the warps would part
+    if (__syncthreads_or(bad)) {
+      ok = false;
+      break;
+    }
   }
-  const bool ok = !s_fail;
   if (ok)
     for (int q = threadIdx.x; q < d; q += blockDim.x) rd[q] = 1.0 / sqrt(piv[q]);
   __syncthreads();
@@ -190,13 +192,11 @@ __host__ __device__ constexpr size_t factor_smem_bytes(int d) {
 // same in every thread.
 __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, double *P) {
   __shared__ double s_m[2][kPanel], s_piv[kPanel], s_rd[kPanel];
-  __shared__ int s_bad;
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < d * d; e += nt) {
     const int r = e / d, c = e - r * d;
     A[e] = (c <= r) ? S[e] : S[(size_t)c * d + r];
   }
-  if (tid == 0) s_bad = 0;
   __syncthreads();
   for (int k0 = 0; k0 < d; k0 += kPanel) {
     const int w = min(kPanel, d - k0), m = d - k0;
@@ -212,10 +212,11 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
 #pragma unroll
     for (int q = 0; q < kPanel; q++) {
       if (q >= w) break;
+      int bad = 0;
       if (tid < 32) {
         const double p = __shfl_sync(0xffffffffu, x[q], q);
         if (!(p > 0.0)) {
-          if (tid == 0) s_bad = 1;
+          bad = 1;
         } else {
           double u[1] = {x[q]};
           factor_divide(u, p);
@@ -223,13 +224,11 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
           if (tid == q) s_piv[q] = p;
         }
       }
-      __syncthreads();
-      if (s_bad) break;
+      if (__syncthreads_or(bad)) return false;     // the same in every thread
       // the entries right of a row's own diagonal are never used
 #pragma unroll
       for (int c = q + 1; c < kPanel; c++) x[c] = fma(-x[q], s_m[q & 1][c], x[c]);
     }
-    if (s_bad) break;
     if (tid < w) s_rd[tid] = 1.0 / sqrt(s_piv[tid]);
     __syncthreads();
     if (i < m) {
@@ -285,8 +284,7 @@ __device__ inline bool block_cholesky_panels(const double *S, int d, double *A, 
     }
     __syncthreads();
   }
-  __syncthreads();
-  return !s_bad;
+  return true;
 }
 
 // log det = 2 sum log L_ii (L in the lower triangle of A): the logarithms in

@@ -60,7 +60,7 @@ constexpr uint32_t kKmOnes = 4096;                        // constant A operand:
 
 struct __align__(1024) KmSmem {
   __half b1[kKmMaxK * 64];                 // [ch | ch]  (SW128)
-  __half b2[kKmMaxK * 64];                 // [cl | 0]   (SW128)
+  __half b2[kKmMaxK * 64];                 // [cl | n | 0]  (SW128)
   __half a[kKmAStages][kKmTile * 64];      // [xh | xl]  (SW128)
   float x[kKmXStages][kKmTile * kKmD];     // FP32 rows  (SW128, TMA)
   long long acc[kKmMaxK * kKmAccPitch];    // fixed-point sums
@@ -91,11 +91,13 @@ __device__ __forceinline__ void fence_proxy_async_smem_km() {
 // Centroid operands and bound constants (FP64 centroids in); one CTA, a warp
 // per centroid, lane = dimension.  With N = max ||c'|| over the centroids used,
 //   |D_j - (x'.c'_j - ||c'_j||^2 / 2)| <= ||x'|| bc + ac,
-//   bc = 2^-16 N + 2^-18, ac = 2^-18 N^2 / 2 + 2^-18 N + 1e-30:
+//   bc = 2^-16 N + 2^-18, ac = 2^-18 N^2 / 2 + 2^-18 N + 2^-18:
 // the tensor core cuts each of the 16 terms of a product and the accumulator to
 // 2^-23 of the largest (7 products: 7 x 17 x 2^-23 of ||x'|| ||c'||, 17 x 2^-23
 // of ||c'||^2 / 2 for the last), the splits leave 2^-22 of each side, x - g
-// rounds to 2^-24, and halves below FP16's normal range are off by 2^-25.
+// rounds to 2^-24, and halves below FP16's normal range are off by 2^-25: 2^-18
+// of ||x'|| and N cover that of the operands, and the norm's three parts leave up
+// to 2^-25 times the constant 128 however small row and centroid are.
 // A centroid farther from g than every row can be from the nearest one to g
 // (its norm above that one's plus twice the rows' radius) is never chosen and
 // gets n of the padding.  Centroids all far outside the data: bc = inf, every
@@ -147,7 +149,7 @@ k_km_tc_prep(const double *__restrict__ cent, const double *__restrict__ g, doub
     for (int o = 16; o > 0; o >>= 1) hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     if (lane == 0) {
       cconst[0] = hi < kKmFar ? kKmRel * hi + kKmAbs : INFINITY;
-      cconst[1] = kKmRelN * 0.5f * hi * hi + kKmAbs * hi + 1e-30f;
+      cconst[1] = kKmRelN * 0.5f * hi * hi + kKmAbs * hi + kKmAbs;
     }
   }
 }

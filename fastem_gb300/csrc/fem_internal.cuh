@@ -181,6 +181,8 @@ struct fem_km {
   float xmax = 0.f;                // max |x|
   double xg2 = 0.0;                // sum_i ||x_i - g||^2
   double *g = nullptr;             // data mean (device, d)
+  float *gs = nullptr;             // centre of the screens (device, d)
+  int spread = 0;                  // values' typical distance from it: below 2^spread, half that or more
   double *hg = nullptr;            // data mean (host)
   double *out = nullptr;           // device: k x d new centroids, k counts (as double), fit
   double *hout = nullptr;          // pinned host copy

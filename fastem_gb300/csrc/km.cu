@@ -473,6 +473,7 @@ void free_km(fem_km *h) {
   dfree(h->acc);
   dfree(h->cnt);
   dfree(h->g);
+  dfree(h->gs);
   dfree(h->out);
   dfree(h->dstat);
   km_tc_destroy(h);
@@ -486,6 +487,50 @@ void free_km(fem_km *h) {
     if (e) cudaEventDestroy(e), e = nullptr;
   if (h->stream) cudaStreamDestroy(h->stream);
   h->stream = nullptr;
+}
+
+// Centre and spread of the data for the screens, from the statistics' row blocks
+// (merged to 128): per column the median of the blocks' means, and the median of
+// their mean squares around it.  Not the mean: rows far out, which fall into a few
+// blocks, would move it and widen the spread, and with both every row's bound.
+void screen_frame(fem_km *h, const std::vector<double> &h1, const std::vector<double> &h2, const std::vector<float> &c,
+                  int G, int64_t rpb, std::vector<float> &gs) {
+  const int d = h->d, per = (G + 127) / 128;
+  auto median = [](std::vector<double> &v) {
+    if (v.empty()) return 0.0;
+    const size_t m = v.size() / 2;
+    std::nth_element(v.begin(), v.begin() + m, v.end());
+    const double hi = v[m];
+    return v.size() % 2 ? hi : 0.5 * (hi + *std::max_element(v.begin(), v.begin() + m));
+  };
+  auto rows = [&](int b0, int b1) { return (double)(std::min(h->n, b1 * rpb) - b0 * rpb); };
+  std::vector<double> v, sq((G + per - 1) / per, 0.0);
+  float big = 0.f;
+  for (int q = 0; q < d; q++) {
+    v.clear();
+    for (int b0 = 0; b0 < G; b0 += per) {
+      const int b1 = std::min(G, b0 + per);
+      double a = 0.0;
+      for (int b = b0; b < b1; b++) a += h1[(size_t)b * d + q];
+      const double n = rows(b0, b1);
+      if (n > 0.0 && std::isfinite(a)) v.push_back((double)c[q] + a / n);
+    }
+    gs[q] = (float)median(v);
+    big = std::max(big, std::fabs(gs[q]));
+    for (int b0 = 0; b0 < G; b0 += per) {
+      const int b1 = std::min(G, b0 + per);
+      double a = 0.0, a2 = 0.0;
+      for (int b = b0; b < b1; b++) a += h1[(size_t)b * d + q], a2 += h2[(size_t)b * d + q];
+      const double n = rows(b0, b1), o = (double)gs[q] - (double)c[q];
+      if (n > 0.0) sq[b0 / per] += std::max(0.0, (a2 - 2.0 * o * a) / n + o * o);
+    }
+  }
+  v.clear();
+  for (double t : sq)
+    if (std::isfinite(t)) v.push_back(t);
+  // no less than FP32 resolves at the centre
+  const double rms = std::max(std::sqrt(median(v) / d), std::max((double)big * 5.9604645e-8, 1e-32));
+  std::frexp(rms, &h->spread);
 }
 
 int upload_km(fem_km *h, const float *X, int64_t ld, cudaMemcpyKind kind) {
@@ -541,7 +586,11 @@ int upload_km(fem_km *h, const float *X, int64_t ld, cudaMemcpyKind kind) {
   const double lg = std::log2((double)std::max(mx, 1e-30f)) + std::log2((double)n);
   h->xmax = mx;
   h->shift = (int)std::min(40.0, std::floor(61.0 - std::ceil(lg)));
+  std::vector<float> gs(d);
+  screen_frame(h, h1, h2, c, G, rpb, gs);
   FEM_CUDA(cudaMemcpyAsync(h->g, h->hg, d * 8, cudaMemcpyHostToDevice, h->stream));
+  FEM_CUDA(cudaMemcpyAsync(h->gs, gs.data(), d * 4, cudaMemcpyHostToDevice, h->stream));
+  FEM_CUDA(cudaStreamSynchronize(h->stream));
   h->have_data = true;
   return FEM_OK;
 }
@@ -616,6 +665,7 @@ int fem_km_create(int d, int64_t n, int k, const fem_km_config *cfg, fem_km **ou
       (st = dalloc(&h->cent, (size_t)k * d)) || (st = dalloc(&h->centf, (size_t)k * d)) ||
       (st = dalloc(&h->cnorm, k)) || (st = dalloc(&h->acc, (size_t)h->grid * k * d)) ||
       (st = dalloc(&h->cnt, (size_t)h->grid * k)) || (st = dalloc(&h->g, d)) ||
+      (st = dalloc(&h->gs, d)) ||
       (st = dalloc(&h->out, (size_t)k * d + 2 * k)) || (st = dalloc(&h->dstat, 1)))
     return fail(st);
   if (cudaMallocHost(&h->hout, ((size_t)k * d + 2 * k) * 8) != cudaSuccess ||

@@ -1,9 +1,11 @@
 // km_tc.cu -- Lloyd k-means assignment as a tcgen05 GEMM plus argmin
 // (NaiveKMA::ComputeMSEAndCorrect, Clust/KMAlgorithm.cpp:205-255, for d = 32).
 //
-// Distances are translation invariant, so both sides are first centred on the
-// data mean g (as float) and scaled by a power of two (every |x'| <= 32):
-// x' = t (x - g), c' = t (c - g).  For a tile of 128 points the tensor cores form
+// Distances are translation invariant, so both sides are first centred on a point g
+// amid the data and scaled by a power of two that brings the values' typical
+// distance from it to 1/4..1/2: x' = t (x - g), c' = t (c - g).  (Scaled by max |x|,
+// an offset or one row far out pushes all others below FP16's normal range and
+// leaves them open.)  For a tile of 128 points the tensor cores form
 //   D_j = x'.c'_j - ||c'_j||^2 / 2,   ||x' - c'_j||^2 = ||x'||^2 - 2 D_j,
 // for all K <= 256 centroids in FP32 (TMEM), from FP16 splits:
 //   A row  = [xh | xl]            (64 halves, one 128-byte swizzled row)
@@ -31,6 +33,7 @@
 // the tensor cores (128 16-byte loads a row less).  HBM would take 0.33.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 
 #include "km_kernels.cuh"
@@ -50,11 +53,11 @@ constexpr int kKmAStages = 2;
 constexpr int kKmAccPitch = kKmD + 1;    // padded rows of the fixed-point sums
 constexpr int kKmThreads = 14 * 32;
 constexpr uint32_t kKmXBytes = kKmTile * kKmD * 4;       // 16 KB FP32 tile
-// bound constants (see k_km_tc_prep)
+// constants of the bound (see k_km_tc_prep)
 constexpr float kKmRel = 1.52587890625e-5f;               // 2^-16
 constexpr float kKmRelN = 3.814697265625e-6f;             // 2^-18
 constexpr float kKmAbs = 3.814697265625e-6f;              // 2^-18
-constexpr float kKmRadius = 182.f;                        // ||x'|| <= 32 sqrt(32)
+constexpr int kKmMany = 16;                               // candidates that a row's dimensions are spread over lanes for
 constexpr float kKmFar = 3600.f;                          // ||c'||^2 / 256 within FP16 up to 4095
 constexpr uint32_t kKmOnes = 4096;                        // constant A operand: 128 rows x 32 bytes
 
@@ -65,9 +68,9 @@ struct __align__(1024) KmSmem {
   float x[kKmXStages][kKmTile * kKmD];     // FP32 rows  (SW128, TMA)
   long long acc[kKmMaxK * kKmAccPitch];    // fixed-point sums
   __half ones[kKmOnes / 2];                // every 16 bytes: 128 128 128 0 0 0 0 0
-  float bc, ac;                            // bound on any D: ||x'|| bc + ac
+  float lo, hi;                            // smallest ||c'||, largest that is used
   alignas(16) float g[kKmD];               // -t g
-  float xn[kKmXStages][kKmTile];           // ||x|| of the rows of each X stage
+  float slack[kKmXStages][kKmTile];        // per row of each X stage twice the bound on any D, inf: every centroid
   int cnt[kKmMaxK];
   unsigned cand[8][kKmMaxK / 32][32];      // per epilogue warp: a row's candidate centroids, 32 a word, first = top bit
   uint64_t b_full, x_full[kKmXStages], x_empty[kKmXStages], a_full[kKmAStages], a_empty[kKmAStages],
@@ -79,7 +82,7 @@ static_assert(sizeof(KmSmem) + 1024 <= 232448, "k-means kernel shared memory");
 struct KmTcPlanImpl {
   CUtensorMap tm_x, tm_b1, tm_b2;
   __half *b1 = nullptr, *b2 = nullptr;   // Kp x 64
-  float *cconst = nullptr;               // bound slope and offset
+  float *cconst = nullptr;               // smallest ||c'||, largest that is used
   int *err = nullptr;
   int kp = 0;
 };
@@ -88,26 +91,32 @@ __device__ __forceinline__ void fence_proxy_async_smem_km() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Centroid operands and bound constants (FP64 centroids in); one CTA, a warp
-// per centroid, lane = dimension.  With N = max ||c'|| over the centroids used,
-//   |D_j - (x'.c'_j - ||c'_j||^2 / 2)| <= ||x'|| bc + ac,
-//   bc = 2^-16 N + 2^-18, ac = 2^-18 N^2 / 2 + 2^-18 N + 2^-18:
+// Centroid operands (FP64 centroids in); one CTA, a warp per centroid, lane =
+// dimension.  With N = ||c'_j||,
+//   |D_j - (x'.c'_j - ||c'_j||^2 / 2)| <= B(N) = ||x'|| (2^-16 N + 2^-18) +
+//                                         2^-18 N^2 / 2 + 2^-18 N + 2^-18:
 // the tensor core cuts each of the 16 terms of a product and the accumulator to
 // 2^-23 of the largest (7 products: 7 x 17 x 2^-23 of ||x'|| ||c'||, 17 x 2^-23
 // of ||c'||^2 / 2 for the last), the splits leave 2^-22 of each side, x - g
 // rounds to 2^-24, and halves below FP16's normal range are off by 2^-25: 2^-18
 // of ||x'|| and N cover that of the operands, and the norm's three parts leave up
 // to 2^-25 times the constant 128 however small row and centroid are.
-// A centroid farther from g than every row can be from the nearest one to g
-// (its norm above that one's plus twice the rows' radius) is never chosen and
-// gets n of the padding.  Centroids all far outside the data: bc = inf, every
-// centroid a candidate.
+//
+// A row's nearest centroid is no farther from g than L = l + 2 ||x'||, l the
+// smallest ||c'||: the centroid at l is at most l + ||x'|| away.  The rows screen
+// with B(min(h, 1.01 L + 1/8)), h the largest norm used.  A centroid beyond that,
+// at N, has D_j at least (0.01 N + 1/8) / 1.01 N / 2 below the one at l, more
+// than B(N) and the row's bound together (||x'|| <= N / 2), so it is neither the
+// largest nor the one left out, and one centroid far out does not open every row.
+// Beyond kKmFar a centroid gets n of the padding, and rows that could be its
+// (1.01 L + 1/8 > kKmFar: rows far out, or all centroids far outside the data) take
+// every centroid as a candidate.
 __global__ void __launch_bounds__(1024)
-k_km_tc_prep(const double *__restrict__ cent, const double *__restrict__ g, double t, int K, int Kp,
+k_km_tc_prep(const double *__restrict__ cent, const float *__restrict__ g, double t, int K, int Kp,
              __half *__restrict__ b1, __half *__restrict__ b2, float *__restrict__ cconst) {
   __shared__ float nrm[kKmMaxK], red[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double gq = (double)(float)g[lane];
+  const double gq = (double)g[lane];
   for (int j = warp; j < K; j += 32) {
     const double c = t * (cent[(size_t)j * kKmD + lane] - gq);
     double s = c * c;
@@ -120,10 +129,9 @@ k_km_tc_prep(const double *__restrict__ cent, const double *__restrict__ g, doub
   for (int j = lane; j < K; j += 32) lo = fminf(lo, nrm[j]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-  const float cut = 1.01f * (lo + 2.f * kKmRadius);
   float hi = 0.f;
   for (int j = warp; j < Kp; j += 32) {
-    const bool used = j < K && nrm[j] <= cut;
+    const bool used = j < K && nrm[j] <= kKmFar;
     double c = used ? t * (cent[(size_t)j * kKmD + lane] - gq) : 0.0;
     const __half ch = __double2half(c);
     b1[(size_t)j * 64 + lane] = b1[(size_t)j * 64 + 32 + lane] = ch;              // [ch | ch]
@@ -148,8 +156,8 @@ k_km_tc_prep(const double *__restrict__ cent, const double *__restrict__ g, doub
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     if (lane == 0) {
-      cconst[0] = hi < kKmFar ? kKmRel * hi + kKmAbs : INFINITY;
-      cconst[1] = kKmRelN * 0.5f * hi * hi + kKmAbs * hi + kKmAbs;
+      cconst[0] = lo;
+      cconst[1] = hi;
     }
   }
 }
@@ -165,7 +173,7 @@ __global__ void __launch_bounds__(kKmThreads, 1)
 k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_b1,
                const __grid_constant__ CUtensorMap tm_b2, const float *__restrict__ cconst,
                const double *__restrict__ cent, const float *__restrict__ centf,
-               const float *__restrict__ cnorm, const float *__restrict__ X, const double *__restrict__ gmean, int64_t n,
+               const float *__restrict__ cnorm, const float *__restrict__ X, const float *__restrict__ gs, int64_t n,
                int K, int Kp, float xscale, int32_t *__restrict__ labels,
                long long *__restrict__ accg, int *__restrict__ cntg, float scale, float scale_hi, int lo_bits,
                int64_t epoch, DevStatus *st, int *err) {
@@ -179,10 +187,10 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   for (int j = threadIdx.x; j < kKmMaxK; j += blockDim.x) S.cnt[j] = 0;
   for (uint32_t e = threadIdx.x; e < kKmOnes / 2; e += blockDim.x) S.ones[e] = __float2half((e & 7) < 3 ? 128.f : 0.f);
   fence_proxy_async_smem_km();
-  if (threadIdx.x < kKmD) S.g[threadIdx.x] = -xscale * (float)gmean[threadIdx.x];
+  if (threadIdx.x < kKmD) S.g[threadIdx.x] = -xscale * gs[threadIdx.x];
   if (threadIdx.x == 0) {
-    S.bc = cconst[0];
-    S.ac = cconst[1];
+    S.lo = cconst[0];
+    S.hi = cconst[1];
     mbar_init(&S.b_full, 1);
     for (int s = 0; s < kKmXStages; s++) mbar_init(&S.x_full[s], 1), mbar_init(&S.x_empty[s], 4);
     for (int s = 0; s < kKmAStages; s++) mbar_init(&S.a_full[s], 4), mbar_init(&S.a_empty[s], 1);
@@ -281,8 +289,11 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         ar[c2 ^ (r & 7)] = make_uint4(hh[0], hh[1], hh[2], hh[3]);
         ar[(4 + c2) ^ (r & 7)] = make_uint4(ll[0], ll[1], ll[2], ll[3]);
       }
-      // ||x'|| rounded up a little so that the bound stays an upper bound
-      S.xn[s][r] = sqrtf(ss) * 1.00001f;
+      // the row's bound on D (see k_km_tc_prep), ||x'|| rounded up a little; here,
+      // since the epilogue has no issue slots to spare
+      const float xn = sqrtf(ss) * 1.00001f, reach = fmaf(1.01f, fmaf(2.f, xn, S.lo), 0.125f), cn = fminf(S.hi, reach);
+      const float bound = fmaf(xn, fmaf(kKmRel, cn, kKmAbs), fmaf(fmaf(0.5f * kKmRelN, cn, kKmAbs), cn, kKmAbs));
+      S.slack[s][r] = reach <= kKmFar ? 2.01f * bound : INFINITY;      // (a row with NaN: every centroid)
       fence_proxy_async_smem_km();
       __syncwarp();
       if (lane == 0) mbar_arrive(&S.a_full[as]);
@@ -306,7 +317,7 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       tc_fence_after();
       // the warp's 32 rows, lane = dimension, for the sums: taken now, so that the
       // stage is free for the next copy while this tile is scanned
-      const float xn = S.xn[s][r];
+      const float slack = S.slack[s][r];
       float xr[32];
 #pragma unroll
       for (int rr = 0; rr < 32; rr++) {
@@ -335,9 +346,9 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       const float mv = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
       const int64_t row = (blockIdx.x + i * gridDim.x) * kKmTile + r;
       // the winner's exact value is at least mv - bound, so the reference's
-      // choice has D > thr (bound inf: every centroid)
-      const float thr = mv - 2.01f * fmaf(xn, S.bc, S.ac);
-      const bool all = !(thr > -INFINITY);         // (a row with NaN too)
+      // choice has D > thr
+      const float thr = mv - slack;
+      const bool all = !(slack < INFINITY);
       const float2 thr2 = make_float2(thr, thr), neg = make_float2(-1.f, -1.f);
       unsigned (*cw)[32] = S.cand[warp - 6];
       int cnt = 0, lab = -1;
@@ -377,6 +388,49 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       for (unsigned open = __ballot_sync(0xffffffffu, row < n && cnt > 1); open; open &= open - 1) {
         const int b = __ffs(open) - 1;
         const float xv = __ldg(X + (row - lane + b) * kKmD + lane);
+        if (__shfl_sync(0xffffffffu, cnt, b) > kKmMany) {
+          // the same over all centroids, lane = centroid: a row far outside the data
+          // has every one as its candidate, a chain of K reductions the other way
+          auto dist32 = [&](int j) {
+            float s = 0.f;
+#pragma unroll 8
+            for (int q = 0; q < kKmD; q++) {
+              const float t = __shfl_sync(0xffffffffu, xv, q) - centf[(size_t)min(j, K - 1) * kKmD + q];
+              s = fmaf(t, t, s);
+            }
+            return s;
+          };
+          float U = INFINITY;
+          for (int j0 = 0; j0 < K; j0 += 32) {
+            const float s = dist32(j0 + lane);
+            if (j0 + lane < K) U = fminf(U, s + km_bound32(s, cnorm[j0 + lane]));
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) U = fminf(U, __shfl_xor_sync(0xffffffffu, U, o));
+          double best = DBL_MAX;
+          int l = INT_MAX;
+          for (int j0 = 0; j0 < K; j0 += 32) {
+            const int j = j0 + lane;
+            const float s = dist32(j);
+            const bool in = j < K && s - km_bound32(s, cnorm[min(j, K - 1)]) <= U;
+            if (!__any_sync(0xffffffffu, in)) continue;
+            double d64 = 0.0;
+#pragma unroll 4
+            for (int q = 0; q < kKmD; q++) {
+              const double t = __dsub_rn(cent[(size_t)min(j, K - 1) * kKmD + q], (double)__shfl_sync(0xffffffffu, xv, q));
+              d64 = __dadd_rn(d64, __dmul_rn(t, t));
+            }
+            if (in && d64 < best) best = d64, l = j;     // a lane's centroids come in index order
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int ol = __shfl_xor_sync(0xffffffffu, l, o);
+            if (ob < best || (ob == best && ol < l)) best = ob, l = ol;
+          }
+          if (lane == b) lab = l == INT_MAX ? -1 : l;
+          continue;
+        }
         auto dist = [&](int j) {
           const float t = xv - centf[(size_t)j * kKmD + lane];
           float sj = t * t;
@@ -529,9 +583,10 @@ void km_tc_destroy(fem_km *h) {
 int km_tc_assign(fem_km *h) {
   KmTcPlanImpl *p = static_cast<KmTcPlanImpl *>(h->tc);
   int xe = 0;
-  std::frexp((double)std::max(h->xmax, 1e-25f), &xe);      // |x| <= xmax < 2^xe, |x - g| < 2^(xe + 1)
-  const int te = std::max(-110, 4 - xe);
-  k_km_tc_prep<<<1, 1024, 0, h->stream>>>(h->cent, h->g, std::ldexp(1.0, te), h->k, p->kp, p->b1, p->b2, p->cconst);
+  std::frexp((double)std::max(h->xmax, 1e-25f), &xe);      // |x| <= xmax < 2^xe
+  // 2^te brings the data's spread to 1/4..1/2 (rows up to 3600 times that far out are screened)
+  const int te = -1 - std::min(125, h->spread);
+  k_km_tc_prep<<<1, 1024, 0, h->stream>>>(h->cent, h->gs, std::ldexp(1.0, te), h->k, p->kp, p->b1, p->b2, p->cconst);
   FEM_CUDA(cudaGetLastError());
   // |x| 2^shift < 2^bits: hi takes bits / 2 of them, lo the lo_bits below; both
   // sums stay within 32 bits for `rows` rows of one centroid.  From 1024 rows on
@@ -543,7 +598,7 @@ int km_tc_assign(fem_km *h) {
   const int64_t epoch = w32 ? rows / kKmTile / 2 * 2 - 2 : h->n;   // even: the two groups alternate
 #define FEM_KT(W)                                                                                                \
   k_km_assign_tc<W><<<h->grid, kKmThreads, sizeof(KmSmem) + 1024, h->stream>>>(                                  \
-      p->tm_x, p->tm_b1, p->tm_b2, p->cconst, h->cent, h->centf, h->cnorm, h->X, h->g, h->n, h->k, p->kp,        \
+      p->tm_x, p->tm_b1, p->tm_b2, p->cconst, h->cent, h->centf, h->cnorm, h->X, h->gs, h->n, h->k, p->kp,        \
       ldexpf(1.f, te), h->labels, h->acc, h->cnt, ldexpf(1.f, h->shift), ldexpf(1.f, hi_bits - xe), lo_bits, epoch, h->dstat, p->err)
   if (w32)
     FEM_KT(true);

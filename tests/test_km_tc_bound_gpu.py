@@ -36,3 +36,19 @@ def test_labels_are_the_fp64_argmin(gpu_lib, oracle, case, gap):
         _, cg = km.ComputeMSEAndCorrectCounts(C.copy())
         assert np.array_equal(km.Assignment(), lo)
         assert np.array_equal(cg, co)
+
+
+@pytest.mark.parametrize("case", [{}] + CASES + [dict(outlier=1e7)], ids=lambda c: "_".join("%s%g" % i for i in c.items()))
+def test_an_offset_or_an_outlier_opens_few_rows(gpu_lib, oracle, case):
+    """The screen decides nearly every row whatever the data's offset, and
+    whatever one row or one centroid far out does to the largest value."""
+    n, k = 20000, 256
+    X, C = data(n, k, 1.0, **case)
+    for far in (0.0, 1e4):
+        C[9, :] += far
+        with CudaKMA(32, n, k, precision="mixed", repair=False) as km:
+            km.SetDataset(X)
+            lo = oracle.km_iterate(X, C, repair=False)[3]
+            km.ComputeMSEAndCorrect(C.copy())
+            assert np.array_equal(km.Assignment(), lo)
+            assert km.Stats()["rechecked"] <= n // 100

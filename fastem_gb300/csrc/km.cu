@@ -86,10 +86,10 @@ k_km_stats(const float *__restrict__ X, int64_t n, int d, int64_t rows_per_block
   }
 }
 
-// centroids -> float copy and norm, and for the FP32 path the copy around the
-// data mean (as float) and half its squared norm; one warp per centroid
+// centroids -> float copy and norm, and for the FP32 path the copy around g (as
+// float) and half its squared norm; one warp per centroid
 __global__ void __launch_bounds__(128)
-k_km_prep(const double *__restrict__ cent, const double *__restrict__ g, int K, int d, float *__restrict__ centf,
+k_km_prep(const double *__restrict__ cent, const float *__restrict__ g, int K, int d, float *__restrict__ centf,
           float *__restrict__ cnorm, float *__restrict__ centg, float *__restrict__ hnorm) {
   const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= K) return;
@@ -99,7 +99,7 @@ k_km_prep(const double *__restrict__ cent, const double *__restrict__ g, int K, 
     centf[(size_t)j * d + q] = (float)c;
     s = fma(c, c, s);
     if (centg) {
-      const double cg = c - (double)(float)g[q];
+      const double cg = c - (double)g[q];
       centg[(size_t)j * d + q] = (float)cg;
       h = fma(cg, cg, h);
     }
@@ -134,13 +134,19 @@ __device__ __forceinline__ float bound_f32(float s, float cn, int d) {
 // =================================================== FP32 assignment
 // Every warp takes its own share of the rows, 32 R at a time (R rows per
 // lane, in registers), and screens all centroids by
-//   w_j = ||c'_j||^2 / 2 - x'.c'_j     (x' = x - g, c' = c - g; ||x - c||^2 =
-//                                       ||x'||^2 + 2 w_j),
+//   w_j = ||c'_j||^2 / 2 - x'.c'_j     (x' = x - g, c' = c - g, g amid the data;
+//                                       ||x - c||^2 = ||x'||^2 + 2 w_j),
 // D products per (row, centroid) where the difference form takes 2 D
-// operations, keeping the two smallest.  With u = 2^-24 the computed w_j is within
-//   B = 1.05 (D + 6) u (||x'|| ||c'||max + ||c'||max^2 / 2)
-// of the exact one (rounding of x', c', ||c'||^2 and the D-term sum), so a row
-// whose two smallest differ by more than 2 B is decided.  The others, few, go
+// operations, keeping the two smallest.  With u = 2^-24 and N = ||c'_j|| the computed
+// w_j is within
+//   B(N) = 1.05 (D + 6) u (||x'|| N + N^2 / 2)
+// of the exact one (rounding of x', c', ||c'||^2 and the D-term sum).  A row's
+// nearest centroid is no farther from g than L = l + 2 ||x'||, l the smallest
+// ||c'||; one beyond 1.01 L, at N, has w_j at least 0.0049 N^2 above the one at l,
+// more than B(N) and B(1.01 L) together, so it is never the smallest.  A row whose
+// two smallest differ by more than 2 B(min(||c'||max, 1.01 L)) is therefore decided
+// (with ||c'||max alone one centroid at 10^4 opened every row of unit blobs: N =
+// 1000003, D = 64, K = 100 43 ms an iteration, without it 0.62).  The others, few, go
 // through the difference form by the whole warp (lane = centroid): FP32 with
 // the bound of bound_f32, then the reference's FP64 sums among the centroids
 // that remain, lowest index on ties.  Rows are added to exact fixed-point sums
@@ -256,7 +262,7 @@ __device__ int km_decide(const float *__restrict__ x, const float *__restrict__ 
 
 template <int D>
 __global__ void __launch_bounds__(KmShape<D>::kThreads)
-k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const double *__restrict__ gmean,
+k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const float *__restrict__ gs,
                 const float *__restrict__ centg, const float *__restrict__ hnorm, const float *__restrict__ centf,
                 const float *__restrict__ cnorm, const double *__restrict__ cent, int32_t *__restrict__ labels,
                 long long *__restrict__ accg, int *__restrict__ cntg, float scale, DevStatus *st) {
@@ -267,9 +273,9 @@ k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const double *__r
   float *sH = sC + (size_t)K * D;                       // K
   int *sCnt = (int *)(sH + K);                          // K
   __shared__ __align__(16) float sG[D < 4 ? 4 : D];
-  __shared__ float sMax[T / 32];
+  __shared__ float sMax[T / 32], sMin[T / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float hmax = 0.f;
+  float hmax = 0.f, hmin = INFINITY;
   for (int e = tid; e < K * D; e += T) {
     sAcc[e] = 0;
     sC[e] = -centg[e];                                  // w = h + x'.(-c')
@@ -278,16 +284,17 @@ k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const double *__r
     const float h = hnorm[j];
     sCnt[j] = 0;
     sH[j] = h;
-    hmax = fmaxf(hmax, h);
+    hmax = fmaxf(hmax, h), hmin = fminf(hmin, h);
   }
-  if (tid < D) sG[tid] = (float)gmean[tid];
+  if (tid < D) sG[tid] = gs[tid];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) hmax = fmaxf(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
-  if (lane == 0) sMax[warp] = hmax;
+  for (int o = 16; o > 0; o >>= 1)
+    hmax = fmaxf(hmax, __shfl_xor_sync(0xffffffffu, hmax, o)), hmin = fminf(hmin, __shfl_xor_sync(0xffffffffu, hmin, o));
+  if (lane == 0) sMax[warp] = hmax, sMin[warp] = hmin;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < T / 32; w++) hmax = fmaxf(hmax, sMax[w]);
-  const float cmax = sqrtf(2.f * hmax) * 1.00001f;
+  for (int w = 0; w < T / 32; w++) hmax = fmaxf(hmax, sMax[w]), hmin = fminf(hmin, sMin[w]);
+  const float cmax = sqrtf(2.f * hmax) * 1.00001f, clo = sqrtf(2.f * hmin) * 1.0101f;   // ||c'||max, 1.01 l
   const bool track = st->track_changes;
   constexpr float kU = 5.9604645e-8f * 1.05f * (D + 6);
   int64_t rechecks = 0;
@@ -335,7 +342,8 @@ k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const double *__r
       const int64_t row = base + 32 * r + lane;
       const bool in = row < r1;
       // the last term covers the reference's own FP64 rounding
-      const float B = fmaf(kU, fmaf(xn[r], cmax, 0.5f * cmax * cmax), 1e-13f * fmaf(xn[r], xn[r], cmax * cmax)) + 1e-30f;
+      const float cn = fminf(cmax, fmaf(2.02f, xn[r], clo));
+      const float B = fmaf(kU, fmaf(xn[r], cn, 0.5f * cn * cn), 1e-13f * fmaf(xn[r], xn[r], cn * cn)) + 1e-30f;
       int lab = j1[r];
       unsigned open = __ballot_sync(0xffffffffu, in && !(m2[r] - m1[r] > 2.1f * B));
       while (open) {
@@ -426,7 +434,7 @@ int km_launch_assign_f32(fem_km *h) {
   case DD:                                                                                                     \
     FEM_CUDA(allow_dyn_smem(k_km_assign_f32<DD>, sm));                                                         \
     k_km_assign_f32<DD><<<h->grid, KmShape<DD>::kThreads, sm, h->stream>>>(                                    \
-        h->X, h->n, K, h->g, h->centg, h->hnorm, h->centf, h->cnorm, h->cent, h->labels, h->acc, h->cnt,       \
+        h->X, h->n, K, h->gs, h->centg, h->hnorm, h->centf, h->cnorm, h->cent, h->labels, h->acc, h->cnt,       \
         ldexpf(1.f, h->shift), h->dstat);                                                                      \
     break;
   switch (D) {
@@ -749,7 +757,7 @@ static int km_iterate(fem_km *h, double *centroids, double *fit, int64_t *counts
   *h->hstat = z;
   FEM_CUDA(cudaMemcpyAsync(h->dstat, h->hstat, sizeof(DevStatus), cudaMemcpyHostToDevice, h->stream));
   FEM_CUDA(cudaMemcpyAsync(h->cent, centroids, kd * 8, cudaMemcpyHostToDevice, h->stream));
-  k_km_prep<<<(K + 3) / 4, 128, 0, h->stream>>>(h->cent, h->g, K, d, h->centf, h->cnorm, h->centg, h->hnorm);
+  k_km_prep<<<(K + 3) / 4, 128, 0, h->stream>>>(h->cent, h->gs, K, d, h->centf, h->cnorm, h->centg, h->hnorm);
   FEM_CUDA(cudaGetLastError());
   FEM_CUDA(cudaEventRecord(h->ev[0], h->stream));
   if (h->cfg.precision == FEM_PREC_MIXED)

@@ -147,10 +147,10 @@ static_assert(kZACol + kZA * kZAStage <= 512 && 3 * kZDCol + kZN <= kZACol, "cov
 constexpr int kSIn = 4;                  // input ring (blocks)
 constexpr int kSSteps = kBlk / 16;
 constexpr int kSA = 6;                   // TMEM A ring (steps)
-constexpr int kSAcc = 16;                // blocks a zh xh^T accumulator spans
+constexpr int kSAcc = 16;                // blocks a zh xg^T accumulator spans
 constexpr int kSWin = 64;                // blocks an FP32 register sum spans (4096 rows)
 constexpr int kSRows = 2048;             // rows an FP32 diagonal sum spans
-// TMEM columns: [pair] zh [xh; 1]^T, [pair] the small products, A ring (per pair 8 hi + 8 lo a step)
+// TMEM columns: [pair] zh [xg; 1]^T, [pair] the small products, A ring (per pair 8 hi + 8 lo a step)
 constexpr int kSN = kD + 16;             // accumulator columns per pair: 64 sums, sum z, 15 unused
 constexpr uint32_t kSCross = 2 * kSN, kSACol = 4 * kSN, kSAStage = 32;
 // warps 0 TMA, 1 MMA, 2 posteriors, 3 none; 4..19 producers (4 groups); 20..27 flush (a group of 4 per pair)
@@ -162,8 +162,8 @@ constexpr int kSRegLaunch = 72, kSRegCtl = 24, kSRegProd = 72, kSRegFlush = 96;
 static_assert(128 * kSRegCtl + 512 * kSRegProd + 256 * kSRegFlush <= kSThreads * kSRegLaunch, "register split");
 static_assert(kSACol + kSA * kSAStage <= 512, "split covariance TMEM columns");
 struct __align__(1024) SSmem {
-  __half bh[kSIn][kSN * kBlk];                       // rows 0..63 xh^T (TMA, SW128), row 64 ones, 65..79 zero
-  __half bl[kSIn][kD * kBlk], bm[kSIn][kD * kBlk];   // xl^T, xm^T
+  __half bh[kSIn][kSN * kBlk];                       // rows 0..63 xg^T (TMA, SW128), row 64 ones, 65..79 zero
+  __half bl[kSIn][kD * kBlk], bm[kSIn][kD * kBlk];   // xr^T, xm^T
   float x[kSIn][kBlk * kD];                          // FP32 rows (TMA)
   __half rh[kSIn][4 * kBlk], rl[kSIn][4 * kBlk];     // posteriors of the CTA's 4 components
   float rf[kSIn][4 * kBlk];                          // hi + lo
@@ -178,14 +178,15 @@ static_assert(sizeof(SSmem) + 1024 <= 232448, "split covariance shared memory");
 struct TcEmPlan {
   CUtensorMap tm_xh, tm_xl, tm_wh, tm_wl;      // E-step
   CUtensorMap tm_rh, tm_rl, tm_xht, tm_xlt;    // means
-  CUtensorMap tm_xmt;                          // split covariance
+  CUtensorMap tm_xgt, tm_xrt, tm_xmt;          // split covariance
   CUtensorMap tm_x32, tm_rh4, tm_rl4;          // covariances
   __half *Wh = nullptr, *Wl = nullptr;  // (K*d) x d, permuted rows
   float *bias = nullptr;                // K*d, permuted
   float *clo = nullptr;                 // log coefficient - float(log coefficient)
   __half *Rh = nullptr, *Rl = nullptr;  // K x np posteriors hi / lo
-  __half *XhT = nullptr, *XlT = nullptr;  // d x np, in units of each dimension (x_unit)
-  __half *XmT = nullptr;                // their remainder (split covariance only)
+  __half *XhT = nullptr, *XlT = nullptr;  // d x np: fp16(x) and the rest
+  // split covariance only, d x np: x in units of its dimension (x_unit): nearest integer, rest, what FP16 leaves of it
+  __half *XgT = nullptr, *XrT = nullptr, *XmT = nullptr;
   int64_t np = 0;                       // padded row pitch (multiple of 64)
   float *lsc = nullptr;                 // E-step scratch: egrid x 2 x K x 256
   double *epart = nullptr;              // per-CTA log-likelihood
@@ -196,7 +197,7 @@ struct TcEmPlan {
   float *chi = nullptr;                 // float(log coefficient); -inf for padding components
   float *X64 = nullptr;                 // n x 64 zero-padded FP32 rows when d < 64
   int *err = nullptr;                   // device status of the bounded waits
-  float *amax = nullptr;                // upload: largest |x| of every dimension, then of all (FP16 range check)
+  float *amax = nullptr;                // upload: largest |x| of every dimension (split covariance), then of all (FP16 range check)
   float *zunit = nullptr;               // split covariance: unit of z per component and dimension
   int *roles = nullptr;                 // bounded-wait expiry self-test: which waits gave up
   int egrid = 0, mgrid = 0, cgx = 0, cgy = 0;
@@ -216,12 +217,13 @@ __device__ __forceinline__ void store_post(__half *Rh, __half *Rl, size_t o, flo
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
-// Columns of X^T are held in units of a power of two, h = 2^(E - 10) with 2^E
-// <= max |x| < 2^(E + 1) over the column: x = h (xh + xl), xh an integer of at
-// most 2^11 (exact in FP16), |xl| <= 1/2 in FP16 (2^-24 of the column's
-// maximum); the split covariance adds what is left, xm.  Products of xh with a weight on a grid add up exactly in FP32
-// while they stay below 2^24 units, where the tensor core's truncation of a
-// floating split would cut every addition.
+// The split covariance's columns of X^T are in units of a power of two, h = 2^(E -
+// 10) with 2^E <= max |x| < 2^(E + 1) over the column: x = h (xg + xr + xm), xg an
+// integer of at most 2^11 (exact in FP16), |xr| <= 1/2 in FP16, xm what is left.
+// Products of xg with a weight on a grid add up exactly in FP32 while they stay
+// below 2^24 units, where the tensor core's truncation of a floating split would
+// cut every addition.  (xg + xr alone are exact to 2^-24 of the column's maximum
+// only, so the forms that read two parts take fp16(x) and its rest, 2^-22 of x.)
 __device__ __forceinline__ int x_unit_exp(float cmax) { return cmax > 0.f ? max(ilogbf(cmax), -110) - 10 : 0; }
 __device__ __forceinline__ float x_unit(float cmax) { return ldexpf(1.f, x_unit_exp(cmax)); }
 
@@ -649,7 +651,7 @@ k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n
   }
 #pragma unroll
   for (int u = 1; u < kFMSplit; u++) s += red[u][q];
-  const double m = s * (double)x_unit(cmax[q]) / s1;
+  const double m = s / s1;
   if (q < d) mu[(size_t)j * d + q] = m;
   muf[(size_t)j * kD + q] = q < d ? (float)m : 0.f;
   zunit[(size_t)j * kD + q] = q < d ? z_unit(sigma[((size_t)j * d + q) * d + q], cmax[q]) : 1.f;
@@ -928,8 +930,7 @@ __global__ void k_final_cov_tc(const double *__restrict__ cpart, const double *_
 // kFlushBlocks blocks (double buffered in TMEM).
 __global__ void __launch_bounds__(kZThreads, 1)
 k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUtensorMap tm_xlt,
-         const __grid_constant__ CUtensorMap tm_rh4, const float *__restrict__ muf, const float *__restrict__ cmax,
-         int64_t n,
+         const __grid_constant__ CUtensorMap tm_rh4, const float *__restrict__ muf, int64_t n,
          int64_t blocks_per_chunk, double *__restrict__ cpart, int *err) {
   extern __shared__ uint8_t smem_raw[];
   ZSmem &S = smem_aligned<ZSmem>(smem_raw);
@@ -1027,7 +1028,6 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
     const int a = 32 * (quad & 1) + lane;        // dimension = TMEM lane within the slot
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     float mu[2];
-    const float2 hx = f2(x_unit(cmax[a]));       // x = hx (xh + xl)
 #pragma unroll
     for (int pr = 0; pr < 2; pr++) mu[pr] = muf[(size_t)(cg * 4 + 2 * pr + slot) * kD + a];
     bool ok = true;
@@ -1040,7 +1040,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
       const uint8_t *rowl = reinterpret_cast<const uint8_t *>(S.bl[st]) + a * 128;
 #pragma unroll 1
       for (int kb = part * kSteps; kb < (part + 1) * kSteps; kb++) {
-        // x / hx = xh + xl (exact in FP32) of the 16 points of this K step, dimension a
+        // x = xh + xl (exact in FP32) of the 16 points of this K step, dimension a
         float2 x[8];
 #pragma unroll
         for (int hc = 0; hc < 2; hc++) {
@@ -1064,7 +1064,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
           uint32_t packed[8];
 #pragma unroll
           for (int q = 0; q < 8; q++) {
-            const float2 dz = __ffma2_rn(x[q], hx, nm);
+            const float2 dz = __fadd2_rn(x[q], nm);
             const __half2 z = __hmul2(__floats2half2_rn(dz.x, dz.y), *reinterpret_cast<const __half2 *>(&rw[q]));
             packed[q] = *reinterpret_cast<const uint32_t *>(&z);
           }
@@ -1133,8 +1133,7 @@ k_cov_zx(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUt
 constexpr int kFCRows = 8;
 __global__ void __launch_bounds__(512)
 k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const double *__restrict__ psum,
-               const double *__restrict__ mu, const float *__restrict__ muf, const float *__restrict__ cmax,
-               double *__restrict__ sigma) {
+               const double *__restrict__ mu, const float *__restrict__ muf, double *__restrict__ sigma) {
   const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
   const int a0 = blockIdx.y * kFCRows;
   // S[a][b] = sum z_a x_b for the block's rows a, and S[b][a] for its columns
@@ -1169,8 +1168,7 @@ k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const do
     const int i = e / kD, a = a0 + i, b = e - i * kD;
     if (a >= d || b >= d || b < a) continue;
     const double ma = muf[(size_t)j * kD + a], mb = muf[(size_t)j * kD + b];
-    // the sums' columns are in units of the x column
-    const double ca = sr[i][b] * x_unit(cmax[b]) - sz[a] * mb, cb = sc[b][i] * x_unit(cmax[a]) - sz[b] * ma;
+    const double ca = sr[i][b] - sz[a] * mb, cb = sc[b][i] - sz[b] * ma;
     const double v = 0.5 * (ca + cb) * inv - (mu[(size_t)j * d + a] - ma) * (mu[(size_t)j * d + b] - mb);
     Sg[a * d + b] = v;
     Sg[b * d + a] = v;
@@ -1180,10 +1178,11 @@ k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const do
 // ================================================ covariances (split z x^T)
 // The z x^T form above with z = r (x - mu) split into FP16 hi + lo as well,
 // for fits whose components hold too few points for z's single rounding to
-// average out:  sum z x^T = sum zh xh^T + (sum zh (xl + xm)^T + sum zl (xh + xl)^T).
+// average out, and x = xg + xr + xm in units of its dimension:
+//   sum z x^T = sum zh xg^T + (sum zh (xr + xm)^T + sum zl (xg + xr)^T).
 // To reach the accuracy of FP32 sums on CUDA cores:
 //  * the tensor core truncates its FP32 accumulator, so z is put on a grid as x
-//    is (z_unit: zh an integer, |zl| <= 1/2): zh xh^T then adds up exactly below
+//    is (z_unit: zh an integer, |zl| <= 1/2): zh xg^T then adds up exactly below
 //    2^24 units, which kSAcc blocks of a component rarely reach (beyond it,
 //    truncation is as for any FP32 sum).  With a floating split every addition
 //    truncates: 4e-8 to 7e-8 off where FP32 sums on CUDA cores are at 1e-8;
@@ -1209,7 +1208,7 @@ k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const do
 // d = 64, K = 32 1.19 -> 0.32 ms; error of Sigma (Frobenius) against 64-bit
 // sums over the same posteriors 8e-9 and 9e-9 (CUDA cores 8e-9 and 1.6e-8).
 __global__ void __launch_bounds__(kSThreads, 1)
-k_cov_split(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUtensorMap tm_xlt,
+k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ CUtensorMap tm_xrt,
             const __grid_constant__ CUtensorMap tm_xmt, const __grid_constant__ CUtensorMap tm_x32,
             const __grid_constant__ CUtensorMap tm_rh4, const __grid_constant__ CUtensorMap tm_rl4,
             const float *__restrict__ muf, const float *__restrict__ cmax, const float *__restrict__ zunit, int64_t n,
@@ -1267,8 +1266,8 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ 
           if (!(ok = mbar_wait_lazy(&S.in_empty[st], ((t / kSIn) & 1) ^ 1, err, 128))) break;
           const int p0 = (int)(r0 + (int64_t)t * kBlk);
           mbar_expect_tx(&S.in_full[st], kInBytes);
-          tma_load_2d(S.bh[st], &tm_xht, &S.in_full[st], p0, 0);
-          tma_load_2d(S.bl[st], &tm_xlt, &S.in_full[st], p0, 0);
+          tma_load_2d(S.bh[st], &tm_xgt, &S.in_full[st], p0, 0);
+          tma_load_2d(S.bl[st], &tm_xrt, &S.in_full[st], p0, 0);
           tma_load_2d(S.bm[st], &tm_xmt, &S.in_full[st], p0, 0);
           tma_load_2d(S.x[st], &tm_x32, &S.in_full[st], 0, p0);
           tma_load_2d(S.rh[st], &tm_rh4, &S.in_full[st], p0, cg * 4);
@@ -1608,8 +1607,8 @@ __global__ void k_prep_w(const double *__restrict__ linv, const double *__restri
   }
 }
 
-// largest |x| of every dimension (cmax[0..63], zero for dimensions >= d) and
-// of all (cmax[64]); cmax starts at zero
+// largest |x| of every dimension (cmax[0..d - 1], zero at the start): the units of
+// the split covariance
 __global__ void __launch_bounds__(256)
 k_col_max(const float *__restrict__ X, int64_t n, int d, float *__restrict__ cmax) {
   __shared__ int sm[kD];
@@ -1625,22 +1624,25 @@ k_col_max(const float *__restrict__ X, int64_t n, int d, float *__restrict__ cma
     atomicMax(&sm[c], __float_as_int(m));
   }
   __syncthreads();
-  if (threadIdx.x < d) {
-    // non-negative floats order like their bits
-    atomicMax(reinterpret_cast<int *>(cmax) + threadIdx.x, sm[threadIdx.x]);
-    atomicMax(reinterpret_cast<int *>(cmax) + kD, sm[threadIdx.x]);
-  }
+  // non-negative floats order like their bits
+  if (threadIdx.x < d) atomicMax(reinterpret_cast<int *>(cmax) + threadIdx.x, sm[threadIdx.x]);
 }
 
-// row-major: x -> xh = fp16(x), xl = fp16(x - xh); transposed (d x np): x /
-// x_unit -> its nearest integer xh, the rest xl, and with XmT what FP16 leaves of it
+// x -> xh = fp16(x), xl = fp16(x - xh), row-major and transposed (d x np) (rows of
+// d < 64 values are zero-padded to 64; X64 receives the padded FP32 rows when it is
+// not null), and the largest |x|.  UNITS: the split covariance's three parts as well.
+template <bool UNITS>
 __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half *__restrict__ Xh,
                           __half *__restrict__ Xl, __half *__restrict__ XhT, __half *__restrict__ XlT,
-                          __half *__restrict__ XmT, int64_t np, float *__restrict__ X64, const float *__restrict__ cmax) {
-  __shared__ __half th[kD][65], tl[kD][65], tm[kD][65];
+                          __half *__restrict__ XgT, __half *__restrict__ XrT, __half *__restrict__ XmT, int64_t np,
+                          float *__restrict__ X64, const float *__restrict__ cmax, float *__restrict__ amax) {
+  constexpr int kParts = UNITS ? 5 : 2;
+  __shared__ __half t[kParts][kD][65];
   __shared__ float sinv[kD];
-  if (threadIdx.x < kD) sinv[threadIdx.x] = ldexpf(1.f, -x_unit_exp(cmax[threadIdx.x]));
+  if (UNITS && threadIdx.x < kD) sinv[threadIdx.x] = ldexpf(1.f, -x_unit_exp(cmax[threadIdx.x]));
   __syncthreads();
+  __half *const out[5] = {XhT, XlT, XgT, XrT, XmT};
+  float m = 0.f;
   const int64_t nt = (n + 63) / 64;
   for (int64_t tile = blockIdx.x; tile < nt; tile += gridDim.x) {
     const int64_t r0 = tile * 64;
@@ -1651,26 +1653,31 @@ __global__ void k_split_x(const float *__restrict__ X, int64_t n, int d, __half 
         if (X64) X64[(r0 + r) * kD + c] = x;
         const __half h = __float2half_rn(x);
         const __half l = __float2half_rn(x - __half2float(h));
-        Xh[(r0 + r) * kD + c] = h;
-        Xl[(r0 + r) * kD + c] = l;
-        const float u = x * sinv[c], ui = rintf(u);
-        th[c][r] = __float2half_rn(ui);
-        const __half ul = __float2half_rn(u - ui);
-        tl[c][r] = ul;
-        if (XmT) tm[c][r] = __float2half_rn((u - ui) - __half2float(ul));
+        Xh[(r0 + r) * kD + c] = t[0][c][r] = h;
+        Xl[(r0 + r) * kD + c] = t[1][c][r] = l;
+        m = fmaxf(m, fabsf(x));
+        if constexpr (UNITS) {
+          const float u = x * sinv[c], ui = rintf(u);
+          const __half ur = __float2half_rn(u - ui);
+          t[2][c][r] = __float2half_rn(ui);
+          t[3][c][r] = ur;
+          t[4][c][r] = __float2half_rn((u - ui) - __half2float(ur));
+        }
       }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 64 * kD; e += blockDim.x) {
       const int c = e / 64, r = e - c * 64;
-      if (r0 + r < n) {
-        XhT[(size_t)c * np + r0 + r] = th[c][r];
-        XlT[(size_t)c * np + r0 + r] = tl[c][r];
-        if (XmT) XmT[(size_t)c * np + r0 + r] = tm[c][r];
-      }
+      if (r0 + r < n)
+#pragma unroll
+        for (int p = 0; p < kParts; p++) out[p][(size_t)c * np + r0 + r] = t[p][c][r];
     }
     __syncthreads();
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+  // non-negative floats order like their bits
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
 }
 
 // one warp, a lane's terms first, then a fixed tree
@@ -1817,9 +1824,13 @@ int em_tc_create(fem_em *h) {
       split_rows(n, kBlk, p->cgx, sms, 12.0, &p->cgy, &p->srows);
       FEM_TRY(dalloc(&p->cpart, (size_t)p->cgx * p->cgy * 2 * kD * 128));
       FEM_TRY(dalloc(&p->dpart, (size_t)p->cgx * p->cgy * 4 * 4 * kD));
-      FEM_TRY(dalloc(&p->XmT, (size_t)kD * p->np));
-      FEM_TRY(encode_tmap_2d(&p->tm_xmt, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p->XmT, (uint64_t)n, kD, kBlk, kD,
-                             CU_TENSOR_MAP_SWIZZLE_128B, (uint64_t)p->np * 2));
+      __half **parts[3] = {&p->XgT, &p->XrT, &p->XmT};
+      CUtensorMap *maps[3] = {&p->tm_xgt, &p->tm_xrt, &p->tm_xmt};
+      for (int q = 0; q < 3; q++) {
+        FEM_TRY(dalloc(parts[q], (size_t)kD * p->np));
+        FEM_TRY(encode_tmap_2d(maps[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, *parts[q], (uint64_t)n, kD, kBlk, kD,
+                               CU_TENSOR_MAP_SWIZZLE_128B, (uint64_t)p->np * 2));
+      }
     }
   } else {
     p->cgy = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks, (4 * sms + p->cgx - 1) / p->cgx));
@@ -1872,6 +1883,8 @@ void em_tc_destroy(fem_em *h) {
   dfree(p->Rl);
   dfree(p->XhT);
   dfree(p->XlT);
+  dfree(p->XgT);
+  dfree(p->XrT);
   dfree(p->XmT);
   dfree(p->lsc);
   dfree(p->epart);
@@ -1895,9 +1908,9 @@ int em_tc_upload(fem_em *h) {
   float *amax = p->amax;
   FEM_CUDA(cudaMemsetAsync(amax, 0, (kD + 1) * sizeof(float), h->stream));
   const int blocks = (int)std::min<int64_t>(4 * sm_count(), (h->n + 63) / 64);
-  k_col_max<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, amax);
-  k_split_x<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, h->Xhi, h->Xlo, p->XhT, p->XlT, p->XmT, p->np,
-                                            p->X64, amax);
+  if (p->srows) k_col_max<<<blocks, 256, 0, h->stream>>>(h->X, h->n, h->d, amax);
+  (p->srows ? k_split_x<true> : k_split_x<false>)<<<blocks, 256, 0, h->stream>>>(
+      h->X, h->n, h->d, h->Xhi, h->Xlo, p->XhT, p->XlT, p->XgT, p->XrT, p->XmT, p->np, p->X64, amax, amax + kD);
   float m = 0.f;
   cudaMemcpyAsync(&m, amax + kD, sizeof(float), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -1949,8 +1962,8 @@ int em_tc_mstep(fem_em *h) {
     timing_begin(h, 8);
     if (p->srows) {
       k_cov_split<<<dim3(p->cgx, p->cgy), kSThreads, ssmem_bytes(), h->stream>>>(
-          p->tm_xht, p->tm_xlt, p->tm_xmt, p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf, p->amax, p->zunit, h->n, p->srows, p->cpart, p->dpart,
-          p->err);
+          p->tm_xgt, p->tm_xrt, p->tm_xmt, p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf, p->amax, p->zunit, h->n, p->srows,
+          p->cpart, p->dpart, p->err);
       FEM_CUDA(cudaGetLastError());
       timing_begin(h, 9);
       k_final_cov_split<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(
@@ -1970,11 +1983,11 @@ int em_tc_mstep(fem_em *h) {
   timing_begin(h, 8);
   if (cov_zx_enabled()) {
     k_cov_zx<<<dim3(p->cgx, p->cgy), kZThreads, zsmem_bytes(), h->stream>>>(
-        p->tm_xht, p->tm_xlt, p->tm_rh4, p->muf, p->amax, h->n, bpc, p->cpart, p->err);
+        p->tm_xht, p->tm_xlt, p->tm_rh4, p->muf, h->n, bpc, p->cpart, p->err);
     FEM_CUDA(cudaGetLastError());
     timing_begin(h, 9);
-    k_final_cov_zx<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, p->amax,
-                                                                          h->sigma);
+    k_final_cov_zx<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(p->cpart, p->cgx, p->cgy, h->d, h->psum,
+                                                                          h->mu, p->muf, h->sigma);
   } else {
     k_cov_tc<<<dim3(p->cgx, p->cgy), kCThreads, csmem_bytes(), h->stream>>>(p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf,
                                                                            h->n, bpc, p->cpart, p->dpart, p->err);

@@ -96,10 +96,14 @@ __device__ __forceinline__ void factor_divide(double (&u)[N], double p) {
 template <int NS>
 __device__ inline bool block_factor_smem(double *A, double *W, double *piv, double *rd, double *m, int d, int ld) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nu = (blockDim.x >> 5) - 1;
+  // by column parity: warp 0 may be in the next column, and set its flag, before
+  // the slowest warp has read this one's behind the column's only barrier
+  __shared__ int s_fail[2];
+  if (threadIdx.x < 2) s_fail[threadIdx.x] = 0;
+  __syncthreads();
   bool ok = true;
   for (int k = -1; k < d - 1; k++) {
     const double *mk = m + (k & 1) * d;
-    int bad = 0;
     if (warp == 0) {
       const int c = k + 1;
       double u[NS];
@@ -113,7 +117,7 @@ __device__ inline bool block_factor_smem(double *A, double *W, double *piv, doub
       const double p = __shfl_sync(0xffffffffu, u[0], 0);
       const long long pb = __double_as_longlong(p);
       if (pb <= 0 || pb > 0x7ff0000000000000LL) {    // !(p > 0), without waiting for the FP64 pipe
-        bad = 1;
+        if (lane == 0) s_fail[k & 1] = 1;
       } else {
         double *mc = m + (c & 1) * d;
 #pragma unroll
@@ -149,9 +153,8 @@ __device__ inline bool block_factor_smem(double *A, double *W, double *piv, doub
         }
       }
     }
-    // the barrier carries the verdict: a flag in shared memory could already hold
-    // the next column's when a slow warp reads it, and the warps would part
-    if (__syncthreads_or(bad)) {
+    __syncthreads();
+    if (s_fail[k & 1]) {
       ok = false;
       break;
     }

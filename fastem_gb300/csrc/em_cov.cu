@@ -152,7 +152,8 @@ template <typename T, int TB, bool TRI, class Src>
 __global__ void __launch_bounds__(kCvThreads, sizeof(T) == 4 ? 2 : 1)
 k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T *__restrict__ mu, int mu_ld,
             double *__restrict__ part, int nb, int nblk, int64_t rows_per_chunk, int upc, int G, int TP, int xpitch,
-            int rpitch, int cjmax) {
+            int rpitch, int cjmax, const int *__restrict__ gate) {
+  if (gate && !(gate[0] | gate[1])) return;
   constexpr int NE = cv_ne(TB, TRI);
   // FP32 blocks of 8 x 8: two columns per instruction
   constexpr bool PK = sizeof(T) == 4 && TB == 8 && !TRI;
@@ -369,7 +370,8 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
 // fits to a chain of L2 loads (d = 24, K = 21: 248 -> 9 us).
 __global__ void __launch_bounds__(256)
 k_final_cov(const double *__restrict__ part, int chunks, int K, int d, int nb, int nblk, int TB, int tri,
-            const double *__restrict__ psum, double *__restrict__ sigma) {
+            const double *__restrict__ psum, double *__restrict__ sigma, const int *__restrict__ gate) {
+  if (gate && !(gate[0] | gate[1])) return;
   __shared__ double red[8][32];
   const int units = K * nblk, ne = tri ? TB * (TB + 1) / 2 : TB * TB;
   const int64_t per = (int64_t)units * ne;
@@ -650,7 +652,7 @@ int em_means_plain(fem_em *h) {
 
 // partials + FP64 finalisation for one posterior source
 template <typename T, class Src>
-static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld) {
+static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld, const int *gate = nullptr) {
   const CovPlan &p = h->cov;
   const int d = h->d, K = h->k;
   if (p.smem > kCvMaxSmem) {
@@ -663,7 +665,7 @@ static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld) {
     FEM_CUDA(allow_dyn_smem(k_cov_units<T, TB, TRI, Src>, p.smem));                                            \
     k_cov_units<T, TB, TRI, Src><<<grid, kCvThreads, p.smem, h->stream>>>(                                     \
         h->X, h->n, d, K, src, mu, mu_ld, h->cpart, p.nb, p.nblk, p.rows, p.upc, p.G, p.TP, p.xpitch, p.rpitch, \
-        p.cj);                                                                                                 \
+        p.cj, gate);                                                                                           \
   } while (0)
   if (p.TB == 4)
     FEM_CV(4, true);
@@ -675,13 +677,14 @@ static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld) {
   FEM_CUDA(cudaGetLastError());
   const int64_t per = (int64_t)K * p.nblk * (p.tri ? p.TB * (p.TB + 1) / 2 : p.TB * p.TB);
   k_final_cov<<<(unsigned)((per + 31) / 32), 256, 0, h->stream>>>(h->cpart, p.chunks, K, d, p.nb, p.nblk, p.TB, p.tri,
-                                                                  h->psum, h->sigma);
+                                                                  h->psum, h->sigma, gate);
   FEM_CUDA(cudaGetLastError());
   return FEM_OK;
 }
 
-int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld) {
-  FEM_TRY((cov_pass<float, PostHiLo>(h, PostHiLo{Rh, Rl, pitch}, muf, mu_ld)));
+int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld,
+                const int *gate) {
+  FEM_TRY((cov_pass<float, PostHiLo>(h, PostHiLo{Rh, Rl, pitch}, muf, mu_ld, gate)));
   h->launches += 2;
   return FEM_OK;
 }

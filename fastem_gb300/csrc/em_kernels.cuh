@@ -32,9 +32,11 @@ int em_means_plain(fem_em *h);
 CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo);
 int em_cov_plain(fem_em *h);
 // the mixed path's covariance on CUDA cores in FP32 (for small components):
-// posteriors as FP16 hi + lo, means as float with row stride mu_ld
-int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld);
-// true when the mixed path (after em_tc_create) computes covariances with em_cov_hilo
+// posteriors as FP16 hi + lo, means as float with row stride mu_ld; with a gate
+// (device, two words) only when one of them is set
+int em_cov_hilo(fem_em *h, const __half *Rh, const __half *Rl, int64_t pitch, const float *muf, int mu_ld,
+                const int *gate);
+// true when the mixed path (after em_tc_create) may compute covariances with em_cov_hilo
 bool em_tc_cuda_core_cov(const fem_em *h);
 // device posteriors of the mixed path: FP16 hi / lo, component-major, row pitch
 void em_tc_posteriors(fem_em *h, const __half **rh, const __half **rl, int64_t *pitch);

@@ -147,8 +147,10 @@ static_assert(kZACol + kZA * kZAStage <= 512 && 3 * kZDCol + kZN <= kZACol, "cov
 constexpr int kSIn = 4;                  // input ring (blocks)
 constexpr int kSSteps = kBlk / 16;
 constexpr int kSA = 6;                   // TMEM A ring (steps)
-constexpr int kSAcc = 16;                // blocks a zh xg^T accumulator spans
+constexpr int kSAccLong = 16, kSAccShort = 4;   // blocks a zh xg^T accumulator spans
+constexpr int kSAccWeight = 24;          // the short span from 1 / 24 of all posterior weight in one component on
 constexpr int kSWin = 64;                // blocks an FP32 register sum spans (4096 rows)
+constexpr int kSCrossWin = 256;          // blocks the small products' accumulator spans
 constexpr int kSRows = 2048;             // rows an FP32 diagonal sum spans
 // TMEM columns: [pair] zh [xg; 1]^T, [pair] the small products, A ring (per pair 8 hi + 8 lo a step)
 constexpr int kSN = kD + 16;             // accumulator columns per pair: 64 sums, sum z, 15 unused
@@ -156,9 +158,10 @@ constexpr uint32_t kSCross = 2 * kSN, kSACol = 4 * kSN, kSAStage = 32;
 // warps 0 TMA, 1 MMA, 2 posteriors, 3 none; 4..19 producers (4 groups); 20..27 flush (a group of 4 per pair)
 constexpr int kSThreads = 28 * 32;
 constexpr int kSProd0 = 4, kSFlush0 = 20;
-// registers per thread after the split: 128 threads x 24 + 512 x 72 + 256 x
-// 96 = 64512 = the launch's 896 x 72
-constexpr int kSRegLaunch = 72, kSRegCtl = 24, kSRegProd = 72, kSRegFlush = 96;
+// registers per thread after the split: 128 threads x 56 + 512 x 64 + 256 x 96 =
+// 64512 = the launch's 896 x 72 (with 24, 72, 96 the MMA warp spills in its loop: N =
+// 2^20, d = 64, K = 128 5.93 ms against 5.32; 40, 64, 104: 5.36)
+constexpr int kSRegLaunch = 72, kSRegCtl = 56, kSRegProd = 64, kSRegFlush = 96;
 static_assert(128 * kSRegCtl + 512 * kSRegProd + 256 * kSRegFlush <= kSThreads * kSRegLaunch, "register split");
 static_assert(kSACol + kSA * kSAStage <= 512, "split covariance TMEM columns");
 struct __align__(1024) SSmem {
@@ -170,7 +173,7 @@ struct __align__(1024) SSmem {
   float mu[4][kD];                                   // means of the CTA's components in column units
   float zs[4][kD], zm[4][kD];                        // 1 / zunit, -mu / zunit
   uint64_t in_full[kSIn], rf_full[kSIn], in_empty[kSIn], a_full[kSA], a_empty[kSA], acc_full, acc_empty, cross_full,
-      mma_done;
+      cross_empty, mma_done;
   uint32_t tmem_base;
 };
 static_assert(sizeof(SSmem) + 1024 <= 232448, "split covariance shared memory");
@@ -199,6 +202,7 @@ struct TcEmPlan {
   int *err = nullptr;                   // device status of the bounded waits
   float *amax = nullptr;                // upload: largest |x| of every dimension (split covariance), then of all (FP16 range check)
   float *zunit = nullptr;               // split covariance: unit of z per component and dimension
+  int *coarse = nullptr;                // split covariance: grids too coarse, [0] before the sums and [1] by their result
   int *roles = nullptr;                 // bounded-wait expiry self-test: which waits gave up
   int egrid = 0, mgrid = 0, cgx = 0, cgy = 0;
   int64_t srows = 0;                    // split form: rows per chunk (0: not used)
@@ -228,14 +232,27 @@ __device__ __forceinline__ int x_unit_exp(float cmax) { return cmax > 0.f ? max(
 __device__ __forceinline__ float x_unit(float cmax) { return ldexpf(1.f, x_unit_exp(cmax)); }
 
 // unit of z = r (x - mu) in the split covariance: 2^-9 of the standard
-// deviation that the E-step used (sigma: its covariance's diagonal entry), so
+// deviation that the E-step used (var: its covariance's diagonal entry), so
 // most rows are integers below 2^11, but no less than keeps |z| <= 2 max|x|
-// below 2^15 units whatever sigma says
+// below 2^15 units whatever var says, and no more than 2^-9 of max |x|
 __device__ __forceinline__ float z_unit(double var, float cmax) {
   const int lo = x_unit_exp(cmax) - 3;
   int e = lo;
-  if (var > 1e-60 && var < 1e60) e = max(lo, ilogb(sqrt(var)) - 9);
-  return ldexpf(1.f, min(e, 100));
+  if (var > 1e-60 && var < 1e60) e = max(lo, min(ilogb(sqrt(var)) - 9, lo + 4));
+  return ldexpf(1.f, e);
+}
+
+// The split covariance's grids against the standard deviation sd of a component's
+// dimension: z has 2^-13 of its unit left out, the tensor core cuts sums that an
+// offset makes large, and the unit follows the column's maximum.  Up to max |x| = 32
+// sd and a unit of 2^-8 sd the split form is as exact as FP32 sums on CUDA cores,
+// beyond that those are formed (rms error of Sigma_ab / (sd_a sd_b) against 64-bit
+// sums, N = 2^18, d = 64, K = 128, split and CUDA cores: 1.7e-9 and 2.0e-9 at 12 sd,
+// 2.4e-9 and 1.9e-9 at 37, 5.6e-9 and 1.8e-9 at 100, 2.4e-8 and 1.8e-9 at 340).
+constexpr float kSRange = 32.f, kSUnits = 256.f;
+__device__ __forceinline__ bool split_too_coarse(double var, float cmax, float zunit) {
+  const float sd = (float)sqrt(var);
+  return cmax > 0.f && !(cmax <= kSRange * sd && kSUnits * zunit <= sd);
 }
 
 // ============================================================== E-step
@@ -512,8 +529,9 @@ k_estep_tc(const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CU
 __global__ void __launch_bounds__(192, 1)
 k_means_tc(const __grid_constant__ CUtensorMap tm_rh, const __grid_constant__ CUtensorMap tm_rl,
            const __grid_constant__ CUtensorMap tm_xht, const __grid_constant__ CUtensorMap tm_xlt,
-           int64_t n, double *__restrict__ part, int *err) {
+           int64_t n, double *__restrict__ part, int *coarse, int *err) {
   extern __shared__ uint8_t smem_raw[];
+  if (blockIdx.x == 0 && threadIdx.x < 2) coarse[threadIdx.x] = 0;   // this M-step's
   MSmem &S = smem_aligned<MSmem>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t nblocks = (n + kBlk - 1) / kBlk;
@@ -632,7 +650,8 @@ constexpr int kFMSplit = 4, kFMCols = kD + 1;
 __global__ void __launch_bounds__(kFMSplit * kFMCols)
 k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n, double *__restrict__ mu,
                  double *__restrict__ pi, double *__restrict__ psum, float *__restrict__ muf,
-                 const float *__restrict__ cmax, const double *__restrict__ sigma, float *__restrict__ zunit) {
+                 const float *__restrict__ cmax, const double *__restrict__ sigma, float *__restrict__ zunit,
+                 int *__restrict__ coarse) {
   const int j = blockIdx.x, q = threadIdx.x % kFMCols, w = threadIdx.x / kFMCols;
   __shared__ double red[kFMSplit][kFMCols];
   double s = 0.0;
@@ -654,7 +673,10 @@ k_final_means_tc(const double *__restrict__ part, int G, int K, int d, int64_t n
   const double m = s / s1;
   if (q < d) mu[(size_t)j * d + q] = m;
   muf[(size_t)j * kD + q] = q < d ? (float)m : 0.f;
-  zunit[(size_t)j * kD + q] = q < d ? z_unit(sigma[((size_t)j * d + q) * d + q], cmax[q]) : 1.f;
+  const double var = q < d ? sigma[((size_t)j * d + q) * d + q] : 1.0;
+  const float zu = q < d ? z_unit(var, cmax[q]) : 1.f;
+  zunit[(size_t)j * kD + q] = zu;
+  if (q < d && split_too_coarse(var, cmax[q], zu)) coarse[0] = 1;
 }
 
 // ========================================================= covariances
@@ -1183,36 +1205,46 @@ k_final_cov_zx(const double *__restrict__ cpart, int gx, int gy, int d, const do
 // To reach the accuracy of FP32 sums on CUDA cores:
 //  * the tensor core truncates its FP32 accumulator, so z is put on a grid as x
 //    is (z_unit: zh an integer, |zl| <= 1/2): zh xg^T then adds up exactly below
-//    2^24 units, which kSAcc blocks of a component rarely reach (beyond it,
-//    truncation is as for any FP32 sum).  With a floating split every addition
-//    truncates: 4e-8 to 7e-8 off where FP32 sums on CUDA cores are at 1e-8;
-//  * the small products have an accumulator of their own over the chunk; z
-//    comes from the FP32 rows, and x on the B side has a third part xm;
+//    2^24 units.  Sums pass that more often the more rows a component has among
+//    them, so the accumulator spans 16 blocks where none of the CTA's components
+//    has a 24th of all weight and 4 elsewhere (rms error of Sigma_ab / (sd_a sd_b)
+//    with 16 throughout: K = 12 3.2e-9, half the weight in one of 128 1.3e-8; now
+//    1.2e-9 and 2.5e-9; CUDA cores 1.5e-9 and 4.2e-9).  With a floating split every
+//    addition truncates: 4e-8 to 7e-8 off where CUDA cores are at 1e-8;
+//  * the small products have an accumulator of their own (over a whole chunk its
+//    truncation shows: N = 2^20, K = 128 1.4e-9, every kSCrossWin blocks 9e-10, CUDA
+//    cores 1.1e-9); z comes from the FP32 rows, and x on the B side has a third
+//    part xm;
 //  * x on the B side is shared by all components and so not centred: a sum
 //    holds (sum z) mu^T, random and |mu| / sigma times larger than what is
 //    wanted.  A row of ones in B gives sum zh (exact) and sum zl beside the
 //    sums, and flush warps take the product off before they add to FP32
 //    registers (round to nearest); those go to FP64 every kSWin blocks;
 //  * the diagonal is summed by the producers from the unrounded z (FP32 over
-//    at most kSRows rows, then FP64).
+//    at most kSRows rows, then FP64);
+//  * where a grid is too coarse for a component (split_too_coarse, by the E-step's
+//    covariances before and by the result behind) the sums are formed on CUDA cores
+//    instead: this kernel or that one returns at once.
 // Sums are in units of z (rows) and x (columns), whatever the data's scale.
 // Warp roles: 0 TMA, 1 MMA, 2 turns the posteriors into FP32 once per block;
 // four producer groups of 4 warps, group g forming step g of every block (a
-// warp's lanes and dimensions as in k_cov_zx); a flush group of 4 warps per pair, 64 sums per thread (which is why the
-// registers are split unevenly).
+// warp's lanes and dimensions as in k_cov_zx); a flush group of 4 warps per pair, 64
+// sums per thread (which is why the registers are split unevenly).
 // What bounds it: shared memory, read by producers (x, posteriors) and by the
 // 40 MMAs of a block (B), written by TMA, ~1800 of the ~3000 cycles a block
 // takes; without 24 of the MMAs it is 13 % faster, with waits that sleep
 // instead of polling no different.  GB300, with its finalisation, against the
-// FP32 CUDA-core form: N = 2^20, d = 64, K = 128 20.7 -> 5.4 ms, N = 200000,
-// d = 64, K = 32 1.19 -> 0.32 ms; error of Sigma (Frobenius) against 64-bit
-// sums over the same posteriors 8e-9 and 9e-9 (CUDA cores 8e-9 and 1.6e-8).
+// FP32 CUDA-core form: N = 2^20, d = 64, K = 128 20.7 -> 5.3 ms, N = 250000,
+// d = 64, K = 24 0.98 -> 0.35 ms; error of Sigma (Frobenius) against 64-bit
+// sums over the same posteriors 9.5e-9 and 1.0e-8 (CUDA cores 1.0e-8 and 1.7e-8).
 __global__ void __launch_bounds__(kSThreads, 1)
 k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ CUtensorMap tm_xrt,
             const __grid_constant__ CUtensorMap tm_xmt, const __grid_constant__ CUtensorMap tm_x32,
             const __grid_constant__ CUtensorMap tm_rh4, const __grid_constant__ CUtensorMap tm_rl4,
             const float *__restrict__ muf, const float *__restrict__ cmax, const float *__restrict__ zunit, int64_t n,
-            int64_t rows_per_chunk, double *__restrict__ cpart, double *__restrict__ dpart, int *err) {
+            int64_t rows_per_chunk, const double *__restrict__ psum, int K, double *__restrict__ cpart,
+            double *__restrict__ dpart, const int *__restrict__ coarse, int *err) {
+  if (coarse[0]) return;
   extern __shared__ uint8_t smem_raw[];
   SSmem &S = smem_aligned<SSmem>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1229,9 +1261,13 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ 
     mbar_init(&S.acc_full, 1);
     mbar_init(&S.acc_empty, 8);
     mbar_init(&S.cross_full, 1);
+    mbar_init(&S.cross_empty, 8);
     mbar_init(&S.mma_done, 1);
     fence_mbar_init();
   }
+  double wmax = 0.0;
+  for (int q = 0; q < 4 && 4 * cg + q < K; q++) wmax = fmax(wmax, psum[4 * cg + q]);
+  const int am = (kSAccWeight * wmax <= (double)n ? kSAccLong : kSAccShort) - 1;   // span - 1
   // 16-byte chunk c of row r stored at c ^ (r & 7)
   for (int e = threadIdx.x; e < kSIn * 16 * kBlk; e += blockDim.x) {
     const int st = e / (16 * kBlk), rem = e - st * 16 * kBlk;
@@ -1281,7 +1317,7 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ 
       if (elect_one()) {
         bool ok = true;
         constexpr uint32_t id = idesc_f16(128, kD), idn = idesc_f16(128, kSN);
-        uint32_t sl = 0, sp = 0;                   // operand slot and its phase
+        uint32_t sl = 0, sp = 0, ap = 0;           // operand slot and its phase; accumulator phase
         for (int t = 0; t < mine && ok; t++) {
           const int st = t % kSIn;
           if (!(ok = mbar_wait(&S.in_full[st], (t / kSIn) & 1, err))) break;
@@ -1292,30 +1328,34 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ 
             if (!(ok = mbar_wait(&S.a_full[sl], sp, err))) break;
             tc_fence_after();
             const uint32_t at = tbase + kSACol + sl * kSAStage;
+            if (t % kSCrossWin == 0 && kb == 0) {
+              if (!(ok = mbar_wait(&S.cross_empty, ((t / kSCrossWin) & 1) ^ 1, err))) break;
+              tc_fence_after();
+            }
 #pragma unroll
             for (int pr = 0; pr < 2; pr++) {
               // +32 bytes per 16-point step inside the 128-byte swizzle row
               const uint32_t dc = tbase + kSCross + pr * kSN, ah = at + 16 * pr, al = ah + 8;
-              mma_f16_ta(dc, al, dbh + 2 * kb, idn, (t | kb) != 0);
+              mma_f16_ta(dc, al, dbh + 2 * kb, idn, (t % kSCrossWin | kb) != 0);
               mma_f16_ta(dc, al, dbl + 2 * kb, id, 1);
               mma_f16_ta(dc, ah, dbl + 2 * kb, id, 1);
               mma_f16_ta(dc, ah, dbm + 2 * kb, id, 1);
             }
-            if (t % kSAcc == 0 && kb == 0) {
-              if (!(ok = mbar_wait(&S.acc_empty, ((t / kSAcc) & 1) ^ 1, err))) break;
+            if ((t & am) == 0 && kb == 0) {
+              if (!(ok = mbar_wait(&S.acc_empty, ap ^ 1, err))) break;
               tc_fence_after();
             }
 #pragma unroll
             for (int pr = 0; pr < 2; pr++)
-              mma_f16_ta(tbase + pr * kSN, at + 16 * pr, dbh + 2 * kb, idn, (t % kSAcc != 0) || kb);
+              mma_f16_ta(tbase + pr * kSN, at + 16 * pr, dbh + 2 * kb, idn, (t & am) || kb);
             mma_commit(&S.a_empty[sl]);
             if (++sl == kSA) sl = 0, sp ^= 1;
           }
           if (!ok) break;
           mma_commit(&S.in_empty[st]);
-          if (t % kSAcc == kSAcc - 1 || t + 1 == mine) mma_commit(&S.acc_full);
+          if ((t & am) == am || t + 1 == mine) mma_commit(&S.acc_full), ap ^= 1;
+          if (t % kSCrossWin == kSCrossWin - 1 || t + 1 == mine) mma_commit(&S.cross_full);
         }
-        if (ok) mma_commit(&S.cross_full);
         mma_commit(&S.mma_done);
         mbar_wait_drain(&S.mma_done, 0);
       }
@@ -1451,18 +1491,22 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ 
       }
     };
     bool ok = true, first = true;
-    for (int t0 = 0; t0 < mine && ok; t0 += kSAcc) {
-      const int t1 = std::min(mine, t0 + kSAcc);
-      if (!(ok = mbar_wait_lazy_warp(&S.acc_full, (t0 / kSAcc) & 1, err, 500))) break;
+    uint32_t ap = 0;
+    for (int t0 = 0; t0 < mine && ok; t0 += am + 1, ap ^= 1) {
+      const int t1 = std::min(mine, t0 + am + 1);
+      if (!(ok = mbar_wait_lazy_warp(&S.acc_full, ap, err, 500))) break;
       tc_fence_after();
       take(ta);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&S.acc_empty);
-      if (t1 == mine) {
-        if (!(ok = mbar_wait_warp(&S.cross_full, 0, err))) break;
+      if (t1 == mine || t1 % kSCrossWin == 0) {
+        if (!(ok = mbar_wait_warp(&S.cross_full, ((t1 - 1) / kSCrossWin) & 1, err))) break;
         tc_fence_after();
         take(ta + kSCross);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.cross_empty);
       }
       if (t1 == mine || t1 % kSWin == 0) {
 #pragma unroll
@@ -1483,11 +1527,13 @@ k_cov_split(const __grid_constant__ CUtensorMap tm_xgt, const __grid_constant__ 
 
 // Sigma_j = sym(sum z (x - muf)^T) / N_j - (mu - muf)(mu - muf)^T, the
 // producers' sums on the diagonal; chunks summed in order (FP64).
-// A CTA owns rows 16 blockIdx.y .. + 15 of component blockIdx.x.
+// A CTA owns rows 8 blockIdx.y .. + 7 of component blockIdx.x.
 __global__ void __launch_bounds__(512)
 k_final_cov_split(const double *__restrict__ cpart, const double *__restrict__ dpart, int gx, int gy, int d,
                   const double *__restrict__ psum, const double *__restrict__ mu, const float *__restrict__ muf,
-                  const float *__restrict__ cmax, const float *__restrict__ zunit, double *__restrict__ sigma) {
+                  const float *__restrict__ cmax, const float *__restrict__ zunit, double *__restrict__ sigma,
+                  int *coarse) {
+  if (coarse[0]) return;
   const int j = blockIdx.x, grp = j / 4, c = j % 4, pr = c >> 1, slot = c & 1;
   const int a0 = blockIdx.y * kFCRows;
   __shared__ double sr[kFCRows][kD + 1], sc[kD][kFCRows + 1], sd[kFCRows];
@@ -1524,6 +1570,7 @@ k_final_cov_split(const double *__restrict__ cpart, const double *__restrict__ d
     const double t = a == b ? sd[i] * ga * ga
                             : 0.5 * (sr[i][b] * (ga * x_unit(cmax[b])) + sc[b][i] * (gb * x_unit(cmax[a])));
     const double v = t * inv - da * db;
+    if (a == b && split_too_coarse(v, cmax[a], zunit[(size_t)j * kD + a])) coarse[1] = 1;
     Sg[a * d + b] = v;
     Sg[b * d + a] = v;
   }
@@ -1765,7 +1812,7 @@ static bool cov_zx_enabled() {
 // 8 x 8 blocks of the triangle, so it is ahead up to d = 32 (N = 10^5, K = 12,
 // d = 32: 86 against 130 us; N = 200003, K = 21, d = 24: 147 against 240) and
 // the split form above (N = 500000, K = 64, d = 48: 1.3 against 3.5 ms; N =
-// 2^20, K = 128, d = 64: 5.4 against 20.7 ms), once every SM has 16 or more of
+// 2^20, K = 128, d = 64: 5.3 against 20.7 ms), once every SM has 16 or more of
 // its (64-point block, 4-component group) units to pay for a CTA's start and
 // end (K = 8, d = 64: N = 20000, 4 a SM, 57 against 102 us; N = 100000, 20 a
 // SM, 227 against 143 us).
@@ -1809,6 +1856,7 @@ int em_tc_create(fem_em *h) {
   FEM_TRY(dalloc(&p->amax, kD + 1));
   FEM_CUDA(cudaMemset(p->amax, 0, (kD + 1) * sizeof(float)));
   FEM_TRY(dalloc(&p->zunit, (size_t)K * kD));
+  FEM_TRY(dalloc(&p->coarse, 2));
   FEM_TRY(dalloc(&p->roles, 4));
   const int64_t npairs = ((n + kTileM - 1) / kTileM + 1) / 2;
   p->egrid = (int)std::min<int64_t>(sms, npairs);
@@ -1867,9 +1915,7 @@ int em_tc_create(fem_em *h) {
   return FEM_OK;
 }
 
-bool em_tc_cuda_core_cov(const fem_em *h) {
-  return h->tc && em_tc_small_components(h->n, h->k, h->d) && !h->tc->srows;
-}
+bool em_tc_cuda_core_cov(const fem_em *h) { return h->tc && em_tc_small_components(h->n, h->k, h->d); }
 
 void em_tc_destroy(fem_em *h) {
   em_wide_destroy(h);
@@ -1897,6 +1943,7 @@ void em_tc_destroy(fem_em *h) {
   dfree(p->err);
   dfree(p->amax);
   dfree(p->zunit);
+  dfree(p->coarse);
   dfree(p->roles);
   delete p;
   h->tc = nullptr;
@@ -1953,27 +2000,26 @@ int em_tc_mstep(fem_em *h) {
   TcEmPlan *p = h->tc;
   const int K = h->k;
   k_means_tc<<<p->mgrid, 192, msmem_bytes(), h->stream>>>(p->tm_rh, p->tm_rl, p->tm_xht, p->tm_xlt, h->n,
-                                                           p->mpart, p->err);
+                                                           p->mpart, p->coarse, p->err);
   FEM_CUDA(cudaGetLastError());
   k_final_means_tc<<<K, kFMSplit * kFMCols, 0, h->stream>>>(p->mpart, p->mgrid, K, h->d, h->n, h->mu, h->pi, h->psum,
-                                                               p->muf, p->amax, h->sigma, p->zunit);
+                                                               p->muf, p->amax, h->sigma, p->zunit, p->coarse);
   FEM_CUDA(cudaGetLastError());
   if (em_tc_small_components(h->n, h->k, h->d)) {
     timing_begin(h, 8);
     if (p->srows) {
       k_cov_split<<<dim3(p->cgx, p->cgy), kSThreads, ssmem_bytes(), h->stream>>>(
-          p->tm_xgt, p->tm_xrt, p->tm_xmt, p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf, p->amax, p->zunit, h->n, p->srows,
-          p->cpart, p->dpart, p->err);
+          p->tm_xgt, p->tm_xrt, p->tm_xmt, p->tm_x32, p->tm_rh4, p->tm_rl4, p->muf, p->amax, p->zunit, h->n, p->srows, h->psum,
+          K, p->cpart, p->dpart, p->coarse, p->err);
       FEM_CUDA(cudaGetLastError());
-      timing_begin(h, 9);
       k_final_cov_split<<<dim3(K, (h->d + kFCRows - 1) / kFCRows), 512, 0, h->stream>>>(
-          p->cpart, p->dpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, p->amax, p->zunit, h->sigma);
+          p->cpart, p->dpart, p->cgx, p->cgy, h->d, h->psum, h->mu, p->muf, p->amax, p->zunit, h->sigma, p->coarse);
       FEM_CUDA(cudaGetLastError());
       h->launches += 2;
-    } else {
-      FEM_TRY(em_cov_hilo(h, p->Rh, p->Rl, p->np, p->muf, kD));
-      timing_begin(h, 9);
     }
+    // the only form, or where the split one's grids are too coarse
+    FEM_TRY(em_cov_hilo(h, p->Rh, p->Rl, p->np, p->muf, kD, p->srows ? p->coarse : nullptr));
+    timing_begin(h, 9);
     k_flag_timeout<<<1, 32, 0, h->stream>>>(h->dstat, p->err);
     h->launches += 3;
     return FEM_OK;

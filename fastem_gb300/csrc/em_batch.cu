@@ -121,7 +121,8 @@ __device__ __forceinline__ double group_sum(const float *v, int n, int stride) {
     lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(x, b)));
     hi = t;
   }
-  return n > 1 ? (double)hi + (double)lo : (double)hi;
+  // an infinite sum has no error term (inf - inf above)
+  return isfinite(hi) ? (double)hi + (double)lo : (double)hi;
 }
 
 // deterministic block sum, result in thread 0

@@ -110,21 +110,6 @@ __device__ __forceinline__ double bwarp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
-// sum of n FP32 values `stride` apart, in order, to FP64: the rounding errors of
-// the FP32 additions are carried along exactly (two-sum), so three FP64
-// operations suffice instead of 2 n, which the FP64 pipe's rate would make a
-// tenth of a covariance item's time
-__device__ __forceinline__ double group_sum(const float *v, int n, int stride) {
-  float hi = v[0], lo = 0.f;
-  for (int g = 1; g < n; g++) {
-    const float x = v[g * stride], t = __fadd_rn(hi, x), b = __fsub_rn(t, hi);
-    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(x, b)));
-    hi = t;
-  }
-  // an infinite sum has no error term (inf - inf above)
-  return isfinite(hi) ? (double)hi + (double)lo : (double)hi;
-}
-
 // deterministic block sum, result in thread 0
 template <int NT>
 __device__ double bblock_sum(double v, double *red) {

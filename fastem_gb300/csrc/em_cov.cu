@@ -227,8 +227,8 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
   };
 
   bool first = true;
-  // adds the FP32 sums into this CTA's FP64 partials (or stores them); the
-  // groups' sums of a unit are added in T first, in group order
+  // adds the FP32 sums into this CTA's FP64 partials (or stores them), the groups'
+  // sums of a unit in group order and without FP32 rounding (group_sum)
   auto flush = [&](bool more) {
     if constexpr (PK) {
 #pragma unroll
@@ -256,10 +256,9 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
       const int live = min(upc, units - u0);
       for (int i = tid; i < live * NE; i += kCvThreads) {
         const int e = i / live, u = i - e * live;
-        T s = red[e * kCvThreads + u];
-        for (int q = 1; q < G; q++) s += red[e * kCvThreads + q * upc + u];
+        const double s = group_sum(red + e * kCvThreads + u, G, upc);
         double *p = o + (size_t)e * units + u;
-        *p = first ? (double)s : *p + (double)s;
+        *p = first ? s : *p + s;
       }
       __syncthreads();
     }

@@ -1,9 +1,11 @@
 // em_tri.cuh -- ||W t||^2 for a lower-triangular W in shared memory and several
 // points per thread, and the online log-sum-exp, shared by the single-fit and
 // batched E-steps (MatrixEMBase::BlockDensities and PostProcessDensityMatrix,
-// EM2/MatrixEM.cpp:39-51,69-81).
+// EM2/MatrixEM.cpp:39-51,69-81), and the addition of point groups' sums in the
+// M-steps (EM2/MatrixEM.cpp:309-378).
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 namespace fem {
@@ -131,6 +133,26 @@ __device__ __forceinline__ void lse_add(float l, float &mx, float &se) {
   const float a = l > mx ? fmaf(se, e, 1.f) : se + e;
   se = l > -INFINITY ? a : se;
   mx = fmaxf(l, mx);
+}
+
+// sum of n FP32 values `stride` apart, in order, to FP64: the rounding errors of
+// the FP32 additions are carried along exactly (two-sum), so three FP64
+// operations suffice instead of 2 n, which the FP64 pipe's rate would make a
+// tenth of a covariance item's time
+__device__ __forceinline__ double group_sum(const float *v, int n, int stride) {
+  float hi = v[0], lo = 0.f;
+  for (int g = 1; g < n; g++) {
+    const float x = v[g * stride], t = __fadd_rn(hi, x), b = __fsub_rn(t, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(x, b)));
+    hi = t;
+  }
+  // an infinite sum has no error term (inf - inf above)
+  return isfinite(hi) ? (double)hi + (double)lo : (double)hi;
+}
+__device__ __forceinline__ double group_sum(const double *v, int n, int stride) {
+  double s = v[0];
+  for (int g = 1; g < n; g++) s += v[g * stride];
+  return s;
 }
 
 }  // namespace fem

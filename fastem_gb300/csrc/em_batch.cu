@@ -59,7 +59,6 @@ constexpr int kBCChunk = 4096;   // points per covariance item
 constexpr int kBMTile = 128;     // points staged per means tile
 constexpr int kBCTile = 128;     // points staged per covariance tile
 constexpr int kBatchSyncEvery = 8;
-constexpr size_t kStageDoubles = (size_t)1 << 19;   // parameter staging ring (4 MB)
 constexpr int kTimeMarks = 15;   // timing events per sweep (see collect_timing)
 constexpr int kClasses = 4;      // D = 4, 8, 16, 32
 
@@ -1136,8 +1135,7 @@ struct fem_em_batch {
   double *epart = nullptr, *mpart = nullptr, *cpart = nullptr;
   double *trace = nullptr, *etrace = nullptr;
   int *nactive = nullptr, *hnactive = nullptr;   // device / pinned host
-  double *stage = nullptr;          // pinned staging ring of the parameters (doubles)
-  size_t stage_n = 0, stage_at = 0;
+  double *stage = nullptr;          // pinned staging of one fit's parameters
   EItem *eitems = nullptr;
   MItem *mitems = nullptr;
   CItem *citems = nullptr;
@@ -1589,9 +1587,9 @@ extern "C" int fem_em_batch_create_tuned(int nfits, const int *d, const int64_t 
       return fail(FEM_ERR_CUDA);
     }
   }
-  b->stage_n = kStageDoubles;
-  for (int f = 0; f < nfits; f++) b->stage_n = std::max(b->stage_n, (size_t)k[f] * (1 + d[f] + d[f] * d[f]));
-  if (cudaMallocHost((void **)&b->stage, b->stage_n * sizeof(double)) != cudaSuccess ||
+  size_t stage = 0;                 // the largest fit's parameters (doubles)
+  for (int f = 0; f < nfits; f++) stage = std::max(stage, (size_t)k[f] * (1 + d[f] + d[f] * d[f]));
+  if (cudaMallocHost((void **)&b->stage, stage * sizeof(double)) != cudaSuccess ||
       cudaMallocHost((void **)&b->hnactive, sizeof(int)) != cudaSuccess) {
     set_error("pinned allocation failed");
     return fail(FEM_ERR_CUDA);
@@ -1667,20 +1665,9 @@ extern "C" int fem_em_batch_upload_packed(fem_em_batch *b, const float *X) {
   return FEM_OK;
 }
 
-// n doubles of the pinned staging ring: parameters go in and out in one copy per
-// fit, and a copy in need not have finished when the call returns (192 fits:
-// 27 us a call with three or four waited-for pageable copies).  Wrapping around
-// waits for the copies in flight.
-static int stage_params(fem_em_batch *b, size_t n, double **h) {
-  if (b->stage_at + n > b->stage_n) {
-    FEM_CUDA(cudaStreamSynchronize(b->stream));
-    b->stage_at = 0;
-  }
-  *h = b->stage + b->stage_at;
-  b->stage_at += n;
-  return FEM_OK;
-}
-
+// Parameters go in and out in one copy per fit through pinned memory (192 fits: 27
+// us a call with three or four pageable copies); the copy is done, and its errors
+// are known, when the call returns.
 extern "C" int fem_em_batch_set_params(fem_em_batch *b, int fit, const double *pi, const double *mu,
                                        const double *sigma) {
   FEM_TRY(check_fit(b, fit));
@@ -1691,12 +1678,12 @@ extern "C" int fem_em_batch_set_params(fem_em_batch *b, int fit, const double *p
   const BFit &F = b->hfits[fit];
   const size_t nk = F.k, nm = nk * F.d, ns = nm * F.d;
   FEM_CUDA(cudaSetDevice(b->cfg.device));
-  double *h = nullptr;
-  FEM_TRY(stage_params(b, nk + nm + ns, &h));
+  double *h = b->stage;
   memcpy(h, pi, nk * sizeof(double));
   memcpy(h + nk, mu, nm * sizeof(double));
   memcpy(h + nk + nm, sigma, ns * sizeof(double));
   FEM_CUDA(cudaMemcpyAsync(F.pi, h, (nk + nm + ns) * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+  FEM_CUDA(cudaStreamSynchronize(b->stream));
   b->have_params[fit] = 1;
   return FEM_OK;
 }
@@ -1706,8 +1693,7 @@ extern "C" int fem_em_batch_get_params(fem_em_batch *b, int fit, double *pi, dou
   const BFit &F = b->hfits[fit];
   FEM_CUDA(cudaSetDevice(b->cfg.device));
   const size_t nk = F.k, nm = nk * F.d, ns = nm * F.d;
-  double *h = nullptr;
-  FEM_TRY(stage_params(b, nk + nm + ns, &h));
+  double *h = b->stage;
   const size_t want = sigma ? nk + nm + ns : mu ? nk + nm : pi ? nk : 0;   // up to the last one asked for
   if (want) FEM_CUDA(cudaMemcpyAsync(h, F.pi, want * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   FEM_CUDA(cudaStreamSynchronize(b->stream));

@@ -182,6 +182,7 @@ struct fem_km {
   double xg2 = 0.0;                // sum_i ||x_i - g||^2
   double *g = nullptr;             // data mean (device, d)
   float *gs = nullptr;             // centre of the screens (device, d)
+  int *range = nullptr;            // centroids' smallest and largest distance from it (km_tc.cu)
   int spread = 0;                  // values' typical distance from it: below 2^spread, half that or more
   double *hg = nullptr;            // data mean (host)
   double *out = nullptr;           // device: k x d new centroids, k counts (as double), fit

@@ -87,10 +87,12 @@ k_km_stats(const float *__restrict__ X, int64_t n, int d, int64_t rows_per_block
 }
 
 // centroids -> float copy and norm, and for the FP32 path the copy around g (as
-// float) and half its squared norm; one warp per centroid
+// float) and half its squared norm; one warp per centroid.  Clears the range of
+// norms that the tensor-core path's preparation collects.
 __global__ void __launch_bounds__(128)
 k_km_prep(const double *__restrict__ cent, const float *__restrict__ g, int K, int d, float *__restrict__ centf,
-          float *__restrict__ cnorm, float *__restrict__ centg, float *__restrict__ hnorm) {
+          float *__restrict__ cnorm, float *__restrict__ centg, float *__restrict__ hnorm, int *__restrict__ range) {
+  if (blockIdx.x == 0 && threadIdx.x < 2) range[threadIdx.x] = 0;
   const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= K) return;
   double s = 0.0, h = 0.0;
@@ -482,6 +484,7 @@ void free_km(fem_km *h) {
   dfree(h->cnt);
   dfree(h->g);
   dfree(h->gs);
+  dfree(h->range);
   dfree(h->out);
   dfree(h->dstat);
   km_tc_destroy(h);
@@ -673,7 +676,7 @@ int fem_km_create(int d, int64_t n, int k, const fem_km_config *cfg, fem_km **ou
       (st = dalloc(&h->cent, (size_t)k * d)) || (st = dalloc(&h->centf, (size_t)k * d)) ||
       (st = dalloc(&h->cnorm, k)) || (st = dalloc(&h->acc, (size_t)h->grid * k * d)) ||
       (st = dalloc(&h->cnt, (size_t)h->grid * k)) || (st = dalloc(&h->g, d)) ||
-      (st = dalloc(&h->gs, d)) ||
+      (st = dalloc(&h->gs, d)) || (st = dalloc(&h->range, 2)) ||
       (st = dalloc(&h->out, (size_t)k * d + 2 * k)) || (st = dalloc(&h->dstat, 1)))
     return fail(st);
   if (cudaMallocHost(&h->hout, ((size_t)k * d + 2 * k) * 8) != cudaSuccess ||
@@ -757,7 +760,7 @@ static int km_iterate(fem_km *h, double *centroids, double *fit, int64_t *counts
   *h->hstat = z;
   FEM_CUDA(cudaMemcpyAsync(h->dstat, h->hstat, sizeof(DevStatus), cudaMemcpyHostToDevice, h->stream));
   FEM_CUDA(cudaMemcpyAsync(h->cent, centroids, kd * 8, cudaMemcpyHostToDevice, h->stream));
-  k_km_prep<<<(K + 3) / 4, 128, 0, h->stream>>>(h->cent, h->gs, K, d, h->centf, h->cnorm, h->centg, h->hnorm);
+  k_km_prep<<<(K + 3) / 4, 128, 0, h->stream>>>(h->cent, h->gs, K, d, h->centf, h->cnorm, h->centg, h->hnorm, h->range);
   FEM_CUDA(cudaGetLastError());
   FEM_CUDA(cudaEventRecord(h->ev[0], h->stream));
   if (h->cfg.precision == FEM_PREC_MIXED)

@@ -183,7 +183,7 @@ struct fem_km {
   double *g = nullptr;             // data mean (device, d)
   float *gs = nullptr;             // centre of the screens (device, d)
   int *range = nullptr;            // centroids' smallest and largest distance from it (km_tc.cu)
-  int spread = 0;                  // values' typical distance from it: below 2^spread, half that or more
+  float *xscale = nullptr;         // power of two that brings the data's spread around it to 1/2..1
   double *hg = nullptr;            // data mean (host)
   double *out = nullptr;           // device: k x d new centroids, k counts (as double), fit
   double *hout = nullptr;          // pinned host copy

@@ -2,8 +2,8 @@
 // (NaiveKMA::ComputeMSEAndCorrect, Clust/KMAlgorithm.cpp:205-255, for d = 32).
 //
 // Distances are translation invariant, so both sides are first centred on a point g
-// amid the data and scaled by a power of two that brings the values' typical
-// distance from it to 1/4..1/2: x' = t (x - g), c' = t (c - g).  (Scaled by max |x|,
+// amid the data and scaled by a power of two that brings the rows' typical largest
+// distance from it to 1/2..1: x' = t (x - g), c' = t (c - g).  (Scaled by max |x|,
 // an offset or one row far out pushes all others below FP16's normal range and
 // leaves them open.)  For a tile of 128 points the tensor cores form
 //   D_j = x'.c'_j - ||c'_j||^2 / 2,   ||x' - c'_j||^2 = ||x'||^2 - 2 D_j,
@@ -113,11 +113,11 @@ __device__ __forceinline__ void fence_proxy_async_smem_km() {
 // (1.01 L + 1/8 > kKmFar: rows far out, or all centroids far outside the data) take
 // every centroid as a candidate.
 __global__ void __launch_bounds__(128)
-k_km_tc_prep(const double *__restrict__ cent, const float *__restrict__ g, double t, int K, int Kp,
+k_km_tc_prep(const double *__restrict__ cent, const float *__restrict__ g, const float *__restrict__ xscale, int K, int Kp,
              __half *__restrict__ b1, __half *__restrict__ b2, int *__restrict__ range) {
   const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= Kp) return;
-  double c = j < K ? t * (cent[(size_t)j * kKmD + lane] - (double)g[lane]) : 0.0, n = c * c;
+  double c = j < K ? (double)*xscale * (cent[(size_t)j * kKmD + lane] - (double)g[lane]) : 0.0, n = c * c;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
   const float nrm = (float)sqrt(n);
@@ -153,12 +153,13 @@ k_km_assign_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_b2, const int *__restrict__ range,
                const double *__restrict__ cent, const float *__restrict__ centf,
                const float *__restrict__ cnorm, const float *__restrict__ X, const float *__restrict__ gs, int64_t n,
-               int K, int Kp, float xscale, int32_t *__restrict__ labels,
+               int K, int Kp, const float *__restrict__ xscale_at, int32_t *__restrict__ labels,
                long long *__restrict__ accg, int *__restrict__ cntg, float scale, float scale_hi, int lo_bits,
                int64_t epoch, DevStatus *st, int *err) {
   extern __shared__ uint8_t smem_raw[];
   KmSmem &S = smem_aligned<KmSmem>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float xscale = *xscale_at;
   const int64_t ntiles = (n + kKmTile - 1) / kKmTile;
   const int64_t mine = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
@@ -561,9 +562,7 @@ int km_tc_assign(fem_km *h) {
   KmTcPlanImpl *p = static_cast<KmTcPlanImpl *>(h->tc);
   int xe = 0;
   std::frexp((double)std::max(h->xmax, 1e-25f), &xe);      // |x| <= xmax < 2^xe
-  // 2^te brings the data's spread to 1/4..1/2 (rows up to 3600 times that far out are screened)
-  const int te = -1 - std::min(125, h->spread);
-  k_km_tc_prep<<<p->kp / 4, 128, 0, h->stream>>>(h->cent, h->gs, std::ldexp(1.0, te), h->k, p->kp, p->b1, p->b2, h->range);
+  k_km_tc_prep<<<p->kp / 4, 128, 0, h->stream>>>(h->cent, h->gs, h->xscale, h->k, p->kp, p->b1, p->b2, h->range);
   FEM_CUDA(cudaGetLastError());
   // |x| 2^shift < 2^bits: hi takes bits / 2 of them, lo the lo_bits below; both
   // sums stay within 32 bits for `rows` rows of one centroid.  From 1024 rows on
@@ -576,7 +575,7 @@ int km_tc_assign(fem_km *h) {
 #define FEM_KT(W)                                                                                                \
   k_km_assign_tc<W><<<h->grid, kKmThreads, sizeof(KmSmem) + 1024, h->stream>>>(                                  \
       p->tm_x, p->tm_b1, p->tm_b2, h->range, h->cent, h->centf, h->cnorm, h->X, h->gs, h->n, h->k, p->kp,        \
-      ldexpf(1.f, te), h->labels, h->acc, h->cnt, ldexpf(1.f, h->shift), ldexpf(1.f, hi_bits - xe), lo_bits, epoch, h->dstat, p->err)
+      h->xscale, h->labels, h->acc, h->cnt, ldexpf(1.f, h->shift), ldexpf(1.f, hi_bits - xe), lo_bits, epoch, h->dstat, p->err)
   if (w32)
     FEM_KT(true);
   else

@@ -52,3 +52,21 @@ def test_an_offset_or_an_outlier_opens_few_rows(gpu_lib, oracle, case):
             km.ComputeMSEAndCorrect(C.copy())
             assert np.array_equal(km.Assignment(), lo)
             assert km.Stats()["rechecked"] <= n // 100
+
+
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_mostly_equal_rows_open_few(gpu_lib, oracle, shuffled):
+    """Four of five rows the same, sorted first or mixed in: the others are
+    screened as well."""
+    n, k = 30000, 64
+    X, C = data(n, k, 5.0, seed=4)
+    X[:4 * n // 5] = 0.0
+    C[0] = 0.0
+    if shuffled:
+        X = X[np.random.default_rng(1).permutation(n)]
+    with CudaKMA(32, n, k, precision="mixed", repair=False) as km:
+        km.SetDataset(X)
+        lo = oracle.km_iterate(X, C, repair=False)[3]
+        km.ComputeMSEAndCorrect(C.copy())
+        assert np.array_equal(km.Assignment(), lo)
+        assert km.Stats()["rechecked"] <= n // 100

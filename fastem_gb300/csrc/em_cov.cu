@@ -13,8 +13,8 @@
 // written to shared memory and a tile costs one barrier.  Bound by the
 // FP32 pipe: 64 of the 88 FP32 operations per point and unit are the products
 // (16 subtractions and 8 multiplications by r beside them) and, at 77 % of its
-// rate, by the 128-bit shared-memory loads; in FP64 by the FP64 pipe (2 per
-// clock and SM).  FP32 8 x 8 blocks multiply two columns per instruction
+// rate, by the 128-bit shared-memory loads; in FP64 (d <= 8; k_cov_staged above) by
+// the FP64 pipe (2 per clock and SM).  FP32 8 x 8 blocks multiply two columns per instruction
 // (N = 250007, d = 16, K = 200: 0.89 -> 0.68 ms; copies without a division per
 // element 0.65).  On the GB300, against a kernel that wrote sqrt(r) (x - mu)
 // of every component to shared memory and used one thread per block:
@@ -363,6 +363,117 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
   flush(false);
 }
 
+// FP64 with more than one block per dimension.  The FP64 pipe is all that counts, and
+// k_cov_units would spend 104 of its operations per point and 8 x 8 unit on 64
+// products (conversions, differences and weights formed by every unit).  Here a CTA's
+// rows are turned into u = x - mu_j and w = r_ij u for its cj components once per
+// tile, in shared memory, and a unit only multiplies.  Partials as k_cov_units leaves
+// them.  M-steps on the GB300, N = 60000, by the kernel that staged sqrt(r) (x - mu)
+// and used one thread per block, by k_cov_units, and here: d = 9, K = 200 3.80, 7.33,
+// 3.30 ms; d = 20, K = 60 3.67, 4.58, 2.35; d = 32, K = 20 3.66, 2.33, 1.66; d = 64, K =
+// 60 17.9, 26.8, 15.7; d = 256, K = 9 37.9, 52.0, 34.7; N = 5000, d = 32, K = 9 0.48,
+// 0.15, 0.12.
+template <int TB>
+__global__ void __launch_bounds__(kCvThreads, TB == 8 ? 1 : 2)
+k_cov_staged(const float *__restrict__ X, int64_t n, int d, int K, PostTyped<double> R, const double *__restrict__ mu,
+             double *__restrict__ part, int nb, int nblk, int64_t rows_per_chunk, int upc, int G, int TP, int xpitch,
+             int rpitch, int cjmax) {
+  constexpr int NE = TB * TB;
+  extern __shared__ __align__(16) unsigned char cv_smem[];
+  const int tid = threadIdx.x, units = K * nblk, u0 = blockIdx.x * upc;
+  const int j_lo = u0 / nblk, cj = min(K - 1, (u0 + upc - 1) / nblk) - j_lo + 1;
+  const int g = tid / upc, ul = tid - g * upc, unit = u0 + ul;
+  const bool act = g < G && unit < units;
+  const size_t xbytes = (size_t)TP * xpitch * sizeof(float), buf_bytes = xbytes + (size_t)cjmax * rpitch * sizeof(double);
+  const int dp = nb * TB, zp = dp + 2;              // row pitch of u and w
+  double *su = reinterpret_cast<double *>(cv_smem + 2 * buf_bytes), *sw = su + (size_t)cjmax * TP * zp;
+  int j = j_lo, bi = 0, bj = 0;
+  if (act) {
+    j = unit / nblk;
+    int b = unit - j * nblk;
+    while (b >= nb - bi) {
+      b -= nb - bi;
+      bi++;
+    }
+    bj = bi + b;
+  }
+  double acc[NE];
+#pragma unroll
+  for (int e = 0; e < NE; e++) acc[e] = 0.0;
+  const int64_t c0 = (int64_t)blockIdx.y * rows_per_chunk, c1 = min(n, c0 + rows_per_chunk);
+  auto stage = [&](int buf, int64_t t0) {
+    float *sx = reinterpret_cast<float *>(cv_smem + buf * buf_bytes);
+    if ((d & 3) == 0) {
+      for (CvWalk w(d >> 2); w.row < TP; w.next()) {
+        const bool v = t0 + w.row < c1;
+        cv_copy16(sx + w.row * xpitch + 4 * w.col, X + (v ? (t0 + w.row) * d + 4 * w.col : 0), v);
+      }
+    } else {
+      for (CvWalk w(d); w.row < TP; w.next()) {
+        const bool v = t0 + w.row < c1;
+        cv_copy4(sx + w.row * xpitch + w.col, X + (v ? (t0 + w.row) * d + w.col : 0), v);
+      }
+    }
+    R.stage(cv_smem + buf * buf_bytes + xbytes, rpitch, j_lo, cj, t0, TP, c1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  stage(0, c0);
+  int buf = 0;
+  for (int64_t t0 = c0; t0 < c1; t0 += TP, buf ^= 1) {
+    if (t0 + TP < c1)
+      stage(buf ^ 1, t0 + TP);
+    else
+      asm volatile("cp.async.commit_group;\n" ::: "memory");   // keeps the wait count uniform
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    const float *sx = reinterpret_cast<const float *>(cv_smem + buf * buf_bytes);
+    const double *sr = reinterpret_cast<const double *>(cv_smem + buf * buf_bytes + xbytes);
+    const int live = (int)min((int64_t)TP, c1 - t0);
+    for (CvWalk w(dp); w.row < cj * TP; w.next()) {
+      const int jj = w.row / TP, p = w.row - jj * TP, q = w.col;
+      if (p >= live) continue;
+      const double u = q < d ? (double)sx[p * xpitch + q] - __ldg(mu + (size_t)(j_lo + jj) * d + q) : 0.0;
+      su[(size_t)w.row * zp + q] = u;
+      sw[(size_t)w.row * zp + q] = sr[jj * rpitch + p] * u;
+    }
+    __syncthreads();
+    if (act) {
+      const double *wa = sw + (size_t)(j - j_lo) * TP * zp + bi * TB, *ub = su + (size_t)(j - j_lo) * TP * zp + bj * TB;
+#pragma unroll 1
+      for (int p = g; p < live; p += G) {
+        double a[TB], b[TB];
+#pragma unroll
+        for (int q = 0; q < TB; q += 2) {
+          const double2 va = *reinterpret_cast<const double2 *>(wa + p * zp + q);
+          const double2 vb = *reinterpret_cast<const double2 *>(ub + p * zp + q);
+          a[q] = va.x, a[q + 1] = va.y, b[q] = vb.x, b[q + 1] = vb.y;
+        }
+#pragma unroll
+        for (int e = 0; e < NE; e++) acc[e] = fma(a[e / TB], b[e % TB], acc[e]);
+      }
+    }
+    __syncthreads();
+  }
+  double *o = part + (size_t)blockIdx.y * NE * units + u0;
+  if (G == 1) {
+    if (act)
+#pragma unroll
+      for (int e = 0; e < NE; e++) o[(size_t)e * units + ul] = acc[e];
+    return;
+  }
+  double *red = reinterpret_cast<double *>(cv_smem);   // NE x 256, over the tiles
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < NE; e++) red[e * kCvThreads + tid] = acc[e];
+  __syncthreads();
+  const int live = min(upc, units - u0);
+  for (int i = tid; i < live * NE; i += kCvThreads) {
+    const int e = i / live, u = i - e * live;
+    o[(size_t)e * units + u] = group_sum(red + e * kCvThreads + u, G, upc);
+  }
+}
+
 // Covs_j = CovSum_j / PosteriorSum_j, upper mirrored to lower (EM2/MatrixEM.cpp:370-373).
 // 32 consecutive elements per CTA, the chunks split over 8 threads each and
 // combined in a fixed order: one thread per element left the sums of small
@@ -581,11 +692,46 @@ void split_rows(int64_t n, int TP, int gx, int slots, double extra, int *chunks,
   }
 }
 
+// Schedule of k_cov_staged with TB x TB blocks; returns its FP64 operations per row, 0
+// where no tile fits (every d and k of the FP64 form has one that does)
+static double staged_plan(int d, int64_t n, int k, int TB, CovPlan *out) {
+  CovPlan p{};
+  p.TB = TB;
+  p.nb = (d + TB - 1) / TB;
+  p.nblk = p.nb * (p.nb + 1) / 2;
+  split_units(k * p.nblk, &p.gx, &p.upc, &p.G);
+  p.cj = std::min(k, (p.upc + p.nblk - 2) / p.nblk + 1);
+  p.xpitch = (d + 3) & ~3;
+  const size_t red = p.G > 1 ? (size_t)TB * TB * kCvThreads * sizeof(double) : 0;
+  const size_t most = kCvMaxSmem / (TB == 8 ? 1 : 2) - 1024;
+  for (int tile = 64;; tile /= 2) {
+    if (tile < 8) return 0.0;
+    p.TP = (p.G * std::max(1, tile / p.G) + 1) & ~1;
+    p.rpitch = p.TP + 2;
+    p.smem = std::max(red, 2 * ((size_t)p.TP * p.xpitch * sizeof(float) + (size_t)p.cj * p.rpitch * sizeof(double)) +
+                               2 * (size_t)p.cj * p.TP * (p.nb * TB + 2) * sizeof(double));
+    if (p.smem <= most) break;
+  }
+  split_rows(n, p.TP, p.gx, (TB == 8 ? 1 : 2) * sm_count(), 2.0, &p.chunks, &p.rows);
+  p.part = (size_t)p.chunks * k * p.nblk * TB * TB;
+  *out = p;
+  return p.gx * ((double)p.upc * TB * TB + 3.0 * p.cj * p.nb * TB);
+}
+
 // Schedule of the covariance sums for one handle (fixed by its shape).
 //
-//  TB, tri   8 x 8 blocks; one triangular block when d <= 8 (4 x 4 when d <= 4)
+//  TB, tri   8 x 8 blocks; one triangular block when d <= 8 (4 x 4 when d <= 4).  FP64
+//            with d > 8: k_cov_staged by 4 x 4 or 8 x 8 blocks, whichever takes fewer
+//            operations (4 x 4 pads and doubles less, 8 x 8 stages a component's rows
+//            for more products: d = 9, K = 200 3.3 against 5.7 ms, d = 64, K = 60 15.7
+//            against 16.9, d = 256, K = 9 45.6 against 34.7, N = 60000)
 //  units     split as split_units says, rows as split_rows says
 CovPlan cov_plan(int d, int64_t n, int k, bool fp64, bool hilo) {
+  if (fp64 && d > 8) {
+    CovPlan q[2];
+    const double c4 = staged_plan(d, n, k, 4, &q[0]), c8 = staged_plan(d, n, k, 8, &q[1]);
+    return q[c4 > 0.0 && (c8 == 0.0 || c4 <= c8) ? 0 : 1];
+  }
   CovPlan p{};
   p.TB = d <= 4 ? 4 : 8;
   p.nb = (d + p.TB - 1) / p.TB;
@@ -666,12 +812,21 @@ static int cov_pass(fem_em *h, Src src, const T *mu, int mu_ld, const int *gate 
         h->X, h->n, d, K, src, mu, mu_ld, h->cpart, p.nb, p.nblk, p.rows, p.upc, p.G, p.TP, p.xpitch, p.rpitch, \
         p.cj, gate);                                                                                           \
   } while (0)
-  if (p.TB == 4)
+  if (p.TB == 4 && p.tri) {
     FEM_CV(4, true);
-  else if (p.tri)
+  } else if (p.tri) {
     FEM_CV(8, true);
-  else
+  } else if constexpr (sizeof(T) == 4) {
     FEM_CV(8, false);
+  } else {
+    auto launch = [&](auto kern) -> int {
+      FEM_CUDA(allow_dyn_smem(kern, p.smem));
+      kern<<<grid, kCvThreads, p.smem, h->stream>>>(h->X, h->n, d, K, src, mu, h->cpart, p.nb, p.nblk, p.rows, p.upc, p.G,
+                                                    p.TP, p.xpitch, p.rpitch, p.cj);
+      return FEM_OK;
+    };
+    FEM_TRY(p.TB == 8 ? launch(k_cov_staged<8>) : launch(k_cov_staged<4>));
+  }
 #undef FEM_CV
   FEM_CUDA(cudaGetLastError());
   const int64_t per = (int64_t)K * p.nblk * (p.tri ? p.TB * (p.TB + 1) / 2 : p.TB * p.TB);

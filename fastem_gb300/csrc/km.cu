@@ -579,27 +579,21 @@ int upload_km(fem_km *h, const float *X, int64_t ld, cudaMemcpyKind kind) {
   // data mean, max |x| -> fixed-point shift, sum ||x - g||^2, in one pass
   const int G = (int)std::min<int64_t>(4 * (int64_t)sm_count(), (n + 255) / 256);
   const int64_t rpb = (n + G - 1) / G;
-  std::vector<float> c(d);
-  FEM_CUDA(cudaMemcpyAsync(c.data(), h->X, (size_t)d * 4, cudaMemcpyDeviceToHost, h->stream));
-  FEM_CUDA(cudaStreamSynchronize(h->stream));
-  float *dc = nullptr;
   double *s1 = nullptr, *s2 = nullptr;
   float *amax = nullptr;
-  FEM_TRY(dalloc(&dc, d));
   FEM_TRY(dalloc(&s1, (size_t)G * d));
   FEM_TRY(dalloc(&s2, (size_t)G * d));
   FEM_TRY(dalloc(&amax, G));
-  FEM_CUDA(cudaMemcpyAsync(dc, c.data(), (size_t)d * 4, cudaMemcpyHostToDevice, h->stream));
-  k_km_stats<<<G, 256, 0, h->stream>>>(h->X, n, d, rpb, dc, s1, s2, amax);
+  k_km_stats<<<G, 256, 0, h->stream>>>(h->X, n, d, rpb, h->X, s1, s2, amax);
   k_km_centre<<<d, kFrameRows, 0, h->stream>>>(h->X, n, d, h->gs);
   k_km_spread<<<1, kFrameRows, 0, h->stream>>>(h->X, n, d, h->gs, h->xscale);
   std::vector<double> h1((size_t)G * d), h2((size_t)G * d);
-  std::vector<float> hm(G);
+  std::vector<float> hm(G), c(d);
+  cudaMemcpyAsync(c.data(), h->X, (size_t)d * 4, cudaMemcpyDeviceToHost, h->stream);
   cudaMemcpyAsync(h1.data(), s1, h1.size() * 8, cudaMemcpyDeviceToHost, h->stream);
   cudaMemcpyAsync(h2.data(), s2, h2.size() * 8, cudaMemcpyDeviceToHost, h->stream);
   cudaMemcpyAsync(hm.data(), amax, hm.size() * 4, cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  dfree(dc);
   dfree(s1);
   dfree(s2);
   dfree(amax);

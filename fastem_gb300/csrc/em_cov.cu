@@ -228,7 +228,10 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
 
   bool first = true;
   // adds the FP32 sums into this CTA's FP64 partials (or stores them), the groups'
-  // sums of a unit in group order and without FP32 rounding (group_sum)
+  // sums of a unit in group order: in T as long as they span kCvRows rows together,
+  // else without FP32 rounding (group_sum, two more FP64 conversions and additions a
+  // sum: N = 200003, d = 24, K = 21, 658 rows a CTA, 5 us a sweep)
+  int rows = 0;                                     // of each group since the last flush
   auto flush = [&](bool more) {
     if constexpr (PK) {
 #pragma unroll
@@ -256,7 +259,15 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
       const int live = min(upc, units - u0);
       for (int i = tid; i < live * NE; i += kCvThreads) {
         const int e = i / live, u = i - e * live;
-        const double s = group_sum(red + e * kCvThreads + u, G, upc);
+        const T *v = red + e * kCvThreads + u;
+        double s;
+        if (rows * G <= kCvRows) {
+          T t = v[0];
+          for (int q = 1; q < G; q++) t += v[q * upc];
+          s = (double)t;
+        } else {
+          s = group_sum(v, G, upc);
+        }
         double *p = o + (size_t)e * units + u;
         *p = first ? s : *p + s;
       }
@@ -272,7 +283,7 @@ k_cov_units(const float *__restrict__ X, int64_t n, int d, int K, Src R, const T
   };
 
   stage(0, c0);
-  int buf = 0, rows = 0;
+  int buf = 0;
   const int tile_rows = TP / G;
   const int roff = (j - j_lo) * rpitch, rlo = cj * rpitch;
   for (int64_t t0 = c0; t0 < c1; t0 += TP, buf ^= 1) {

@@ -212,8 +212,12 @@ __device__ __forceinline__ float bound_f32(float s, float cn, int d) {
 // more than B(N) and B(1.01 L) together, so it is never the smallest.  A row whose
 // two smallest differ by more than 2 B(min(||c'||max, 1.01 L)) is therefore decided
 // (with ||c'||max alone one centroid at 10^4 opened every row of unit blobs: N =
-// 1000003, D = 64, K = 100 43 ms an iteration, without it 0.62).  The others, few, go
-// through the difference form by the whole warp (lane = centroid): FP32 with
+// 1000003, D = 64, K = 100 43 ms an iteration, without it 0.62).  Where several
+// of a warp's 32 rows stay open (centroids close together, far from g) each lane first
+// tries its own in the difference form: with D >= 32 that costs as much as deciding
+// two rows, with 8 and 16 about five (20 centroids in each of 5 blobs, D = 64: 13.2 ->
+// 1.3 ms, one row per thread 1.8; D = 2, K = 700 0.42 -> 0.53, so not there).  The
+// others, few, go through the difference form by the whole warp (lane = centroid): FP32 with
 // the bound of bound_f32, then the reference's FP64 sums among the centroids
 // that remain, lowest index on ties.  Rows are added to exact fixed-point sums
 // in shared memory (a float times 2^shift is exact), so the order is free.
@@ -266,6 +270,35 @@ __device__ __forceinline__ void km_screen(const float2 (*x)[D / 2], const float 
   }
 }
 
+// a lane's own row in the difference form over all centroids around g: the nearest,
+// and whether FP32 tells it from every other.  q: ||x'|| plus the largest ||c'|| that
+// counts (km_screen's callers); x' and c' are rounded, so a distance is off by what
+// bound_f32 says with q for ||c||, and farther centroids are out of reach of theirs.
+template <int D>
+__device__ __forceinline__ bool km_differences(const float2 (&x)[D / 2], const float *sC, int K, float q, int *j1) {
+  constexpr float u = 5.9604645e-8f;  // 2^-24
+  const float e1 = 2.f * 2.01f * u * q, e0 = 2.f * (u * q) * (u * q) + 1e-30f;
+  float U = INFINITY, l1 = INFINITY, l2 = INFINITY;
+  *j1 = -1;
+#pragma unroll 1
+  for (int j = 0; j < K; j++) {
+    const float2 *c = reinterpret_cast<const float2 *>(sC + j * D);     // -c'
+    float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < D / 2; p++) {
+      const float2 t = __fadd2_rn(x[p], c[p]);
+      s2 = km_ffma2(t, t, s2);
+    }
+    const float s = s2.x + s2.y, e = fmaf(2.f * (D + 4) * u, s, fmaf(e1, sqrtf(s), e0)), lb = s - e;
+    U = fminf(U, s + e);
+    if (lb < l1)
+      l2 = l1, l1 = lb, *j1 = j;
+    else
+      l2 = fminf(l2, lb);
+  }
+  return l2 > U;
+}
+
 // the reference's choice for one row, by the whole warp: -1 when no centroid
 // compares (a row with NaN); *fp64 when FP64 had to decide
 template <int D>
@@ -275,14 +308,29 @@ __device__ int km_decide(const float *__restrict__ x, const float *__restrict__ 
   float xr[D];
 #pragma unroll
   for (int q = 0; q < D; q++) xr[q] = x[q];
+  // 16 bytes a load where the registers allow it: the lanes' rows lie a row apart
+  auto dist = [&](int j) {
+    float s = 0.f;
+    if constexpr (D >= 32) {
+      const float4 *c = reinterpret_cast<const float4 *>(centf + (size_t)j * D);
+#pragma unroll
+      for (int q = 0; q < D / 4; q++) {
+        const float4 v = __ldg(c + q);
+        const float t0 = xr[4 * q] - v.x, t1 = xr[4 * q + 1] - v.y, t2 = xr[4 * q + 2] - v.z, t3 = xr[4 * q + 3] - v.w;
+        s = fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, s))));
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < D; q++) {
+        const float t = xr[q] - centf[(size_t)j * D + q];
+        s = fmaf(t, t, s);
+      }
+    }
+    return s;
+  };
   float U = INFINITY;
   for (int j = lane; j < K; j += 32) {
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < D; q++) {
-      const float t = xr[q] - centf[(size_t)j * D + q];
-      s = fmaf(t, t, s);
-    }
+    const float s = dist(j);
     U = fminf(U, s + bound_f32(s, cnorm[j], D));
   }
 #pragma unroll
@@ -290,12 +338,7 @@ __device__ int km_decide(const float *__restrict__ x, const float *__restrict__ 
   double best = DBL_MAX;
   int lab = INT_MAX, cand = 0, only = INT_MAX;
   for (int j = lane; j < K; j += 32) {
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < D; q++) {
-      const float t = xr[q] - centf[(size_t)j * D + q];
-      s = fmaf(t, t, s);
-    }
+    const float s = dist(j);
     if (s - bound_f32(s, cnorm[j], D) <= U) cand++, only = min(only, j);
   }
 #pragma unroll
@@ -306,12 +349,7 @@ __device__ int km_decide(const float *__restrict__ x, const float *__restrict__ 
   *fp64 = cand > 1;
   if (cand <= 1) return cand == 1 ? only : -1;
   for (int j = lane; j < K; j += 32) {
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < D; q++) {
-      const float t = xr[q] - centf[(size_t)j * D + q];
-      s = fmaf(t, t, s);
-    }
+    const float s = dist(j);
     if (s - bound_f32(s, cnorm[j], D) <= U) {
       const double s64 = dist64(cent + (size_t)j * D, xr, D);
       if (s64 < best) best = s64, lab = j;       // a lane's centroids come in index order
@@ -412,6 +450,14 @@ k_km_assign_f32(const float *__restrict__ X, int64_t n, int K, const float *__re
       const float B = fmaf(kU, fmaf(xn[r], cn, 0.5f * cn * cn), 1e-13f * fmaf(xn[r], xn[r], cn * cn)) + 1e-30f;
       int lab = j1[r];
       unsigned open = __ballot_sync(0xffffffffu, in && !(m2[r] - m1[r] > 2.1f * B));
+      if constexpr (D >= 8) {
+        if (__popc(open) >= (D >= 32 ? 2 : 5)) {
+          int l;
+          const bool told = km_differences<D>(x[r], sC, K, xn[r] + cn, &l);
+          if (told && (open >> lane & 1)) lab = l;
+          open &= ~__ballot_sync(0xffffffffu, told);
+        }
+      }
       while (open) {
         const int b = __ffs(open) - 1;
         open &= open - 1;
